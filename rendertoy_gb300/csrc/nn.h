@@ -62,7 +62,10 @@ struct ConvDgrad {
   int mask_relu;
   bf16* din;         // [P][Cin] (s1's channels upsampled when s1.up)
   int* err;
-  int ctw = 256;     // row-tile kernel: input channels per tile (multiple of 16, <= 256)
+  // Both given (only where conv_dgrad_splits says so): instead of din, s1's
+  // channels go to dlow [P / 4][C1], summed over each 2 x 2 block (nearest
+  // upsampling's gradient), and s2's to dskip [P][C2].
+  bf16 *dlow = nullptr, *dskip = nullptr;
 };
 
 struct ConvWgrad {
@@ -80,6 +83,9 @@ struct ConvWgrad {
 
 cudaError_t conv_fwd(const ConvFwd& a, cudaStream_t st);
 cudaError_t conv_dgrad(const ConvDgrad& a, cudaStream_t st);
+// whether conv_dgrad can write an upsampled + skip concatenation's gradient
+// straight to its two sources (dlow, dskip)
+bool conv_dgrad_splits(const ConvDgrad& a);
 cudaError_t conv_wgrad(const ConvWgrad& a, cudaStream_t st);
 // pixels per weight-gradient CTA: enough CTAs for about eight per SM, each
 // summing a multiple of 64 pixels

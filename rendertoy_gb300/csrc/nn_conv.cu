@@ -33,6 +33,7 @@
 #include <cudaTypedefs.h>
 
 #include "nn.h"
+#include "nn_tile.h"
 #include "tc_core.cuh"
 
 namespace rtx {
@@ -234,42 +235,6 @@ __device__ __forceinline__ bool produce(int n, uint64_t* full, uint64_t* empty, 
   return true;
 }
 
-// produce() for units that arrive as tensor copies: the producer warps
-// still copy what every MMA needs (pre, then wbar), then thread 32 alone
-// issues each unit's copies (issue(unit, stage, bar)) into its stage once
-// the stage is free, with one arrival carrying the unit's `tx` bytes.
-// `issued` counts the units it issued.
-template <int S, class Pre, class Issue>
-__device__ __forceinline__ bool produce_tma(int n, uint64_t* full, uint64_t* empty, uint64_t* wbar, uint32_t tx,
-                                            Pre&& pre, Issue&& issue, int& issued) {
-  const int pw = (threadIdx.x >> 5) - 1, lane = threadIdx.x & 31;
-  issued = 0;
-  if (wbar) {
-    pre(pw, lane);
-    tc::cp_async_commit();
-    tc::cp_async_wait<0>();
-    tc::fence_proxy_async();
-    tc::mbar_arrive(wbar);
-  }
-  if (threadIdx.x != 32) return true;
-  for (int u = 0; u < n; ++u) {
-    const int st = u % S;
-    if (u >= S && !tc::mbar_wait(&empty[st], (uint32_t)(u / S - 1) & 1u)) return false;
-    tc::mbar_arrive_expect_tx(&full[st], tx);
-    issue(u, st, &full[st]);
-    issued = u + 1;
-  }
-  return true;
-}
-
-// After a timed-out wait: thread 32 waits (bounded) for the tensor copies it
-// issued last on each stage, so that none lands after the CTA has left.
-template <int S>
-__device__ __forceinline__ void drain_tma(uint64_t* full, int issued) {
-  if (threadIdx.x != 32) return;
-  for (int u = max(0, issued - S); u < issued; ++u) tc::mbar_wait(&full[u % S], (uint32_t)(u / S) & 1u);
-}
-
 // One accumulation over n slices (the weight gradient).  Returns true,
 // uniformly, once every MMA has completed; false (error flag set) when a
 // bounded wait ran out.
@@ -367,10 +332,10 @@ struct TileBars {
 };
 
 template <int S>
-__device__ __forceinline__ void tile_bars_init(TileBars& b, uint32_t full_count = kLoadStride) {
+__device__ __forceinline__ void tile_bars_init(TileBars& b) {
   if (threadIdx.x == 0) {
     for (int i = 0; i < S; ++i) {
-      tc::mbar_init(&b.full[i], full_count);
+      tc::mbar_init(&b.full[i], kLoadStride);
       tc::mbar_init(&b.empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -382,13 +347,12 @@ __device__ __forceinline__ void tile_bars_init(TileBars& b, uint32_t full_count 
   }
 }
 
-template <int S, bool kTma = false, class Pre, class Load, class Mma, class Epi, class Issue>
+template <int S, class Pre, class Load, class Mma, class Epi>
 __device__ __forceinline__ bool ws_tiles(int n_tiles, int nsl, TileBars& b, Pre&& pre, Load&& load, Mma&& mma,
-                                         Epi&& epi, int* err, Issue&& issue, uint32_t tx) {
+                                         Epi&& epi, int* err) {
   const int tid = threadIdx.x, warp = tid >> 5;
   const int n = n_tiles * nsl;
   bool ok = true;
-  int issued = 0;
   if (warp == 0) {
     if (tid == 0) {
       if (n > 0) ok = tc::mbar_wait(&b.wbar, 0u);
@@ -404,10 +368,7 @@ __device__ __forceinline__ bool ws_tiles(int n_tiles, int nsl, TileBars& b, Pre&
       }
     }
   } else if (warp <= kProducerWarps) {
-    if constexpr (kTma)
-      ok = produce_tma<S>(n, b.full, b.empty, &b.wbar, tx, pre, issue, issued);
-    else
-      ok = produce<S>(n, b.full, b.empty, &b.wbar, pre, load);
+    ok = produce<S>(n, b.full, b.empty, &b.wbar, pre, load);
   } else {
     for (int i = 0; i < n_tiles; ++i) {
       const int buf = i & 1;
@@ -422,10 +383,7 @@ __device__ __forceinline__ bool ws_tiles(int n_tiles, int nsl, TileBars& b, Pre&
     }
   }
   ok = __syncthreads_and(ok);
-  if (!ok) {
-    if constexpr (kTma) drain_tma<S>(b.full, issued);
-    if ((tid & 31) == 0) atomicOr(err, tc::kErrMbarTimeout);
-  }
+  if (!ok && (tid & 31) == 0) atomicOr(err, tc::kErrMbarTimeout);
   return ok;
 }
 
@@ -533,15 +491,12 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_fwd(ConvFwd a) {
 // ---------------------------------------------------------------------------
 constexpr int kHalo = 130;                                  // pixels x0 - 1 .. x0 + 128
 constexpr uint32_t kHaloBytes = 3 * 2 * kHalo * 16;          // rows x chunks x pixels x 16 B
-constexpr uint32_t kHaloStage = (kHaloBytes + 1023) & ~1023u;  // 1 KB aligned for tensor copies
 
 // smem byte offset of chunk c (of 2) of halo pixel h in halo row r
 __device__ __forceinline__ uint32_t halo_off(int r, int c, int h) { return ((r * 2 + c) * kHalo + h) * 16; }
 
-template <int S, bool kRes, bool kTma = false>
-__global__ void __launch_bounds__(kTileThreads, 1)
-    k_conv_fwd_rows(ConvFwd a, const __grid_constant__ CUtensorMap tm_halo,
-                    const __grid_constant__ CUtensorMap tm_w) {
+template <int S, bool kRes>
+__global__ void __launch_bounds__(kTileThreads, 1) k_conv_fwd_rows(ConvFwd a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) TileBars bars;
   __shared__ uint32_t tmem_slot;
@@ -552,13 +507,9 @@ __global__ void __launch_bounds__(kTileThreads, 1)
   const int nsl = a.Cin / 16;
   const uint32_t ncols = a.Cout <= 32 ? 32 : (a.Cout <= 64 ? 64 : (a.Cout <= 128 ? 128 : 256));
   const uint32_t tap_bytes = (uint32_t)a.Cout * 32;
-  // tensor copies: the halo, then (streamed weights) the slice's nine weight
-  // tiles from the next 1 KB boundary
-  const uint32_t stage = kTma ? kHaloStage + (kRes ? 0u : (9 * tap_bytes + 1023u) & ~1023u)
-                              : (kRes ? kHaloBytes : kHaloBytes + 9 * tap_bytes);
-  const uint32_t w_off = kTma ? kHaloStage : kHaloBytes;  // weights within a streamed stage
+  const uint32_t stage = kRes ? kHaloBytes : kHaloBytes + 9 * tap_bytes;
   if (warp == 0) tc::tmem_alloc(&tmem_slot, 2 * ncols);
-  tile_bars_init<S>(bars, kTma ? 1 : kLoadStride);
+  tile_bars_init<S>(bars);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
@@ -602,7 +553,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
   };
   auto mma = [&](int, int st, int buf, int s) {
     const uint32_t sh = s0 + st * stage;
-    const uint32_t sb = kRes ? sw + (uint32_t)s * 9 * tap_bytes : sh + w_off;
+    const uint32_t sb = kRes ? sw + (uint32_t)s * 9 * tap_bytes : sh + kHaloBytes;
     // A: pixel groups 128 B apart (SBO), channel chunks one halo row apart
     // (LBO); tap t starts (dy + 1) halo rows and 1 + dx pixels in (offsets in
     // the descriptors' 16-byte address units)
@@ -637,140 +588,7 @@ __global__ void __launch_bounds__(kTileThreads, 1)
       }
     }
   };
-  // tensor-copy form: the unit's halo slice as one box of the source map
-  auto issue = [&](int u, int st, uint64_t* bar) {
-    const int i = u / nsl, s = u - i * nsl;
-    int n, y, x0;
-    tile_of(i, n, y, x0);
-    tc::tma_load_5d(s0 + st * stage, &tm_halo, 0, x0 - 1, 2 * s, y - 1, n, bar);
-    // the slice's nine [Cout x 16] weight tiles, tap-major
-    if (!kRes) tc::tma_load_5d(s0 + st * stage + w_off, &tm_w, 0, 0, 2 * s, 0, 0, bar);
-  };
-  ws_tiles<S, kTma>(n_tiles, nsl, bars, pre, load, mma, epi, a.err, issue, kHaloBytes + (kRes ? 0u : 9 * tap_bytes));
-  tc_end(tmem, 2 * ncols);
-}
-
-// data gradient, row tiles: din[p] = sum_t dout[p - off(t)] wt_t, the same
-// halo scheme over dout (slices of 16 of its channels, shifts negated).  A
-// tile is (image row, 128 pixels, 256 input channels); the channel tile
-// varies fastest, so neighbouring CTAs read the same dout halo.  Resident
-// weights: [channel tile][slice][tap] tiles of NTmax x 16.
-template <int S, bool kRes, bool kTma = false>
-__global__ void __launch_bounds__(kTileThreads, 1)
-    k_conv_dgrad_rows(ConvDgrad a, const __grid_constant__ CUtensorMap tm_halo,
-                      const __grid_constant__ CUtensorMap tm_w) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ __align__(8) TileBars bars;
-  __shared__ uint32_t tmem_slot;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int TR = (a.W + 127) / 128, nt = (a.Cin + a.ctw - 1) / a.ctw;
-  const int T = a.N * a.H * TR * nt;
-  const int n_tiles = (int)blockIdx.x < T ? (T - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-  const int nsl = a.Cout / 16;
-  const int ntm = min(a.ctw, a.Cin);  // widest channel tile
-  const uint32_t ncols = ntm <= 32 ? 32 : (ntm <= 64 ? 64 : (ntm <= 128 ? 128 : 256));
-  const uint32_t tap_bytes = (uint32_t)ntm * 32;
-  const uint32_t stage = kTma ? kHaloStage + (kRes ? 0u : (9 * tap_bytes + 1023u) & ~1023u)
-                              : (kRes ? kHaloBytes : kHaloBytes + 9 * tap_bytes);
-  const uint32_t w_off = kTma ? kHaloStage : kHaloBytes;  // weights within a streamed stage
-  if (warp == 0) tc::tmem_alloc(&tmem_slot, 2 * ncols);
-  tile_bars_init<S>(bars, kTma ? 1 : kLoadStride);
-  tc::fence_before();
-  __syncthreads();
-  tc::fence_after();
-  const uint32_t tmem = tmem_slot;
-  const uint32_t s0 = tc::smem_u32(smem), sw = s0 + S * stage;
-  auto tile_of = [&](int i, int& n, int& y, int& x0, int& ct) {
-    const int j = (int)blockIdx.x + i * (int)gridDim.x;
-    const int rx = j / nt;
-    ct = j - rx * nt;
-    const int row = rx / TR;
-    x0 = (rx - row * TR) * 128;
-    n = row / a.H;
-    y = row - n * a.H;
-  };
-  auto pre = [&](int pw, int lane) {
-    if (kRes)  // q -> (channel tile, slice, tap, row, chunk)
-      for (int q = pw * 32 + lane; q < nt * nsl * 9 * ntm * 2; q += kProducerWarps * 32) {
-        const int kc = q & 1, row = (q >> 1) % ntm, set = (q >> 1) / ntm;  // set = (ct * nsl + sl) * 9 + t
-        const int t = set % 9, cs = set / 9, sl = cs % nsl, c = cs / nsl;
-        const int ch = c * a.ctw + row;
-        chunk_async(sw + set * tap_bytes + tc::tile_offset(row, 8 * kc, 16),
-                    ch < a.Cin ? a.wt + ((size_t)ch * 9 + t) * a.Cout + sl * 16 + 8 * kc : nullptr, a.wt);
-      }
-  };
-  auto load = [&](int u, int st, int lane) {
-    const int i = u / nsl, s = u - i * nsl;
-    int n, y, x0, ct;
-    tile_of(i, n, y, x0, ct);
-    const uint32_t sh = s0 + st * stage;
-    const int o0 = s * 16;
-    for (int q = lane; q < 3 * kHalo * 2; q += kLoadStride) {
-      const int c = q & 1, h = (q >> 1) % kHalo, r = (q >> 1) / kHalo;
-      const int yy = y + r - 1, xx = x0 + h - 1;
-      const bf16* p = (yy >= 0 && yy < a.H && xx >= 0 && xx < a.W)
-                          ? a.dout + (((size_t)n * a.H + yy) * a.W + xx) * a.Cout + o0 + 8 * c
-                          : nullptr;
-      chunk_async(sh + halo_off(r, c, h), p, a.dout);
-    }
-    if (!kRes) {
-      const int n0 = ct * a.ctw, NT = min(a.ctw, a.Cin - n0);
-      for (int q = lane; q < 9 * NT * 2; q += kLoadStride) {
-        const int kc = q & 1, row = (q >> 1) % NT, t = (q >> 1) / NT;
-        chunk_async(sh + kHaloBytes + t * tap_bytes + tc::tile_offset(row, 8 * kc, 16),
-                    a.wt + ((size_t)(n0 + row) * 9 + t) * a.Cout + o0 + 8 * kc, a.wt);
-      }
-    }
-  };
-  auto mma = [&](int u, int st, int buf, int s) {
-    int n, y, x0, ct;
-    tile_of(u / nsl, n, y, x0, ct);
-    const int NT = min(a.ctw, a.Cin - ct * a.ctw);
-    const uint32_t idesc = tc::make_idesc_bf16(128, NT);
-    const uint32_t sh = s0 + st * stage;
-    const uint32_t sb = kRes ? sw + (uint32_t)(ct * nsl + s) * 9 * tap_bytes : sh + w_off;
-    const uint64_t ah = tc::make_desc(sh, kHalo * 16, 128), bw = tc::make_desc(sb, 128, 256);
-    const uint32_t d = tmem + buf * ncols;
-#pragma unroll
-    for (int t = 0; t < 9; ++t) {
-      const int dy = t / 3 - 1, dx = t % 3 - 1;
-      tc::mma_bf16(d, ah + ((1 - dy) * 2 * kHalo + 1 - dx), bw + t * (tap_bytes >> 4), idesc, s > 0 || t > 0);
-    }
-  };
-  auto epi = [&](int i, int buf) {
-    const int q = warp & 3;
-    int n, y, x0, ct;
-    tile_of(i, n, y, x0, ct);
-    const int n0 = ct * a.ctw, NT = min(a.ctw, a.Cin - n0);
-    const int x = x0 + q * 32 + lane;
-    const size_t p = ((size_t)n * a.H + y) * a.W + x;
-    const uint32_t taddr = tmem + buf * ncols + ((uint32_t)(q * 32) << 16);
-    for (int c0 = 0; c0 < NT; c0 += 8) {
-      float v[8];
-      tc::tmem_ld8(taddr + c0, v);
-      if (x < a.W) {
-        if (a.mask_relu) {
-          float sv[8];
-          bf16x8_to_f32(src_chunk(a.s1, a.s2, a.N, a.H, a.W, n, y, x, n0 + c0), sv);
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            if (!(sv[k] > 0.0f)) v[k] = 0.0f;
-        }
-        *reinterpret_cast<uint4*>(a.din + p * a.Cin + n0 + c0) = f32_to_bf16x8(v);
-      }
-    }
-  };
-  // tensor-copy form: the unit's dout halo slice as one box of dout's map
-  auto issue = [&](int u, int st, uint64_t* bar) {
-    const int i = u / nsl, s = u - i * nsl;
-    int n, y, x0, ct;
-    tile_of(i, n, y, x0, ct);
-    tc::tma_load_5d(s0 + st * stage, &tm_halo, 0, x0 - 1, 2 * s, y - 1, n, bar);
-    // the slice's nine [ntm x 16] tiles of the channel tile (rows past Cin
-    // read zeros), tap-major
-    if (!kRes) tc::tma_load_5d(s0 + st * stage + w_off, &tm_w, 0, 0, 2 * s, (ct * a.ctw) >> 3, 0, bar);
-  };
-  ws_tiles<S, kTma>(n_tiles, nsl, bars, pre, load, mma, epi, a.err, issue, kHaloBytes + (kRes ? 0u : 9 * tap_bytes));
+  ws_tiles<S>(n_tiles, nsl, bars, pre, load, mma, epi, a.err);
   tc_end(tmem, 2 * ncols);
 }
 
@@ -1185,9 +1003,9 @@ static bool use_rows(int W, int Ck) { return W >= 64 && Ck % 16 == 0; }
 // past half the SM so that a second CTA never waits on the first one's TMEM
 // columns.  Resident weights take a 7-stage halo ring; streamed weights the
 // deepest ring (6, 4 or 2 stages) that fits 200 KB.
-template <class KR, class K6, class K4, class K2, class Args>
+template <class KR, class K6, class K4, class K2>
 static cudaError_t launch_tiles(KR kr, K6 k6, K4 k4, K2 k2, bool res, size_t stage, size_t res_bytes, long long T,
-                                const Args& a, const CUtensorMap& tm, const CUtensorMap& tw, cudaStream_t st) {
+                                const ConvFwd& a, cudaStream_t st) {
   if (T <= 0) return cudaSuccess;
   int S = 7;
   size_t smem = 7 * stage + res_bytes;
@@ -1200,7 +1018,7 @@ static cudaError_t launch_tiles(KR kr, K6 k6, K4 k4, K2 k2, bool res, size_t sta
   cudaError_t e;
 #define RTX_LAUNCH_TILES(K)                                                                          \
   if ((e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))) return e; \
-  K<<<grid, kTileThreads, smem, st>>>(a, tm, tw);
+  K<<<grid, kTileThreads, smem, st>>>(a);
   if (res) {
     RTX_LAUNCH_TILES(kr)
   } else if (S == 6) {
@@ -1248,24 +1066,6 @@ static bool chunk_major_map(CUtensorMap* m, const void* base, int imgs, int H, i
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Tensor map of a [rows][9][K] BF16 weight array (rows, K multiples of 16)
-// viewed as 5-D (8 of K, row % 8, K chunk, row / 8, tap) with a box of (8, 8,
-// 2, box_rows / 8, 9): a slice's nine K-major [box_rows x 16] tiles land
-// tap-major in the no-swizzle core-matrix layout (tc::tile_offset).  False
-// if it cannot be encoded.
-static bool weight_map(CUtensorMap* m, const void* base, int rows, int K, int box_rows) {
-  const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-  if (!enc || (reinterpret_cast<uintptr_t>(base) & 15) || rows % 8 || K % 16 || box_rows % 8 || box_rows > 2048)
-    return false;
-  const cuuint64_t dims[5] = {8, 8, (cuuint64_t)(K / 8), (cuuint64_t)(rows / 8), 9};
-  const cuuint64_t strides[4] = {(cuuint64_t)9 * K * 2, 16, (cuuint64_t)8 * 9 * K * 2, (cuuint64_t)K * 2};
-  const cuuint32_t box[5] = {8, 8, 2, (cuuint32_t)(box_rows / 8), 9};
-  const cuuint32_t es[5] = {1, 1, 1, 1, 1};
-  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, es,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // weights kept in shared memory by the persistent kernels up to this size
 // (128 KB: with 1 KB-aligned tensor-copy halo stages, 7 x 13 KB + 128 KB
 // fits the 227 KB of a CTA; measured 0.75 % faster per training step than 96)
@@ -1275,24 +1075,14 @@ cudaError_t conv_fwd(const ConvFwd& a, cudaStream_t st) {
   long long P = (long long)a.N * a.H * a.W;
   if (a.Cout % 16 || a.Cout > 256 || a.Cin % 8) return cudaErrorInvalidValue;
   if (use_rows(a.W, a.Cin)) {
+    cudaError_t e = cudaSuccess;
+    if (conv_tile_fwd(a, st, &e)) return e;
     const size_t wbytes = (size_t)9 * a.Cin * a.Cout * 2;
     const bool res = wbytes <= kResidentWeights;
-    // one full-resolution source: halo slices (and streamed weight tiles)
-    // arrive as tensor copies, if the maps encode
-    CUtensorMap tm{}, tw{};
-    const bool tma = kConvTma && !a.s2.ptr && !a.s1.up && a.s1.C == a.Cin &&
-                     chunk_major_map(&tm, a.s1.ptr, a.N, a.H, a.W, a.Cin, kHalo, 2, 3) &&
-                     (res || weight_map(&tw, a.w, a.Cout, a.Cin, a.Cout));
-    const size_t wtiles = (size_t)9 * a.Cout * 32;
-    const size_t stage = tma ? kHaloStage + (res ? 0 : (wtiles + 1023) / 1024 * 1024)
-                             : (res ? kHaloBytes : kHaloBytes + wtiles);
+    const size_t stage = res ? kHaloBytes : kHaloBytes + (size_t)9 * a.Cout * 32;
     const long long T = (long long)a.N * a.H * ((a.W + 127) / 128);
-    if (tma)
-      return launch_tiles(k_conv_fwd_rows<7, true, true>, k_conv_fwd_rows<6, false, true>,
-                          k_conv_fwd_rows<4, false, true>, k_conv_fwd_rows<2, false, true>, res, stage,
-                          res ? wbytes : 0, T, a, tm, tw, st);
     return launch_tiles(k_conv_fwd_rows<7, true>, k_conv_fwd_rows<6, false>, k_conv_fwd_rows<4, false>,
-                        k_conv_fwd_rows<2, false>, res, stage, res ? wbytes : 0, T, a, tm, tw, st);
+                        k_conv_fwd_rows<2, false>, res, stage, res ? wbytes : 0, T, a, st);
   }
   size_t stage = 128 * kSlice * 2 + (size_t)a.Cout * kSlice * 2;
   const dim3 grid((unsigned)((P + 127) / 128));
@@ -1300,44 +1090,17 @@ cudaError_t conv_fwd(const ConvFwd& a, cudaStream_t st) {
                        stage, a, st);
 }
 
+bool conv_dgrad_splits(const ConvDgrad& a) {
+  return use_rows(a.W, a.Cout) && a.s1.up && a.s2.ptr && a.Cin % 16 == 0 && a.s1.C % 16 == 0 && a.H % 2 == 0 &&
+         a.W % 2 == 0;
+}
+
 cudaError_t conv_dgrad(const ConvDgrad& a, cudaStream_t st) {
   long long P = (long long)a.N * a.H * a.W;
   if (a.Cin % 16 || a.Cout % 8) return cudaErrorInvalidValue;
-  const int nt = (a.Cin + 255) / 256;
-  if (use_rows(a.W, a.Cout)) {
-    ConvDgrad b = a;
-    b.ctw = std::min(256, a.Cin);
-    const size_t wbytes = (size_t)nt * b.ctw * 9 * a.Cout * 2;
-    const bool res = wbytes <= kResidentWeights;
-    if (!res) {
-      // streamed weights: split the channels into the fewest equal tiles
-      // (multiples of 16) whose stage lets at least four stages fit
-      for (int k = 1; k <= 16; ++k) {
-        const int w = ((a.Cin + k - 1) / k + 15) / 16 * 16;
-        if (w > 256) continue;
-        b.ctw = w;
-        if (4 * (kHaloBytes + (size_t)9 * w * 32) <= 200 * 1024) break;
-      }
-    }
-    const int ntb = (a.Cin + b.ctw - 1) / b.ctw;
-    // dout's halo slices (and streamed weight tiles) arrive as tensor
-    // copies, if the maps encode
-    CUtensorMap tm{}, tw{};
-    const int ntm = std::min(b.ctw, a.Cin);  // rows of the widest channel tile
-    const bool tma = kConvTma && a.Cout % 16 == 0 &&
-                     chunk_major_map(&tm, a.dout, a.N, a.H, a.W, a.Cout, kHalo, 2, 3) &&
-                     (res || weight_map(&tw, a.wt, a.Cin, a.Cout, ntm));
-    const size_t wtiles = (size_t)9 * ntm * 32;
-    const size_t stage = tma ? kHaloStage + (res ? 0 : (wtiles + 1023) / 1024 * 1024)
-                             : (res ? kHaloBytes : kHaloBytes + (size_t)9 * b.ctw * 32);
-    const long long T = (long long)a.N * a.H * ((a.W + 127) / 128) * ntb;
-    if (tma)
-      return launch_tiles(k_conv_dgrad_rows<7, true, true>, k_conv_dgrad_rows<6, false, true>,
-                          k_conv_dgrad_rows<4, false, true>, k_conv_dgrad_rows<2, false, true>, res, stage,
-                          res ? wbytes : 0, T, b, tm, tw, st);
-    return launch_tiles(k_conv_dgrad_rows<7, true>, k_conv_dgrad_rows<6, false>, k_conv_dgrad_rows<4, false>,
-                        k_conv_dgrad_rows<2, false>, res, stage, res ? wbytes : 0, T, b, tm, tw, st);
-  }
+  cudaError_t e = cudaSuccess;
+  if (use_rows(a.W, a.Cout) && conv_tile_dgrad(a, st, &e)) return e;
+  if (a.dlow || a.dskip) return cudaErrorNotSupported;  // only the tile kernel splits its output
   int nb = std::min(256, a.Cin);
   size_t stage = 128 * kSlice * 2 + (size_t)nb * kSlice * 2;
   const dim3 grid((unsigned)((P + 127) / 128), (a.Cin + 255) / 256);

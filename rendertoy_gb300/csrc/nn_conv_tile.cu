@@ -1,0 +1,665 @@
+// nn_conv_tile.cu — forward and data-gradient 3 x 3 convolutions on the
+// tcgen05 tensor cores from swizzled tensor copies (TMA).
+//
+// Work unit: a tile of 8 x 16 pixels (the 128 accumulator lanes of one MMA),
+// lane m = pixel (m % 8, m / 8).  Per slab of KC input channels (32; 16 where
+// a channel count asks for it) one tensor copy brings the tile's halo,
+// 10 x 18 pixels of KC channels, into shared memory in the swizzled K-major
+// layout whose rows are one pixel (KC * 2 bytes).  The swizzle is a function
+// of the address alone, so a descriptor may start at any pixel: tap (dy, dx)
+// reads the same halo (dy + 1) * 10 + dx + 1 pixels further on, its eight-lane
+// groups one halo row (10 pixels) apart.  Every source byte is copied 1.4
+// times per tile and never gathered per tap.
+//
+// What bounds it: an MMA of 128 pixels x N outputs x 16 channels reads its
+// 4 KB A operand from shared memory (32 clocks at 128 B per clock) plus 32 N
+// bytes of B, so below N = 128 a step costs about 32 + N / 4 clocks and the
+// tensor pipe cannot fill; a tensor copy moves about one row (here 64 B) per
+// 1.2 clocks (measured: 52 B per clock and SM for 64-byte rows, 13 B for the
+// 16-byte rows of an unswizzled halo, which bounded the row kernels this
+// replaces).
+//
+// k_conv_tile: the order of additions is slab of 16 channels, then tap (rows
+// of 64 pixels or more).  Forms:
+//   one or two full-resolution sources, MT = 1 or 2 vertically adjacent tiles
+//   per unit (2 when weights are streamed: each slab's nine weight tiles then
+//   serve 256 pixels);
+//   kUp: the first source at half resolution (nearest upsampling).  A tile is
+//   8 x 16 low-resolution pixels, i.e. 16 x 32 outputs in four parity classes
+//   (py, px), each with its own accumulator.  Output (2 y + py, 2 x + px)
+//   reads low pixel (y + floor((py + dy) / 2), x + floor((px + dx) / 2)): for
+//   one parity class and tap a constant shift of the low-resolution halo.  A
+//   skip source is read through four tensor maps, one per parity plane
+//   (strides of two pixels and two rows), in which taps are shifts again.  So
+//   neither source is expanded, and weights serve four MMAs per fetch.
+// k_conv_narrow: the order of additions is tap, then 16 channels (rows
+// shorter than 64 pixels): the tile's halo of all slabs stays resident while
+// weights stream by (tap, slabs); an upsampled source is expanded into the
+// halo by the copying warps.
+//
+// Roles (320 threads, one CTA per SM, persistent): thread 0 issues the MMAs,
+// thread 32 the tensor copies, warps 2 .. 9 the epilogue (two warps per 32
+// accumulator lanes, taking alternate chunks of 16 columns).
+#include <algorithm>
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
+#include "nn.h"
+#include "nn_tile.h"
+#include "tc_core.cuh"
+
+namespace rtx {
+namespace nn {
+
+namespace {
+
+constexpr int kThreadsT = 320, kEpiWarps = 8;
+constexpr int kMaxS = 8;
+constexpr int kHW = 10, kPW = 9;  // halo width: full- and low-resolution tiles, parity planes
+
+__host__ __device__ constexpr uint32_t up1k(uint32_t b) { return (b + 1023u) & ~1023u; }
+// bytes of a unit's A region
+__host__ __device__ constexpr uint32_t halo_bytes(int KC, int MT) { return (uint32_t)kHW * (16 * MT + 2) * KC * 2; }
+__host__ __device__ constexpr uint32_t plane_bytes(int KC) { return (uint32_t)kPW * 17 * KC * 2; }
+
+struct TileArgs {
+  int H, W;                 // output resolution
+  int tx, ty, n_tiles;      // tiles per image row / column; images x ty x tx x n-tiles
+  int ntn, NT, Nout;        // output-channel tiles of NT (multiples of 16)
+  int nslab1, nslab;        // slabs of the first source, of both
+  int S, nbuf;              // ring stages, accumulator buffers
+  uint32_t stage, w_off;    // ring stage bytes, weights within a streamed stage
+  int flip;                 // data gradient: taps mirrored
+  uint32_t ncols;           // TMEM columns allocated
+  // epilogue
+  const float* bias;
+  int relu;
+  bf16* out;
+  float* out_f32;
+  // data gradient: the sources (ReLU mask), and where the gradient goes
+  Src s1, s2;
+  int mask_relu;
+  bf16 *din, *dlow, *dskip;
+  int* err;
+  // narrow form
+  int G, nhalo, up1;        // slabs per weight unit, halo buffers, expand the first source
+  uint32_t halo_stride;
+  const bf16* x1;
+  int C1;
+};
+
+struct TileMaps {
+  CUtensorMap w, s1, s2[4];
+};
+
+struct Bars {
+  uint64_t full[kMaxS], empty[kMaxS], accf[2], acce[2], wbar, hfull[2], hempty[2];
+};
+
+__device__ __forceinline__ void tma4(uint32_t dst, const void* m, int c0, int c1, int c2, int c3, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
+      "l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(tc::smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void tma3(uint32_t dst, const void* m, int c0, int c1, int c2, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(tc::smem_u32(bar))
+      : "memory");
+}
+
+// 16 FP32 columns of this thread's accumulator lane
+__device__ __forceinline__ void tmem_ld16(uint32_t t, float* v) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(t)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<uint32_t*>(&h);
+}
+__device__ __forceinline__ float2 unpack2(uint32_t u) {
+  return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u));
+}
+
+// 32 bytes to p: one store where p allows it, else two
+__device__ __forceinline__ void st32(void* p, const uint32_t* u, bool wide) {
+  if (wide) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(u[0]), "r"(u[1]), "r"(u[2]),
+                 "r"(u[3]), "r"(u[4]), "r"(u[5]), "r"(u[6]), "r"(u[7])
+                 : "memory");
+  } else {
+    uint4* q = reinterpret_cast<uint4*>(p);
+    q[0] = make_uint4(u[0], u[1], u[2], u[3]);
+    q[1] = make_uint4(u[4], u[5], u[6], u[7]);
+  }
+}
+
+struct Tile {
+  int n, x0, y0, nt;  // image, tile origin (in tiles' own resolution), output-channel tile
+};
+__device__ __forceinline__ Tile tile_of(const TileArgs& a, int i, int th) {
+  Tile t;
+  int j = (int)blockIdx.x + i * (int)gridDim.x;
+  t.nt = j % a.ntn;
+  j /= a.ntn;
+  t.x0 = (j % a.tx) * 8;
+  j /= a.tx;
+  t.y0 = (j % a.ty) * th;
+  t.n = j / a.ty;
+  return t;
+}
+
+// 16 channels [c, c + 8), [c + 8, c + 16) of the sources at (n, y, x), for the ReLU mask
+__device__ __forceinline__ uint4 mask8(const TileArgs& a, int n, int y, int x, int c) {
+  const Src& s = c < a.s1.C ? a.s1 : a.s2;
+  const int cc = c < a.s1.C ? c : c - a.s1.C;
+  const size_t p = s.up ? ((size_t)n * (a.H >> 1) + (y >> 1)) * (a.W >> 1) + (x >> 1)
+                        : ((size_t)n * a.H + y) * a.W + x;
+  return __ldg(reinterpret_cast<const uint4*>(s.ptr + p * s.C + cc));
+}
+
+constexpr int kBatch = 4;  // chunks whose mask loads are in flight together
+
+// One tile's epilogue for one warp: chunks of 16 columns half, half + 2, ...
+// of the NA accumulators.  `wait` blocks until the accumulators are complete;
+// the first batch's mask loads are issued before it.
+template <int NA, bool kUp, bool kDg, class Wait>
+__device__ __forceinline__ bool tile_epilogue(const TileArgs& a, const Tile& t, uint32_t tmem, int warp, int lane,
+                                              uint4 (*xch)[2], Wait&& wait) {
+  const int q = warp & 3, half = (warp - 2) >> 2;
+  const int m = q * 32 + lane, mx = m & 7, my = m >> 3;
+  const int n0 = t.nt * a.NT, nch = min(a.NT, a.Nout - n0) >> 4;
+  const int total = NA * nch;
+  const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16);
+  auto pixel = [&](int acc, int& y, int& x) {
+    if (kUp) {
+      x = 2 * (t.x0 + mx) + (acc & 1);
+      y = 2 * (t.y0 + my) + (acc >> 1);
+    } else {
+      x = t.x0 + mx;
+      y = t.y0 + 16 * acc + my;
+    }
+    return x < a.W && y < a.H;
+  };
+  bool ready = false;
+  for (int j0 = half; j0 < total; j0 += 2 * kBatch) {
+    uint4 mk[kBatch][2];
+    if (kDg && a.mask_relu) {
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        const int j = j0 + 2 * b;
+        mk[b][0] = mk[b][1] = make_uint4(0, 0, 0, 0);
+        if (j < total) {
+          const int acc = j / nch, c = n0 + (j - acc * nch) * 16;
+          int y, x;
+          if (pixel(acc, y, x)) {
+            mk[b][0] = mask8(a, t.n, y, x, c);
+            mk[b][1] = mask8(a, t.n, y, x, c + 8);
+          }
+        }
+      }
+    }
+    if (!ready) {
+      if (!wait()) return false;
+      ready = true;
+    }
+#pragma unroll
+    for (int b = 0; b < kBatch; ++b) {
+      const int j = j0 + 2 * b;
+      if (j >= total) break;
+      const int acc = j / nch, cc = (j - acc * nch) * 16, c = n0 + cc;
+      int y, x;
+      const bool ok = pixel(acc, y, x);
+      const size_t p = ((size_t)t.n * a.H + y) * a.W + x;
+      float v[16];
+      tmem_ld16(lanes + acc * a.NT + cc, v);
+      if (!kDg) {
+        if (a.bias) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) v[k] += __ldg(a.bias + c + k);
+        }
+        if (a.relu) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) v[k] = fmaxf(v[k], 0.0f);
+        }
+        if (ok && a.out) {
+          uint32_t u[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) u[k] = pack2(v[2 * k], v[2 * k + 1]);
+          bf16* d = a.out + p * a.Nout + c;
+          st32(d, u, (reinterpret_cast<uintptr_t>(a.out) & 31) == 0);
+        }
+        if (ok && a.out_f32) {
+          float* d = a.out_f32 + p * a.Nout + c;
+          const uintptr_t al = reinterpret_cast<uintptr_t>(a.out_f32);
+          if ((al & 15) == 0) {
+            st32(d, reinterpret_cast<const uint32_t*>(v), (al & 31) == 0);
+            st32(d + 8, reinterpret_cast<const uint32_t*>(v) + 8, (al & 31) == 0);
+          } else {
+#pragma unroll
+            for (int k = 0; k < 16; ++k) d[k] = v[k];
+          }
+        }
+      } else {
+        if (a.mask_relu) {
+          const uint32_t* w = reinterpret_cast<const uint32_t*>(mk[b]);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            const float2 s = unpack2(w[k]);
+            if (!(s.x > 0.0f)) v[2 * k] = 0.0f;
+            if (!(s.y > 0.0f)) v[2 * k + 1] = 0.0f;
+          }
+        }
+        uint32_t u[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) u[k] = pack2(v[2 * k], v[2 * k + 1]);
+        if (!a.dlow) {
+          if (ok) {
+            bf16* d = a.din + p * a.Nout + c;
+            st32(d, u, (reinterpret_cast<uintptr_t>(a.din) & 31) == 0);
+          }
+        } else if (c >= a.s1.C) {
+          if (ok) {
+            bf16* d = a.dskip + p * a.s2.C + (c - a.s1.C);
+            st32(d, u, (reinterpret_cast<uintptr_t>(a.dskip) & 31) == 0);
+          }
+        } else {
+          // gradient of nearest upsampling: the 2 x 2 blocks of the warp's
+          // 8 x 4 pixels, summed in FP32 in row order from the BF16 values;
+          // each of a block's four lanes sums four channels
+          xch[lane][0] = make_uint4(u[0], u[1], u[2], u[3]);
+          xch[lane][1] = make_uint4(u[4], u[5], u[6], u[7]);
+          __syncwarp();
+          const int lx = lane & 7, ly = lane >> 3, sub = (ly & 1) * 2 + (lx & 1);
+          const int base = (ly & ~1) * 8 + (lx & ~1);
+          float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const uint2 g = reinterpret_cast<const uint2*>(xch[base + (k >> 1) * 8 + (k & 1)])[sub];
+            const float2 g0 = unpack2(g.x), g1 = unpack2(g.y);
+            s[0] += g0.x;
+            s[1] += g0.y;
+            s[2] += g1.x;
+            s[3] += g1.y;
+          }
+          __syncwarp();
+          if (ok) {
+            const size_t pl = ((size_t)t.n * (a.H >> 1) + (y >> 1)) * (a.W >> 1) + (x >> 1);
+            *reinterpret_cast<uint2*>(a.dlow + pl * a.s1.C + c + 4 * sub) =
+                make_uint2(pack2(s[0], s[1]), pack2(s[2], s[3]));
+          }
+        }
+      }
+    }
+  }
+  if (!ready) return wait();
+  return true;
+}
+
+// swizzled K-major descriptor: 8-row groups `sbo` bytes apart
+template <int KC>
+__device__ __forceinline__ uint64_t kdesc(uint32_t addr, uint32_t sbo) {
+  constexpr uint64_t layout = KC == 32 ? 4 : 6;  // 64- / 32-byte swizzle
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46) |
+         (layout << 61);
+}
+
+__device__ __forceinline__ void bars_init(Bars& b, int S) {
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < S; ++i) {
+      tc::mbar_init(&b.full[i], 1);
+      tc::mbar_init(&b.empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&b.accf[i], 1);
+      tc::mbar_init(&b.acce[i], kEpiWarps * 32);
+      tc::mbar_init(&b.hfull[i], 1 + 32);
+      tc::mbar_init(&b.hempty[i], 1);
+    }
+    tc::mbar_init(&b.wbar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+}
+
+template <int KC, int MT, bool kUp, bool kRes, bool kDg>
+__global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, const __grid_constant__ TileMaps tm) {
+  constexpr int NA = kUp ? 4 : MT;
+  constexpr int RB = KC * 2;  // bytes of a pixel row
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ __align__(8) Bars bars;
+  __shared__ uint32_t tmem_slot;
+  __shared__ uint4 xch[kDg ? kEpiWarps : 1][32][2];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n_tiles = (int)blockIdx.x < a.n_tiles ? (a.n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  if (warp == 0) tc::tmem_alloc(&tmem_slot, a.ncols);
+  bars_init(bars, a.S);
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = tmem_slot, s0 = tc::smem_u32(smem), sw = s0 + a.S * a.stage;
+  const uint32_t tap_bytes = (uint32_t)a.NT * RB, slab_w = 9 * tap_bytes;
+  bool ok = true;
+  if (warp == 0) {
+    if (lane == 0) {
+      if (kRes && n_tiles > 0) ok = tc::mbar_wait(&bars.wbar, 0u);
+      int st = 0;
+      uint32_t ph = 0;
+      for (int i = 0; i < n_tiles && ok; ++i) {
+        const Tile t = tile_of(a, i, kUp ? 16 : 16 * MT);
+        const int buf = a.nbuf == 2 ? (i & 1) : 0, lap = a.nbuf == 2 ? (i >> 1) : i;
+        if (lap > 0) ok = tc::mbar_wait(&bars.acce[buf], (uint32_t)(lap - 1) & 1u);
+        const uint32_t idesc = tc::make_idesc_bf16(128, min(a.NT, a.Nout - t.nt * a.NT));
+        const uint32_t d = tmem + buf * NA * a.NT;
+        for (int s = 0; s < a.nslab && ok; ++s) {
+          ok = tc::mbar_wait(&bars.full[st], ph);
+          if (!ok) break;
+          tc::fence_after();
+          const uint32_t sa = s0 + st * a.stage;
+          const bool skip = kUp && s >= a.nslab1;
+          const uint32_t sb = kRes ? sw + (uint32_t)(t.nt * a.nslab + s) * slab_w : sa + a.w_off;
+          const uint64_t bd = kdesc<KC>(sb, 8 * RB);
+          const uint32_t tap16 = tap_bytes >> 4;
+#pragma unroll
+          for (int ks = 0; ks < KC / 16; ++ks) {
+            const uint64_t ad = kdesc<KC>(sa + 32 * ks, (skip ? kPW : kHW) * RB);
+            const bool acc0 = s > 0 || ks > 0;
+            if (!skip) {
+#pragma unroll
+              for (int tap = 0; tap < 9; ++tap) {
+                const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+#pragma unroll
+                for (int c = 0; c < NA; ++c) {
+                  int off;
+                  if (kUp)
+                    off = (((c >> 1) + dy + 2) / 2) * kHW + ((c & 1) + dx + 2) / 2;  // floor(./2) + 1
+                  else
+                    off = (16 * c + (kDg ? 1 - dy : 1 + dy)) * kHW + (kDg ? 1 - dx : 1 + dx);
+                  tc::mma_bf16(d + c * a.NT, ad + (uint64_t)(off * RB >> 4), bd + 2 * ks + (uint64_t)tap * tap16, idesc,
+                               acc0 || tap > 0);
+                }
+              }
+            } else {
+#pragma unroll
+              for (int tap = 0; tap < 9; ++tap) {
+                const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                  // parity plane (qy, qx), shifts oy + qy, ox + qx of it
+                  const int Y = (c >> 1) + dy, X = (c & 1) + dx, qy = Y & 1, qx = X & 1;
+                  const int oy = (Y - qy) / 2, ox = (X - qx) / 2;
+                  const uint32_t off = (2 * qy + qx) * up1k(plane_bytes(KC)) + ((oy + qy) * kPW + ox + qx) * RB;
+                  tc::mma_bf16(d + c * a.NT, ad + (uint64_t)(off >> 4), bd + 2 * ks + (uint64_t)tap * tap16, idesc,
+                               acc0 || tap > 0);
+                }
+              }
+            }
+          }
+          tc::mma_commit(&bars.empty[st]);
+          if (s == a.nslab - 1) tc::mma_commit(&bars.accf[buf]);
+          if (++st == a.S) {
+            st = 0;
+            ph ^= 1u;
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      if (kRes && n_tiles > 0) {
+        tc::mbar_arrive_expect_tx(&bars.wbar, (uint32_t)(a.ntn * a.nslab) * slab_w);
+        for (int k = 0; k < a.ntn * a.nslab; ++k)
+          tma3(sw + k * slab_w, &tm.w, (k % a.nslab) * KC, (k / a.nslab) * a.NT, 0, &bars.wbar);
+      }
+      int st = 0, issued = 0;
+      uint32_t ph = 1;  // a fresh barrier's preceding phase reads complete
+      for (int i = 0; i < n_tiles && ok; ++i) {
+        const Tile t = tile_of(a, i, kUp ? 16 : 16 * MT);
+        for (int s = 0; s < a.nslab; ++s) {
+          ok = tc::mbar_wait(&bars.empty[st], ph);
+          if (!ok) break;
+          const bool first = s < a.nslab1;
+          const uint32_t sa = s0 + st * a.stage;
+          const uint32_t ab = kUp ? (first ? halo_bytes(KC, 1) : 4 * plane_bytes(KC)) : halo_bytes(KC, MT);
+          tc::mbar_arrive_expect_tx(&bars.full[st], ab + (kRes ? 0u : slab_w));
+          if (!kUp || first) {
+            const int c0 = (first ? s : s - a.nslab1) * KC;
+            tma4(sa, first ? &tm.s1 : &tm.s2[0], c0, t.x0 - 1, t.y0 - 1, t.n, &bars.full[st]);
+          } else {
+#pragma unroll
+            for (int pl = 0; pl < 4; ++pl)  // plane (qy, qx) starts at shift -qy, -qx
+              tma4(sa + pl * up1k(plane_bytes(KC)), &tm.s2[pl], (s - a.nslab1) * KC, t.x0 - (pl & 1),
+                   t.y0 - (pl >> 1), t.n, &bars.full[st]);
+          }
+          if (!kRes) tma3(sa + a.w_off, &tm.w, s * KC, t.nt * a.NT, 0, &bars.full[st]);
+          ++issued;
+          if (++st == a.S) {
+            st = 0;
+            ph ^= 1u;
+          }
+        }
+      }
+      if (!ok) {
+        // a wait ran out: wait (bounded) for the copies issued last on each
+        // stage, so that none lands after the CTA has left
+        for (int u = max(0, issued - a.S); u < issued; ++u) tc::mbar_wait(&bars.full[u % a.S], (uint32_t)(u / a.S) & 1u);
+      }
+    }
+  } else {
+    for (int i = 0; i < n_tiles && ok; ++i) {
+      const Tile t = tile_of(a, i, kUp ? 16 : 16 * MT);
+      const int buf = a.nbuf == 2 ? (i & 1) : 0, lap = a.nbuf == 2 ? (i >> 1) : i;
+      ok = tile_epilogue<NA, kUp, kDg>(a, t, tmem + buf * NA * a.NT, warp, lane, xch[kDg ? warp - 2 : 0], [&] {
+        const bool w = __all_sync(0xffffffffu, tc::mbar_wait(&bars.accf[buf], (uint32_t)lap & 1u));
+        tc::fence_after();
+        return w;
+      });
+      tc::fence_before();
+      tc::mbar_arrive(&bars.acce[buf]);
+    }
+  }
+  if (!__syncthreads_and(ok) && lane == 0) atomicOr(a.err, tc::kErrMbarTimeout);
+  tc::fence_before();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tmem, a.ncols);
+}
+
+}  // namespace
+
+// ---------------------------------------------------------------------------
+// host
+// ---------------------------------------------------------------------------
+static PFN_cuTensorMapEncodeTiled_v12000 encoder() {
+  static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      p = nullptr;
+    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+  }();
+  return fn;
+}
+
+static CUtensorMapSwizzle swizzle_of(int KC) {
+  return KC == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : (KC == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+}
+
+bool pixel_map(CUtensorMap* m, const bf16* base, int imgs, int H, int W, int C, int step, int KC, int bw, int bh) {
+  const PFN_cuTensorMapEncodeTiled_v12000 enc = encoder();
+  if (!enc || (reinterpret_cast<uintptr_t>(base) & 15) || C % 8 || H <= 0 || W <= 0) return false;
+  // `step` 2: every second pixel of every second row (a parity plane of the
+  // image that starts at `base`, H x W counted in plane pixels)
+  const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)imgs};
+  const cuuint64_t row = (cuuint64_t)W * step * C * 2;
+  const cuuint64_t strides[3] = {(cuuint64_t)step * C * 2, (cuuint64_t)step * row, (cuuint64_t)H * step * row};
+  const cuuint32_t box[4] = {(cuuint32_t)KC, (cuuint32_t)bw, (cuuint32_t)bh, 1};
+  const cuuint32_t es[4] = {1, 1, 1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(base), dims, strides, box, es,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_of(KC), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// [rows][9][K] weights as (K, row, tap); a box of (KC, NT, taps) lands tap-major
+static bool tap_map(CUtensorMap* m, const bf16* base, int rows, int K, int KC, int NT, int taps) {
+  const PFN_cuTensorMapEncodeTiled_v12000 enc = encoder();
+  if (!enc || (reinterpret_cast<uintptr_t>(base) & 15) || K % 8) return false;
+  const cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, 9};
+  const cuuint64_t strides[2] = {(cuuint64_t)9 * K * 2, (cuuint64_t)K * 2};
+  const cuuint32_t box[3] = {(cuuint32_t)KC, (cuuint32_t)NT, (cuuint32_t)taps};
+  const cuuint32_t es[3] = {1, 1, 1};
+  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<bf16*>(base), dims, strides, box, es,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_of(KC), CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+int tile_sm_count() {
+  static int n = 0;
+  if (!n) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+      n = 152;
+  }
+  return n;
+}
+
+static uint32_t pow2_cols(uint32_t c) {
+  uint32_t p = 32;
+  while (p < c) p *= 2;
+  return p;
+}
+
+constexpr uint32_t kSmem = 216 * 1024;  // dynamic shared memory a CTA may plan with
+
+template <int KC, int MT, bool kUp, bool kRes, bool kDg>
+static cudaError_t launch_tile(const TileArgs& a, const TileMaps& m, size_t smem, cudaStream_t st) {
+  auto k = k_conv_tile<KC, MT, kUp, kRes, kDg>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e) return e;
+  k<<<std::min(a.n_tiles, tile_sm_count()), kThreadsT, smem, st>>>(a, m);
+  return cudaGetLastError();
+}
+
+// The wide (slab-major) form.  kDg: the data gradient (taps mirrored, single
+// source dout).  False: not a shape (or alignment) it takes.
+template <int KC, bool kDg>
+static bool plan_wide(TileArgs a, const Src& x1, const Src& x2, const bf16* w, int imgs, cudaStream_t st,
+                      cudaError_t* e) {
+  const bool up = !kDg && x1.up;
+  const int K = x1.C + x2.C, K1 = x1.C;
+  a.nslab1 = K1 / KC;
+  a.nslab = K / KC;
+  TileMaps m{};
+  auto weights = [&](int NT) { return (size_t)9 * NT * KC * 2; };
+  // resident weights when they leave room for three halo stages
+  const uint32_t stage_a = up ? std::max(up1k(halo_bytes(KC, 1)), x2.ptr ? 4 * up1k(plane_bytes(KC)) : 0u)
+                              : up1k(halo_bytes(KC, 1));
+  a.ntn = (a.Nout + 255) / 256;
+  a.NT = ((a.Nout + a.ntn - 1) / a.ntn + 15) / 16 * 16;
+  const int NA1 = up ? 4 : 1;
+  const size_t res_bytes = (size_t)a.ntn * a.nslab * weights(a.NT);
+  const bool fits = NA1 * a.NT <= 512;
+  const bool res = fits && res_bytes + 3 * (size_t)stage_a <= kSmem && res_bytes < (1u << 20);
+  int MT = 1;
+  if (!res) {
+    // streamed weights: two tiles per unit (four parity classes when
+    // upsampling), output tiles of at most 128 channels, so that the
+    // accumulators of two units fit TMEM and at least two stages fit
+    MT = up ? 1 : 2;
+    a.ntn = (a.Nout + 127) / 128;
+    for (;; ++a.ntn) {
+      a.NT = ((a.Nout + a.ntn - 1) / a.ntn + 15) / 16 * 16;
+      const size_t s = (up ? stage_a : up1k(halo_bytes(KC, 2))) + up1k((uint32_t)weights(a.NT));
+      if (2 * s <= kSmem || a.NT <= 16) break;
+    }
+  }
+  const uint32_t sa = (up || MT == 1) ? stage_a : up1k(halo_bytes(KC, 2));
+  a.w_off = sa;
+  a.stage = res ? sa : sa + up1k((uint32_t)weights(a.NT));
+  a.S = (int)std::min<size_t>(kMaxS, (kSmem - (res ? res_bytes : 0)) / a.stage);
+  if (a.S < 2) return false;
+  const int NA = up ? 4 : MT;
+  a.nbuf = 2 * NA * a.NT <= 512 ? 2 : 1;
+  a.ncols = pow2_cols(a.nbuf * NA * a.NT);
+  const int th = up ? 32 : 16 * MT, tw = up ? 16 : 8;
+  a.tx = (a.W + tw - 1) / tw;
+  a.ty = (a.H + th - 1) / th;
+  const long long T = (long long)imgs * a.tx * a.ty * a.ntn;
+  if (T > (1LL << 30)) return false;
+  a.n_tiles = (int)T;
+  if (!tap_map(&m.w, w, a.Nout, K, KC, a.NT, 9)) return false;
+  if (up) {
+    if (!pixel_map(&m.s1, x1.ptr, imgs, a.H / 2, a.W / 2, x1.C, 1, KC, kHW, 18)) return false;
+    if (x2.ptr)
+      for (int pl = 0; pl < 4; ++pl)
+        if (!pixel_map(&m.s2[pl], x2.ptr + ((size_t)(pl >> 1) * a.W + (pl & 1)) * x2.C, imgs, a.H / 2, a.W / 2, x2.C, 2,
+                       KC, kPW, 17))
+          return false;
+  } else {
+    if (!pixel_map(&m.s1, x1.ptr, imgs, a.H, a.W, x1.C, 1, KC, kHW, 16 * MT + 2)) return false;
+    if (x2.ptr && !pixel_map(&m.s2[0], x2.ptr, imgs, a.H, a.W, x2.C, 1, KC, kHW, 16 * MT + 2)) return false;
+  }
+  // past half the SM's shared memory: one CTA per SM (TMEM columns)
+  const size_t smem = std::max<size_t>((size_t)a.S * a.stage + (res ? res_bytes : 0), 116 * 1024);
+  if constexpr (!kDg) {
+    if (up) {
+      *e = res ? launch_tile<KC, 1, true, true, false>(a, m, smem, st)
+               : launch_tile<KC, 1, true, false, false>(a, m, smem, st);
+      return true;
+    }
+  }
+  *e = res ? launch_tile<KC, 1, false, true, kDg>(a, m, smem, st) : launch_tile<KC, 2, false, false, kDg>(a, m, smem, st);
+  return true;
+}
+
+bool conv_tile_fwd(const ConvFwd& c, cudaStream_t st, cudaError_t* e) {
+  const int g = c.s2.ptr ? (c.s1.C | c.s2.C) : c.s1.C;
+  if (g % 16 || c.Cout % 16 || c.s2.up || (c.s1.up && (c.H % 2 || c.W % 2))) return false;
+  if (c.out && (reinterpret_cast<uintptr_t>(c.out) & 15)) return false;
+  TileArgs a{};
+  a.H = c.H;
+  a.W = c.W;
+  a.Nout = c.Cout;
+  a.bias = c.bias;
+  a.relu = c.relu;
+  a.out = c.out;
+  a.out_f32 = c.out_f32;
+  a.err = c.err;
+  const Src s2 = c.s2.ptr ? c.s2 : Src{nullptr, 0, 0};
+  return g % 32 == 0 ? plan_wide<32, false>(a, c.s1, s2, c.w, c.N, st, e)
+                     : plan_wide<16, false>(a, c.s1, s2, c.w, c.N, st, e);
+}
+
+bool conv_tile_dgrad(const ConvDgrad& c, cudaStream_t st, cudaError_t* e) {
+  if (c.Cout % 16 || c.Cin % 16) return false;
+  TileArgs a{};
+  a.H = c.H;
+  a.W = c.W;
+  a.Nout = c.Cin;
+  a.s1 = c.s1;
+  a.s2 = c.s2;
+  a.mask_relu = c.mask_relu;
+  a.din = c.din;
+  a.dlow = c.dlow;
+  a.dskip = c.dskip;
+  a.flip = 1;
+  a.err = c.err;
+  const Src d{c.dout, c.Cout, 0}, none{nullptr, 0, 0};
+  return c.Cout % 32 == 0 ? plan_wide<32, true>(a, d, none, c.wt, c.N, st, e)
+                          : plan_wide<16, true>(a, d, none, c.wt, c.N, st, e);
+}
+
+}  // namespace nn
+}  // namespace rtx

@@ -322,7 +322,7 @@ cudaError_t UNet::backward(int N, int H, int W, int* err, cudaStream_t st) {
     if (i == 0) break;  // the input needs no gradient
     // data gradient into the sources
     bool pooled = l.d.s1 == tP1 || l.d.s1 == tP2 || l.d.s1 == tP3 || l.d.s1 == tP4;
-    ConvDgrad d;
+    ConvDgrad d{};
     d.dout = dout;
     d.Cout = l.d.cout_pad;
     d.wt = I.wbf + l.wt_off;
@@ -335,12 +335,19 @@ cudaError_t UNet::backward(int N, int H, int W, int* err, cudaStream_t st) {
     d.mask_relu = pooled ? 0 : 1;  // pooled inputs are not ReLU outputs
     d.err = err;
     if (l.d.s2 >= 0) {
-      d.din = I.dcat;
-      if ((e = conv_dgrad(d, st))) return e;
-      int c1 = kTC[l.d.s1], c2 = kTC[l.d.s2];
-      if ((e = upsample_grad(I.dcat, l.cin_pad, 0, I.dact[l.d.s1], N, h, w, c1, st))) return e;
-      if ((e = take_channels(I.dcat, l.cin_pad, c1, I.dact[l.d.s2], P, c2, st))) return e;
-      I.launches += 3;
+      if (conv_dgrad_splits(d)) {
+        d.dlow = I.dact[l.d.s1];
+        d.dskip = I.dact[l.d.s2];
+        if ((e = conv_dgrad(d, st))) return e;
+        ++I.launches;
+      } else {
+        d.din = I.dcat;
+        if ((e = conv_dgrad(d, st))) return e;
+        int c1 = kTC[l.d.s1], c2 = kTC[l.d.s2];
+        if ((e = upsample_grad(I.dcat, l.cin_pad, 0, I.dact[l.d.s1], N, h, w, c1, st))) return e;
+        if ((e = take_channels(I.dcat, l.cin_pad, c1, I.dact[l.d.s2], P, c2, st))) return e;
+        I.launches += 3;
+      }
     } else {
       d.din = I.dact[l.d.s1];
       if ((e = conv_dgrad(d, st))) return e;

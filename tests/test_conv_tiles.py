@@ -1,0 +1,99 @@
+"""The tile convolutions (8 x 16-pixel tiles from swizzled tensor copies) at
+the sizes where they can go wrong, against the FP64 oracle on the same BF16
+values: one pixel past and short of a tile, single rows, odd low-resolution
+sizes, 16- and 32-channel slabs, resident and streamed weights, several
+output-channel tiles, rings that wrap.  Tolerance: FP32 accumulation of at
+most 9 x 288 products, |err| <= K 2^-24 sum |x w| in the worst case; 1e-4
+relative (1e-5 of the largest value for sums that cancel) is above it for
+these inputs and far below any indexing mistake.  Gradients in BF16 add one
+rounding (2^-8)."""
+import numpy as np
+import pytest
+
+from oracle import unet_oracle as U
+
+pytestmark = pytest.mark.gpu
+
+CASES = [  # N, H, W, C1, up1, C2, Cout
+    (1, 1, 64, 32, 0, 0, 16),      # one row, the narrowest row-order width
+    (1, 17, 65, 32, 0, 0, 32),     # one pixel past a tile both ways
+    (2, 15, 71, 16, 0, 0, 32),     # 16-channel slabs, one pixel short
+    (1, 16, 72, 48, 0, 16, 48),    # two full-resolution sources, 16-channel slabs
+    (1, 33, 80, 64, 0, 32, 96),    # two sources, 32-channel slabs
+    (1, 33, 64, 128, 0, 0, 160),   # streamed weights: two tiles per unit, two output tiles
+    (1, 20, 66, 96, 0, 0, 256),    # four output tiles of streamed weights
+    (1, 34, 66, 64, 1, 32, 32),    # upsampled + skip, odd low-resolution size
+    (1, 18, 80, 32, 1, 0, 64),     # upsampled source alone
+    (2, 32, 64, 96, 1, 64, 64),    # upsampled + skip, streamed weights
+    (1, 18, 68, 160, 1, 128, 128),  # 288 inputs: two output tiles of four accumulators
+    (1, 20, 70, 48, 1, 16, 16),    # upsampled + skip, 16-channel slabs
+    (6, 48, 128, 32, 0, 0, 32),    # several tiles per CTA: rings and accumulators wrap
+    (6, 32, 128, 64, 1, 32, 32),
+]
+
+
+def bits(x):
+    f = U.to_bf16(x).astype(np.float32)
+    return (f.view(np.uint32) >> 16).astype(np.uint16)
+
+
+def val(b):
+    return (b.astype(np.uint32) << 16).view(np.float32).astype(np.float64)
+
+
+def inputs(c, seed):
+    N, H, W, C1, up, C2, Cout = c
+    rng = np.random.RandomState(seed)
+    x1 = bits(np.maximum(rng.normal(size=(N, H // 2, W // 2, C1) if up else (N, H, W, C1)), 0.0))
+    x2 = bits(np.maximum(rng.normal(size=(N, H, W, C2)), 0.0)) if C2 else None
+    w = bits(rng.normal(0, np.sqrt(2.0 / (9 * (C1 + C2))), (Cout, 9, C1 + C2)))
+    x = U.upsample2(val(x1)) if up else val(x1)
+    if C2:
+        x = np.concatenate([x, val(x2)], 3)
+    dout = bits(rng.normal(size=(N, H, W, Cout)))
+    return x1, x2, w, x, dout, rng.normal(0, 0.1, Cout).astype(np.float32)
+
+
+@pytest.mark.parametrize("c", CASES)
+def test_forward(ctx, c):
+    x1, x2, w, x, _, b = inputs(c, 1)
+    out = ctx.conv3x3_fwd(x1, w, c[6], x2=x2, up1=bool(c[4]), bias=b, relu=True)
+    ref = np.maximum(U.conv3x3(x, val(w).reshape(c[6], 3, 3, -1), b.astype(np.float64)), 0.0)
+    np.testing.assert_allclose(out, ref, rtol=1e-4, atol=1e-5 * np.abs(ref).max())
+
+
+@pytest.mark.parametrize("c", CASES)
+def test_data_gradient(ctx, c):
+    x1, x2, w, x, dout, _ = inputs(c, 2)
+    wt = np.ascontiguousarray(w.transpose(2, 1, 0))
+    din = ctx.conv3x3_dgrad(dout, wt, x1, x2=x2, up1=bool(c[4]), mask_relu=True)
+    ref = np.where(x > 0.0, U.conv3x3_dgrad(val(dout), val(w).reshape(c[6], 3, 3, -1)), 0.0)
+    np.testing.assert_allclose(val(din), ref, rtol=2.0 ** -7, atol=1e-5 * np.abs(ref).max())
+
+
+@pytest.mark.parametrize("shape", [(1, 64, 80), (2, 80, 144)])
+def test_network_gradients(ctx, shape):
+    """The whole network at sizes whose upper levels take the tile kernels
+    (the data gradients of the decoder write their two sources directly): no
+    layer's gradient further from exact FP64 than twice what BF16 storage
+    itself moves it, as for the narrow network."""
+    N, H, W = shape
+    rng = np.random.RandomState(H + W)
+    raw = np.zeros((N, H, W, 11), np.float32)
+    raw[..., :3] = rng.exponential(0.6, (N, H, W, 3))
+    raw[..., 3:10] = rng.uniform(0, 1, (N, H, W, 7))
+    raw[..., 10] = 16.0
+    target = (raw[..., :3] * rng.uniform(0.5, 1.5, (N, H, W, 3))).astype(np.float32)
+    ctx.dn_init(5)
+    p = U.init_params(9).astype(np.float32)
+    ctx.dn_set_params(p)
+    loss = ctx.dn_loss_grads(raw, target)
+    g = ctx.dn_get_grads()
+    lo, go = U.UNet(p.astype(np.float64), bf16=True).loss_and_grads(raw, target)
+    _, gf = U.UNet(p.astype(np.float64), bf16=False).loss_and_grads(raw, target)
+    assert abs(loss - lo) <= 1e-4 * lo
+    rel = lambda a, b: np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-30)  # noqa: E731
+    for i, r in enumerate(U.layer_table()[0]):
+        for off, n in ((r["w_off"], r["cout_pad"] * 9 * r["cin_pad"]), (r["b_off"], r["cout_pad"])):
+            a, b, c = g[off:off + n], go[off:off + n], gf[off:off + n]
+            assert rel(a, c) <= 2.0 * rel(b, c) + 2e-3, (i, rel(a, c), rel(b, c))
