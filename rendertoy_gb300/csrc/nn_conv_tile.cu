@@ -38,8 +38,9 @@
 // halo by the copying warps.
 //
 // Roles (320 threads, one CTA per SM, persistent): thread 0 issues the MMAs,
-// thread 32 the tensor copies, warps 2 .. 9 the epilogue (two warps per 32
-// accumulator lanes, taking alternate chunks of 16 columns).
+// thread 32 the tensor copies, warps 2 .. 9 the epilogue (two groups of four
+// warps on alternate tiles, up to four accumulators in flight; both groups on
+// each tile of kUp's four accumulators).
 #include <algorithm>
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -54,7 +55,7 @@ namespace nn {
 namespace {
 
 constexpr int kThreadsT = 320, kEpiWarps = 8;
-constexpr int kMaxS = 8;
+constexpr int kMaxS = 8, kMaxBuf = 4;
 constexpr int kHW = 10, kPW = 9;  // halo width: full- and low-resolution tiles, parity planes
 
 __host__ __device__ constexpr uint32_t up1k(uint32_t b) { return (b + 1023u) & ~1023u; }
@@ -93,7 +94,7 @@ struct TileMaps {
 };
 
 struct Bars {
-  uint64_t full[kMaxS], empty[kMaxS], accf[2], acce[2], wbar, hfull[2], hempty[2];
+  uint64_t full[kMaxS], empty[kMaxS], accf[kMaxBuf], acce[kMaxBuf], wbar, hfull[2], hempty[2];
 };
 
 __device__ __forceinline__ void tma4(uint32_t dst, const void* m, int c0, int c1, int c2, int c3, uint64_t* bar) {
@@ -149,17 +150,35 @@ __device__ __forceinline__ void st32(void* p, const uint32_t* u, bool wide) {
 struct Tile {
   int n, x0, y0, nt;  // image, tile origin (in tiles' own resolution), output-channel tile
 };
-__device__ __forceinline__ Tile tile_of(const TileArgs& a, int i, int th) {
-  Tile t;
-  int j = (int)blockIdx.x + i * (int)gridDim.x;
-  t.nt = j % a.ntn;
-  j /= a.ntn;
-  t.x0 = (j % a.tx) * 8;
-  j /= a.tx;
-  t.y0 = (j % a.ty) * th;
-  t.n = j / a.ty;
-  return t;
-}
+// Tiles first, first + step, ... in (image, y, x, output tile) order, without
+// a division per tile.
+struct TileIter {
+  int nt, x, y, n, snt, sx, sy, sn;
+  __device__ __forceinline__ TileIter(const TileArgs& a, int first, int step) {
+    nt = first % a.ntn;
+    first /= a.ntn;
+    x = first % a.tx;
+    first /= a.tx;
+    y = first % a.ty;
+    n = first / a.ty;
+    snt = step % a.ntn;
+    step /= a.ntn;
+    sx = step % a.tx;
+    step /= a.tx;
+    sy = step % a.ty;
+    sn = step / a.ty;
+  }
+  __device__ __forceinline__ void next(const TileArgs& a) {
+    nt += snt;
+    x += sx;
+    y += sy;
+    n += sn;
+    if (nt >= a.ntn) nt -= a.ntn, ++x;
+    if (x >= a.tx) x -= a.tx, ++y;
+    if (y >= a.ty) y -= a.ty, ++n;
+  }
+  __device__ __forceinline__ Tile tile(int th) const { return Tile{n, x * 8, y * th, nt}; }
+};
 
 // 16 channels [c, c + 8), [c + 8, c + 16) of the sources at (n, y, x), for the ReLU mask
 __device__ __forceinline__ uint4 mask8(const TileArgs& a, int n, int y, int x, int c) {
@@ -172,13 +191,16 @@ __device__ __forceinline__ uint4 mask8(const TileArgs& a, int n, int y, int x, i
 
 constexpr int kBatch = 4;  // chunks whose mask loads are in flight together
 
-// One tile's epilogue for one warp: chunks of 16 columns half, half + 2, ...
-// of the NA accumulators.  `wait` blocks until the accumulators are complete;
-// the first batch's mask loads are issued before it.
-template <int NA, bool kUp, bool kDg, class Wait>
+// One tile's epilogue for one warp: chunks first, first + step, ... of 16
+// columns of the NA accumulators, for its 32 lanes (at least one chunk).  `wait` blocks until the accumulators are
+// complete; the first batch's mask loads are issued before it.  `release`
+// runs once the last column is in registers: the MMAs of a later tile need
+// not wait for this one's stores.
+template <int NA, bool kUp, bool kDg, class Wait, class Release>
 __device__ __forceinline__ bool tile_epilogue(const TileArgs& a, const Tile& t, uint32_t tmem, int warp, int lane,
-                                              uint4 (*xch)[2], Wait&& wait) {
-  const int q = warp & 3, half = (warp - 2) >> 2;
+                                              uint4 (*xch)[2], const float* bias, int first, int step, Wait&& wait,
+                                              Release&& release) {
+  const int q = warp & 3;
   const int m = q * 32 + lane, mx = m & 7, my = m >> 3;
   const int n0 = t.nt * a.NT, nch = min(a.NT, a.Nout - n0) >> 4;
   const int total = NA * nch;
@@ -194,12 +216,12 @@ __device__ __forceinline__ bool tile_epilogue(const TileArgs& a, const Tile& t, 
     return x < a.W && y < a.H;
   };
   bool ready = false;
-  for (int j0 = half; j0 < total; j0 += 2 * kBatch) {
+  for (int j0 = first; j0 < total; j0 += kBatch * step) {
     uint4 mk[kBatch][2];
     if (kDg && a.mask_relu) {
 #pragma unroll
       for (int b = 0; b < kBatch; ++b) {
-        const int j = j0 + 2 * b;
+        const int j = j0 + b * step;
         mk[b][0] = mk[b][1] = make_uint4(0, 0, 0, 0);
         if (j < total) {
           const int acc = j / nch, c = n0 + (j - acc * nch) * 16;
@@ -217,7 +239,7 @@ __device__ __forceinline__ bool tile_epilogue(const TileArgs& a, const Tile& t, 
     }
 #pragma unroll
     for (int b = 0; b < kBatch; ++b) {
-      const int j = j0 + 2 * b;
+      const int j = j0 + b * step;
       if (j >= total) break;
       const int acc = j / nch, cc = (j - acc * nch) * 16, c = n0 + cc;
       int y, x;
@@ -225,10 +247,17 @@ __device__ __forceinline__ bool tile_epilogue(const TileArgs& a, const Tile& t, 
       const size_t p = ((size_t)t.n * a.H + y) * a.W + x;
       float v[16];
       tmem_ld16(lanes + acc * a.NT + cc, v);
+      if (j + step >= total) release();
       if (!kDg) {
         if (a.bias) {
 #pragma unroll
-          for (int k = 0; k < 16; ++k) v[k] += __ldg(a.bias + c + k);
+          for (int k = 0; k < 16; k += 4) {
+            const float4 b4 = *reinterpret_cast<const float4*>(bias + c + k);
+            v[k] += b4.x;
+            v[k + 1] += b4.y;
+            v[k + 2] += b4.z;
+            v[k + 3] += b4.w;
+          }
         }
         if (a.relu) {
 #pragma unroll
@@ -304,7 +333,6 @@ __device__ __forceinline__ bool tile_epilogue(const TileArgs& a, const Tile& t, 
       }
     }
   }
-  if (!ready) return wait();
   return true;
 }
 
@@ -316,15 +344,17 @@ __device__ __forceinline__ uint64_t kdesc(uint32_t addr, uint32_t sbo) {
          (layout << 61);
 }
 
-__device__ __forceinline__ void bars_init(Bars& b, int S) {
+__device__ __forceinline__ void bars_init(Bars& b, int S, int readers) {
   if (threadIdx.x == 0) {
     for (int i = 0; i < S; ++i) {
       tc::mbar_init(&b.full[i], 1);
       tc::mbar_init(&b.empty[i], 1);
     }
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < kMaxBuf; ++i) {
       tc::mbar_init(&b.accf[i], 1);
-      tc::mbar_init(&b.acce[i], kEpiWarps * 32);
+      tc::mbar_init(&b.acce[i], readers);
+    }
+    for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&b.hfull[i], 1 + 32);
       tc::mbar_init(&b.hempty[i], 1);
     }
@@ -337,14 +367,18 @@ template <int KC, int MT, bool kUp, bool kRes, bool kDg>
 __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, const __grid_constant__ TileMaps tm) {
   constexpr int NA = kUp ? 4 : MT;
   constexpr int RB = KC * 2;  // bytes of a pixel row
+  constexpr int kTH = kUp ? 16 : 16 * MT;
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) Bars bars;
   __shared__ uint32_t tmem_slot;
   __shared__ uint4 xch[kDg ? kEpiWarps : 1][32][2];
+  __shared__ __align__(16) float bias[kDg ? 4 : 256];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tiles = (int)blockIdx.x < a.n_tiles ? (a.n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   if (warp == 0) tc::tmem_alloc(&tmem_slot, a.ncols);
-  bars_init(bars, a.S);
+  bars_init(bars, a.S, kUp ? kEpiWarps * 32 : kEpiWarps * 16);
+  if (!kDg && a.bias)
+    for (int k = tid; k < a.Nout; k += kThreadsT) bias[k] = a.bias[k];
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
@@ -354,12 +388,12 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
   if (warp == 0) {
     if (lane == 0) {
       if (kRes && n_tiles > 0) ok = tc::mbar_wait(&bars.wbar, 0u);
-      int st = 0;
-      uint32_t ph = 0;
-      for (int i = 0; i < n_tiles && ok; ++i) {
-        const Tile t = tile_of(a, i, kUp ? 16 : 16 * MT);
-        const int buf = a.nbuf == 2 ? (i & 1) : 0, lap = a.nbuf == 2 ? (i >> 1) : i;
-        if (lap > 0) ok = tc::mbar_wait(&bars.acce[buf], (uint32_t)(lap - 1) & 1u);
+      int st = 0, buf = 0;
+      uint32_t ph = 0, bph = 1;  // a fresh barrier's preceding phase reads complete
+      TileIter it(a, (int)blockIdx.x, (int)gridDim.x);
+      for (int i = 0; i < n_tiles && ok; ++i, it.next(a)) {
+        const Tile t = it.tile(kTH);
+        ok = tc::mbar_wait(&bars.acce[buf], bph);
         const uint32_t idesc = tc::make_idesc_bf16(128, min(a.NT, a.Nout - t.nt * a.NT));
         const uint32_t d = tmem + buf * NA * a.NT;
         for (int s = 0; s < a.nslab && ok; ++s) {
@@ -413,6 +447,10 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
             ph ^= 1u;
           }
         }
+        if (++buf == a.nbuf) {
+          buf = 0;
+          bph ^= 1u;
+        }
       }
     }
   } else if (warp == 1) {
@@ -424,8 +462,9 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
       }
       int st = 0, issued = 0;
       uint32_t ph = 1;  // a fresh barrier's preceding phase reads complete
-      for (int i = 0; i < n_tiles && ok; ++i) {
-        const Tile t = tile_of(a, i, kUp ? 16 : 16 * MT);
+      TileIter it(a, (int)blockIdx.x, (int)gridDim.x);
+      for (int i = 0; i < n_tiles && ok; ++i, it.next(a)) {
+        const Tile t = it.tile(kTH);
         for (int s = 0; s < a.nslab; ++s) {
           ok = tc::mbar_wait(&bars.empty[st], ph);
           if (!ok) break;
@@ -457,16 +496,27 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
       }
     }
   } else {
-    for (int i = 0; i < n_tiles && ok; ++i) {
-      const Tile t = tile_of(a, i, kUp ? 16 : 16 * MT);
-      const int buf = a.nbuf == 2 ? (i & 1) : 0, lap = a.nbuf == 2 ? (i >> 1) : i;
-      ok = tile_epilogue<NA, kUp, kDg>(a, t, tmem + buf * NA * a.NT, warp, lane, xch[kDg ? warp - 2 : 0], [&] {
-        const bool w = __all_sync(0xffffffffu, tc::mbar_wait(&bars.accf[buf], (uint32_t)lap & 1u));
-        tc::fence_after();
-        return w;
-      });
-      tc::fence_before();
-      tc::mbar_arrive(&bars.acce[buf]);
+    // The two groups of four warps take alternate tiles; a tile of four
+    // accumulators (kUp) they share, in alternate chunks.  (Alternate tiles
+    // need two accumulator buffers: with one, a group would skip every second
+    // phase of its barrier.)
+    const int g = (warp - 2) >> 2;
+    constexpr int kStep = kUp ? 1 : 2;
+    TileIter it(a, (int)(blockIdx.x + (kUp ? 0 : g) * gridDim.x), kStep * (int)gridDim.x);
+    for (int i = kUp ? 0 : g; i < n_tiles && ok; i += kStep, it.next(a)) {
+      const Tile t = it.tile(kTH);
+      const int buf = i % a.nbuf, lap = i / a.nbuf;
+      ok = tile_epilogue<NA, kUp, kDg>(
+          a, t, tmem + buf * NA * a.NT, warp, lane, xch[kDg ? warp - 2 : 0], bias, kUp ? g : 0, kUp ? 2 : 1,
+          [&] {
+            const bool w = __all_sync(0xffffffffu, tc::mbar_wait(&bars.accf[buf], (uint32_t)lap & 1u));
+            tc::fence_after();
+            return w;
+          },
+          [&] {
+            tc::fence_before();
+            tc::mbar_arrive(&bars.acce[buf]);
+          });
     }
   }
   if (!__syncthreads_and(ok) && lane == 0) atomicOr(a.err, tc::kErrMbarTimeout);
@@ -591,7 +641,8 @@ static bool plan_wide(TileArgs a, const Src& x1, const Src& x2, const bf16* w, i
   a.S = (int)std::min<size_t>(kMaxS, (kSmem - (res ? res_bytes : 0)) / a.stage);
   if (a.S < 2) return false;
   const int NA = up ? 4 : MT;
-  a.nbuf = 2 * NA * a.NT <= 512 ? 2 : 1;
+  a.nbuf = std::min(kMaxBuf, 512 / (NA * a.NT));
+  if (!up && a.nbuf < 2) return false;
   a.ncols = pow2_cols(a.nbuf * NA * a.NT);
   const int th = up ? 32 : 16 * MT, tw = up ? 16 : 8;
   a.tx = (a.W + tw - 1) / tw;
