@@ -37,10 +37,10 @@
 // weights stream by (tap, slabs); an upsampled source is expanded into the
 // halo by the copying warps.
 //
-// Roles (320 threads, one CTA per SM, persistent): thread 0 issues the MMAs,
-// thread 32 the tensor copies, warps 2 .. 9 the epilogue (two groups of four
-// warps on alternate tiles, up to four accumulators in flight; both groups on
-// each tile of kUp's four accumulators).
+// Roles (576 threads, one CTA per SM, persistent): warp 0 issues the MMAs,
+// thread 32 the tensor copies, warps 2 .. 17 are four epilogue groups of four
+// warps, on alternate tiles (up to four accumulator buffers) or, for kUp, one
+// accumulator each.
 #include <algorithm>
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -54,7 +54,7 @@ namespace nn {
 
 namespace {
 
-constexpr int kThreadsT = 320, kEpiWarps = 8;
+constexpr int kEpiWarps = 16, kThreadsT = 64 + 32 * kEpiWarps;
 constexpr int kMaxS = 8, kMaxBuf = 4;
 constexpr int kHW = 10, kPW = 9;  // halo width: full- and low-resolution tiles, parity planes
 
@@ -112,6 +112,17 @@ __device__ __forceinline__ void tma3(uint32_t dst, const void* m, int c0, int c1
       : "memory");
 }
 
+// One lane of a converged warp
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+  return p != 0;
+}
+// The whole warp waits; the result is the same on every lane
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity));
+}
+
 // 16 FP32 columns of this thread's accumulator lane
 __device__ __forceinline__ void tmem_ld16(uint32_t t, float* v) {
   uint32_t r[16];
@@ -124,6 +135,22 @@ __device__ __forceinline__ void tmem_ld16(uint32_t t, float* v) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ void tmem_ld32(uint32_t t, float* v) {
+  uint32_t r[32];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
+      "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(t)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
@@ -180,156 +207,157 @@ struct TileIter {
   __device__ __forceinline__ Tile tile(int th) const { return Tile{n, x * 8, y * th, nt}; }
 };
 
-// 16 channels [c, c + 8), [c + 8, c + 16) of the sources at (n, y, x), for the ReLU mask
-__device__ __forceinline__ uint4 mask8(const TileArgs& a, int n, int y, int x, int c) {
-  const Src& s = c < a.s1.C ? a.s1 : a.s2;
-  const int cc = c < a.s1.C ? c : c - a.s1.C;
-  const size_t p = s.up ? ((size_t)n * (a.H >> 1) + (y >> 1)) * (a.W >> 1) + (x >> 1)
-                        : ((size_t)n * a.H + y) * a.W + x;
-  return __ldg(reinterpret_cast<const uint4*>(s.ptr + p * s.C + cc));
+// 16 output columns (channels c .. c + 15 of this lane's pixel p) of a
+// forward convolution
+__device__ __forceinline__ void store_fwd(const TileArgs& a, float* v, int c, size_t p, bool ok, const float* bias) {
+  if (a.bias) {
+#pragma unroll
+    for (int k = 0; k < 16; k += 4) {
+      const float4 b4 = *reinterpret_cast<const float4*>(bias + c + k);
+      v[k] += b4.x;
+      v[k + 1] += b4.y;
+      v[k + 2] += b4.z;
+      v[k + 3] += b4.w;
+    }
+  }
+  if (a.relu) {
+#pragma unroll
+    for (int k = 0; k < 16; ++k) v[k] = fmaxf(v[k], 0.0f);
+  }
+  if (!ok) return;
+  if (a.out) {
+    uint32_t u[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) u[k] = pack2(v[2 * k], v[2 * k + 1]);
+    st32(a.out + p * a.Nout + c, u, (reinterpret_cast<uintptr_t>(a.out) & 31) == 0);
+  }
+  if (a.out_f32) {
+    float* d = a.out_f32 + p * a.Nout + c;
+    const uintptr_t al = reinterpret_cast<uintptr_t>(a.out_f32);
+    if ((al & 15) == 0) {
+      st32(d, reinterpret_cast<const uint32_t*>(v), (al & 31) == 0);
+      st32(d + 8, reinterpret_cast<const uint32_t*>(v) + 8, (al & 31) == 0);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) d[k] = v[k];
+    }
+  }
 }
 
-constexpr int kBatch = 4;  // chunks whose mask loads are in flight together
+// The same for a data gradient: the ReLU mask (`mk`: the source's 16 BF16
+// values), then din, or the two sources' gradients.  Warp-wide.
+__device__ __forceinline__ void store_dgrad(const TileArgs& a, float* v, const uint4* mk, int c, size_t p, size_t plow,
+                                            bool ok, int lane, uint4 (*xch)[2]) {
+  if (a.mask_relu) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(mk);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float2 s = unpack2(w[k]);
+      if (!(s.x > 0.0f)) v[2 * k] = 0.0f;
+      if (!(s.y > 0.0f)) v[2 * k + 1] = 0.0f;
+    }
+  }
+  uint32_t u[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) u[k] = pack2(v[2 * k], v[2 * k + 1]);
+  if (!a.dlow) {
+    if (ok) st32(a.din + p * a.Nout + c, u, (reinterpret_cast<uintptr_t>(a.din) & 31) == 0);
+  } else if (c >= a.s1.C) {
+    if (ok) st32(a.dskip + p * a.s2.C + (c - a.s1.C), u, (reinterpret_cast<uintptr_t>(a.dskip) & 31) == 0);
+  } else {
+    // gradient of nearest upsampling: the 2 x 2 blocks of the warp's 8 x 4
+    // pixels, summed in FP32 in row order from the BF16 values; each of a
+    // block's four lanes sums four channels
+    xch[lane][0] = make_uint4(u[0], u[1], u[2], u[3]);
+    xch[lane][1] = make_uint4(u[4], u[5], u[6], u[7]);
+    __syncwarp();
+    const int lx = lane & 7, ly = lane >> 3, sub = (ly & 1) * 2 + (lx & 1);
+    const int base = (ly & ~1) * 8 + (lx & ~1);
+    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint2 g = reinterpret_cast<const uint2*>(xch[base + (k >> 1) * 8 + (k & 1)])[sub];
+      const float2 g0 = unpack2(g.x), g1 = unpack2(g.y);
+      s[0] += g0.x;
+      s[1] += g0.y;
+      s[2] += g1.x;
+      s[3] += g1.y;
+    }
+    __syncwarp();
+    if (ok)
+      *reinterpret_cast<uint2*>(a.dlow + plow * a.s1.C + c + 4 * sub) = make_uint2(pack2(s[0], s[1]), pack2(s[2], s[3]));
+  }
+}
 
-// One tile's epilogue for one warp: chunks first, first + step, ... of 16
-// columns of the NA accumulators, for its 32 lanes (at least one chunk).  `wait` blocks until the accumulators are
-// complete; the first batch's mask loads are issued before it.  `release`
-// runs once the last column is in registers: the MMAs of a later tile need
-// not wait for this one's stores.
-template <int NA, bool kUp, bool kDg, class Wait, class Release>
-__device__ __forceinline__ bool tile_epilogue(const TileArgs& a, const Tile& t, uint32_t tmem, int warp, int lane,
-                                              uint4 (*xch)[2], const float* bias, int first, int step, Wait&& wait,
+// The epilogue of accumulators [acc0, acc1) of a tile for one warp (its 32
+// lanes, every column).  `wait` blocks until the accumulators are complete;
+// a data gradient's first mask loads are issued before it.  `release` runs
+// once the last column is in registers: the MMAs of a later tile need not
+// wait for this one's stores.  Returns false when the wait ran out.
+template <bool kUp, bool kDg, class Wait, class Release>
+__device__ __forceinline__ bool tile_epilogue(const TileArgs& a, const Tile& t, uint32_t tmem, int acc0, int acc1,
+                                              int warp, int lane, uint4 (*xch)[2], const float* bias, Wait&& wait,
                                               Release&& release) {
   const int q = warp & 3;
   const int m = q * 32 + lane, mx = m & 7, my = m >> 3;
-  const int n0 = t.nt * a.NT, nch = min(a.NT, a.Nout - n0) >> 4;
-  const int total = NA * nch;
+  const int n0 = t.nt * a.NT, nt = min(a.NT, a.Nout - n0);
   const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16);
-  auto pixel = [&](int acc, int& y, int& x) {
-    if (kUp) {
-      x = 2 * (t.x0 + mx) + (acc & 1);
-      y = 2 * (t.y0 + my) + (acc >> 1);
-    } else {
-      x = t.x0 + mx;
-      y = t.y0 + 16 * acc + my;
-    }
-    return x < a.W && y < a.H;
-  };
   bool ready = false;
-  for (int j0 = first; j0 < total; j0 += kBatch * step) {
-    uint4 mk[kBatch][2];
-    if (kDg && a.mask_relu) {
+  for (int acc = acc0; acc < acc1; ++acc) {
+    const int x = kUp ? 2 * (t.x0 + mx) + (acc & 1) : t.x0 + mx;
+    const int y = kUp ? 2 * (t.y0 + my) + (acc >> 1) : t.y0 + 16 * acc + my;
+    const bool ok = x < a.W && y < a.H;
+    const size_t p = ((size_t)t.n * a.H + y) * a.W + x;
+    const size_t plow = ((size_t)t.n * (a.H >> 1) + (y >> 1)) * (a.W >> 1) + (x >> 1);
+    const uint32_t taddr = lanes + acc * a.NT;
+    if constexpr (kDg) {
+      constexpr int kAhead = 4;  // 16-channel chunks whose mask loads are in flight together
+      const size_t p1 = a.s1.up ? plow : p, p2 = a.s2.up ? plow : p;
+      for (int c0 = 0; c0 < nt; c0 += 16 * kAhead) {
+        uint4 mk[kAhead][2];
+        if (a.mask_relu) {
 #pragma unroll
-      for (int b = 0; b < kBatch; ++b) {
-        const int j = j0 + b * step;
-        mk[b][0] = mk[b][1] = make_uint4(0, 0, 0, 0);
-        if (j < total) {
-          const int acc = j / nch, c = n0 + (j - acc * nch) * 16;
-          int y, x;
-          if (pixel(acc, y, x)) {
-            mk[b][0] = mask8(a, t.n, y, x, c);
-            mk[b][1] = mask8(a, t.n, y, x, c + 8);
-          }
+          for (int b = 0; b < kAhead; ++b)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int c = n0 + c0 + 16 * b + 8 * h;
+              mk[b][h] = make_uint4(0, 0, 0, 0);
+              if (ok && c0 + 16 * b < nt)
+                mk[b][h] = __ldg(reinterpret_cast<const uint4*>(c < a.s1.C ? a.s1.ptr + p1 * a.s1.C + c
+                                                                           : a.s2.ptr + p2 * a.s2.C + (c - a.s1.C)));
+            }
+        }
+        if (!ready) {
+          if (!wait()) return false;
+          ready = true;
+        }
+#pragma unroll
+        for (int b = 0; b < kAhead; ++b) {
+          if (c0 + 16 * b >= nt) break;
+          float v[16];
+          tmem_ld16(taddr + c0 + 16 * b, v);
+          if (acc == acc1 - 1 && c0 + 16 * b + 16 >= nt) release();
+          store_dgrad(a, v, mk[b], n0 + c0 + 16 * b, p, plow, ok, lane, xch);
         }
       }
-    }
-    if (!ready) {
-      if (!wait()) return false;
-      ready = true;
-    }
-#pragma unroll
-    for (int b = 0; b < kBatch; ++b) {
-      const int j = j0 + b * step;
-      if (j >= total) break;
-      const int acc = j / nch, cc = (j - acc * nch) * 16, c = n0 + cc;
-      int y, x;
-      const bool ok = pixel(acc, y, x);
-      const size_t p = ((size_t)t.n * a.H + y) * a.W + x;
-      float v[16];
-      tmem_ld16(lanes + acc * a.NT + cc, v);
-      if (j + step >= total) release();
-      if (!kDg) {
-        if (a.bias) {
-#pragma unroll
-          for (int k = 0; k < 16; k += 4) {
-            const float4 b4 = *reinterpret_cast<const float4*>(bias + c + k);
-            v[k] += b4.x;
-            v[k + 1] += b4.y;
-            v[k + 2] += b4.z;
-            v[k + 3] += b4.w;
-          }
-        }
-        if (a.relu) {
-#pragma unroll
-          for (int k = 0; k < 16; ++k) v[k] = fmaxf(v[k], 0.0f);
-        }
-        if (ok && a.out) {
-          uint32_t u[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) u[k] = pack2(v[2 * k], v[2 * k + 1]);
-          bf16* d = a.out + p * a.Nout + c;
-          st32(d, u, (reinterpret_cast<uintptr_t>(a.out) & 31) == 0);
-        }
-        if (ok && a.out_f32) {
-          float* d = a.out_f32 + p * a.Nout + c;
-          const uintptr_t al = reinterpret_cast<uintptr_t>(a.out_f32);
-          if ((al & 15) == 0) {
-            st32(d, reinterpret_cast<const uint32_t*>(v), (al & 31) == 0);
-            st32(d + 8, reinterpret_cast<const uint32_t*>(v) + 8, (al & 31) == 0);
-          } else {
-#pragma unroll
-            for (int k = 0; k < 16; ++k) d[k] = v[k];
-          }
-        }
-      } else {
-        if (a.mask_relu) {
-          const uint32_t* w = reinterpret_cast<const uint32_t*>(mk[b]);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const float2 s = unpack2(w[k]);
-            if (!(s.x > 0.0f)) v[2 * k] = 0.0f;
-            if (!(s.y > 0.0f)) v[2 * k + 1] = 0.0f;
-          }
-        }
-        uint32_t u[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) u[k] = pack2(v[2 * k], v[2 * k + 1]);
-        if (!a.dlow) {
-          if (ok) {
-            bf16* d = a.din + p * a.Nout + c;
-            st32(d, u, (reinterpret_cast<uintptr_t>(a.din) & 31) == 0);
-          }
-        } else if (c >= a.s1.C) {
-          if (ok) {
-            bf16* d = a.dskip + p * a.s2.C + (c - a.s1.C);
-            st32(d, u, (reinterpret_cast<uintptr_t>(a.dskip) & 31) == 0);
-          }
-        } else {
-          // gradient of nearest upsampling: the 2 x 2 blocks of the warp's
-          // 8 x 4 pixels, summed in FP32 in row order from the BF16 values;
-          // each of a block's four lanes sums four channels
-          xch[lane][0] = make_uint4(u[0], u[1], u[2], u[3]);
-          xch[lane][1] = make_uint4(u[4], u[5], u[6], u[7]);
-          __syncwarp();
-          const int lx = lane & 7, ly = lane >> 3, sub = (ly & 1) * 2 + (lx & 1);
-          const int base = (ly & ~1) * 8 + (lx & ~1);
-          float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const uint2 g = reinterpret_cast<const uint2*>(xch[base + (k >> 1) * 8 + (k & 1)])[sub];
-            const float2 g0 = unpack2(g.x), g1 = unpack2(g.y);
-            s[0] += g0.x;
-            s[1] += g0.y;
-            s[2] += g1.x;
-            s[3] += g1.y;
-          }
-          __syncwarp();
-          if (ok) {
-            const size_t pl = ((size_t)t.n * (a.H >> 1) + (y >> 1)) * (a.W >> 1) + (x >> 1);
-            *reinterpret_cast<uint2*>(a.dlow + pl * a.s1.C + c + 4 * sub) =
-                make_uint2(pack2(s[0], s[1]), pack2(s[2], s[3]));
-          }
-        }
+    } else {
+      if (!ready) {
+        if (!wait()) return false;
+        ready = true;
+      }
+      int c = 0;
+      for (; c + 32 <= nt; c += 32) {
+        float v[32];
+        tmem_ld32(taddr + c, v);
+        if (acc == acc1 - 1 && c + 32 == nt) release();
+        store_fwd(a, v, n0 + c, p, ok, bias);
+        store_fwd(a, v + 16, n0 + c + 16, p, ok, bias);
+      }
+      if (c < nt) {
+        float v[16];
+        tmem_ld16(taddr + c, v);
+        if (acc == acc1 - 1) release();
+        store_fwd(a, v, n0 + c, p, ok, bias);
       }
     }
   }
@@ -376,7 +404,7 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tiles = (int)blockIdx.x < a.n_tiles ? (a.n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   if (warp == 0) tc::tmem_alloc(&tmem_slot, a.ncols);
-  bars_init(bars, a.S, kUp ? kEpiWarps * 32 : kEpiWarps * 16);
+  bars_init(bars, a.S, kUp ? kEpiWarps * 32 : 128);
   if (!kDg && a.bias)
     for (int k = tid; k < a.Nout; k += kThreadsT) bias[k] = a.bias[k];
   tc::fence_before();
@@ -386,28 +414,33 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
   const uint32_t tap_bytes = (uint32_t)a.NT * RB, slab_w = 9 * tap_bytes;
   bool ok = true;
   if (warp == 0) {
-    if (lane == 0) {
-      if (kRes && n_tiles > 0) ok = tc::mbar_wait(&bars.wbar, 0u);
-      int st = 0, buf = 0;
-      uint32_t ph = 0, bph = 1;  // a fresh barrier's preceding phase reads complete
-      TileIter it(a, (int)blockIdx.x, (int)gridDim.x);
-      for (int i = 0; i < n_tiles && ok; ++i, it.next(a)) {
-        const Tile t = it.tile(kTH);
-        ok = tc::mbar_wait(&bars.acce[buf], bph);
-        const uint32_t idesc = tc::make_idesc_bf16(128, min(a.NT, a.Nout - t.nt * a.NT));
-        const uint32_t d = tmem + buf * NA * a.NT;
-        for (int s = 0; s < a.nslab && ok; ++s) {
-          ok = tc::mbar_wait(&bars.full[st], ph);
-          if (!ok) break;
-          tc::fence_after();
-          const uint32_t sa = s0 + st * a.stage;
-          const bool skip = kUp && s >= a.nslab1;
-          const uint32_t sb = kRes ? sw + (uint32_t)(t.nt * a.nslab + s) * slab_w : sa + a.w_off;
-          const uint64_t bd = kdesc<KC>(sb, 8 * RB);
-          const uint32_t tap16 = tap_bytes >> 4;
+    // The whole warp walks the units, so that descriptors and loop state stay
+    // in uniform registers; one elected lane issues a slab's MMAs and commits
+    // (issued from a single-lane loop, every MMA cost ~47 clocks of the
+    // issuing thread and every tile ~600 more: 108 -> 88 us for 32 -> 32
+    // channels at 32 x 256^2).
+    if (kRes && n_tiles > 0) ok = warp_wait(&bars.wbar, 0u);
+    int st = 0, buf = 0;
+    uint32_t ph = 0, bph = 1;  // a fresh barrier's preceding phase reads complete
+    TileIter it(a, (int)blockIdx.x, (int)gridDim.x);
+    const uint32_t tap16 = tap_bytes >> 4;
+    for (int i = 0; i < n_tiles && ok; ++i, it.next(a)) {
+      ok = warp_wait(&bars.acce[buf], bph);
+      const uint32_t idesc = tc::make_idesc_bf16(128, min(a.NT, a.Nout - it.nt * a.NT));
+      const uint32_t d = tmem + buf * NA * a.NT;
+      for (int s = 0; s < a.nslab && ok; ++s) {
+        ok = warp_wait(&bars.full[st], ph);
+        if (!ok) break;
+        tc::fence_after();
+        const uint32_t sa = s0 + st * a.stage;
+        const bool skip = kUp && s >= a.nslab1;
+        const uint32_t sb = kRes ? sw + (uint32_t)(it.nt * a.nslab + s) * slab_w : sa + a.w_off;
+        const uint64_t bd = kdesc<KC>(sb, 8 * RB);
+        const uint64_t ad0 = kdesc<KC>(sa, (skip ? kPW : kHW) * RB);
+        if (elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < KC / 16; ++ks) {
-            const uint64_t ad = kdesc<KC>(sa + 32 * ks, (skip ? kPW : kHW) * RB);
+            const uint64_t ad = ad0 + 2 * ks;
             const bool acc0 = s > 0 || ks > 0;
             if (!skip) {
 #pragma unroll
@@ -442,15 +475,16 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
           }
           tc::mma_commit(&bars.empty[st]);
           if (s == a.nslab - 1) tc::mma_commit(&bars.accf[buf]);
-          if (++st == a.S) {
-            st = 0;
-            ph ^= 1u;
-          }
         }
-        if (++buf == a.nbuf) {
-          buf = 0;
-          bph ^= 1u;
+        __syncwarp();
+        if (++st == a.S) {
+          st = 0;
+          ph ^= 1u;
         }
+      }
+      if (++buf == a.nbuf) {
+        buf = 0;
+        bph ^= 1u;
       }
     }
   } else if (warp == 1) {
@@ -496,27 +530,28 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
       }
     }
   } else {
-    // The two groups of four warps take alternate tiles; a tile of four
-    // accumulators (kUp) they share, in alternate chunks.  (Alternate tiles
-    // need two accumulator buffers: with one, a group would skip every second
-    // phase of its barrier.)
-    const int g = (warp - 2) >> 2;
-    constexpr int kStep = kUp ? 1 : 2;
-    TileIter it(a, (int)(blockIdx.x + (kUp ? 0 : g) * gridDim.x), kStep * (int)gridDim.x);
-    for (int i = kUp ? 0 : g; i < n_tiles && ok; i += kStep, it.next(a)) {
-      const Tile t = it.tile(kTH);
-      const int buf = i % a.nbuf, lap = i / a.nbuf;
-      ok = tile_epilogue<NA, kUp, kDg>(
-          a, t, tmem + buf * NA * a.NT, warp, lane, xch[kDg ? warp - 2 : 0], bias, kUp ? g : 0, kUp ? 2 : 1,
-          [&] {
-            const bool w = __all_sync(0xffffffffu, tc::mbar_wait(&bars.accf[buf], (uint32_t)lap & 1u));
-            tc::fence_after();
-            return w;
-          },
-          [&] {
-            tc::fence_before();
-            tc::mbar_arrive(&bars.acce[buf]);
-          });
+    // Groups of four warps: each takes every groups-th tile, or (kUp) one of
+    // each tile's four accumulators.  A group must not be given a buffer
+    // whose previous phase it cannot know to be complete, so there are no
+    // more groups on alternate tiles than buffers.
+    const int g = (warp - 2) >> 2, groups = kUp ? 1 : min(kEpiWarps / 4, a.nbuf), g0 = kUp ? 0 : g;
+    if (g0 < groups) {
+      TileIter it(a, (int)(blockIdx.x + g0 * gridDim.x), groups * (int)gridDim.x);
+      for (int i = g0; i < n_tiles && ok; i += groups, it.next(a)) {
+        const Tile t = it.tile(kTH);
+        const int buf = i % a.nbuf, lap = i / a.nbuf;
+        ok = tile_epilogue<kUp, kDg>(
+            a, t, tmem + buf * NA * a.NT, kUp ? g : 0, kUp ? g + 1 : MT, warp, lane, xch[kDg ? warp - 2 : 0], bias,
+            [&] {
+              const bool w = warp_wait(&bars.accf[buf], (uint32_t)lap & 1u);
+              tc::fence_after();
+              return w;
+            },
+            [&] {
+              tc::fence_before();
+              tc::mbar_arrive(&bars.acce[buf]);
+            });
+      }
     }
   }
   if (!__syncthreads_and(ok) && lane == 0) atomicOr(a.err, tc::kErrMbarTimeout);
@@ -591,7 +626,7 @@ static uint32_t pow2_cols(uint32_t c) {
   return p;
 }
 
-constexpr uint32_t kSmem = 216 * 1024;  // dynamic shared memory a CTA may plan with
+constexpr uint32_t kSmem = 208 * 1024;  // dynamic shared memory a CTA may plan with
 
 template <int KC, int MT, bool kUp, bool kRes, bool kDg>
 static cudaError_t launch_tile(const TileArgs& a, const TileMaps& m, size_t smem, cudaStream_t st) {
