@@ -29,8 +29,6 @@
 // MMAs that read it have completed.  The gathers of later slices therefore
 // overlap the MMAs of earlier ones, and no thread stalls on its own loads.
 #include <algorithm>
-#include <cuda.h>
-#include <cudaTypedefs.h>
 
 #include "nn.h"
 #include "nn_tile.h"
@@ -202,10 +200,6 @@ __device__ __forceinline__ bool conv_ring(int n, uint64_t* bars, Load&& load, Mm
 // load(unit, stage, lane) copies with item stride kLoadStride.
 constexpr int kProducerWarps = 7;
 constexpr int kLoadStride = 32;
-#ifndef RTX_CONV_TMA
-#define RTX_CONV_TMA 1
-#endif
-constexpr bool kConvTma = RTX_CONV_TMA != 0;  // tensor copies where a source allows them
 
 // pre(pw, lane) issues copies every MMA needs (resident weights, split over
 // the producer warps); the warp waits for them and its 32 lanes arrive on
@@ -233,86 +227,6 @@ __device__ __forceinline__ bool produce(int n, uint64_t* full, uint64_t* empty, 
     tc::mbar_arrive(&full[pw]);
   }
   return true;
-}
-
-// One accumulation over n slices (the weight gradient).  Returns true,
-// uniformly, once every MMA has completed; false (error flag set) when a
-// bounded wait ran out.
-template <int S, class Load, class Mma>
-__device__ __forceinline__ bool ws_ring(int n, uint64_t* full, uint64_t* empty, Load&& load, Mma&& mma, int* err) {
-  const int tid = threadIdx.x;
-  bool ok = true;
-  if (tid < 32) {
-    if (tid == 0) {
-      for (int it = 0; it < n; ++it) {
-        const int st = it % S;
-        if (!tc::mbar_wait(&full[st], (uint32_t)(it / S) & 1u)) {
-          ok = false;
-          break;
-        }
-        tc::fence_after();
-        mma(it, st);
-        tc::mma_commit(&empty[st]);
-      }
-    }
-  } else {
-    ok = produce<S>(n, full, empty, nullptr, [](int, int) {}, load);
-  }
-  // the last commit covers every MMA (waited after a plain barrier, so the
-  // producers do not spin while the MMAs drain)
-  bool fin = __syncthreads_and(ok);
-  if (fin && n > 0) fin = tc::mbar_wait(&empty[(n - 1) % S], (uint32_t)((n - 1) / S) & 1u);
-  fin = __syncthreads_and(fin);
-  if (!fin && (tid & 31) == 0) atomicOr(err, tc::kErrMbarTimeout);
-  tc::fence_after();
-  return fin;
-}
-
-// The same accumulation fed by tensor copies (TMA): thread 32 issues unit
-// it's copies into stage it % S once the MMAs of unit it - S have released
-// it (one arrival carrying the unit's byte count, `tx`), thread 0 issues the
-// MMAs.  On a timed-out wait the issuing thread waits (bounded) for the
-// copies it issued last on each stage before the CTA leaves, so that none
-// lands in released shared memory.
-template <int S, class Issue, class Mma>
-__device__ __forceinline__ bool tma_ring(int n, uint64_t* full, uint64_t* empty, uint32_t tx, Issue&& issue,
-                                         Mma&& mma, int* err) {
-  const int tid = threadIdx.x;
-  bool ok = true;
-  int issued = 0;
-  if (tid == 0) {
-    for (int it = 0; it < n; ++it) {
-      const int st = it % S;
-      if (!tc::mbar_wait(&full[st], (uint32_t)(it / S) & 1u)) {
-        ok = false;
-        break;
-      }
-      tc::fence_after();
-      mma(it, st);
-      tc::mma_commit(&empty[st]);
-    }
-  } else if (tid == 32) {
-    for (int it = 0; it < n; ++it) {
-      const int st = it % S;
-      if (it >= S && !tc::mbar_wait(&empty[st], (uint32_t)(it / S - 1) & 1u)) {
-        ok = false;
-        break;
-      }
-      tc::mbar_arrive_expect_tx(&full[st], tx);
-      issue(it, st, &full[st]);
-      issued = it + 1;
-    }
-  }
-  bool fin = __syncthreads_and(ok);
-  if (fin && n > 0) fin = tc::mbar_wait(&empty[(n - 1) % S], (uint32_t)((n - 1) / S) & 1u);
-  fin = __syncthreads_and(fin);
-  if (!fin) {
-    if (tid == 32)
-      for (int it = max(0, issued - S); it < issued; ++it) tc::mbar_wait(&full[it % S], (uint32_t)(it / S) & 1u);
-    if ((tid & 31) == 0) atomicOr(err, tc::kErrMbarTimeout);
-  }
-  tc::fence_after();
-  return fin;
 }
 
 // Persistent tiles (kTileThreads = 12 warps): thread 0 issues MMAs, warps
@@ -753,201 +667,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_wgrad(ConvWgrad a) {
 }
 
 // ---------------------------------------------------------------------------
-// weight gradient, row tiles: a CTA owns source channels [c0, c0 + CR)
-// (CR <= 48) for all nine taps and sums over a run of row tiles (TW pixels
-// of one image row, TW = 64 or 128).  GEMM M = output channels (the 128
-// accumulator lanes; lanes >= Cout are never read), N = CR per tap, K = the
-// tile's pixels, both operands MN-major:
-//   A = the dout tile, chunk g of pixel k at (g * TW + k) * 16
-//   B = the 3-row source halo, chunk ch of pixel h of row r at
-//       ((r * CR / 8 + ch) * (TW + 2) + h) * 16
-// Tap t = (dy, dx) reads halo row dy + 1 shifted by dx pixels (any 16-byte
-// shift of an MN-major operand whose K neighbours are 16 B apart is a legal
-// start address) into accumulator columns [t * CR, t * CR + CR).  Per tile a
-// CTA copies the dout tile and the halo once, so the source is read about
-// three times and dout Cin / CR times, against nine and 9 Cin / 128 times in
-// k_conv_wgrad.  The accumulator lives in TMEM across all of the CTA's tiles;
-// one set of FP32 atomics per CTA combines the runs.
-//
-// kSwap (narrow outputs, Cout <= 56, and Cin >= 64): the operands trade
-// places.  M = the CTA's source channels (up to 128 accumulator lanes; the
-// MMA reads 128 rows of the halo, and rows past CR land in lanes that are
-// never read), N = Cout, A = the halo read at each tap's shift, B = the dout
-// tile; tap t accumulates in columns [t * Cout, t * Cout + Cout), 9 Cout <=
-// 512.  With M = Cout = 32 three quarters of every MMA would be padding; with
-// M = 96 source channels one quarter is, and one CTA covers all channels, so
-// dout is read once per tile.
-//
-// kTma (single, full-resolution source; Cin a multiple of the CTA's
-// channels): each unit's halo and dout tile arrive as two tensor copies
-// into the same layouts.  The source map is NHWC viewed as 5-D (8 channels,
-// x, channel chunk, y, image), so a box of (8, TW + 2, CR / 8, 3, 1) lands
-// row, chunk, pixel major -- the layout above -- with zeros outside the
-// image; dout's map is the same view of [rows][W][Cout] with a box of
-// (8, TW, Cout / 8, 1, 1).  Stages are 1 KB aligned for the copies.
-// ---------------------------------------------------------------------------
-template <int S, bool kSwap, bool kTma>
-__global__ void __launch_bounds__(kThreads, 1)
-    k_conv_wgrad_row(ConvWgrad a, const __grid_constant__ CUtensorMap tm_src,
-                     const __grid_constant__ CUtensorMap tm_dout) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ __align__(8) uint64_t full[S], empty[S];
-  __shared__ uint32_t tmem_slot;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int TW = a.tw, TW2 = a.tw + 2;
-  const int c0 = blockIdx.x * a.cr;
-  const int CR = min(a.cr, a.Cin - c0);  // this CTA's channels (multiple of 16)
-  const int nch = CR >> 3, nco = a.Cout >> 3;
-  const int TR = (a.W + TW - 1) / TW;  // tiles per image row
-  const int T = a.N * a.H * TR;
-  const int tb = blockIdx.y * a.tiles_per_cta;
-  const int n_tiles = max(0, min(a.tiles_per_cta, T - tb));
-  const uint32_t ncols = (!kSwap && 9 * a.cr <= 256) ? 256 : 512;
-  const uint32_t dout_bytes = (uint32_t)a.Cout * TW * 2;
-  const uint32_t tx = dout_bytes + 3u * (a.cr >> 3) * TW2 * 16;  // one unit's bytes
-  const uint32_t stage = kTma ? (tx + 1023u) & ~1023u : tx;
-  if (warp == 0) tc::tmem_alloc(&tmem_slot, ncols);
-  if (tid == 0) {
-    for (int i = 0; i < S; ++i) {
-      tc::mbar_init(&full[i], kTma ? 1 : kLoadStride);
-      tc::mbar_init(&empty[i], 1);
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  tc::fence_before();
-  __syncthreads();
-  tc::fence_after();
-  const uint32_t tmem = tmem_slot;
-  const uint32_t idesc = tc::make_idesc_bf16(128, kSwap ? a.Cout : CR, true, true);
-  const uint32_t s0 = tc::smem_u32(smem);
-  // a producer's starting item and the per-iteration step of the two copy
-  // loops (items: dout = (pixel k, chunk g), g fastest; halo = (row r, pixel
-  // h, chunk ch), ch fastest, so neighbouring threads read contiguous bytes)
-  const int pt = lane;
-  const int d_g0 = pt % nco, d_k0 = pt / nco, d_dg = kLoadStride % nco, d_dk = kLoadStride / nco;
-  const int h_c0 = pt % nch, h_p0 = pt / nch, h_dc = kLoadStride % nch, h_dp = kLoadStride / nch;
-  auto load = [&](int slice, int st, int ptid) {
-    const uint32_t sd = s0 + st * stage, sh = sd + dout_bytes;
-    const int j = tb + slice;
-    const int row = j / TR, x0 = (j - row * TR) * TW;  // row = n * H + y
-    const int n = row / a.H, y = row - n * a.H;
-    const bf16* drow = a.dout + (size_t)row * a.W * a.Cout;
-    for (int i = ptid, g = d_g0, k = d_k0; i < TW * nco; i += kLoadStride) {
-      const bf16* p = x0 + k < a.W ? drow + (size_t)(x0 + k) * a.Cout + g * 8 : nullptr;
-      chunk_async(sd + (g * TW + k) * 16, p, a.dout);
-      g += d_dg;
-      k += d_dk;
-      if (g >= nco) {
-        g -= nco;
-        ++k;
-      }
-    }
-    int r = 0, h = h_p0;
-    while (h >= TW2) {
-      h -= TW2;
-      ++r;
-    }
-    for (int i = ptid, ch = h_c0; i < 3 * TW2 * nch; i += kLoadStride) {
-      const bf16* p = src_ptr(a.s1, a.s2, a.H, a.W, n, y + r - 1, x0 + h - 1, c0 + 8 * ch);
-      chunk_async(sh + ((r * nch + ch) * TW2 + h) * 16, p, a.s1.ptr);
-      ch += h_dc;
-      h += h_dp;
-      if (ch >= nch) {
-        ch -= nch;
-        ++h;
-      }
-      while (h >= TW2) {
-        h -= TW2;
-        ++r;
-      }
-    }
-  };
-  auto mma = [&](int it, int st) {
-    const bool first = it == 0;
-    const uint32_t sd = s0 + st * stage, sh = sd + dout_bytes;
-    // descriptors built once; a K step (16 pixels) is +256 B = +16 in the
-    // address field, tap t's B starts (dy + 1) halo rows and 1 + dx pixels in
-    const uint64_t ad0 = tc::make_desc(sd, 128, TW * 16), bh = tc::make_desc(sh, 128, TW2 * 16);
-    const int nks = TW / 16;
-#pragma unroll 1
-    for (int t = 0; t < 9; ++t) {
-      const int dy = t / 3 - 1, dx = t % 3 - 1;
-      const uint64_t hd = bh + ((dy + 1) * nch * TW2 + 1 + dx);
-      if (kSwap) {  // A = the shifted halo (M = channels), B = the dout tile
-        const uint32_t d = tmem + t * a.Cout;
-        tc::mma_bf16(d, hd, ad0, idesc, !first);
-#pragma unroll 8
-        for (int ks = 1; ks < nks; ++ks) tc::mma_bf16(d, hd + 16 * ks, ad0 + 16 * ks, idesc, true);
-      } else {
-        const uint32_t d = tmem + t * CR;
-        tc::mma_bf16(d, ad0, hd, idesc, !first);
-#pragma unroll 8
-        for (int ks = 1; ks < nks; ++ks) tc::mma_bf16(d, ad0 + 16 * ks, hd + 16 * ks, idesc, true);
-      }
-    }
-  };
-  // the tensor-copy form: unit `slice` of this CTA (its row tile) as two boxes
-  auto issue = [&](int slice, int st, uint64_t* bar) {
-    const uint32_t sd = s0 + st * stage, sh = sd + dout_bytes;
-    const int j = tb + slice;
-    const int row = j / TR, x0 = (j - row * TR) * TW;  // row = n * H + y
-    const int n = row / a.H, y = row - n * a.H;
-    tc::tma_load_5d(sh, &tm_src, 0, x0 - 1, c0 >> 3, y - 1, n, bar);
-    tc::tma_load_5d(sd, &tm_dout, 0, x0, 0, row, 0, bar);
-  };
-  bool ok;
-  if constexpr (kTma)
-    ok = tma_ring<S>(n_tiles, full, empty, tx, issue, mma, a.err);
-  else
-    ok = ws_ring<S>(n_tiles, full, empty, load, mma, a.err);
-  const int lw = warp & 3;
-  if (kSwap) {
-    // warp w reads lanes 32 (w % 4) .. + 31 (source channel c0 + ch), half
-    // w / 4 of the 9 Cout / 8 column chunks (tap t, output channels o0 ..)
-    const int ch = lw * 32 + lane;
-    const uint32_t taddr = tmem + ((uint32_t)(lw * 32) << 16);
-    const int nq = 9 * nco, q0 = (warp >> 2) * (nq >> 1), q1 = (warp >> 2) ? nq : (nq >> 1);
-    if (ok && n_tiles > 0 && lw * 32 < CR) {
-      for (int q = q0; q < q1; ++q) {
-        float v[8];
-        tc::tmem_ld8(taddr + q * 8, v);  // warp-wide: every lane loads, valid lanes add
-        if (ch < CR) {
-          const int t = q / nco, o0 = (q - t * nco) * 8;
-#pragma unroll
-          for (int k = 0; k < 8; ++k) atomicAdd(a.dw + ((size_t)(o0 + k) * 9 + t) * a.Cin + c0 + ch, v[k]);
-        }
-      }
-    }
-    tc_end(tmem, ncols);
-    return;
-  }
-  if (ok && n_tiles > 0 && lw * 32 < a.Cout) {
-    // warp w reads lanes 32 (w % 4) .. + 31 (output channel o), half w / 4 of
-    // the 9 CR / 8 column chunks
-    const int o = lw * 32 + lane;
-    const uint32_t taddr = tmem + ((uint32_t)(lw * 32) << 16);
-    const int nq = 9 * nch, q0 = (warp >> 2) * (nq >> 1), q1 = (warp >> 2) ? nq : (nq >> 1);
-    const bool vec = ((reinterpret_cast<uintptr_t>(a.dw) & 15) == 0);
-    for (int q = q0; q < q1; ++q) {
-      float v[8];
-      tc::tmem_ld8(taddr + q * 8, v);
-      if (o < a.Cout) {
-        const int t = q / nch, cl = (q - t * nch) * 8;
-        float* d = a.dw + ((size_t)o * 9 + t) * a.Cin + c0 + cl;
-        if (vec) {
-          atomicAdd(reinterpret_cast<float4*>(d), make_float4(v[0], v[1], v[2], v[3]));
-          atomicAdd(reinterpret_cast<float4*>(d + 4), make_float4(v[4], v[5], v[6], v[7]));
-        } else {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) atomicAdd(d + i, v[i]);
-        }
-      }
-    }
-  }
-  tc_end(tmem, ncols);
-}
-
-// ---------------------------------------------------------------------------
 // Stages of the ring for a B tile of nb rows: 3 stages up to 128 rows, 2
 // beyond (72 KB per CTA for nb <= 64, at most 96 KB otherwise).
 static int stages_for(int nb) { return nb <= 128 ? 3 : 2; }
@@ -1032,40 +751,6 @@ static cudaError_t launch_tiles(KR kr, K6 k6, K4 k4, K2 k2, bool res, size_t sta
   return cudaGetLastError();
 }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point (null if
-// the driver does not provide it)
-static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) !=
-            cudaSuccess ||
-        q != cudaDriverEntryPointSuccess)
-      p = nullptr;
-    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-  }();
-  return fn;
-}
-
-// Tensor map of an [imgs][H][W][C] BF16 tensor (C a multiple of 8) viewed as
-// 5-D (8 channels, x, channel chunk, y, image), with a box of (8, box_w,
-// box_chunks, box_rows, 1): the box lands in shared memory row, chunk,
-// pixel major, 16 bytes per (pixel, chunk).  False if it cannot be encoded.
-static bool chunk_major_map(CUtensorMap* m, const void* base, int imgs, int H, int W, int C, int box_w,
-                            int box_chunks, int box_rows) {
-  const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-  if (!enc || (reinterpret_cast<uintptr_t>(base) & 15) || C % 8 || box_w > 256 || box_chunks > 256 ||
-      box_rows > 256)
-    return false;
-  const cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)(C / 8), (cuuint64_t)H, (cuuint64_t)imgs};
-  const cuuint64_t strides[4] = {(cuuint64_t)C * 2, 16, (cuuint64_t)W * C * 2, (cuuint64_t)H * W * C * 2};
-  const cuuint32_t box[5] = {8, (cuuint32_t)box_w, (cuuint32_t)box_chunks, (cuuint32_t)box_rows, 1};
-  const cuuint32_t es[5] = {1, 1, 1, 1, 1};
-  return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(base), dims, strides, box, es,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // weights kept in shared memory by the persistent kernels up to this size
 // (128 KB: with 1 KB-aligned tensor-copy halo stages, 7 x 13 KB + 128 KB
 // fits the 227 KB of a CTA; measured 0.75 % faster per training step than 96)
@@ -1117,109 +802,11 @@ int wgrad_pixels_per_cta(long long P, int Cout, int Cin) {
   return (int)std::max(64LL, std::min(per, 1LL << 30));
 }
 
-// Channels per CTA of the row-tile weight gradient (16, 32 or 48; the last
-// range may be narrower): fewest ranges, weighing each range's fixed dout
-// copy against its width.
-static int wgrad_row_channels(int Cin, int Cout) {
-  int best = 16;
-  long long best_cost = -1;
-  for (int cr : {48, 32, 16}) {
-    if (cr > Cin) continue;
-    long long cost = (long long)((Cin + cr - 1) / cr) * (cr + Cout / 4 + 8);
-    if (best_cost < 0 || cost < best_cost) best = cr, best_cost = cost;
-  }
-  return best;
-}
-
-// The row-tile weight gradient with S ring stages (2..7): each stage has its
-// own producer warp, so a deeper ring is also more warps copying at once
-// (tensor-copy form: one issuing thread for all stages).
-template <bool kSwap, bool kTma>
-static cudaError_t launch_wgrad_row(int S, dim3 grid, size_t smem, const ConvWgrad& a, const CUtensorMap& ms,
-                                    const CUtensorMap& md, cudaStream_t st) {
-  auto go = [&](auto kern) -> cudaError_t {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e) return e;
-    kern<<<grid, kThreads, smem, st>>>(a, ms, md);
-    return cudaGetLastError();
-  };
-  switch (S) {
-    case 7: return go(k_conv_wgrad_row<7, kSwap, kTma>);
-    case 6: return go(k_conv_wgrad_row<6, kSwap, kTma>);
-    case 5: return go(k_conv_wgrad_row<5, kSwap, kTma>);
-    case 4: return go(k_conv_wgrad_row<4, kSwap, kTma>);
-    case 3: return go(k_conv_wgrad_row<3, kSwap, kTma>);
-    default: return go(k_conv_wgrad_row<2, kSwap, kTma>);
-  }
-}
-
-cudaError_t conv_wgrad(const ConvWgrad& a0, cudaStream_t st) {
-  long long P = (long long)a0.N * a0.H * a0.W;
-  if (P >= (1LL << 31) || a0.Cout % 16 || a0.Cout > 256) return cudaErrorInvalidValue;
-  constexpr size_t kRing = 190 * 1024;  // shared memory for the ring
-  auto stages = [&](size_t stage) { return (int)std::min<size_t>(kProducerWarps, kRing / stage); };
-  if (use_rows(a0.W, a0.Cin) && 9 * a0.Cout <= 512 && a0.Cin >= 64) {
-    // narrow outputs: source channels on the accumulator lanes (kSwap)
-    ConvWgrad a = a0;
-    const int nr = (a.Cin + 127) / 128;
-    a.cr = (a.Cin + nr - 1) / nr;
-    a.cr = (a.cr + 15) / 16 * 16;
-    const int nch = a.cr / 8;
-    auto stage_of = [&](int tw) { return (size_t)a.Cout * tw * 2 + (size_t)3 * nch * (tw + 2) * 16; };
-    // the tile width whose ring is deepest (ties: the wider tile)
-    a.tw = stages(stage_of(32)) > stages(stage_of(64)) ? 32 : 64;
-    const size_t stage = stage_of(a.tw);
-    const int S = std::max(2, stages(stage));
-    const long long T = (long long)a.N * a.H * ((a.W + a.tw - 1) / a.tw);
-    const int TW2 = a.tw + 2;
-    // the MMA's A operand spans 128 channel rows of a halo row: at the last
-    // stage's last halo row that reaches past the halo by this much
-    const size_t a_over = ((size_t)(16 - std::min(nch, 16)) * TW2 + a.tw + 2) * 16;
-    const long long ctas = (long long)sm_count();  // 512 TMEM columns: one CTA per SM
-    const long long npg = std::max(1LL, ctas / nr);
-    a.tiles_per_cta = (int)((T + npg - 1) / npg);
-    const unsigned gy = (unsigned)((T + a.tiles_per_cta - 1) / a.tiles_per_cta);
-    const CUtensorMap none{};
-    return launch_wgrad_row<true, false>(S, dim3(nr, gy), S * stage + a_over, a, none, none, st);
-  }
-  if (use_rows(a0.W, a0.Cin) && a0.Cout <= 128) {
-    ConvWgrad a = a0;
-    a.cr = wgrad_row_channels(a.Cin, a.Cout);
-    const int nr = (a.Cin + a.cr - 1) / a.cr;
-    a.tw = a.W >= 128 ? 128 : 64;
-    // a single full-resolution source whose channels split evenly over the
-    // CTAs: the tensor-copy form, if both maps encode
-    CUtensorMap ms{}, md{};
-    const bool tma = kConvTma && !a.s2.ptr && !a.s1.up && a.Cin % a.cr == 0 &&
-                     chunk_major_map(&ms, a.s1.ptr, a.N, a.H, a.W, a.Cin, a.tw + 2, a.cr / 8, 3) &&
-                     chunk_major_map(&md, a.dout, 1, a.N * a.H, a.W, a.Cout, a.tw, a.Cout / 8, 1);
-    const size_t tx = (size_t)a.Cout * a.tw * 2 + (size_t)3 * (a.cr / 8) * (a.tw + 2) * 16;
-    const size_t stage = tma ? (tx + 1023) / 1024 * 1024 : tx;
-    // the MMA's A operand spans 128 rows of TW pixels; rows past Cout are
-    // read (and their accumulator lanes ignored), so they must lie inside the
-    // allocation
-    const size_t a_span = (size_t)256 * a.tw;
-    size_t extra = a_span > stage ? a_span - stage : 0;
-    // at most 4 stages with producer warps: deeper rings (narrower tiles, or
-    // more stages of the same tile) measured 0-10 % slower on these layers.
-    // Tensor copies: as deep as fits, but not so deep that it costs the
-    // second CTA per SM that a 256-column accumulator allows.
-    int S = std::max(2, tma ? stages(stage) : std::min(4, stages(stage)));
-    if (tma && 9 * a.cr <= 256 && 2 * stage + extra <= 110 * 1024)
-      S = std::min(S, (int)((110 * 1024 - extra) / stage));
-    const int per_sm = (9 * a.cr <= 256 && S * stage + extra <= 110 * 1024) ? 2 : 1;
-    // one CTA per SM when it takes all 512 TMEM columns: a second CTA on the
-    // SM would wait in its allocation for the first to finish
-    if (per_sm == 1 && S * stage + extra < 116 * 1024) extra = 116 * 1024 - S * stage;
-    const long long T = (long long)a.N * a.H * ((a.W + a.tw - 1) / a.tw);
-    const long long ctas = (long long)sm_count() * per_sm;
-    const long long npg = std::max(1LL, ctas / nr);
-    a.tiles_per_cta = (int)((T + npg - 1) / npg);
-    const unsigned gy = (unsigned)((T + a.tiles_per_cta - 1) / a.tiles_per_cta);
-    if (tma) return launch_wgrad_row<false, true>(S, dim3(nr, gy), S * stage + extra, a, ms, md, st);
-    return launch_wgrad_row<false, false>(S, dim3(nr, gy), S * stage + extra, a, ms, md, st);
-  }
-  const ConvWgrad& a = a0;
+cudaError_t conv_wgrad(const ConvWgrad& a, cudaStream_t st) {
+  long long P = (long long)a.N * a.H * a.W;
+  if (P >= (1LL << 31) || a.Cout % 16 || a.Cout > 256) return cudaErrorInvalidValue;
+  cudaError_t e = cudaSuccess;
+  if (conv_tile_wgrad(a, st, &e)) return e;
   size_t stage = 128 * kSlice * 2 + (size_t)a.Cout * kSlice * 2;
   dim3 grid((9 * a.Cin + 127) / 128, (unsigned)((P + a.pix_per_cta - 1) / a.pix_per_cta));
   return launch_staged(k_conv_wgrad<4>, k_conv_wgrad<3>, k_conv_wgrad<2>, stages_for(a.Cout), grid, stage, a, st);

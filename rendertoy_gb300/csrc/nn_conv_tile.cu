@@ -46,8 +46,8 @@
 #include <cudaTypedefs.h>
 
 #include "nn.h"
+#include "nn_tile.cuh"
 #include "nn_tile.h"
-#include "tc_core.cuh"
 
 namespace rtx {
 namespace nn {
@@ -58,7 +58,6 @@ constexpr int kEpiWarps = 16, kThreadsT = 64 + 32 * kEpiWarps;
 constexpr int kMaxS = 8, kMaxBuf = 4;
 constexpr int kHW = 10, kPW = 9;  // halo width: full- and low-resolution tiles, parity planes
 
-__host__ __device__ constexpr uint32_t up1k(uint32_t b) { return (b + 1023u) & ~1023u; }
 // bytes of a unit's A region
 __host__ __device__ constexpr uint32_t halo_bytes(int KC, int MT) { return (uint32_t)kHW * (16 * MT + 2) * KC * 2; }
 __host__ __device__ constexpr uint32_t plane_bytes(int KC) { return (uint32_t)kPW * 17 * KC * 2; }
@@ -96,62 +95,6 @@ struct TileMaps {
 struct Bars {
   uint64_t full[kMaxS], empty[kMaxS], accf[kMaxBuf], acce[kMaxBuf], wbar, hfull[2], hempty[2];
 };
-
-__device__ __forceinline__ void tma4(uint32_t dst, const void* m, int c0, int c1, int c2, int c3, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(dst),
-      "l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(tc::smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ void tma3(uint32_t dst, const void* m, int c0, int c1, int c2, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-      "l"(m), "r"(c0), "r"(c1), "r"(c2), "r"(tc::smem_u32(bar))
-      : "memory");
-}
-
-// One lane of a converged warp
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
-  return p != 0;
-}
-// The whole warp waits; the result is the same on every lane
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) {
-  return __all_sync(0xffffffffu, tc::mbar_wait(bar, parity));
-}
-
-// 16 FP32 columns of this thread's accumulator lane
-__device__ __forceinline__ void tmem_ld16(uint32_t t, float* v) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(t)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t t, float* v) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
-      "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(t)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
@@ -581,14 +524,13 @@ static CUtensorMapSwizzle swizzle_of(int KC) {
   return KC == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : (KC == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
 }
 
-bool pixel_map(CUtensorMap* m, const bf16* base, int imgs, int H, int W, int C, int step, int KC, int bw, int bh) {
+bool pixel_map(CUtensorMap* m, const bf16* base, int imgs, int H, int W, int C, int step_x, int step_y, int KC, int bw,
+               int bh) {
   const PFN_cuTensorMapEncodeTiled_v12000 enc = encoder();
   if (!enc || (reinterpret_cast<uintptr_t>(base) & 15) || C % 8 || H <= 0 || W <= 0) return false;
-  // `step` 2: every second pixel of every second row (a parity plane of the
-  // image that starts at `base`, H x W counted in plane pixels)
   const cuuint64_t dims[4] = {(cuuint64_t)C, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)imgs};
-  const cuuint64_t row = (cuuint64_t)W * step * C * 2;
-  const cuuint64_t strides[3] = {(cuuint64_t)step * C * 2, (cuuint64_t)step * row, (cuuint64_t)H * step * row};
+  const cuuint64_t row = (cuuint64_t)W * step_x * C * 2;
+  const cuuint64_t strides[3] = {(cuuint64_t)step_x * C * 2, (cuuint64_t)step_y * row, (cuuint64_t)H * step_y * row};
   const cuuint32_t box[4] = {(cuuint32_t)KC, (cuuint32_t)bw, (cuuint32_t)bh, 1};
   const cuuint32_t es[4] = {1, 1, 1, 1};
   return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(base), dims, strides, box, es,
@@ -687,15 +629,15 @@ static bool plan_wide(TileArgs a, const Src& x1, const Src& x2, const bf16* w, i
   a.n_tiles = (int)T;
   if (!tap_map(&m.w, w, a.Nout, K, KC, a.NT, 9)) return false;
   if (up) {
-    if (!pixel_map(&m.s1, x1.ptr, imgs, a.H / 2, a.W / 2, x1.C, 1, KC, kHW, 18)) return false;
+    if (!pixel_map(&m.s1, x1.ptr, imgs, a.H / 2, a.W / 2, x1.C, 1, 1, KC, kHW, 18)) return false;
     if (x2.ptr)
       for (int pl = 0; pl < 4; ++pl)
         if (!pixel_map(&m.s2[pl], x2.ptr + ((size_t)(pl >> 1) * a.W + (pl & 1)) * x2.C, imgs, a.H / 2, a.W / 2, x2.C, 2,
-                       KC, kPW, 17))
+                       2, KC, kPW, 17))
           return false;
   } else {
-    if (!pixel_map(&m.s1, x1.ptr, imgs, a.H, a.W, x1.C, 1, KC, kHW, 16 * MT + 2)) return false;
-    if (x2.ptr && !pixel_map(&m.s2[0], x2.ptr, imgs, a.H, a.W, x2.C, 1, KC, kHW, 16 * MT + 2)) return false;
+    if (!pixel_map(&m.s1, x1.ptr, imgs, a.H, a.W, x1.C, 1, 1, KC, kHW, 16 * MT + 2)) return false;
+    if (x2.ptr && !pixel_map(&m.s2[0], x2.ptr, imgs, a.H, a.W, x2.C, 1, 1, KC, kHW, 16 * MT + 2)) return false;
   }
   // past half the SM's shared memory: one CTA per SM (TMEM columns)
   const size_t smem = std::max<size_t>((size_t)a.S * a.stage + (res ? res_bytes : 0), 116 * 1024);

@@ -13,11 +13,14 @@ namespace nn {
 bool conv_tile_fwd(const ConvFwd& a, cudaStream_t st, cudaError_t* e);
 bool conv_tile_dgrad(const ConvDgrad& a, cudaStream_t st, cudaError_t* e);
 
-// Tensor map of an [imgs][H * step][W * step][C] BF16 tensor as (C, x, y,
-// image) over every step-th pixel and row, swizzled boxes of KC channels x bw
-// x bh pixels (KC * 2 bytes per pixel row; zeros outside the image).  False
-// if it cannot be encoded.
-bool pixel_map(CUtensorMap* m, const bf16* base, int imgs, int H, int W, int C, int step, int KC, int bw, int bh);
+bool conv_tile_wgrad(const ConvWgrad& a, cudaStream_t st, cudaError_t* e);
+
+// Tensor map of a BF16 NHWC tensor's every step_x-th pixel of every step_y-th
+// row as (C, x, y, image), H x W counted in those pixels: swizzled boxes of KC
+// channels (KC * 2 bytes per pixel row) x bw x bh pixels, zeros outside.
+// False if it cannot be encoded.
+bool pixel_map(CUtensorMap* m, const bf16* base, int imgs, int H, int W, int C, int step_x, int step_y, int KC, int bw,
+               int bh);
 int tile_sm_count();
 
 }  // namespace nn

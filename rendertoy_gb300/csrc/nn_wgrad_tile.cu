@@ -1,0 +1,392 @@
+// nn_wgrad_tile.cu — 3 x 3 weight gradients on the tcgen05 tensor cores from
+// swizzled tensor copies (TMA):
+//   dw[o, t, c] += sum over pixels p of dout[p, o] src[p + off(t), c]
+//
+// A GEMM over the pixels of 8 x TR-pixel tiles, both operands MN-major (a
+// shared-memory row is one pixel's KO outputs or CB source channels).  All
+// nine taps of a KO x CB block come from one MMA per 16 pixels: the operands'
+// "atoms" (groups of KO or CB elements along M or N) may overlap in shared
+// memory, so
+//   M = 4 atoms of KO outputs, atom i = the dout tile one pixel row further
+//       down (rows y - 1 + i): with the source row fixed that is tap dy = 1 - i
+//       (i = 3 is padding),
+//   N = 3 atoms of CB channels, atom d = the source tile one pixel further
+//       right (columns x - 1 + d): tap dx = d - 1.
+// dout carries a halo of one row above and below, the source of one column
+// left and right; both read zeros outside the image, so every (pixel, tap)
+// pair inside it is counted once.  Against M = the output channels and one
+// MMA per tap (the row kernels this replaces) a 32 x 32 block costs 56 clocks
+// per 16 pixels instead of 9 x 40, and every byte is copied about once.
+//
+// A source at half resolution (read upsampled) is expanded into the same
+// layout by the eight warps that later run the epilogue: 16-byte cp.async
+// copies, one unit ahead.
+//
+// A CTA owns one or more groups of CB channels for its outputs, keeps their
+// accumulators in TMEM over a run of tiles and adds them to dw with FP32
+// atomics at the run's end.  FP32 accumulation in the tensor core truncates: a
+// run of n MMAs loses about n 2^-26 of a sum that grows steadily (measured
+// 1.3e-5 after 864 of them), so a CTA's range is cut into runs no longer than
+// the earlier kernels' (run_pixels), alternating between two sets of
+// accumulators where TMEM holds them.
+#include <algorithm>
+#include <cmath>
+#include <cuda.h>
+
+#include "nn.h"
+#include "nn_tile.cuh"
+#include "nn_tile.h"
+
+namespace rtx {
+namespace nn {
+
+namespace {
+
+constexpr int kThreadsW = 320, kMaxSW = 8;
+
+struct WgradArgs {
+  int KO, CB, ao, G;        // block sizes; o-blocks and channel groups of a CTA
+  int Cout, Cin;            // outputs; dw's channel stride
+  int C1, C2, ng1, ng;      // the sources' channels; channel groups of the first, of both
+  int up1;                  // the first source is expanded from half resolution
+  const bf16* x1;
+  int H, W;
+  int ngc;                  // CTA columns: sets of G channel groups (x o-block sets)
+  int TR, tx, ty;           // tile rows, tiles per image row / column
+  int tiles, per;           // all tiles, tiles per CTA
+  int run, sets;            // tiles per run, accumulator sets that runs alternate between
+  int S;
+  uint32_t stage, dbytes, sbytes, src_off;  // ring stage; bytes of one dout / source box (1 KB steps); source offset
+  uint32_t ncols;
+  float* dw;
+  int* err;
+};
+struct WgradMaps {
+  CUtensorMap dout, src[2];
+};
+
+__device__ __forceinline__ uint64_t mn_desc(uint32_t addr, uint32_t atom, uint32_t group, int K) {
+  const uint64_t layout = K == 32 ? 4 : 6;  // 64- / 32-byte swizzle
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((atom >> 4) & 0x3FFFu) << 16) |
+         ((uint64_t)((group >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (layout << 61);
+}
+
+// dw[o, t, c .. c + 7] += v
+__device__ __forceinline__ void add8(const WgradArgs& a, int o, int t, int c, const float* v) {
+  float* d = a.dw + ((size_t)o * 9 + t) * a.Cin + c;
+  if ((reinterpret_cast<uintptr_t>(d) & 15) == 0) {
+    atomicAdd(reinterpret_cast<float4*>(d), make_float4(v[0], v[1], v[2], v[3]));
+    atomicAdd(reinterpret_cast<float4*>(d + 4), make_float4(v[4], v[5], v[6], v[7]));
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) atomicAdd(d + k, v[k]);
+  }
+}
+
+// Walks a CTA's tiles in order
+struct Walk {
+  int x, y, img;
+  __device__ __forceinline__ Walk(const WgradArgs& a, int t) {
+    x = t % a.tx;
+    t /= a.tx;
+    y = t % a.ty;
+    img = t / a.ty;
+  }
+  __device__ __forceinline__ void next(const WgradArgs& a) {
+    if (++x == a.tx) {
+      x = 0;
+      if (++y == a.ty) {
+        y = 0;
+        ++img;
+      }
+    }
+  }
+};
+
+constexpr int kExpanders = 8;  // warps
+
+__global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, const __grid_constant__ WgradMaps tm) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ __align__(8) uint64_t full[kMaxSW], empty[kMaxSW], done[2], drained[2];
+  __shared__ uint32_t tmem_slot;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int gc = (int)blockIdx.x % a.ngc, go = (int)blockIdx.x / a.ngc;
+  const int g0 = gc * a.G, gn = min(a.G, a.ng - g0);               // channel groups g0 .. g0 + gn - 1
+  const int nup = a.up1 ? max(0, min(gn, a.ng1 - g0)) : 0;         // of which expanded (the first ones)
+  const int ob0 = go * a.ao, on = min(a.ao, a.Cout / a.KO - ob0);  // o-blocks
+  const int t0 = (int)blockIdx.y * a.per, n = max(0, min(a.per, a.tiles - t0));
+  if (warp == 0) tc::tmem_alloc(&tmem_slot, a.ncols);
+  if (tid == 0) {
+    for (int i = 0; i < a.S; ++i) {
+      tc::mbar_init(&full[i], 1 + (nup ? kExpanders : 0));
+      tc::mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&done[i], 1);
+      tc::mbar_init(&drained[i], kExpanders * 32);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = tmem_slot, s0 = tc::smem_u32(smem);
+  const uint32_t ncb = 3 * a.CB;  // accumulator columns of a block
+  bool ok = true;
+  if (warp == 0) {
+    const uint32_t idesc = tc::make_idesc_bf16(128, ncb, true, true);
+    const uint32_t drow = 8 * a.KO * 2, srow = 10 * a.CB * 2;       // a pixel row of the tile
+    const uint32_t dstep = 2 * drow >> 4, sstep = 2 * srow >> 4;    // 16 pixels further
+    int st = 0, left = 0, set = a.sets - 1;
+    uint32_t ph = 0, set_ph = 0;  // fresh barriers: the phase before reads complete
+    for (int u = 0; u < n && ok; ++u) {
+      const bool fresh = left == 0;  // first unit of a run
+      if (fresh) {
+        left = min(a.run, n - u);
+        if (++set == a.sets) {
+          set = 0;
+          set_ph ^= 1u;
+        }
+        ok = warp_wait(&drained[set], set_ph);
+      }
+      const uint32_t set_col = set * a.ao * a.G * ncb;
+      --left;
+      ok = ok && warp_wait(&full[st], ph);
+      if (!ok) break;
+      tc::fence_after();
+      const uint32_t sd = s0 + st * a.stage, ss = sd + a.src_off;
+      if (elect_one()) {
+        for (int o = 0; o < on; ++o) {
+          const uint64_t ad = mn_desc(sd + o * a.dbytes, drow, drow, a.KO);
+          for (int g = 0; g < gn; ++g) {
+            const uint64_t bd = mn_desc(ss + g * a.sbytes, a.CB * 2, srow, a.CB);
+            const uint32_t d = tmem + set_col + (o * a.G + g) * ncb;
+#pragma unroll 4
+            for (int ks = 0; ks < a.TR / 2; ++ks)
+              tc::mma_bf16(d, ad + (uint64_t)(ks * dstep), bd + (uint64_t)(ks * sstep), idesc, !fresh || ks > 0);
+          }
+        }
+        tc::mma_commit(&empty[st]);
+        if (left == 0) tc::mma_commit(&done[set]);
+      }
+      __syncwarp();
+      if (++st == a.S) {
+        st = 0;
+        ph ^= 1u;
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int st = 0, issued = 0;
+      uint32_t ph = 1;
+      Walk w(a, t0);
+      const uint32_t bytes = (uint32_t)on * (uint32_t)((a.TR + 2) * 8 * a.KO * 2) +
+                             (uint32_t)(gn - nup) * (uint32_t)(a.TR * 10 * a.CB * 2);
+      for (int u = 0; u < n; ++u, w.next(a)) {
+        ok = tc::mbar_wait(&empty[st], ph);
+        if (!ok) break;
+        const uint32_t sd = s0 + st * a.stage;
+        tc::mbar_arrive_expect_tx(&full[st], bytes);
+        for (int o = 0; o < on; ++o)
+          tma4(sd + o * a.dbytes, &tm.dout, (ob0 + o) * a.KO, w.x * 8, w.y * a.TR - 1, w.img, &full[st]);
+        for (int g = nup; g < gn; ++g) {
+          const bool first = g0 + g < a.ng1;
+          tma4(sd + a.src_off + g * a.sbytes, first ? &tm.src[0] : &tm.src[1],
+               (g0 + g - (first ? 0 : a.ng1)) * a.CB, w.x * 8 - 1, w.y * a.TR, w.img, &full[st]);
+        }
+        ++issued;
+        if (++st == a.S) {
+          st = 0;
+          ph ^= 1u;
+        }
+      }
+      if (!ok)
+        for (int u = max(0, issued - a.S); u < issued; ++u) tc::mbar_wait(&full[u % a.S], (uint32_t)(u / a.S) & 1u);
+    }
+  } else {
+    // expand the half-resolution groups: thread -> chunk of 8 channels, every
+    // pxs-th pixel of the TR x 10 halo
+    const int cpp = a.CB >> 3, ch = (tid - 64) % cpp, p0 = (tid - 64) / cpp, pxs = kExpanders * 32 / cpp;
+    const int Hl = a.H >> 1, Wl = a.W >> 1;
+    // epilogue: two warps per 32 lanes, on alternate 8-column chunks
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    const int m = q * 32 + lane, atom = m / a.KO, ol = m - atom * a.KO;
+    const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16);
+    const int nc8 = a.CB >> 3;
+    int st = 0, set = a.sets - 1;
+    uint32_t ph = 1, set_ph = 1;
+    Walk w(a, t0);
+    auto arrive = [&](int stage) {
+      tc::fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&full[stage]);
+    };
+    for (int u0 = 0; u0 < n && ok; u0 += a.run) {
+      if (nup) {
+        int prev = -1;
+        for (int u = u0; u < min(n, u0 + a.run); ++u, w.next(a)) {
+          ok = warp_wait(&empty[st], ph);
+          if (!ok) break;
+          const uint32_t ss = s0 + st * a.stage + a.src_off;
+          for (int h = p0; h < 10 * a.TR; h += pxs) {
+            const int r = h / 10, X = w.x * 8 - 1 + (h - 10 * r), Y = w.y * a.TR + r;
+            const bool in = X >= 0 && X < a.W && Y < a.H;
+            const bf16* px = a.x1 + (((size_t)w.img * Hl + (Y >> 1)) * Wl + (X >> 1)) * a.C1;
+            // 64- / 32-byte swizzle of 16-byte chunks
+            const uint32_t dst = ss + h * a.CB * 2 + ((a.CB == 32 ? ch ^ ((h >> 1) & 3) : ch ^ ((h >> 2) & 1)) << 4);
+            for (int g = 0; g < nup; ++g) {
+              const int c = (g0 + g) * a.CB + 8 * ch;
+              const bool v = in && c < a.C1;
+              tc::cp_async16(dst + g * a.sbytes, v ? px + c : a.x1, v ? 16u : 0u);
+            }
+          }
+          tc::cp_async_commit();
+          if (prev >= 0) {
+            tc::cp_async_wait<1>();
+            arrive(prev);
+          }
+          prev = st;
+          if (++st == a.S) {
+            st = 0;
+            ph ^= 1u;
+          }
+        }
+        tc::cp_async_wait<0>();
+        if (ok && prev >= 0) arrive(prev);
+      }
+      if (++set == a.sets) {
+        set = 0;
+        set_ph ^= 1u;
+      }
+      ok = ok && warp_wait(&done[set], set_ph);
+      tc::fence_after();
+      if (ok && q * 32 / a.KO < 3) {  // some lane of the warp holds a tap
+        for (int o = 0; o < on; ++o)
+          for (int g = 0; g < gn; ++g) {
+            const bool first = g0 + g < a.ng1;
+            const int cl = (g0 + g - (first ? 0 : a.ng1)) * a.CB;  // channel within its source
+            for (int k = half; k < nc8; k += 2) {
+              const int c = cl + 8 * k;
+              const bool live = atom < 3 && c < (first ? a.C1 : a.C2);
+              for (int d = 0; d < 3; ++d) {
+                float v[8];
+                tc::tmem_ld8(lanes + ((set * a.ao + o) * a.G + g) * ncb + d * a.CB + 8 * k, v);
+                if (live) add8(a, (ob0 + o) * a.KO + ol, (2 - atom) * 3 + d, (first ? 0 : a.C1) + c, v);
+              }
+            }
+          }
+      }
+      tc::fence_before();
+      tc::mbar_arrive(&drained[set]);
+    }
+  }
+  if (!__syncthreads_and(ok) && lane == 0) atomicOr(a.err, tc::kErrMbarTimeout);
+  tc::fence_before();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tmem, a.ncols);
+}
+
+constexpr uint32_t kSmemW = 216 * 1024, kPad = 4096;  // kPad: MMA reads of padding atoms past the last stage
+
+// Pixels an accumulator may sum before it is added to dw (see the file
+// comment): the range a CTA of the kernels before this one summed.  Rows of
+// 64 pixels or more: one CTA per SM and set of channels -- all of up to 128
+// where outputs are few, else the width (48, 32 or 16) that weighed a set's
+// fixed cost against its number -- two for 16 channels.  Narrower rows: the
+// gather kernel's, but at least 512 (32 MMAs lose about 4e-7).
+long long run_pixels(const ConvWgrad& c) {
+  const long long P = (long long)c.N * c.H * c.W;
+  long long px;
+  if (c.W >= 64 && c.Cin % 16 == 0 && 9 * c.Cout <= 512 && c.Cin >= 64) {
+    px = P * ((c.Cin + 127) / 128) / tile_sm_count();
+  } else if (c.W >= 64 && c.Cin % 16 == 0 && c.Cout <= 128) {
+    int nr = 1;
+    long long best = -1;
+    for (int cr : {48, 32, 16}) {
+      const int k = (c.Cin + cr - 1) / cr;
+      const long long cost = (long long)k * (cr + c.Cout / 4 + 8);
+      if (cr <= c.Cin && (best < 0 || cost < best)) best = cost, nr = k;
+    }
+    px = P * nr / (tile_sm_count() * (c.Cin <= 16 ? 2 : 1));
+  } else {
+    px = wgrad_pixels_per_cta(P, c.Cout, c.Cin);
+  }
+  return std::max(px, 512LL);
+}
+
+}  // namespace
+
+bool conv_tile_wgrad(const ConvWgrad& c, cudaStream_t st, cudaError_t* e) {
+  if (c.Cout % 16 || c.Cout > 256 || c.s1.C % 8 || c.s2.C % 8 || c.s2.up) return false;
+  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  if (!aligned(c.dout) || !aligned(c.s1.ptr) || !aligned(c.s2.ptr)) return false;
+  if (c.s1.up && (c.H % 2 || c.W % 2)) return false;
+  WgradArgs a{};
+  a.Cout = c.Cout;
+  a.Cin = c.Cin;
+  a.C1 = c.s1.C;
+  a.C2 = c.s2.ptr ? c.s2.C : 0;
+  a.up1 = c.s1.up ? 1 : 0;
+  a.x1 = c.s1.ptr;
+  a.H = c.H;
+  a.W = c.W;
+  a.dw = c.dw;
+  a.err = c.err;
+  a.KO = c.Cout % 32 == 0 ? 32 : 16;
+  const int at = c.Cout / a.KO;
+  a.CB = std::max(a.C1, a.C2) > 16 ? 32 : 16;
+  if (at * 3 * a.CB > 512) a.CB = 16;  // the accumulators of all outputs in 512 columns
+  a.ao = std::min(at, 512 / (3 * a.CB));
+  const int ngo = (at + a.ao - 1) / a.ao;
+  a.ng1 = (a.C1 + a.CB - 1) / a.CB;
+  a.ng = a.ng1 + (a.C2 + a.CB - 1) / a.CB;
+  auto plan = [&](int TR, int G) {
+    a.TR = TR;
+    a.G = G;
+    a.dbytes = up1k((uint32_t)((TR + 2) * 8 * a.KO * 2));
+    a.sbytes = up1k((uint32_t)(TR * 10 * a.CB * 2));
+    a.src_off = a.ao * a.dbytes;
+    a.stage = a.src_off + G * a.sbytes;
+    a.S = (int)std::min<uint32_t>(kMaxSW, (kSmemW - kPad) / a.stage);
+    return a.S;
+  };
+  // One block of outputs (up to 32): a CTA takes every channel group its
+  // accumulators and a three-stage ring allow, so dout is read once; more
+  // outputs: one group per CTA.
+  int G = 1;
+  if (at == 1)
+    while (G < a.ng && (G + 1) * 3 * a.CB <= 512 && plan(8, G + 1) >= 3) ++G;
+  // the tallest tile (up to 32 rows) that leaves three stages
+  int TR = 32;
+  while (TR > 8 && (plan(TR, G) < 3 || c.H <= TR / 2)) TR /= 2;
+  if (plan(TR, G) < 2) return false;
+  a.ngc = (a.ng + G - 1) / G;
+  a.tx = (c.W + 7) / 8;
+  a.ty = (c.H + TR - 1) / TR;
+  const long long T = (long long)c.N * a.tx * a.ty;
+  if (T > (1LL << 30)) return false;
+  a.tiles = (int)T;
+  const int columns = a.ngc * ngo, ranges = std::max(1, tile_sm_count() / columns);
+  a.per = (a.tiles + ranges - 1) / ranges;
+  // equal runs; a tenth over the limit is within what the limit's own
+  // rounding to whole tiles varied by
+  const double over = (double)a.per * 8 * TR / (1.1 * (double)run_pixels(c));
+  const int runs = std::min(a.per, std::max(1, (int)std::ceil(over)));
+  a.run = (a.per + runs - 1) / runs;
+  a.sets = runs > 1 && 2 * a.ao * G * 3 * a.CB <= 512 ? 2 : 1;
+  const uint32_t cols = (uint32_t)(a.sets * a.ao * G * 3 * a.CB);
+  for (a.ncols = 32; a.ncols < cols;) a.ncols *= 2;
+  WgradMaps m{};
+  if (!pixel_map(&m.dout, c.dout, c.N, c.H, c.W, c.Cout, 1, 1, a.KO, 8, TR + 2)) return false;
+  if (!c.s1.up && !pixel_map(&m.src[0], c.s1.ptr, c.N, c.H, c.W, a.C1, 1, 1, a.CB, 10, TR)) return false;
+  if (a.C2 && !pixel_map(&m.src[1], c.s2.ptr, c.N, c.H, c.W, a.C2, 1, 1, a.CB, 10, TR)) return false;
+  // past half the SM's shared memory: one CTA per SM (TMEM columns)
+  const size_t smem = std::max<size_t>((size_t)a.S * a.stage + kPad, 116 * 1024);
+  if ((*e = cudaFuncSetAttribute(k_wgrad_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))) return true;
+  k_wgrad_tile<<<dim3(columns, (a.tiles + a.per - 1) / a.per), kThreadsW, smem, st>>>(a, m);
+  *e = cudaGetLastError();
+  return true;
+}
+
+}  // namespace nn
+}  // namespace rtx

@@ -71,6 +71,25 @@ def test_data_gradient(ctx, c):
     np.testing.assert_allclose(val(din), ref, rtol=2.0 ** -7, atol=1e-5 * np.abs(ref).max())
 
 
+WGRAD_CASES = CASES + [
+    (1, 9, 7, 32, 0, 0, 32),        # an image smaller than a tile
+    (1, 16, 8, 24, 0, 8, 16),       # channel counts that leave part of a group (and 16-output blocks)
+    (2, 12, 20, 40, 1, 24, 48),     # the same, expanded from half resolution
+    (1, 40, 48, 64, 0, 0, 256),     # eight output blocks: 16-channel groups
+    (9, 32, 32, 160, 1, 128, 128),  # several runs per CTA on one set of accumulators
+    (10, 128, 128, 16, 0, 0, 32),   # several runs alternating between two sets
+]
+
+
+@pytest.mark.parametrize("c", WGRAD_CASES)
+def test_weight_gradient(ctx, c):
+    x1, x2, _, x, dout, _ = inputs(c, 3)
+    dw = ctx.conv3x3_wgrad(dout, x1, x2=x2, up1=bool(c[4]))
+    ref, _ = U.conv3x3_wgrad(x, val(dout))
+    ref = ref.reshape(c[6], 9, -1)
+    np.testing.assert_allclose(dw, ref, rtol=1e-4, atol=1e-5 * np.abs(ref).max())
+
+
 @pytest.mark.parametrize("shape", [(1, 64, 80), (2, 80, 144)])
 def test_network_gradients(ctx, shape):
     """The whole network at sizes whose upper levels take the tile kernels
