@@ -759,9 +759,9 @@ constexpr size_t kResidentWeights = 128 * 1024;
 cudaError_t conv_fwd(const ConvFwd& a, cudaStream_t st) {
   long long P = (long long)a.N * a.H * a.W;
   if (a.Cout % 16 || a.Cout > 256 || a.Cin % 8) return cudaErrorInvalidValue;
+  cudaError_t e = cudaSuccess;
+  if (conv_tile_fwd(a, use_rows(a.W, a.Cin), st, &e)) return e;
   if (use_rows(a.W, a.Cin)) {
-    cudaError_t e = cudaSuccess;
-    if (conv_tile_fwd(a, st, &e)) return e;
     const size_t wbytes = (size_t)9 * a.Cin * a.Cout * 2;
     const bool res = wbytes <= kResidentWeights;
     const size_t stage = res ? kHaloBytes : kHaloBytes + (size_t)9 * a.Cout * 32;
@@ -776,15 +776,15 @@ cudaError_t conv_fwd(const ConvFwd& a, cudaStream_t st) {
 }
 
 bool conv_dgrad_splits(const ConvDgrad& a) {
-  return use_rows(a.W, a.Cout) && a.s1.up && a.s2.ptr && a.Cin % 16 == 0 && a.s1.C % 16 == 0 && a.H % 2 == 0 &&
-         a.W % 2 == 0;
+  return conv_tile_takes_dgrad(a, use_rows(a.W, a.Cout)) && a.s1.up && a.s2.ptr && a.s1.C % 16 == 0 &&
+         a.H % 2 == 0 && a.W % 2 == 0;
 }
 
 cudaError_t conv_dgrad(const ConvDgrad& a, cudaStream_t st) {
   long long P = (long long)a.N * a.H * a.W;
   if (a.Cin % 16 || a.Cout % 8) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
-  if (use_rows(a.W, a.Cout) && conv_tile_dgrad(a, st, &e)) return e;
+  if (conv_tile_dgrad(a, use_rows(a.W, a.Cout), st, &e)) return e;
   if (a.dlow || a.dskip) return cudaErrorNotSupported;  // only the tile kernel splits its output
   int nb = std::min(256, a.Cin);
   size_t stage = 128 * kSlice * 2 + (size_t)nb * kSlice * 2;

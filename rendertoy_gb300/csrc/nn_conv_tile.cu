@@ -82,10 +82,9 @@ struct TileArgs {
   bf16 *din, *dlow, *dskip;
   int* err;
   // narrow form
-  int G, nhalo, up1;        // slabs per weight unit, halo buffers, expand the first source
-  uint32_t halo_stride;
+  int G, nhalo;             // slabs per weight unit, halo buffers
+  int up1, C1;              // expand the first source (x1, C1 channels) from half resolution
   const bf16* x1;
-  int C1;
 };
 
 struct TileMaps {
@@ -93,7 +92,7 @@ struct TileMaps {
 };
 
 struct Bars {
-  uint64_t full[kMaxS], empty[kMaxS], accf[kMaxBuf], acce[kMaxBuf], wbar, hfull[2], hempty[2];
+  uint64_t full[kMaxS], empty[kMaxS], accf[kMaxBuf], acce[kMaxBuf], wbar;
 };
 
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
@@ -325,10 +324,6 @@ __device__ __forceinline__ void bars_init(Bars& b, int S, int readers) {
       tc::mbar_init(&b.accf[i], 1);
       tc::mbar_init(&b.acce[i], readers);
     }
-    for (int i = 0; i < 2; ++i) {
-      tc::mbar_init(&b.hfull[i], 1 + 32);
-      tc::mbar_init(&b.hempty[i], 1);
-    }
     tc::mbar_init(&b.wbar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -503,6 +498,193 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
   if (warp == 0) tc::tmem_dealloc(tmem, a.ncols);
 }
 
+// Narrow rows: additions in tap-major order.  The tile's halo of every slab
+// stays in shared memory while the weights stream past it in units of one tap
+// x G slabs; with two halo buffers the next tile's halo loads meanwhile.  An
+// upsampled first source is expanded into the halo by four warps (cp.async),
+// the rest arrives by tensor copy.  Warps 2 .. 5 expand, 6 .. 13 are two
+// epilogue groups on alternate tiles.
+constexpr int kExpandWarps = 4, kNarrowEpi = 8, kThreadsN = 64 + 32 * (kExpandWarps + kNarrowEpi);
+
+struct NarrowBars {
+  uint64_t full[kMaxS], empty[kMaxS], accf[2], acce[2], hfull[2], hempty[2];
+};
+
+template <int KC, bool kDg>
+__global__ void __launch_bounds__(kThreadsN, 1) k_conv_narrow(const TileArgs a, const __grid_constant__ TileMaps tm) {
+  constexpr int RB = KC * 2;
+  constexpr uint32_t kSlab = up1k(halo_bytes(KC, 1));
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ __align__(8) NarrowBars bars;
+  __shared__ uint32_t tmem_slot;
+  __shared__ uint4 xch[kDg ? kNarrowEpi : 1][32][2];
+  __shared__ __align__(16) float bias[kDg ? 4 : 256];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n_tiles = (int)blockIdx.x < a.n_tiles ? (a.n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  if (warp == 0) tc::tmem_alloc(&tmem_slot, a.ncols);
+  if (tid == 0) {
+    for (int i = 0; i < a.S; ++i) {
+      tc::mbar_init(&bars.full[i], 1);
+      tc::mbar_init(&bars.empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&bars.accf[i], 1);
+      tc::mbar_init(&bars.acce[i], 128);
+      tc::mbar_init(&bars.hfull[i], 1 + (a.up1 ? kExpandWarps : 0));
+      tc::mbar_init(&bars.hempty[i], 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (!kDg && a.bias)
+    for (int k = tid; k < a.Nout; k += kThreadsN) bias[k] = a.bias[k];
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = tmem_slot, s0 = tc::smem_u32(smem), sw = s0 + a.nhalo * a.nslab * kSlab;
+  const uint32_t slab_w = (uint32_t)a.NT * RB;
+  const int ngrp = (a.nslab + a.G - 1) / a.G;  // weight units per tap
+  bool ok = true;
+  if (warp == 0) {
+    int st = 0, hb = 0, buf = 0;
+    uint32_t ph = 0, hph = 0, bph = 1;
+    TileIter it(a, (int)blockIdx.x, (int)gridDim.x);
+    for (int i = 0; i < n_tiles && ok; ++i, it.next(a)) {
+      ok = warp_wait(&bars.acce[buf], bph) && warp_wait(&bars.hfull[hb], hph);
+      const uint32_t idesc = tc::make_idesc_bf16(128, min(a.NT, a.Nout - it.nt * a.NT));
+      const uint32_t d = tmem + buf * a.NT, sh = s0 + hb * a.nslab * kSlab;
+      int tap = 0, g = 0;
+      for (int u = 0; u < 9 * ngrp && ok; ++u) {
+        ok = warp_wait(&bars.full[st], ph);
+        if (!ok) break;
+        tc::fence_after();
+        const int dy = tap / 3 - 1, dx = tap - (dy + 1) * 3 - 1;
+        const int off = (kDg ? 1 - dy : 1 + dy) * kHW + (kDg ? 1 - dx : 1 + dx);
+        const int sl0 = g * a.G, sn = min(a.G, a.nslab - sl0);
+        const uint64_t ad = kdesc<KC>(sh + sl0 * kSlab + off * RB, kHW * RB);
+        const uint64_t bd = kdesc<KC>(sw + st * a.stage, 8 * RB);
+        if (elect_one()) {
+          for (int s = 0; s < sn; ++s)
+#pragma unroll
+            for (int ks = 0; ks < KC / 16; ++ks)
+              tc::mma_bf16(d, ad + (uint64_t)(s * (kSlab >> 4) + 2 * ks), bd + (uint64_t)(s * (slab_w >> 4) + 2 * ks), idesc,
+                           u > 0 || s > 0 || ks > 0);
+          tc::mma_commit(&bars.empty[st]);
+          if (u == 9 * ngrp - 1) {
+            tc::mma_commit(&bars.hempty[hb]);
+            tc::mma_commit(&bars.accf[buf]);
+          }
+        }
+        __syncwarp();
+        if (++g == ngrp) {
+          g = 0;
+          ++tap;
+        }
+        if (++st == a.S) {
+          st = 0;
+          ph ^= 1u;
+        }
+      }
+      if (++hb == a.nhalo) {
+        hb = 0;
+        hph ^= 1u;
+      }
+      buf ^= 1;
+      if (buf == 0) bph ^= 1u;
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int st = 0, issued = 0, hb = 0, hissued = 0;
+      uint32_t ph = 1, hph = 1;
+      const int sk = a.up1 ? a.nslab1 : 0;  // expanded slabs are not copied
+      TileIter it(a, (int)blockIdx.x, (int)gridDim.x);
+      for (int i = 0; i < n_tiles && ok; ++i, it.next(a)) {
+        const Tile t = it.tile(16);
+        ok = tc::mbar_wait(&bars.hempty[hb], hph);
+        if (!ok) break;
+        tc::mbar_arrive_expect_tx(&bars.hfull[hb], (uint32_t)(a.nslab - sk) * halo_bytes(KC, 1));
+        for (int s = sk; s < a.nslab; ++s) {
+          const bool first = s < a.nslab1;
+          tma4(s0 + (hb * a.nslab + s) * kSlab, first ? &tm.s1 : &tm.s2[0], (first ? s : s - a.nslab1) * KC, t.x0 - 1,
+               t.y0 - 1, t.n, &bars.hfull[hb]);
+        }
+        ++hissued;
+        if (++hb == a.nhalo) {
+          hb = 0;
+          hph ^= 1u;
+        }
+        for (int u = 0; u < 9 * ngrp; ++u) {
+          ok = tc::mbar_wait(&bars.empty[st], ph);
+          if (!ok) break;
+          const int tap = u / ngrp, sl0 = (u - tap * ngrp) * a.G, sn = min(a.G, a.nslab - sl0);
+          tc::mbar_arrive_expect_tx(&bars.full[st], (uint32_t)sn * slab_w);
+          for (int s = 0; s < sn; ++s)
+            tma3(sw + st * a.stage + s * slab_w, &tm.w, (sl0 + s) * KC, t.nt * a.NT, tap, &bars.full[st]);
+          ++issued;
+          if (++st == a.S) {
+            st = 0;
+            ph ^= 1u;
+          }
+        }
+      }
+      if (!ok) {  // wait (bounded) for the copies in flight before leaving
+        for (int u = max(0, issued - a.S); u < issued; ++u) tc::mbar_wait(&bars.full[u % a.S], (uint32_t)(u / a.S) & 1u);
+        for (int u = max(0, hissued - a.nhalo); u < hissued; ++u)
+          tc::mbar_wait(&bars.hfull[u % a.nhalo], (uint32_t)(u / a.nhalo) & 1u);
+      }
+    }
+  } else if (warp < 2 + kExpandWarps) {
+    if (a.up1) {
+      constexpr int cpp = KC / 8, pxs = kExpandWarps * 32 / cpp;  // 16-byte chunks per pixel
+      const int ch = (tid - 64) % cpp, p0 = (tid - 64) / cpp, Hl = a.H >> 1, Wl = a.W >> 1;
+      int hb = 0;
+      uint32_t hph = 1;
+      TileIter it(a, (int)blockIdx.x, (int)gridDim.x);
+      for (int i = 0; i < n_tiles && ok; ++i, it.next(a)) {
+        const Tile t = it.tile(16);
+        ok = warp_wait(&bars.hempty[hb], hph);
+        if (!ok) break;
+        for (int h = p0; h < kHW * 18; h += pxs) {
+          const int r = h / kHW, X = t.x0 - 1 + (h - kHW * r), Y = t.y0 - 1 + r;
+          const bool in = X >= 0 && X < a.W && Y >= 0 && Y < a.H;
+          const bf16* px = a.x1 + (in ? (((size_t)t.n * Hl + (Y >> 1)) * Wl + (X >> 1)) * a.C1 : 0) + 8 * ch;
+          const uint32_t dst = s0 + hb * a.nslab * kSlab + h * RB + ((KC == 32 ? ch ^ ((h >> 1) & 3) : ch ^ ((h >> 2) & 1)) << 4);
+          for (int s = 0; s < a.nslab1; ++s) tc::cp_async16(dst + s * kSlab, px + s * KC, in ? 16u : 0u);
+        }
+        tc::cp_async_commit();
+        tc::cp_async_wait<0>();
+        tc::fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&bars.hfull[hb]);
+        if (++hb == a.nhalo) {
+          hb = 0;
+          hph ^= 1u;
+        }
+      }
+    }
+  } else {
+    const int g = (warp - 2 - kExpandWarps) >> 2;
+    TileIter it(a, (int)(blockIdx.x + g * gridDim.x), 2 * (int)gridDim.x);
+    for (int i = g; i < n_tiles && ok; i += 2, it.next(a)) {
+      const Tile t = it.tile(16);
+      ok = tile_epilogue<false, kDg>(
+          a, t, tmem + (i & 1) * a.NT, 0, 1, warp, lane, xch[kDg ? warp - 2 - kExpandWarps : 0], bias,
+          [&] {
+            const bool w = warp_wait(&bars.accf[i & 1], (uint32_t)(i >> 1) & 1u);
+            tc::fence_after();
+            return w;
+          },
+          [&] {
+            tc::fence_before();
+            tc::mbar_arrive(&bars.acce[i & 1]);
+          });
+    }
+  }
+  if (!__syncthreads_and(ok) && lane == 0) atomicOr(a.err, tc::kErrMbarTimeout);
+  tc::fence_before();
+  __syncthreads();
+  if (warp == 0) tc::tmem_dealloc(tmem, a.ncols);
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -652,7 +834,61 @@ static bool plan_wide(TileArgs a, const Src& x1, const Src& x2, const bf16* w, i
   return true;
 }
 
-bool conv_tile_fwd(const ConvFwd& c, cudaStream_t st, cudaError_t* e) {
+// The narrow (tap-major) form.  Its halo must fit beside two weight units.
+static bool narrow_fits(int KC, int K) {
+  return (size_t)(K / KC) * up1k(halo_bytes(KC, 1)) + 2 * up1k(128 * KC * 2) <= kSmem;
+}
+
+template <int KC, bool kDg>
+static bool plan_narrow(TileArgs a, const Src& x1, const Src& x2, const bf16* w, int imgs, cudaStream_t st,
+                        cudaError_t* e) {
+  const int K = x1.C + x2.C;
+  if (!narrow_fits(KC, K)) return false;
+  const uint32_t slab = up1k(halo_bytes(KC, 1));
+  a.nslab1 = x1.C / KC;
+  a.nslab = K / KC;
+  a.up1 = x1.up;
+  a.C1 = x1.C;
+  a.x1 = x1.ptr;
+  a.tx = (a.W + 7) / 8;
+  a.ty = (a.H + 15) / 16;
+  const long long T = (long long)imgs * a.tx * a.ty;
+  if (T > (1LL << 24)) return false;
+  // Output-channel tiles of at most 128: the split with the shortest rounds
+  // of tiles over the SMs (an MMA costs max(N / 2, 32 + N / 4) clocks; a
+  // tensor copy one row of its weights per 1.2)
+  double best = 0;
+  for (int k = (a.Nout + 127) / 128; k <= (a.Nout + 31) / 32; ++k) {
+    const int nt = ((a.Nout + k - 1) / k + 15) / 16 * 16, ntn = (a.Nout + nt - 1) / nt;
+    const double step = std::max({nt * 0.5, 32 + nt * 0.25, nt * 1.2 * 16 / KC});
+    const double cost = (double)((T * ntn + tile_sm_count() - 1) / tile_sm_count()) * (step * 9 * (K / 16) + 3000);
+    if (best == 0 || cost < best) best = cost, a.NT = nt, a.ntn = ntn;
+  }
+  a.n_tiles = (int)(T * a.ntn);
+  const size_t unit1 = (size_t)a.NT * KC * 2;
+  a.nhalo = (size_t)2 * a.nslab * slab + 4 * up1k((uint32_t)unit1) <= kSmem ? 2 : 1;
+  const size_t room = kSmem - (size_t)a.nhalo * a.nslab * slab;
+  // weight units of up to 24 KB, of which four fit
+  a.G = (int)std::max<size_t>(1, std::min<size_t>({(size_t)a.nslab, 24 * 1024 / unit1, room / 4 / unit1}));
+  a.stage = up1k((uint32_t)(a.G * unit1));
+  a.S = (int)std::min<size_t>(kMaxS, room / a.stage);
+  if (a.S < 2) return false;
+  a.nbuf = 2;
+  a.ncols = pow2_cols(2 * a.NT);
+  TileMaps m{};
+  if (!tap_map(&m.w, w, a.Nout, K, KC, a.NT, 1)) return false;
+  if (!x1.up && !pixel_map(&m.s1, x1.ptr, imgs, a.H, a.W, x1.C, 1, 1, KC, kHW, 18)) return false;
+  if (x2.ptr && !pixel_map(&m.s2[0], x2.ptr, imgs, a.H, a.W, x2.C, 1, 1, KC, kHW, 18)) return false;
+  if (x1.up && (reinterpret_cast<uintptr_t>(x1.ptr) & 15)) return false;
+  const size_t smem = std::max<size_t>((size_t)a.nhalo * a.nslab * slab + (size_t)a.S * a.stage, 116 * 1024);
+  auto k = k_conv_narrow<KC, kDg>;
+  if ((*e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))) return true;
+  k<<<std::min(a.n_tiles, tile_sm_count()), kThreadsN, smem, st>>>(a, m);
+  *e = cudaGetLastError();
+  return true;
+}
+
+bool conv_tile_fwd(const ConvFwd& c, bool wide, cudaStream_t st, cudaError_t* e) {
   const int g = c.s2.ptr ? (c.s1.C | c.s2.C) : c.s1.C;
   if (g % 16 || c.Cout % 16 || c.s2.up || (c.s1.up && (c.H % 2 || c.W % 2))) return false;
   if (c.out && (reinterpret_cast<uintptr_t>(c.out) & 15)) return false;
@@ -666,12 +902,20 @@ bool conv_tile_fwd(const ConvFwd& c, cudaStream_t st, cudaError_t* e) {
   a.out_f32 = c.out_f32;
   a.err = c.err;
   const Src s2 = c.s2.ptr ? c.s2 : Src{nullptr, 0, 0};
+  if (!wide)
+    return g % 32 == 0 ? plan_narrow<32, false>(a, c.s1, s2, c.w, c.N, st, e)
+                       : plan_narrow<16, false>(a, c.s1, s2, c.w, c.N, st, e);
   return g % 32 == 0 ? plan_wide<32, false>(a, c.s1, s2, c.w, c.N, st, e)
                      : plan_wide<16, false>(a, c.s1, s2, c.w, c.N, st, e);
 }
 
-bool conv_tile_dgrad(const ConvDgrad& c, cudaStream_t st, cudaError_t* e) {
+bool conv_tile_takes_dgrad(const ConvDgrad& c, bool wide) {
   if (c.Cout % 16 || c.Cin % 16) return false;
+  return wide || narrow_fits(c.Cout % 32 == 0 ? 32 : 16, c.Cout);
+}
+
+bool conv_tile_dgrad(const ConvDgrad& c, bool wide, cudaStream_t st, cudaError_t* e) {
+  if (!conv_tile_takes_dgrad(c, wide)) return false;
   TileArgs a{};
   a.H = c.H;
   a.W = c.W;
@@ -685,6 +929,9 @@ bool conv_tile_dgrad(const ConvDgrad& c, cudaStream_t st, cudaError_t* e) {
   a.flip = 1;
   a.err = c.err;
   const Src d{c.dout, c.Cout, 0}, none{nullptr, 0, 0};
+  if (!wide)
+    return c.Cout % 32 == 0 ? plan_narrow<32, true>(a, d, none, c.wt, c.N, st, e)
+                            : plan_narrow<16, true>(a, d, none, c.wt, c.N, st, e);
   return c.Cout % 32 == 0 ? plan_wide<32, true>(a, d, none, c.wt, c.N, st, e)
                           : plan_wide<16, true>(a, d, none, c.wt, c.N, st, e);
 }

@@ -1,5 +1,5 @@
-// nn_tile.h — the tile kernels of nn_conv_tile.cu (forward and data gradient)
-// as nn_conv.cu's launchers see them.  Each returns false when it does not
+// nn_tile.h — the tile kernels of nn_conv_tile.cu (forward, data gradient)
+// and nn_wgrad_tile.cu as nn_conv.cu's launchers see them.  Each returns false when it does not
 // take the shape or alignment (nothing was launched); otherwise *e holds the
 // launch's result.
 #pragma once
@@ -10,8 +10,11 @@
 namespace rtx {
 namespace nn {
 
-bool conv_tile_fwd(const ConvFwd& a, cudaStream_t st, cudaError_t* e);
-bool conv_tile_dgrad(const ConvDgrad& a, cudaStream_t st, cudaError_t* e);
+// wide: additions in slab-major order (the rule for rows of 64 pixels or
+// more), else tap-major
+bool conv_tile_fwd(const ConvFwd& a, bool wide, cudaStream_t st, cudaError_t* e);
+bool conv_tile_takes_dgrad(const ConvDgrad& a, bool wide);
+bool conv_tile_dgrad(const ConvDgrad& a, bool wide, cudaStream_t st, cudaError_t* e);
 
 bool conv_tile_wgrad(const ConvWgrad& a, cudaStream_t st, cudaError_t* e);
 

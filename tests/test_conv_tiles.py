@@ -29,6 +29,12 @@ CASES = [  # N, H, W, C1, up1, C2, Cout
     (1, 20, 70, 48, 1, 16, 16),    # upsampled + skip, 16-channel slabs
     (6, 48, 128, 32, 0, 0, 32),    # several tiles per CTA: rings and accumulators wrap
     (6, 32, 128, 64, 1, 32, 32),
+    # rows shorter than 64 pixels: tap-major order, resident halos
+    (1, 9, 7, 32, 0, 0, 32),       # an image smaller than a tile
+    (2, 17, 63, 16, 0, 32, 48),    # two sources, 16-channel slabs
+    (1, 34, 26, 160, 1, 128, 144),  # upsampled + skip, one halo buffer; 288 inputs: several output tiles
+    (1, 20, 30, 48, 1, 0, 32),     # upsampled source alone, 16-channel slabs
+    (24, 32, 32, 96, 0, 0, 128),   # several tiles per CTA: halos, rings and accumulators wrap
 ]
 
 
@@ -72,7 +78,6 @@ def test_data_gradient(ctx, c):
 
 
 WGRAD_CASES = CASES + [
-    (1, 9, 7, 32, 0, 0, 32),        # an image smaller than a tile
     (1, 16, 8, 24, 0, 8, 16),       # channel counts that leave part of a group (and 16-output blocks)
     (2, 12, 20, 40, 1, 24, 48),     # the same, expanded from half resolution
     (1, 40, 48, 64, 0, 0, 256),     # eight output blocks: 16-channel groups
