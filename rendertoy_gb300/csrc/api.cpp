@@ -97,7 +97,11 @@ struct rtx_context {
   DevBuf nodes, nodes4, tris, shade, geo, mats, emit;
   std::vector<int32_t> emitters;
   // device scratch
-  int* d_err = nullptr;
+  // Error word: mapped pinned host memory that kernels touch only to report
+  // an error, so a synchronous call clears and reads it without a memset and
+  // a copy of its own (5x5 convolution of a 256^2 image: 32.5 -> 21.7 us per call).
+  int* d_err = nullptr;          // device address
+  volatile int* h_err = nullptr;  // the same word on the host
   Counters* d_counters = nullptr;
   PtWorkspace* pt = nullptr;
   DevBuf stage[8];
@@ -126,6 +130,7 @@ struct rtx_context {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   rtx_stats stats{};
   bool pending_timing = false;
+  bool err_busy = false;  // work that may still write the error word was enqueued and not waited for
 };
 
 namespace {
@@ -199,7 +204,15 @@ static SortKeyBounds sort_key_bounds(const Float4Array& nodes4, int root4) {
 
 int begin(rtx_context* c) {
   RTX_CUDA(cudaSetDevice(c->device), "cudaSetDevice");
-  RTX_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream), "cudaMemsetAsync(err)");
+  // Cleared from the host when no earlier call of this context can still be
+  // running; in stream order otherwise (asynchronous calls, captures).
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  RTX_CUDA(cudaStreamIsCapturing(c->stream, &cap), "cudaStreamIsCapturing");
+  if (c->err_busy || cap != cudaStreamCaptureStatusNone)
+    RTX_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream), "cudaMemsetAsync(err)");
+  else
+    *c->h_err = 0;
+  c->err_busy = true;
   RTX_CUDA(cudaEventRecord(c->ev0, c->stream), "cudaEventRecord");
   c->stats.kernel_launches = 0;
   return RTX_OK;
@@ -217,8 +230,8 @@ int finish(rtx_context* c, bool may_async) {
   RTX_CUDA(cudaEventElapsedTime(&ms, c->ev0, c->ev1), "cudaEventElapsedTime");
   c->stats.last_gpu_ms = ms;
   c->pending_timing = false;
-  int herr = 0;
-  RTX_CUDA(cudaMemcpy(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost), "read error word");
+  c->err_busy = false;
+  const int herr = *c->h_err;
   if (herr) {
     std::string m = "kernel error:";
     if (herr & kErrStackOverflow) m += " traversal stack overflow";
@@ -387,7 +400,9 @@ int rtx_create(rtx_context** out, int device) {
   c->own_stream = true;
   if ((e = cudaEventCreate(&c->ev0)) != cudaSuccess) return bail(e);
   if ((e = cudaEventCreate(&c->ev1)) != cudaSuccess) return bail(e);
-  if ((e = cudaMalloc(&c->d_err, sizeof(int))) != cudaSuccess) return bail(e);
+  if ((e = cudaHostAlloc((void**)&c->h_err, sizeof(int), cudaHostAllocMapped)) != cudaSuccess) return bail(e);
+  *c->h_err = 0;
+  if ((e = cudaHostGetDevicePointer((void**)&c->d_err, (void*)c->h_err, 0)) != cudaSuccess) return bail(e);
   if ((e = cudaMalloc(&c->d_counters, sizeof(Counters))) != cudaSuccess) return bail(e);
   if ((e = cudaMemset(c->d_counters, 0, sizeof(Counters))) != cudaSuccess) return bail(e);
   {
@@ -425,7 +440,7 @@ void rtx_destroy(rtx_context* c) {
   c->weights.release();
   c->weights_valid = false;
   if (c->pt) pt_workspace_destroy(c->pt);
-  if (c->d_err) cudaFree(c->d_err);
+  if (c->h_err) cudaFreeHost((void*)c->h_err);
   if (c->d_counters) cudaFree(c->d_counters);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
@@ -523,9 +538,8 @@ int rtx_synchronize(rtx_context* c) {
     c->stats.last_gpu_ms = ms;
     c->pending_timing = false;
   }
-  int herr = 0;
-  RTX_CUDA(cudaMemcpy(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost), "read error word");
-  if (herr) return fail(c, RTX_ERR_DEVICE, "kernel error reported by an asynchronous call");
+  c->err_busy = false;
+  if (*c->h_err) return fail(c, RTX_ERR_DEVICE, "kernel error reported by an asynchronous call");
   return RTX_OK;
 }
 

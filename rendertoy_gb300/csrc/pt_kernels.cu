@@ -1253,7 +1253,9 @@ cudaError_t pt_render(PtWorkspace* ws, const DeviceScene& s, const CamParams& ca
   // idle tail, so fewer, larger waves are faster), at most 2^26 paths and a
   // quarter of the free device memory (kPathBytes = 188 B per path).
   long long wave = p.wave_paths;
-  if (wave <= 0) {
+  if (wave <= 0 && ws->counters && ws->cap >= (size_t)std::min(1LL << 26, total)) {
+    wave = 1LL << 26;  // the workspace holds the whole render: no memory query
+  } else if (wave <= 0) {
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
     long long fit = (long long)(free_b / 4 / kPathBytes);
