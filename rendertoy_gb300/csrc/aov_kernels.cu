@@ -11,6 +11,7 @@ namespace rtx {
 
 enum PrimaryMode { kModeAov = 1, kModeHits = 2 };
 
+template <bool kWide>
 __global__ void __launch_bounds__(64) k_primary(DeviceScene s, CamParams cam, int mode,
                                                 float near_, float inv_range, float* normal,
                                                 float* albedo, float* depth, int* tri_out,
@@ -24,7 +25,7 @@ __global__ void __launch_bounds__(64) k_primary(DeviceScene s, CamParams cam, in
   camera_ray(cam, x, y, o, d);
   float t, u, v;
   VisitCount vc;
-  int h = closest_hit<false>(s, o, d, -1, t, u, v, err, vc);
+  int h = first_hit<kWide>(s, o, d, -1, t, u, v, err, vc);
   size_t p = (size_t)y * cam.W + x;
   if (mode & kModeHits) {
     tri_out[p] = h;
@@ -67,6 +68,7 @@ __global__ void __launch_bounds__(64) k_primary(DeviceScene s, CamParams cam, in
   }
 }
 
+template <bool kWide>
 __global__ void __launch_bounds__(128) k_intersect(DeviceScene s, int n, const float* rays,
                                                    const int* exclude, int* tri_out,
                                                    float* tuv_out, int* err) {
@@ -76,29 +78,30 @@ __global__ void __launch_bounds__(128) k_intersect(DeviceScene s, int n, const f
   F3 o = f3(r[0], r[1], r[2]), d = f3(r[3], r[4], r[5]);
   float t, u, v;
   VisitCount vc;
-  int h = closest_hit<false>(s, o, d, exclude ? exclude[i] : -1, t, u, v, err, vc);
+  int h = first_hit<kWide>(s, o, d, exclude ? exclude[i] : -1, t, u, v, err, vc);
   tri_out[i] = h;
   tuv_out[3 * (size_t)i] = t;
   tuv_out[3 * (size_t)i + 1] = u;
   tuv_out[3 * (size_t)i + 2] = v;
 }
 
-cudaError_t launch_primary(const DeviceScene& s, const CamParams& cam, int mode, float near_,
+cudaError_t launch_primary(const DeviceScene& s, const CamParams& cam, int mode, bool wide, float near_,
                            float far_, float* normal, float* albedo, float* depth, int* tri,
                            float* tuv, int* err, cudaStream_t st, int* launches) {
   int tiles = ((cam.W + 7) >> 3) * ((cam.H + 7) >> 3);
   // DepthBufferRenderer: div_far_minus_near = 1 / (far - near), in float
   float inv_range = 1.0f / (far_ - near_);
-  k_primary<<<tiles, 64, 0, st>>>(s, cam, mode, near_, inv_range, normal, albedo, depth, tri,
-                                  tuv, err);
+  auto k = wide ? k_primary<true> : k_primary<false>;
+  k<<<tiles, 64, 0, st>>>(s, cam, mode, near_, inv_range, normal, albedo, depth, tri, tuv, err);
   ++*launches;
   return cudaGetLastError();
 }
 
-cudaError_t launch_intersect(const DeviceScene& s, int n, const float* rays, const int* exclude,
+cudaError_t launch_intersect(const DeviceScene& s, bool wide, int n, const float* rays, const int* exclude,
                              int* tri, float* tuv, int* err, cudaStream_t st, int* launches) {
   if (n <= 0) return cudaSuccess;
-  k_intersect<<<(n + 127) / 128, 128, 0, st>>>(s, n, rays, exclude, tri, tuv, err);
+  auto k = wide ? k_intersect<true> : k_intersect<false>;
+  k<<<(n + 127) / 128, 128, 0, st>>>(s, n, rays, exclude, tri, tuv, err);
   ++*launches;
   return cudaGetLastError();
 }

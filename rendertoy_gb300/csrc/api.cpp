@@ -1508,7 +1508,7 @@ static int primary_pass(rtx_context* c, const float* cam, int W, int H, int mode
   }
   CamParams cp = make_cam_params(cam, W, H);
   int launches = 0;
-  cudaError_t e = launch_primary(c->ds, cp, mode, near_, far_, (float*)an.dev, (float*)aa.dev,
+  cudaError_t e = launch_primary(c->ds, cp, mode, c->traversal == 2, near_, far_, (float*)an.dev, (float*)aa.dev,
                                  (float*)ad.dev, (int*)at.dev, (float*)au.dev, c->d_err,
                                  c->stream, &launches);
   c->stats.kernel_launches = launches;
@@ -1542,7 +1542,7 @@ int rtx_intersect(rtx_context* c, int n, const float* rays, const int32_t* exclu
   if ((r = bind_out(c, tri_out, (size_t)n * 4, 2, at))) return r;
   if ((r = bind_out(c, tuv_out, (size_t)n * 12, 3, au))) return r;
   int launches = 0;
-  cudaError_t e = launch_intersect(c->ds, n, (const float*)ar.dev, (const int*)ae.dev,
+  cudaError_t e = launch_intersect(c->ds, c->traversal == 2, n, (const float*)ar.dev, (const int*)ae.dev,
                                    (int*)at.dev, (float*)au.dev, c->d_err, c->stream, &launches);
   c->stats.kernel_launches = launches;
   if (e != cudaSuccess) return cuda_fail(c, e, "intersect kernel");

@@ -375,6 +375,7 @@ __global__ void __launch_bounds__(128, RTX_EXTEND_MINB) k_extend_batch(PtArgs a,
 
 // Primary hits of every pixel, traced once per render: all samples of a pixel
 // share its primary ray (renderer.cpp:255-259 has no per-sample jitter).
+template <bool kWide>
 RTX_DEV void primary_px(const DeviceScene& s, const CamParams& cam, float4* out, int* err, Counters* ctr) {
   int tiles_x = (cam.W + 7) >> 3;
   int x = (blockIdx.x % tiles_x) * 8 + (threadIdx.x & 7);
@@ -388,23 +389,26 @@ RTX_DEV void primary_px(const DeviceScene& s, const CamParams& cam, float4* out,
   camera_ray(cam, x, y, o, d);
   float t, u, v;
   VisitCount vc;
-  int h = closest_hit<false>(s, o, d, -1, t, u, v, err, vc);
+  int h = first_hit<kWide>(s, o, d, -1, t, u, v, err, vc);
   out[(size_t)y * cam.W + x] = make_float4(__int_as_float(h), t, u, v);
 }
 
+template <bool kWide>
 __global__ void __launch_bounds__(64) k_primary_cache(DeviceScene s, CamParams cam, float4* out, int* err,
                                                       Counters* ctr) {
-  primary_px(s, cam, out, err, ctr);
+  primary_px<kWide>(s, cam, out, err, ctr);
 }
 
 // A frame of a batch: camera and tree root from the device job table, so that
 // a replayed graph picks up new cameras.
+template <bool kWide>
 __global__ void __launch_bounds__(64) k_primary_cache_job(DeviceScene s, const PtJob* jobs, int j, float4* prim,
                                                           int* err, Counters* ctr) {
   const PtJob& J = jobs[j];
   DeviceScene sj = s;
   sj.root = J.root;
-  primary_px(sj, J.cam, prim + J.pix_begin, err, ctr);
+  sj.root4 = J.root4;
+  primary_px<kWide>(sj, J.cam, prim + J.pix_begin, err, ctr);
 }
 
 // Sort keys (12 bits, 4,096 bins) from the scene bounds the host computed
@@ -1350,12 +1354,12 @@ cudaError_t pt_render(PtWorkspace* ws, const DeviceScene& s, const CamParams& ca
       for (int j = 0; j < p.n_jobs; ++j) {
         const PtJob& J = p.h_jobs[j];  // the launch shape only (W, H)
         int tiles = ((J.cam.W + 7) >> 3) * ((J.cam.H + 7) >> 3);
-        k_primary_cache_job<<<tiles, 64, 0, st>>>(s, p.d_jobs, j, ws->prim, err, d_counters);
+        (p.traversal == 2 ? k_primary_cache_job<true> : k_primary_cache_job<false>)<<<tiles, 64, 0, st>>>(s, p.d_jobs, j, ws->prim, err, d_counters);
         ++*launches;
       }
     } else {
       int tiles = ((p.W + 7) >> 3) * ((p.H + 7) >> 3);
-      k_primary_cache<<<tiles, 64, 0, st>>>(s, cam, ws->prim, err, d_counters);
+      (p.traversal == 2 ? k_primary_cache<true> : k_primary_cache<false>)<<<tiles, 64, 0, st>>>(s, cam, ws->prim, err, d_counters);
       ++*launches;
     }
     prim = ws->prim;

@@ -177,11 +177,11 @@ struct KernelTimer {
 };
 
 // ---- kernel launchers (implemented in the .cu files) ----------------------
-cudaError_t launch_primary(const DeviceScene& s, const CamParams& cam, int mode,
+cudaError_t launch_primary(const DeviceScene& s, const CamParams& cam, int mode, bool wide,
                            float near_, float far_, float* normal, float* albedo,
                            float* depth, int* tri, float* tuv, int* err,
                            cudaStream_t st, int* launches);
-cudaError_t launch_intersect(const DeviceScene& s, int n, const float* rays,
+cudaError_t launch_intersect(const DeviceScene& s, bool wide, int n, const float* rays,
                              const int* exclude, int* tri, float* tuv, int* err,
                              cudaStream_t st, int* launches);
 

@@ -399,6 +399,14 @@ RTX_DEV int trace4(const DeviceScene& s, F3 o, F3 d, int exclude, int target, fl
   return best;
 }
 
+// Closest hit over the tree RTX_OPT_TRAVERSAL selects
+template <bool kWide>
+RTX_DEV int first_hit(const DeviceScene& s, F3 o, F3 d, int exclude, float& t, float& u, float& v, int* err,
+                      VisitCount& vc) {
+  return kWide ? trace4<false, false>(s, o, d, exclude, -1, t, u, v, err, vc)
+               : closest_hit<false>(s, o, d, exclude, t, u, v, err, vc);
+}
+
 // ---------------------------------------------------------------------------
 // Resumable traversal for persistent kernels (Aila & Laine, HPG 2009:
 // while-while loop, speculative postponement of the first leaf, and an exit
