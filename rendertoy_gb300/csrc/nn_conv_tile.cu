@@ -37,10 +37,18 @@
 // weights stream by (tap, slabs); an upsampled source is expanded into the
 // halo by the copying warps.
 //
-// Roles (576 threads, one CTA per SM, persistent): warp 0 issues the MMAs,
-// thread 32 the tensor copies, warps 2 .. 17 are four epilogue groups of four
-// warps, on alternate tiles (up to four accumulator buffers) or, for kUp, one
-// accumulator each.
+// Roles (640 threads, one CTA per SM, persistent): warps 0 .. 3 are service
+// warps, warps 4 .. 19 four epilogue groups of four.  R = 1, 2 or 4 rings, each
+// a set of stages and every R-th tile, as many as stages and accumulators
+// allow.  MMAs are issued by one elected lane of a converged warp, so that
+// descriptors stay in uniform registers.  Such a warp spends ~800 clocks per
+// tile on waits, commits and address work, and only another ring's MMAs fill
+// the tensor pipe meanwhile (640 clocks of MMAs per tile of a 32 -> 32 channel
+// layer: 88 us with one ring, 63 with four at 32 x 256^2; its data gradient 87
+// -> 69).  Up to two rings: one warp issues a ring's MMAs, another its copies;
+// four rings: each warp does both, copies one unit behind (with one ring that
+// was 25 % slower).  The four-accumulator form has 72 MMAs per unit to hide
+// the same work behind: one ring (150 us for d0, 155 with two).
 #include <algorithm>
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -54,8 +62,8 @@ namespace nn {
 
 namespace {
 
-constexpr int kEpiWarps = 16, kThreadsT = 64 + 32 * kEpiWarps;
-constexpr int kMaxS = 8, kMaxBuf = 4;
+constexpr int kService = 4, kEpiWarps = 16, kThreadsT = 32 * (kService + kEpiWarps);
+constexpr int kMaxS = 8, kMaxBuf = 8;
 constexpr int kHW = 10, kPW = 9;  // halo width: full- and low-resolution tiles, parity planes
 
 // bytes of a unit's A region
@@ -67,7 +75,7 @@ struct TileArgs {
   int tx, ty, n_tiles;      // tiles per image row / column; images x ty x tx x n-tiles
   int ntn, NT, Nout;        // output-channel tiles of NT (multiples of 16)
   int nslab1, nslab;        // slabs of the first source, of both
-  int S, nbuf;              // ring stages, accumulator buffers
+  int R, S, nbuf;           // service warps, stages of each one's ring, accumulator buffers
   uint32_t stage, w_off;    // ring stage bytes, weights within a streamed stage
   int flip;                 // data gradient: taps mirrored
   uint32_t ncols;           // TMEM columns allocated
@@ -342,119 +350,146 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tiles = (int)blockIdx.x < a.n_tiles ? (a.n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   if (warp == 0) tc::tmem_alloc(&tmem_slot, a.ncols);
-  bars_init(bars, a.S, kUp ? kEpiWarps * 32 : 128);
+  bars_init(bars, a.R * a.S, kUp ? kEpiWarps * 32 : 128);
   if (!kDg && a.bias)
     for (int k = tid; k < a.Nout; k += kThreadsT) bias[k] = a.bias[k];
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
-  const uint32_t tmem = tmem_slot, s0 = tc::smem_u32(smem), sw = s0 + a.S * a.stage;
+  const uint32_t tmem = tmem_slot, smem0 = tc::smem_u32(smem), sw = smem0 + a.R * a.S * a.stage;
   const uint32_t tap_bytes = (uint32_t)a.NT * RB, slab_w = 9 * tap_bytes;
   bool ok = true;
-  if (warp == 0) {
-    // The whole warp walks the units, so that descriptors and loop state stay
-    // in uniform registers; one elected lane issues a slab's MMAs and commits
-    // (issued from a single-lane loop, every MMA cost ~47 clocks of the
-    // issuing thread and every tile ~600 more: 108 -> 88 us for 32 -> 32
-    // channels at 32 x 256^2).
-    if (kRes && n_tiles > 0) ok = warp_wait(&bars.wbar, 0u);
-    int st = 0, buf = 0;
-    uint32_t ph = 0, bph = 1;  // a fresh barrier's preceding phase reads complete
-    TileIter it(a, (int)blockIdx.x, (int)gridDim.x);
-    const uint32_t tap16 = tap_bytes >> 4;
-    for (int i = 0; i < n_tiles && ok; ++i, it.next(a)) {
-      ok = warp_wait(&bars.acce[buf], bph);
-      const uint32_t idesc = tc::make_idesc_bf16(128, min(a.NT, a.Nout - it.nt * a.NT));
-      const uint32_t d = tmem + buf * NA * a.NT;
-      for (int s = 0; s < a.nslab && ok; ++s) {
-        ok = warp_wait(&bars.full[st], ph);
-        if (!ok) break;
-        tc::fence_after();
-        const uint32_t sa = s0 + st * a.stage;
-        const bool skip = kUp && s >= a.nslab1;
-        const uint32_t sb = kRes ? sw + (uint32_t)(it.nt * a.nslab + s) * slab_w : sa + a.w_off;
-        const uint64_t bd = kdesc<KC>(sb, 8 * RB);
-        const uint64_t ad0 = kdesc<KC>(sa, (skip ? kPW : kHW) * RB);
+  if (warp < kService) {
+    // up to two rings: warps 0, 1 issue MMAs and warps 2, 3 copy; four rings:
+    // each warp does both
+    const bool both = a.R == 4;
+    const int ring = both ? warp : (warp & 1);
+    if (ring < a.R) {
+      uint64_t* const full = bars.full + ring * a.S;
+      uint64_t* const empty = bars.empty + ring * a.S;
+      const uint32_t s0 = smem0 + ring * a.S * a.stage, tap16 = tap_bytes >> 4;
+      const int mine = n_tiles > ring ? (n_tiles - 1 - ring) / a.R + 1 : 0, units = mine * a.nslab;
+      const int first = (int)blockIdx.x + ring * (int)gridDim.x, step = a.R * (int)gridDim.x;
+      // the copying side: units in order, one stage behind the MMAs
+      TileIter ci(a, first, step);
+      int cs = 0, cst = 0, issued = 0;
+      auto copy = [&] {
+        const Tile t = ci.tile(kTH);
+        const bool one = cs < a.nslab1;
+        const uint32_t sa = s0 + cst * a.stage;
+        uint64_t* const bar = &full[cst];
         if (elect_one()) {
+          const uint32_t ab = kUp ? (one ? halo_bytes(KC, 1) : 4 * plane_bytes(KC)) : halo_bytes(KC, MT);
+          tc::mbar_arrive_expect_tx(bar, ab + (kRes ? 0u : slab_w));
+          if (!kUp || one) {
+            tma4(sa, one ? &tm.s1 : &tm.s2[0], (one ? cs : cs - a.nslab1) * KC, t.x0 - 1, t.y0 - 1, t.n, bar);
+          } else {
 #pragma unroll
-          for (int ks = 0; ks < KC / 16; ++ks) {
-            const uint64_t ad = ad0 + 2 * ks;
-            const bool acc0 = s > 0 || ks > 0;
-            if (!skip) {
-#pragma unroll
-              for (int tap = 0; tap < 9; ++tap) {
-                const int dy = tap / 3 - 1, dx = tap % 3 - 1;
-#pragma unroll
-                for (int c = 0; c < NA; ++c) {
-                  int off;
-                  if (kUp)
-                    off = (((c >> 1) + dy + 2) / 2) * kHW + ((c & 1) + dx + 2) / 2;  // floor(./2) + 1
-                  else
-                    off = (16 * c + (kDg ? 1 - dy : 1 + dy)) * kHW + (kDg ? 1 - dx : 1 + dx);
-                  tc::mma_bf16(d + c * a.NT, ad + (uint64_t)(off * RB >> 4), bd + 2 * ks + (uint64_t)tap * tap16, idesc,
-                               acc0 || tap > 0);
-                }
-              }
-            } else {
-#pragma unroll
-              for (int tap = 0; tap < 9; ++tap) {
-                const int dy = tap / 3 - 1, dx = tap % 3 - 1;
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                  // parity plane (qy, qx), shifts oy + qy, ox + qx of it
-                  const int Y = (c >> 1) + dy, X = (c & 1) + dx, qy = Y & 1, qx = X & 1;
-                  const int oy = (Y - qy) / 2, ox = (X - qx) / 2;
-                  const uint32_t off = (2 * qy + qx) * up1k(plane_bytes(KC)) + ((oy + qy) * kPW + ox + qx) * RB;
-                  tc::mma_bf16(d + c * a.NT, ad + (uint64_t)(off >> 4), bd + 2 * ks + (uint64_t)tap * tap16, idesc,
-                               acc0 || tap > 0);
-                }
-              }
-            }
+            for (int pl = 0; pl < 4; ++pl)  // plane (qy, qx) starts at shift -qy, -qx
+              tma4(sa + pl * up1k(plane_bytes(KC)), &tm.s2[pl], (cs - a.nslab1) * KC, t.x0 - (pl & 1),
+                   t.y0 - (pl >> 1), t.n, bar);
           }
-          tc::mma_commit(&bars.empty[st]);
-          if (s == a.nslab - 1) tc::mma_commit(&bars.accf[buf]);
+          if (!kRes) tma3(sa + a.w_off, &tm.w, cs * KC, t.nt * a.NT, 0, bar);
         }
         __syncwarp();
-        if (++st == a.S) {
-          st = 0;
-          ph ^= 1u;
+        ++issued;
+        if (++cst == a.S) cst = 0;
+        if (++cs == a.nslab) {
+          cs = 0;
+          ci.next(a);
         }
-      }
-      if (++buf == a.nbuf) {
-        buf = 0;
-        bph ^= 1u;
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      if (kRes && n_tiles > 0) {
+      };
+      if (kRes && warp == (both ? 0 : 2) && n_tiles > 0 && elect_one()) {
         tc::mbar_arrive_expect_tx(&bars.wbar, (uint32_t)(a.ntn * a.nslab) * slab_w);
         for (int k = 0; k < a.ntn * a.nslab; ++k)
           tma3(sw + k * slab_w, &tm.w, (k % a.nslab) * KC, (k / a.nslab) * a.NT, 0, &bars.wbar);
       }
-      int st = 0, issued = 0;
-      uint32_t ph = 1;  // a fresh barrier's preceding phase reads complete
-      TileIter it(a, (int)blockIdx.x, (int)gridDim.x);
-      for (int i = 0; i < n_tiles && ok; ++i, it.next(a)) {
-        const Tile t = it.tile(kTH);
-        for (int s = 0; s < a.nslab; ++s) {
-          ok = tc::mbar_wait(&bars.empty[st], ph);
-          if (!ok) break;
-          const bool first = s < a.nslab1;
-          const uint32_t sa = s0 + st * a.stage;
-          const uint32_t ab = kUp ? (first ? halo_bytes(KC, 1) : 4 * plane_bytes(KC)) : halo_bytes(KC, MT);
-          tc::mbar_arrive_expect_tx(&bars.full[st], ab + (kRes ? 0u : slab_w));
-          if (!kUp || first) {
-            const int c0 = (first ? s : s - a.nslab1) * KC;
-            tma4(sa, first ? &tm.s1 : &tm.s2[0], c0, t.x0 - 1, t.y0 - 1, t.n, &bars.full[st]);
-          } else {
-#pragma unroll
-            for (int pl = 0; pl < 4; ++pl)  // plane (qy, qx) starts at shift -qy, -qx
-              tma4(sa + pl * up1k(plane_bytes(KC)), &tm.s2[pl], (s - a.nslab1) * KC, t.x0 - (pl & 1),
-                   t.y0 - (pl >> 1), t.n, &bars.full[st]);
+      __syncwarp();
+      if (both || warp >= 2) {
+        while (issued < min(a.S, units)) copy();
+        if (!both) {
+          int st = 0;
+          uint32_t ph = 0;
+          while (issued < units) {
+            ok = warp_wait(&empty[st], ph);
+            if (!ok) break;
+            copy();
+            if (++st == a.S) {
+              st = 0;
+              ph ^= 1u;
+            }
           }
-          if (!kRes) tma3(sa + a.w_off, &tm.w, s * KC, t.nt * a.NT, 0, &bars.full[st]);
-          ++issued;
+        }
+      }
+      const int mmas = both || warp < 2 ? mine : 0;
+      if (kRes && mmas > 0) ok = warp_wait(&bars.wbar, 0u);
+      TileIter it(a, first, step);
+      int st = 0, pst = 0;
+      uint32_t ph = 0, eph = 0;  // phases of the stage in use, of the stage to refill
+      for (int k = 0; k < mmas && ok; ++k, it.next(a)) {
+        const int i = ring + k * a.R, buf = i % a.nbuf, lap = i / a.nbuf;
+        ok = warp_wait(&bars.acce[buf], (uint32_t)(lap - 1) & 1u);  // lap 0: a fresh barrier reads complete
+        const uint32_t idesc = tc::make_idesc_bf16(128, min(a.NT, a.Nout - it.nt * a.NT));
+        const uint32_t d = tmem + buf * NA * a.NT;
+        for (int s = 0; s < a.nslab && ok; ++s) {
+          ok = warp_wait(&full[st], ph);
+          if (!ok) break;
+          tc::fence_after();
+          const uint32_t sa = s0 + st * a.stage;
+          const bool skip = kUp && s >= a.nslab1;
+          const uint32_t sb = kRes ? sw + (uint32_t)(it.nt * a.nslab + s) * slab_w : sa + a.w_off;
+          const uint64_t bd = kdesc<KC>(sb, 8 * RB);
+          const uint64_t ad0 = kdesc<KC>(sa, (skip ? kPW : kHW) * RB);
+          if (elect_one()) {
+#pragma unroll
+            for (int ks = 0; ks < KC / 16; ++ks) {
+              const uint64_t ad = ad0 + 2 * ks;
+              const bool acc0 = s > 0 || ks > 0;
+              if (!skip) {
+#pragma unroll
+                for (int tap = 0; tap < 9; ++tap) {
+                  const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+#pragma unroll
+                  for (int c = 0; c < NA; ++c) {
+                    int off;
+                    if (kUp)
+                      off = (((c >> 1) + dy + 2) / 2) * kHW + ((c & 1) + dx + 2) / 2;  // floor(./2) + 1
+                    else
+                      off = (16 * c + (kDg ? 1 - dy : 1 + dy)) * kHW + (kDg ? 1 - dx : 1 + dx);
+                    tc::mma_bf16(d + c * a.NT, ad + (uint64_t)(off * RB >> 4), bd + 2 * ks + (uint64_t)tap * tap16,
+                                 idesc, acc0 || tap > 0);
+                  }
+                }
+              } else {
+#pragma unroll
+                for (int tap = 0; tap < 9; ++tap) {
+                  const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+#pragma unroll
+                  for (int c = 0; c < 4; ++c) {
+                    // parity plane (qy, qx), shifts oy + qy, ox + qx of it
+                    const int Y = (c >> 1) + dy, X = (c & 1) + dx, qy = Y & 1, qx = X & 1;
+                    const int oy = (Y - qy) / 2, ox = (X - qx) / 2;
+                    const uint32_t off = (2 * qy + qx) * up1k(plane_bytes(KC)) + ((oy + qy) * kPW + ox + qx) * RB;
+                    tc::mma_bf16(d + c * a.NT, ad + (uint64_t)(off >> 4), bd + 2 * ks + (uint64_t)tap * tap16, idesc,
+                                 acc0 || tap > 0);
+                  }
+                }
+              }
+            }
+            tc::mma_commit(&empty[st]);
+            if (s == a.nslab - 1) tc::mma_commit(&bars.accf[buf]);
+          }
+          __syncwarp();
+          // refill the previous unit's stage (pst) once its MMAs are done:
+          // this unit's are queued behind them
+          if (both && (k > 0 || s > 0) && issued < units) {
+            ok = warp_wait(&empty[pst], eph);
+            if (ok) copy();
+            if (++pst == a.S) {
+              pst = 0;
+              eph ^= 1u;
+            }
+          }
           if (++st == a.S) {
             st = 0;
             ph ^= 1u;
@@ -464,7 +499,7 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
       if (!ok) {
         // a wait ran out: wait (bounded) for the copies issued last on each
         // stage, so that none lands after the CTA has left
-        for (int u = max(0, issued - a.S); u < issued; ++u) tc::mbar_wait(&bars.full[u % a.S], (uint32_t)(u / a.S) & 1u);
+        for (int u = max(0, issued - a.S); u < issued; ++u) tc::mbar_wait(&full[u % a.S], (uint32_t)(u / a.S) & 1u);
       }
     }
   } else {
@@ -472,14 +507,14 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
     // each tile's four accumulators.  A group must not be given a buffer
     // whose previous phase it cannot know to be complete, so there are no
     // more groups on alternate tiles than buffers.
-    const int g = (warp - 2) >> 2, groups = kUp ? 1 : min(kEpiWarps / 4, a.nbuf), g0 = kUp ? 0 : g;
+    const int g = (warp - kService) >> 2, groups = kUp ? 1 : min(kEpiWarps / 4, a.nbuf), g0 = kUp ? 0 : g;
     if (g0 < groups) {
       TileIter it(a, (int)(blockIdx.x + g0 * gridDim.x), groups * (int)gridDim.x);
       for (int i = g0; i < n_tiles && ok; i += groups, it.next(a)) {
         const Tile t = it.tile(kTH);
         const int buf = i % a.nbuf, lap = i / a.nbuf;
         ok = tile_epilogue<kUp, kDg>(
-            a, t, tmem + buf * NA * a.NT, kUp ? g : 0, kUp ? g + 1 : MT, warp, lane, xch[kDg ? warp - 2 : 0], bias,
+            a, t, tmem + buf * NA * a.NT, kUp ? g : 0, kUp ? g + 1 : MT, warp, lane, xch[kDg ? warp - kService : 0], bias,
             [&] {
               const bool w = warp_wait(&bars.accf[buf], (uint32_t)lap & 1u);
               tc::fence_after();
@@ -801,6 +836,11 @@ static bool plan_wide(TileArgs a, const Src& x1, const Src& x2, const bf16* w, i
   if (a.S < 2) return false;
   const int NA = up ? 4 : MT;
   a.nbuf = std::min(kMaxBuf, 512 / (NA * a.NT));
+  // service warps: each needs two stages and its own accumulator buffers
+  const int S = a.S;
+  a.R = up ? 1 : (S >= 8 && a.nbuf >= 4 ? 4 : (S >= 4 && a.nbuf >= 2 ? 2 : 1));
+  a.nbuf -= a.nbuf % a.R;
+  a.S = S / a.R;
   if (!up && a.nbuf < 2) return false;
   a.ncols = pow2_cols(a.nbuf * NA * a.NT);
   const int th = up ? 32 : 16 * MT, tw = up ? 16 : 8;
@@ -822,7 +862,7 @@ static bool plan_wide(TileArgs a, const Src& x1, const Src& x2, const bf16* w, i
     if (x2.ptr && !pixel_map(&m.s2[0], x2.ptr, imgs, a.H, a.W, x2.C, 1, 1, KC, kHW, 16 * MT + 2)) return false;
   }
   // past half the SM's shared memory: one CTA per SM (TMEM columns)
-  const size_t smem = std::max<size_t>((size_t)a.S * a.stage + (res ? res_bytes : 0), 116 * 1024);
+  const size_t smem = std::max<size_t>((size_t)a.R * a.S * a.stage + (res ? res_bytes : 0), 116 * 1024);
   if constexpr (!kDg) {
     if (up) {
       *e = res ? launch_tile<KC, 1, true, true, false>(a, m, smem, st)
