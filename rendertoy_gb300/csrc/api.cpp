@@ -2034,9 +2034,8 @@ int rtx_dn_infer(rtx_context* c, const float* input, float* out, int N, int H, i
   if ((r = bind_in(c, input, P * 4 * rtx::nn::kRawCh, 0, ai))) return r;
   if ((r = bind_out(c, out, P * 12, 1, ao))) return r;
   RTX_CUDA(c->dn->reserve((long long)P), "denoiser buffers");
-  cudaError_t e = c->dn->forward((const float*)ai.dev, N, H, W, c->d_err, c->stream);
-  if (e == cudaSuccess) e = c->dn->decode((const float*)ai.dev, (float*)ao.dev, N, H, W, H, W, c->stream);
-  c->stats.kernel_launches = c->dn->last_launches() + 1;
+  cudaError_t e = c->dn->infer((const float*)ai.dev, (float*)ao.dev, N, H, W, c->d_err, c->stream);
+  c->stats.kernel_launches = c->dn->last_launches();
   if (e != cudaSuccess) return cuda_fail(c, e, "denoiser inference");
   if ((r = copy_back(c, ao))) return r;
   return finish(c, all_device({&ai, &ao}));
@@ -2058,14 +2057,18 @@ int rtx_denoise(rtx_context* c, const float* radiance, const float* albedo, cons
   if ((r = bind_in(c, normal, bytes, 2, an))) return r;
   if ((r = bind_in(c, depth, bytes, 3, ad))) return r;
   if ((r = bind_out(c, out, bytes, 4, ao))) return r;
-  RTX_CUDA(c->stage[5].ensure((size_t)Wp * Hp * 4 * rtx::nn::kRawCh), "stage alloc");
   RTX_CUDA(c->dn->reserve((long long)Wp * Hp), "denoiser buffers");
-  float* raw = (float*)c->stage[5].p;
-  cudaError_t e = rtx::nn::pack_passes((const float*)ar.dev, (const float*)aa.dev, (const float*)an.dev,
-                                       (const float*)ad.dev, (float)spp, raw, W, H, Wp, Hp, c->stream);
-  if (e == cudaSuccess) e = c->dn->forward(raw, 1, Hp, Wp, c->d_err, c->stream);
-  if (e == cudaSuccess) e = c->dn->decode(raw, (float*)ao.dev, 1, H, W, Hp, Wp, c->stream);
-  c->stats.kernel_launches = c->dn->last_launches() + 2;
+  // the filters read the radiance while the output is written: an output that
+  // overlaps it reads a copy
+  const float* rad = (const float*)ar.dev;
+  if ((char*)ao.dev < (char*)ar.dev + bytes && (char*)ar.dev < (char*)ao.dev + bytes) {
+    RTX_CUDA(c->stage[5].ensure(bytes), "stage alloc");
+    RTX_CUDA(cudaMemcpyAsync(c->stage[5].p, rad, bytes, cudaMemcpyDeviceToDevice, c->stream), "copy");
+    rad = (const float*)c->stage[5].p;
+  }
+  cudaError_t e = c->dn->denoise(rad, (const float*)aa.dev, (const float*)an.dev,
+                                 (const float*)ad.dev, (float)spp, (float*)ao.dev, W, H, c->d_err, c->stream);
+  c->stats.kernel_launches = c->dn->last_launches();
   if (e != cudaSuccess) return cuda_fail(c, e, "denoise");
   if ((r = copy_back(c, ao))) return r;
   return finish(c, all_device({&ar, &aa, &an, &ad, &ao}));

@@ -53,6 +53,19 @@ struct ConvFwd {
   int* err;
 };
 
+// The kernel-predicting output layer together with what its logits are for:
+// the filtered radiance (out), or the loss and its gradient (dpred, loss).
+struct KpHead {
+  const float* rad;     // radiance of frames stored Hs x Ws, rad_px floats per pixel (RGB first)
+  int rad_px, Hs, Ws;
+  int Hc, Wc;           // frame the taps are clamped to (out: [N][Hc][Wc][3])
+  float* out;
+  const float* target;  // [N][H][W][3]; H = Hc, W = Wc
+  bf16* dpred;          // [P][kPredCh]
+  double* loss;         // += the summed loss
+  float inv;            // 1 / (3 P)
+};
+
 struct ConvDgrad {
   const bf16* dout;  // [P][Cout]
   int Cout;
@@ -79,6 +92,9 @@ struct ConvWgrad {
 };
 
 cudaError_t conv_fwd(const ConvFwd& a, cudaStream_t st);
+// The output layer with its head in one launch; false: not a shape it takes
+// (rows of at least 64 pixels), nothing launched.
+bool conv_head(const ConvFwd& a, const KpHead& h, cudaStream_t st, cudaError_t* e);
 cudaError_t conv_dgrad(const ConvDgrad& a, cudaStream_t st);
 // whether conv_dgrad can write an upsampled + skip concatenation's gradient
 // straight to its two sources (dlow, dskip)

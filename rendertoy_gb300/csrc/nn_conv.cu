@@ -775,6 +775,10 @@ cudaError_t conv_fwd(const ConvFwd& a, cudaStream_t st) {
                        stage, a, st);
 }
 
+bool conv_head(const ConvFwd& a, const KpHead& h, cudaStream_t st, cudaError_t* e) {
+  return use_rows(a.W, a.Cin) && conv_tile_head(a, h, st, e);
+}
+
 bool conv_dgrad_splits(const ConvDgrad& a) {
   return conv_tile_takes_dgrad(a, use_rows(a.W, a.Cout)) && a.s1.up && a.s2.ptr && a.s1.C % 16 == 0 &&
          a.H % 2 == 0 && a.W % 2 == 0;

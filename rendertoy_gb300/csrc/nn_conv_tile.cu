@@ -88,6 +88,7 @@ struct TileArgs {
   Src s1, s2;
   int mask_relu;
   bf16 *din, *dlow, *dskip;
+  KpHead head;              // the output layer with its filter (kHead != 0)
   int* err;
   // narrow form
   int G, nhalo;             // slabs per weight unit, halo buffers
@@ -239,6 +240,132 @@ __device__ __forceinline__ void store_dgrad(const TileArgs& a, float* v, const u
   }
 }
 
+// The output layer's epilogue: the tile's logits become filters in registers
+// (a lane's 32 columns are its pixel's), so neither the FP32 logits nor a
+// second pass over them exists.  kHead 1 filters the radiance, 2 computes the
+// loss and its gradient.  `rad`: the group's 12 x 20 radiance halo (clamped to
+// the frame, made safe), rows kRadRow apart.  Operations and order as the
+// separate kernels (k_kp_apply, k_kp_loss).
+constexpr int kRadRow = 13, kRadTile = 20 * kRadRow * 3;
+constexpr int kHeadGroups = kEpiWarps / 4;
+
+template <int kHead>
+__device__ __forceinline__ void head_pixel(const TileArgs& a, float* l, const float* rad, int mx, int my, const float* tgt,
+                                           size_t p, size_t pc, bool ok, float& part) {
+  float m = l[0];
+#pragma unroll
+  for (int k = 1; k < kKpTaps; ++k) m = fmaxf(m, l[k]);
+  float s = 0.0f;
+#pragma unroll
+  for (int k = 0; k < kKpTaps; ++k) {
+    l[k] = expf(l[k] - m);
+    s += l[k];
+  }
+  const float inv_s = 1.0f / s;
+  float o[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+  for (int k = 0; k < kKpTaps; ++k) {
+    l[k] *= inv_s;
+    const float* c = rad + ((my + k / kKpWidth) * kRadRow + mx + k % kKpWidth) * 3;
+    o[0] += l[k] * c[0];
+    o[1] += l[k] * c[1];
+    o[2] += l[k] * c[2];
+  }
+  if constexpr (kHead == 1) {
+    if (ok) {
+      float* d = a.head.out + 3 * pc;
+      d[0] = o[0];
+      d[1] = o[1];
+      d[2] = o[2];
+    }
+  } else {
+    float g[3], e = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const float d = o[i] - fminf(fmaxf(tgt[i], 0.0f), 65504.0f);
+      const float den = o[i] * o[i] + kRelEps;
+      e += d * d / den;
+      g[i] = 2.0f * d / den * a.head.inv;
+    }
+    if (ok) part += e;
+    // dw_k = sum_c g_c r_c(tap k), formed twice (held, 25 registers spill)
+    auto dw = [&](int k) {
+      const float* c = rad + ((my + k / kKpWidth) * kRadRow + mx + k % kKpWidth) * 3;
+      return g[0] * c[0] + g[1] * c[1] + g[2] * c[2];
+    };
+    float t = 0.0f;
+#pragma unroll
+    for (int k = 0; k < kKpTaps; ++k) t += l[k] * dw(k);
+    if (ok) {
+      uint32_t u[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k)
+        u[k] = pack2(2 * k < kKpTaps ? l[2 * k] * (dw(2 * k) - t) : 0.0f,
+                     2 * k + 1 < kKpTaps ? l[2 * k + 1] * (dw(2 * k + 1) - t) : 0.0f);
+      bf16* d = a.head.dpred + p * kPredCh;
+      const bool wide = (reinterpret_cast<uintptr_t>(a.head.dpred) & 31) == 0;
+      st32(d, u, wide);
+      st32(d + 16, u + 8, wide);
+    }
+  }
+}
+
+template <int kHead, class Wait, class Release>
+__device__ __forceinline__ bool head_epilogue(const TileArgs& a, const Tile& t, uint32_t tmem, int warp, int lane,
+                                              float* rad, const float* bias, double& loss, Wait&& wait,
+                                              Release&& release) {
+  const int q = warp & 3, tid = ((warp - kService) & 3) * 32 + lane, g = (warp - kService) >> 2;
+  const int m = q * 32 + lane, mx = m & 7, my = m >> 3;
+  const KpHead& h = a.head;
+  // this thread's share of the radiance halo, and its target, before the wait
+  float r[2][3], tgt[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int i = tid + 128 * j, yy = i / 12, xx = i - 12 * yy;
+    if (i < 240) {
+      const int y = min(max(t.y0 + yy - 2, 0), h.Hc - 1), x = min(max(t.x0 + xx - 2, 0), h.Wc - 1);
+      const float* s = h.rad + (size_t)h.rad_px * (((size_t)t.n * h.Hs + y) * h.Ws + x);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) r[j][k] = fminf(fmaxf(__ldg(s + k), 0.0f), 65504.0f);
+    }
+  }
+  const int x = t.x0 + mx, y = t.y0 + my;
+  const bool ok = x < h.Wc && y < h.Hc;
+  const size_t p = ((size_t)t.n * a.H + y) * a.W + x, pc = ((size_t)t.n * h.Hc + y) * h.Wc + x;
+  if (kHead == 2 && ok) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) tgt[k] = __ldg(h.target + 3 * p + k);
+  }
+  asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");  // the previous tile's taps are read
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int i = tid + 128 * j, yy = i / 12, xx = i - 12 * yy;
+    if (i < 240)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) rad[(yy * kRadRow + xx) * 3 + k] = r[j][k];
+  }
+  asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");
+  const bool w = wait();
+  float v[32];
+  tmem_ld32(tmem + ((uint32_t)(q * 32) << 16), v);
+  release();
+#pragma unroll
+  for (int k = 0; k < 28; k += 4) {
+    const float4 b4 = *reinterpret_cast<const float4*>(bias + k);
+    v[k] += b4.x;
+    v[k + 1] += b4.y;
+    v[k + 2] += b4.z;
+    v[k + 3] += b4.w;
+  }
+  float part = 0.0f;
+  head_pixel<kHead>(a, v, rad, mx, my, tgt, p, pc, ok, part);
+  if constexpr (kHead == 2) {
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
+    loss += (double)part;
+  }
+  return w;
+}
+
 // The epilogue of accumulators [acc0, acc1) of a tile for one warp (its 32
 // lanes, every column).  `wait` blocks until the accumulators are complete;
 // a data gradient's first mask loads are issued before it.  `release` runs
@@ -337,7 +464,7 @@ __device__ __forceinline__ void bars_init(Bars& b, int S, int readers) {
   }
 }
 
-template <int KC, int MT, bool kUp, bool kRes, bool kDg>
+template <int KC, int MT, bool kUp, bool kRes, bool kDg, int kHead = 0>
 __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, const __grid_constant__ TileMaps tm) {
   constexpr int NA = kUp ? 4 : MT;
   constexpr int RB = KC * 2;  // bytes of a pixel row
@@ -347,6 +474,7 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
   __shared__ uint32_t tmem_slot;
   __shared__ uint4 xch[kDg ? kEpiWarps : 1][32][2];
   __shared__ __align__(16) float bias[kDg ? 4 : 256];
+  __shared__ float rad[kHead ? kHeadGroups : 1][kHead ? kRadTile : 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tiles = (int)blockIdx.x < a.n_tiles ? (a.n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   if (warp == 0) tc::tmem_alloc(&tmem_slot, a.ncols);
@@ -508,23 +636,29 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
     // whose previous phase it cannot know to be complete, so there are no
     // more groups on alternate tiles than buffers.
     const int g = (warp - kService) >> 2, groups = kUp ? 1 : min(kEpiWarps / 4, a.nbuf), g0 = kUp ? 0 : g;
+    double loss = 0.0;
     if (g0 < groups) {
       TileIter it(a, (int)(blockIdx.x + g0 * gridDim.x), groups * (int)gridDim.x);
       for (int i = g0; i < n_tiles && ok; i += groups, it.next(a)) {
         const Tile t = it.tile(kTH);
         const int buf = i % a.nbuf, lap = i / a.nbuf;
-        ok = tile_epilogue<kUp, kDg>(
-            a, t, tmem + buf * NA * a.NT, kUp ? g : 0, kUp ? g + 1 : MT, warp, lane, xch[kDg ? warp - kService : 0], bias,
-            [&] {
-              const bool w = warp_wait(&bars.accf[buf], (uint32_t)lap & 1u);
-              tc::fence_after();
-              return w;
-            },
-            [&] {
-              tc::fence_before();
-              tc::mbar_arrive(&bars.acce[buf]);
-            });
+        auto wait = [&] {
+          const bool w = warp_wait(&bars.accf[buf], (uint32_t)lap & 1u);
+          tc::fence_after();
+          return w;
+        };
+        auto release = [&] {
+          tc::fence_before();
+          tc::mbar_arrive(&bars.acce[buf]);
+        };
+        const uint32_t acc = tmem + buf * NA * a.NT;
+        if constexpr (kHead)
+          ok = head_epilogue<kHead>(a, t, acc, warp, lane, rad[g], bias, loss, wait, release);
+        else
+          ok = tile_epilogue<kUp, kDg>(a, t, acc, kUp ? g : 0, kUp ? g + 1 : MT, warp, lane,
+                                       xch[kDg ? warp - kService : 0], bias, wait, release);
       }
+      if (kHead == 2 && lane == 0) atomicAdd(a.head.loss, loss);
     }
   }
   if (!__syncthreads_and(ok) && lane == 0) atomicOr(a.err, tc::kErrMbarTimeout);
@@ -787,9 +921,9 @@ static uint32_t pow2_cols(uint32_t c) {
 
 constexpr uint32_t kSmem = 208 * 1024;  // dynamic shared memory a CTA may plan with
 
-template <int KC, int MT, bool kUp, bool kRes, bool kDg>
+template <int KC, int MT, bool kUp, bool kRes, bool kDg, int kHead = 0>
 static cudaError_t launch_tile(const TileArgs& a, const TileMaps& m, size_t smem, cudaStream_t st) {
-  auto k = k_conv_tile<KC, MT, kUp, kRes, kDg>;
+  auto k = k_conv_tile<KC, MT, kUp, kRes, kDg, kHead>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e) return e;
   k<<<std::min(a.n_tiles, tile_sm_count()), kThreadsT, smem, st>>>(a, m);
@@ -798,7 +932,7 @@ static cudaError_t launch_tile(const TileArgs& a, const TileMaps& m, size_t smem
 
 // The wide (slab-major) form.  kDg: the data gradient (taps mirrored, single
 // source dout).  False: not a shape (or alignment) it takes.
-template <int KC, bool kDg>
+template <int KC, bool kDg, int kHead = 0>
 static bool plan_wide(TileArgs a, const Src& x1, const Src& x2, const bf16* w, int imgs, cudaStream_t st,
                       cudaError_t* e) {
   const bool up = !kDg && x1.up;
@@ -863,6 +997,11 @@ static bool plan_wide(TileArgs a, const Src& x1, const Src& x2, const bf16* w, i
   }
   // past half the SM's shared memory: one CTA per SM (TMEM columns)
   const size_t smem = std::max<size_t>((size_t)a.R * a.S * a.stage + (res ? res_bytes : 0), 116 * 1024);
+  if constexpr (kHead) {
+    if (up || !res || a.ntn != 1 || a.NT != kPredCh) return false;
+    *e = launch_tile<KC, 1, false, true, false, kHead>(a, m, smem, st);
+    return true;
+  }
   if constexpr (!kDg) {
     if (up) {
       *e = res ? launch_tile<KC, 1, true, true, false>(a, m, smem, st)
@@ -947,6 +1086,21 @@ bool conv_tile_fwd(const ConvFwd& c, bool wide, cudaStream_t st, cudaError_t* e)
                        : plan_narrow<16, false>(a, c.s1, s2, c.w, c.N, st, e);
   return g % 32 == 0 ? plan_wide<32, false>(a, c.s1, s2, c.w, c.N, st, e)
                      : plan_wide<16, false>(a, c.s1, s2, c.w, c.N, st, e);
+}
+
+bool conv_tile_head(const ConvFwd& c, const KpHead& h, cudaStream_t st, cudaError_t* e) {
+  if (c.s1.up || c.s2.ptr || c.s1.C % 32 || c.Cout != kPredCh || !c.bias || c.relu) return false;
+  if (h.dpred && (reinterpret_cast<uintptr_t>(h.dpred) & 15)) return false;
+  TileArgs a{};
+  a.H = c.H;
+  a.W = c.W;
+  a.Nout = c.Cout;
+  a.bias = c.bias;
+  a.head = h;
+  a.err = c.err;
+  const Src none{nullptr, 0, 0};
+  return h.out ? plan_wide<32, false, 1>(a, c.s1, none, c.w, c.N, st, e)
+               : plan_wide<32, false, 2>(a, c.s1, none, c.w, c.N, st, e);
 }
 
 bool conv_tile_takes_dgrad(const ConvDgrad& c, bool wide) {

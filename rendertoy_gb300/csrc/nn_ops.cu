@@ -40,8 +40,9 @@ unsigned blocks(long long n, int t = 256) { return (unsigned)((n + t - 1) / t); 
 __device__ __forceinline__ float sane(float v) { return fminf(fmaxf(v, 0.0f), 65504.0f); }
 
 // Pixel (n, y, x) of frames of Hs x Ws stored pixels, RGB of its raw record
+template <int kPx = kRawCh>
 __device__ __forceinline__ void raw_rgb(const float* raw, long long pix, float* c) {
-  const float* r = raw + (long long)kRawCh * pix;
+  const float* r = raw + (long long)kPx * pix;
   c[0] = sane(r[0]);
   c[1] = sane(r[1]);
   c[2] = sane(r[2]);
@@ -87,21 +88,55 @@ __device__ __forceinline__ long long kp_tap(long long frame0, int x, int y, int 
 
 }  // namespace
 
-// raw [P][kRawCh] -> [P][16] BF16: radiance as log(1 + x), albedo, normal and
-// depth as they are, the samples per pixel as log2(spp) / 16, channels
-// 11..15 zero
+// One pixel's encoded input: radiance as log(1 + x), albedo, normal and depth
+// as they are, the samples per pixel as log2(spp) / 16, channels 11..15 zero
+__device__ __forceinline__ void encode_px(const float* r, bf16* x) {
+  float f[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) f[i] = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) f[i] = log1pf(sane(r[i]));
+#pragma unroll
+  for (int i = 3; i < 10; ++i) f[i] = r[i];
+  f[10] = log2f(fmaxf(r[10], 1.0f)) * (1.0f / 16.0f);
+  st8(x, f);
+  st8(x + 8, f + 8);
+}
+
+// raw [P][kRawCh] -> [P][16] BF16
 __global__ void k_encode_input(const float* __restrict__ raw, bf16* __restrict__ x, long long P) {
   long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= P) return;
   const float* r = raw + (long long)kRawCh * p;
-  float f[16];
+  float f[kRawCh];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) f[i] = 0.0f;
-  for (int i = 0; i < 3; ++i) f[i] = log1pf(sane(r[i]));
-  for (int i = 3; i < 10; ++i) f[i] = r[i];
-  f[10] = log2f(fmaxf(r[10], 1.0f)) * (1.0f / 16.0f);
-  st8(x + 16 * p, f);
-  st8(x + 16 * p + 8, f + 8);
+  for (int i = 0; i < kRawCh; ++i) f[i] = r[i];
+  encode_px(f, x + 16 * p);
+}
+
+// The same from the renderer's passes, without the 44-byte records in between
+// (1920 x 1080: 87 us of packing and 25 of encoding -> XX us; its 168 MB take
+// 25 us).
+__global__ void k_encode_passes(const float* __restrict__ rad, const float* __restrict__ alb,
+                                const float* __restrict__ nrm, const float* __restrict__ dep, float spp,
+                                bf16* __restrict__ x, int W, int H, int Wp) {
+  const int px = blockIdx.x * blockDim.x + threadIdx.x, py = blockIdx.y;
+  if (px >= Wp) return;
+  float f[kRawCh];
+#pragma unroll
+  for (int k = 0; k < kRawCh; ++k) f[k] = 0.0f;
+  if (px < W && py < H) {
+    const long long s = ((long long)py * W + px) * 3;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      f[k] = __ldg(rad + s + k);
+      f[3 + k] = __ldg(alb + s + k);
+      f[6 + k] = __ldg(nrm + s + k);
+    }
+    f[9] = __ldg(dep + s);
+    f[10] = spp;
+  }
+  encode_px(f, x + 16 * ((long long)py * Wp + px));
 }
 
 __global__ void k_avgpool(const bf16* __restrict__ in, bf16* __restrict__ out, int N, int H, int W, int C) {
@@ -359,23 +394,26 @@ __global__ void k_weights_bf16_all(WeightLayouts j) {
 // The denoised radiance: the predicted filter applied to the input radiance,
 // for N frames of Hc x Wc pixels stored as Hs x Ws (the frame is the top-left
 // corner; taps are clamped to it); out [N][Hc][Wc][3].
+// kPx: floats per pixel of `raw` (a record, or the radiance pass itself, whose
+// rows are Wr pixels while pred's are Ws).
+template <int kPx>
 __global__ void k_kp_apply(const float* __restrict__ pred, const float* __restrict__ raw, float* __restrict__ out,
-                           int N, int Hc, int Wc, int Hs, int Ws) {
+                           int N, int Hc, int Wc, int Hs, int Ws, int Hr, int Wr) {
   const long long P = (long long)N * Hc * Wc;
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= P) return;
   const int x = (int)(i % Wc);
   const long long q = i / Wc;
   const int y = (int)(q % Hc);
-  const long long frame0 = (q / Hc) * (long long)Hs * Ws;
-  const long long p = frame0 + (long long)y * Ws + x;
+  const long long n = q / Hc, frame0 = n * Hr * Wr;
+  const long long p = n * Hs * Ws + (long long)y * Ws + x;
   float w[kKpTaps];
   kp_weights(pred + (long long)kPredCh * p, w);
   float o[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
   for (int k = 0; k < kKpTaps; ++k) {
     float c[3];
-    raw_rgb(raw, kp_tap(frame0, x, y, k, Wc, Hc, Ws), c);
+    raw_rgb<kPx>(raw, kp_tap(frame0, x, y, k, Wc, Hc, Wr), c);
     o[0] += w[k] * c[0];
     o[1] += w[k] * c[1];
     o[2] += w[k] * c[2];
@@ -385,30 +423,6 @@ __global__ void k_kp_apply(const float* __restrict__ pred, const float* __restri
   out[3 * i + 2] = o[2];
 }
 
-// the renderer's passes (W x H RGB FP32 each) + their samples per pixel ->
-// raw [Hp][Wp][kRawCh], zero outside the W x H frame
-__global__ void k_pack_passes(const float* __restrict__ rad, const float* __restrict__ alb,
-                              const float* __restrict__ nrm, const float* __restrict__ dep, float spp,
-                              float* __restrict__ raw, int W, int H, int Wp, int Hp) {
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= (long long)Wp * Hp) return;
-  int x = (int)(i % Wp), y = (int)(i / Wp);
-  float* r = raw + (long long)kRawCh * i;
-  if (x >= W || y >= H) {
-    for (int k = 0; k < kRawCh; ++k) r[k] = 0.0f;
-    return;
-  }
-  long long s = ((long long)y * W + x) * 3;
-  for (int k = 0; k < 3; ++k) {
-    r[k] = rad[s + k];
-    r[3 + k] = alb[s + k];
-    r[6 + k] = nrm[s + k];
-  }
-  r[9] = dep[s];
-  r[10] = spp;
-}
-
-// prediction [Hp][Wp][16] (log space) -> radiance W x H RGB
 // ---- launchers ------------------------------------------------------------
 cudaError_t encode_input(const float* raw, bf16* x, long long P, cudaStream_t st) {
   k_encode_input<<<blocks(P), 256, 0, st>>>(raw, x, P);
@@ -482,13 +496,24 @@ cudaError_t weights_bf16_all(const WeightLayouts& j, cudaStream_t st) {
 }
 cudaError_t kp_apply(const float* pred, const float* raw, float* out, int N, int Hc, int Wc, int Hs, int Ws,
                      cudaStream_t st) {
-  k_kp_apply<<<blocks((long long)N * Hc * Wc), 256, 0, st>>>(pred, raw, out, N, Hc, Wc, Hs, Ws);
+  k_kp_apply<kRawCh><<<blocks((long long)N * Hc * Wc), 256, 0, st>>>(pred, raw, out, N, Hc, Wc, Hs, Ws, Hs, Ws);
   return cudaGetLastError();
 }
 
-cudaError_t pack_passes(const float* rad, const float* alb, const float* nrm, const float* dep, float spp,
-                        float* raw, int W, int H, int Wp, int Hp, cudaStream_t st) {
-  k_pack_passes<<<blocks((long long)Wp * Hp), 256, 0, st>>>(rad, alb, nrm, dep, spp, raw, W, H, Wp, Hp);
+cudaError_t kp_apply_passes(const float* pred, const float* rad, float* out, int W, int H, int Wp, cudaStream_t st) {
+  k_kp_apply<3><<<blocks((long long)W * H), 256, 0, st>>>(pred, rad, out, 1, H, W, H, Wp, H, W);
+  return cudaGetLastError();
+}
+
+cudaError_t encode_passes(const float* rad, const float* alb, const float* nrm, const float* dep, float spp, bf16* x,
+                          int W, int H, int Wp, int Hp, cudaStream_t st) {
+  // grid.y is at most 65,535 rows: taller frames in slices
+  for (int y0 = 0; y0 < Hp; y0 += 65535) {
+    const int rows = std::min(65535, Hp - y0);
+    const long long o = 3LL * W * y0;
+    k_encode_passes<<<dim3((Wp + 127) / 128, rows), 128, 0, st>>>(rad + o, alb + o, nrm + o, dep + o, spp,
+                                                                 x + 16LL * Wp * y0, W, H - y0, Wp);
+  }
   return cudaGetLastError();
 }
 

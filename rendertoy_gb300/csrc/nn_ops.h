@@ -46,8 +46,13 @@ cudaError_t weights_bf16_all(const WeightLayouts& layers, cudaStream_t st);
 // frames stored as Hs x Ws pixels (pred and raw share that layout)
 cudaError_t kp_apply(const float* pred, const float* raw, float* out, int N, int Hc, int Wc, int Hs, int Ws,
                      cudaStream_t st);
-cudaError_t pack_passes(const float* rad, const float* alb, const float* nrm, const float* dep, float spp,
-                        float* raw, int W, int H, int Wp, int Hp, cudaStream_t st);
+// the same for one W x H frame given as its radiance pass; pred rows are Wp
+// pixels apart
+cudaError_t kp_apply_passes(const float* pred, const float* rad, float* out, int W, int H, int Wp, cudaStream_t st);
+// the renderer's passes (W x H RGB FP32 each) and their samples per pixel ->
+// the encoded input [Hp][Wp][16], that of a zero record outside the frame
+cudaError_t encode_passes(const float* rad, const float* alb, const float* nrm, const float* dep, float spp, bf16* x,
+                          int W, int H, int Wp, int Hp, cudaStream_t st);
 
 }  // namespace nn
 }  // namespace rtx

@@ -81,8 +81,6 @@ struct UNet::Impl {
   bf16* dcat = nullptr;
   float* pred = nullptr;     // filter logits [P][kPredCh]
   bf16* dpred = nullptr;
-  float* raw = nullptr;     // staged input [P][kRawCh]
-  float* target = nullptr;  // staged target [P][3]
   double* loss = nullptr;
 
   ~Impl() { release(); }
@@ -93,14 +91,12 @@ struct UNet::Impl {
       if (dact[t]) cudaFree(dact[t]);
       act[t] = dact[t] = nullptr;
     }
-    void* ps[] = {dcat, pred, dpred, raw, target};
+    void* ps[] = {dcat, pred, dpred};
     for (void* p : ps)
       if (p) cudaFree(p);
     dcat = nullptr;
     pred = nullptr;
     dpred = nullptr;
-    raw = nullptr;
-    target = nullptr;
     cap = 0;
   }
   void release() {
@@ -127,8 +123,6 @@ struct UNet::Impl {
     if ((e = cudaMalloc(&dcat, ncat * sizeof(bf16)))) return e;
     if ((e = cudaMalloc(&pred, (size_t)P0 * kPredCh * sizeof(float)))) return e;
     if ((e = cudaMalloc(&dpred, (size_t)P0 * kPredCh * sizeof(bf16)))) return e;
-    if ((e = cudaMalloc(&raw, (size_t)P0 * kRawCh * sizeof(float)))) return e;
-    if ((e = cudaMalloc(&target, (size_t)P0 * 3 * sizeof(float)))) return e;
     cap = P0;
     return cudaSuccess;
   }
@@ -245,14 +239,18 @@ cudaError_t UNet::set_state(const float* host_m, const float* host_v, int step, 
   return cudaMemcpyAsync(p_->v, host_v, p_->n_params * 4, cudaMemcpyHostToDevice, st);
 }
 
-cudaError_t UNet::forward(const float* d_raw, int N, int H, int W, int* err, cudaStream_t st) {
+cudaError_t UNet::forward(const float* d_raw, int N, int H, int W, int* err, cudaStream_t st, const KpHead* head,
+                          bool* fused) {
   Impl& I = *p_;
   long long P0 = (long long)N * H * W;
   cudaError_t e;
   if ((e = I.ensure(P0))) return e;
   I.launches = 0;
-  if ((e = encode_input(d_raw, I.act[tX], P0, st))) return e;
-  ++I.launches;
+  if (d_raw) {
+    if ((e = encode_input(d_raw, I.act[tX], P0, st))) return e;
+    ++I.launches;
+  }
+  if (fused) *fused = false;
   for (int i = 0; i < kNumLayers; ++i) {
     const Impl::Layer& l = I.L[i];
     int lev = kTL[l.d.out >= 0 ? l.d.out : tU0];
@@ -276,8 +274,12 @@ cudaError_t UNet::forward(const float* d_raw, int N, int H, int W, int* err, cud
     c.out = l.d.out >= 0 ? I.act[l.d.out] : nullptr;
     c.out_f32 = l.d.out >= 0 ? nullptr : I.pred;
     c.err = err;
-    if ((e = conv_fwd(c, st))) return e;
     ++I.launches;
+    if (i == kNumLayers - 1 && head && conv_head(c, *head, st, &e)) {
+      *fused = true;
+      return e;
+    }
+    if ((e = conv_fwd(c, st))) return e;
   }
   return cudaSuccess;
 }
@@ -365,20 +367,77 @@ cudaError_t UNet::backward(int N, int H, int W, int* err, cudaStream_t st) {
   return cudaSuccess;
 }
 
+// forward + the loss of the filtered radiance and its gradient to the logits
+cudaError_t UNet::loss_pass(const float* d_raw, const float* d_target, int N, int H, int W, int* err, cudaStream_t st) {
+  Impl& I = *p_;
+  cudaError_t e;
+  if ((e = I.ensure((long long)N * H * W))) return e;
+  if ((e = cudaMemsetAsync(I.loss, 0, sizeof(double), st))) return e;
+  KpHead h{};
+  h.rad = d_raw;
+  h.rad_px = kRawCh;
+  h.Hs = h.Hc = H;
+  h.Ws = h.Wc = W;
+  h.target = d_target;
+  h.dpred = I.dpred;
+  h.loss = I.loss;
+  h.inv = 1.0f / (3.0f * (float)((long long)N * H * W));
+  bool fused = false;
+  if ((e = forward(d_raw, N, H, W, err, st, &h, &fused)) || fused) return e;
+  ++I.launches;
+  return kp_loss(I.pred, d_raw, d_target, I.dpred, N, H, W, I.loss, st);
+}
+
+cudaError_t UNet::infer(const float* d_raw, float* d_out, int N, int H, int W, int* err, cudaStream_t st) {
+  Impl& I = *p_;
+  KpHead h{};
+  h.rad = d_raw;
+  h.rad_px = kRawCh;
+  h.Hs = h.Hc = H;
+  h.Ws = h.Wc = W;
+  h.out = d_out;
+  bool fused = false;
+  cudaError_t e;
+  if ((e = forward(d_raw, N, H, W, err, st, &h, &fused)) || fused) return e;
+  ++I.launches;
+  return kp_apply(I.pred, d_raw, d_out, N, H, W, H, W, st);
+}
+
+cudaError_t UNet::denoise(const float* rad, const float* alb, const float* nrm, const float* dep, float spp,
+                          float* d_out, int W, int H, int* err, cudaStream_t st) {
+  Impl& I = *p_;
+  const int Wp = (W + 15) / 16 * 16, Hp = (H + 15) / 16 * 16;
+  cudaError_t e;
+  if ((e = I.ensure((long long)Wp * Hp))) return e;
+  // the encoded input straight from the passes; the filters' taps come from
+  // the radiance pass itself
+  if ((e = encode_passes(rad, alb, nrm, dep, spp, I.act[tX], W, H, Wp, Hp, st))) return e;
+  KpHead h{};
+  h.rad = rad;
+  h.rad_px = 3;
+  h.Hs = h.Hc = H;
+  h.Ws = h.Wc = W;
+  h.out = d_out;
+  bool fused = false;
+  if ((e = forward(nullptr, 1, Hp, Wp, err, st, &h, &fused))) return e;
+  ++I.launches;
+  if (fused) return cudaSuccess;
+  ++I.launches;
+  return kp_apply_passes(I.pred, rad, d_out, W, H, Wp, st);
+}
+
 cudaError_t UNet::train_step(const float* d_raw, const float* d_target, int N, int H, int W, float lr,
                              double* loss_out, int* err, cudaStream_t st) {
   Impl& I = *p_;
   cudaError_t e;
   long long P0 = (long long)N * H * W;
-  if ((e = forward(d_raw, N, H, W, err, st))) return e;
-  if ((e = cudaMemsetAsync(I.loss, 0, sizeof(double), st))) return e;
-  if ((e = kp_loss(I.pred, d_raw, d_target, I.dpred, N, H, W, I.loss, st))) return e;
+  if ((e = loss_pass(d_raw, d_target, N, H, W, err, st))) return e;
   int fwd = I.launches;
   if ((e = backward(N, H, W, err, st))) return e;
   ++I.step;
   if ((e = adam(I.master, I.grad, I.m, I.v, (long long)I.n_params, lr, I.step, st))) return e;
   if ((e = refresh_weights(st))) return e;
-  I.launches += fwd + 3;  // loss, Adam, weight refresh
+  I.launches += fwd + 2;  // Adam, weight refresh
   if (loss_out) {
     double s = 0.0;
     if ((e = cudaMemcpyAsync(&s, I.loss, sizeof(double), cudaMemcpyDeviceToHost, st))) return e;
@@ -393,12 +452,10 @@ cudaError_t UNet::loss_and_grads(const float* d_raw, const float* d_target, int 
   Impl& I = *p_;
   cudaError_t e;
   long long P0 = (long long)N * H * W;
-  if ((e = forward(d_raw, N, H, W, err, st))) return e;
-  if ((e = cudaMemsetAsync(I.loss, 0, sizeof(double), st))) return e;
-  if ((e = kp_loss(I.pred, d_raw, d_target, I.dpred, N, H, W, I.loss, st))) return e;
+  if ((e = loss_pass(d_raw, d_target, N, H, W, err, st))) return e;
   int fwd = I.launches;
   if ((e = backward(N, H, W, err, st))) return e;
-  I.launches += fwd + 1;
+  I.launches += fwd;
   double s = 0.0;
   if ((e = cudaMemcpyAsync(&s, I.loss, sizeof(double), cudaMemcpyDeviceToHost, st))) return e;
   if ((e = cudaStreamSynchronize(st))) return e;
@@ -406,15 +463,7 @@ cudaError_t UNet::loss_and_grads(const float* d_raw, const float* d_target, int 
   return cudaSuccess;
 }
 
-float* UNet::scratch_raw() { return p_->raw; }
-float* UNet::scratch_target() { return p_->target; }
-const float* UNet::prediction() const { return p_->pred; }
 cudaError_t UNet::reserve(long long P0) { return p_->ensure(P0); }
-
-cudaError_t UNet::decode(const float* d_raw, float* d_out, int N, int Hc, int Wc, int Hs, int Ws,
-                         cudaStream_t st) const {
-  return kp_apply(p_->pred, d_raw, d_out, N, Hc, Wc, Hs, Ws, st);
-}
 
 }  // namespace nn
 }  // namespace rtx

@@ -33,7 +33,11 @@ class UNet {
   cudaError_t set_state(const float* host_m, const float* host_v, int step, cudaStream_t st);
 
   // raw [N*H*W][kRawCh] = radiance 3, albedo 3, normal 3, depth 1, spp 1 (FP32)
-  cudaError_t forward(const float* d_raw, int N, int H, int W, int* err, cudaStream_t st);
+  // (nullptr: the encoded input is already in input()).  With a head the
+  // output layer applies it to its logits; *fused tells whether it could (else
+  // the logits are in prediction()).
+  cudaError_t forward(const float* d_raw, int N, int H, int W, int* err, cudaStream_t st,
+                      const KpHead* head = nullptr, bool* fused = nullptr);
   // gradients of the loss of the last forward (d_pred set by the loss)
   cudaError_t backward(int N, int H, int W, int* err, cudaStream_t st);
   // forward + loss against target [N*H*W][3] + backward (no update)
@@ -42,17 +46,16 @@ class UNet {
   // forward + loss + backward + Adam + BF16 weight refresh
   cudaError_t train_step(const float* d_raw, const float* d_target, int N, int H, int W, float lr,
                          double* loss, int* err, cudaStream_t st);
-  // out [N][Hc][Wc][3] = the last forward's predicted filters applied to the
-  // radiance of d_raw (the same input), frames stored as Hs x Ws pixels
-  cudaError_t decode(const float* d_raw, float* d_out, int N, int Hc, int Wc, int Hs, int Ws,
-                     cudaStream_t st) const;
+  // out [N][H][W][3] = the radiance of d_raw under the predicted filters
+  cudaError_t infer(const float* d_raw, float* d_out, int N, int H, int W, int* err, cudaStream_t st);
+  // the same of one W x H frame given as the renderer's passes (RGB FP32 each)
+  cudaError_t denoise(const float* rad, const float* alb, const float* nrm, const float* dep, float spp, float* d_out,
+                      int W, int H, int* err, cudaStream_t st);
 
   cudaError_t reserve(long long P0);  // activation buffers for P0 pixels
-  float* scratch_raw();               // [P0][kRawCh] staging for host inputs
-  float* scratch_target();            // [P0][3]
-  const float* prediction() const;    // [P0][kPredCh] FP32 filter logits
 
  private:
+  cudaError_t loss_pass(const float* d_raw, const float* d_target, int N, int H, int W, int* err, cudaStream_t st);
   cudaError_t refresh_weights(cudaStream_t st);
   struct Impl;
   Impl* p_;

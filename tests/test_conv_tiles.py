@@ -121,3 +121,55 @@ def test_network_gradients(ctx, shape):
         for off, n in ((r["w_off"], r["cout_pad"] * 9 * r["cin_pad"]), (r["b_off"], r["cout_pad"])):
             a, b, c = g[off:off + n], go[off:off + n], gf[off:off + n]
             assert rel(a, c) <= 2.0 * rel(b, c) + 2e-3, (i, rel(a, c), rel(b, c))
+
+
+def _passes(seed, H, W):
+    rng = np.random.RandomState(seed)
+    rad = rng.exponential(0.6, (H, W, 3)).astype(np.float32)
+    rad[rng.uniform(size=(H, W)) < 0.02] = np.nan  # the renderer's rare bad pixels
+    rad[rng.uniform(size=(H, W)) < 0.02, 0] = np.inf
+    alb, nrm = (rng.uniform(0, 1, (H, W, 3)).astype(np.float32) for _ in range(2))
+    dep = np.repeat(rng.uniform(0, 1, (H, W, 1)), 3, 2).astype(np.float32)
+    return rad, alb, nrm, dep
+
+
+@pytest.mark.parametrize("shape", [(33, 64), (50, 130), (17, 40)])
+def test_denoise_frame_and_padding(ctx, shape):
+    """A frame of any size (the filters fused with the output layer from 64
+    padded columns on, separate below) equals the FP64 network on the padded
+    record with its filters clamped to the frame: 2e-2 of the largest value,
+    what BF16 storage moves the network by; and an output that overlaps the
+    radiance gives the same bits."""
+    import torch
+    H, W = shape
+    ctx.dn_init(5)
+    p = U.init_params(4).astype(np.float32)
+    ctx.dn_set_params(p)
+    rad, alb, nrm, dep = _passes(H, H, W)
+    out = ctx.denoise(rad, alb, nrm, dep, 8)
+    Hp, Wp = (H + 15) // 16 * 16, (W + 15) // 16 * 16
+    raw = np.zeros((1, Hp, Wp, 11), np.float32)
+    raw[0, :H, :W] = np.concatenate([rad, alb, nrm, dep[..., :1], np.full((H, W, 1), 8, np.float32)], -1)
+    logits = U.UNet(p.astype(np.float64), bf16=True).forward(raw)[:, :H, :W]
+    ref = U.kp_apply(logits, raw[:, :H, :W])[0]
+    fin = np.abs(ref) < 1e4  # +inf reads 65504: its neighbourhood is judged relatively
+    np.testing.assert_allclose(out[fin], ref[fin], rtol=2e-2, atol=2e-2 * np.abs(ref[fin]).max())
+    np.testing.assert_allclose(out[~fin], ref[~fin], rtol=0.1)
+    dev = [torch.from_numpy(x).cuda() for x in (rad, alb, nrm, dep)]
+    torch.cuda.synchronize()
+    ctx.denoise(*dev, 8, out=dev[0])
+    assert np.array_equal(dev[0].cpu().numpy(), out)
+
+
+@pytest.mark.parametrize("shape", [(1, 48, 64), (2, 80, 144), (1, 32, 48)])
+def test_inference_matches_oracle(ctx, shape):
+    N, H, W = shape
+    ctx.dn_init(5)
+    p = U.init_params(6).astype(np.float32)
+    ctx.dn_set_params(p)
+    rng = np.random.RandomState(W)
+    raw = rng.uniform(0, 1, (N, H, W, 11)).astype(np.float32)
+    raw[..., 10] = 4.0
+    out = ctx.dn_infer(raw)
+    ref = U.UNet(p.astype(np.float64), bf16=True).denoise(raw)
+    np.testing.assert_allclose(out, ref, rtol=2e-2, atol=2e-2 * np.abs(ref).max())
