@@ -244,14 +244,26 @@ __device__ __forceinline__ void store_dgrad(const TileArgs& a, float* v, const u
 // (a lane's 32 columns are its pixel's), so neither the FP32 logits nor a
 // second pass over them exists.  kHead 1 filters the radiance, 2 computes the
 // loss and its gradient.  `rad`: the group's 12 x 20 radiance halo (clamped to
-// the frame, made safe), rows kRadRow apart.  Operations and order as the
+// the frame, made safe).  Operations and order as the
 // separate kernels (k_kp_apply, k_kp_loss).
-constexpr int kRadRow = 13, kRadTile = 20 * kRadRow * 3;
+// Halo pixels are float4s: a tap is one conflict-free 16-byte load (eight
+// neighbouring pixels per quarter warp).
+constexpr int kRadRow = 12, kRadTile = 20 * kRadRow;
 constexpr int kHeadGroups = kEpiWarps / 4;
 
+// Tap k of pixel (mx, my).  volatile: the second pass over the taps loads them
+// again instead of holding 75 values through the softmax's registers.
+__device__ __forceinline__ float4 rad_tap(uint32_t rad, int k) {
+  float4 c;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(c.x), "=f"(c.y), "=f"(c.z), "=f"(c.w)
+               : "r"(rad + ((k / kKpWidth) * kRadRow + k % kKpWidth) * 16));
+  return c;
+}
+
 template <int kHead>
-__device__ __forceinline__ void head_pixel(const TileArgs& a, float* l, const float* rad, int mx, int my, const float* tgt,
-                                           size_t p, size_t pc, bool ok, float& part) {
+__device__ __forceinline__ void head_pixel(const TileArgs& a, float* l, uint32_t rad, const float* tgt, size_t p,
+                                           size_t pc, bool ok, float& part) {
   float m = l[0];
 #pragma unroll
   for (int k = 1; k < kKpTaps; ++k) m = fmaxf(m, l[k]);
@@ -266,10 +278,10 @@ __device__ __forceinline__ void head_pixel(const TileArgs& a, float* l, const fl
 #pragma unroll
   for (int k = 0; k < kKpTaps; ++k) {
     l[k] *= inv_s;
-    const float* c = rad + ((my + k / kKpWidth) * kRadRow + mx + k % kKpWidth) * 3;
-    o[0] += l[k] * c[0];
-    o[1] += l[k] * c[1];
-    o[2] += l[k] * c[2];
+    const float4 c = rad_tap(rad, k);
+    o[0] += l[k] * c.x;
+    o[1] += l[k] * c.y;
+    o[2] += l[k] * c.z;
   }
   if constexpr (kHead == 1) {
     if (ok) {
@@ -288,10 +300,11 @@ __device__ __forceinline__ void head_pixel(const TileArgs& a, float* l, const fl
       g[i] = 2.0f * d / den * a.head.inv;
     }
     if (ok) part += e;
-    // dw_k = sum_c g_c r_c(tap k), formed twice (held, 25 registers spill)
+    // dw_k = sum_c g_c r_c(tap k), formed twice: held, it spills (192 us per
+    // 32 x 256^2 minibatch; so 150)
     auto dw = [&](int k) {
-      const float* c = rad + ((my + k / kKpWidth) * kRadRow + mx + k % kKpWidth) * 3;
-      return g[0] * c[0] + g[1] * c[1] + g[2] * c[2];
+      const float4 c = rad_tap(rad, k);
+      return g[0] * c.x + g[1] * c.y + g[2] * c.z;
     };
     float t = 0.0f;
 #pragma unroll
@@ -310,15 +323,16 @@ __device__ __forceinline__ void head_pixel(const TileArgs& a, float* l, const fl
   }
 }
 
-template <int kHead, class Wait, class Release>
-__device__ __forceinline__ bool head_epilogue(const TileArgs& a, const Tile& t, uint32_t tmem, int warp, int lane,
-                                              float* rad, const float* bias, double& loss, Wait&& wait,
-                                              Release&& release) {
-  const int q = warp & 3, tid = ((warp - kService) & 3) * 32 + lane, g = (warp - kService) >> 2;
-  const int m = q * 32 + lane, mx = m & 7, my = m >> 3;
+// What a tile's head reads from memory: this thread's share of the radiance
+// halo and its pixel's target.  Loaded one tile ahead.
+struct HeadIn {
+  float r[2][3], tgt[3];
+};
+
+template <int kHead>
+__device__ __forceinline__ void head_load(const TileArgs& a, const Tile& t, int warp, int lane, HeadIn& in) {
+  const int tid = ((warp - kService) & 3) * 32 + lane;
   const KpHead& h = a.head;
-  // this thread's share of the radiance halo, and its target, before the wait
-  float r[2][3], tgt[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int i = tid + 128 * j, yy = i / 12, xx = i - 12 * yy;
@@ -326,25 +340,39 @@ __device__ __forceinline__ bool head_epilogue(const TileArgs& a, const Tile& t, 
       const int y = min(max(t.y0 + yy - 2, 0), h.Hc - 1), x = min(max(t.x0 + xx - 2, 0), h.Wc - 1);
       const float* s = h.rad + (size_t)h.rad_px * (((size_t)t.n * h.Hs + y) * h.Ws + x);
 #pragma unroll
-      for (int k = 0; k < 3; ++k) r[j][k] = fminf(fmaxf(__ldg(s + k), 0.0f), 65504.0f);
+      for (int k = 0; k < 3; ++k) in.r[j][k] = __ldg(s + k);
     }
   }
+  if (kHead == 2) {
+    const int m = (warp & 3) * 32 + lane, x = t.x0 + (m & 7), y = t.y0 + (m >> 3);
+    if (x < h.Wc && y < h.Hc) {
+      const float* s = h.target + 3 * (((size_t)t.n * a.H + y) * a.W + x);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) in.tgt[k] = __ldg(s + k);
+    }
+  }
+}
+
+template <int kHead, class Next, class Wait, class Release>
+__device__ __forceinline__ bool head_epilogue(const TileArgs& a, const Tile& t, uint32_t tmem, int warp, int lane,
+                                              float4* rad, const float* bias, HeadIn& in, double& loss, Next&& next,
+                                              Wait&& wait, Release&& release) {
+  const int q = warp & 3, tid = ((warp - kService) & 3) * 32 + lane, g = (warp - kService) >> 2;
+  const int m = q * 32 + lane, mx = m & 7, my = m >> 3;
+  const KpHead& h = a.head;
   const int x = t.x0 + mx, y = t.y0 + my;
   const bool ok = x < h.Wc && y < h.Hc;
   const size_t p = ((size_t)t.n * a.H + y) * a.W + x, pc = ((size_t)t.n * h.Hc + y) * h.Wc + x;
-  if (kHead == 2 && ok) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) tgt[k] = __ldg(h.target + 3 * p + k);
-  }
   asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");  // the previous tile's taps are read
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int i = tid + 128 * j, yy = i / 12, xx = i - 12 * yy;
-    if (i < 240)
-#pragma unroll
-      for (int k = 0; k < 3; ++k) rad[(yy * kRadRow + xx) * 3 + k] = r[j][k];
+    auto sane = [](float v) { return fminf(fmaxf(v, 0.0f), 65504.0f); };
+    if (i < 240) rad[yy * kRadRow + xx] = make_float4(sane(in.r[j][0]), sane(in.r[j][1]), sane(in.r[j][2]), 0.0f);
   }
+  const float tgt[3] = {in.tgt[0], in.tgt[1], in.tgt[2]};
   asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");
+  next(in);
   const bool w = wait();
   float v[32];
   tmem_ld32(tmem + ((uint32_t)(q * 32) << 16), v);
@@ -358,7 +386,7 @@ __device__ __forceinline__ bool head_epilogue(const TileArgs& a, const Tile& t, 
     v[k + 3] += b4.w;
   }
   float part = 0.0f;
-  head_pixel<kHead>(a, v, rad, mx, my, tgt, p, pc, ok, part);
+  head_pixel<kHead>(a, v, tc::smem_u32(rad + my * kRadRow + mx), tgt, p, pc, ok, part);
   if constexpr (kHead == 2) {
     for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
     loss += (double)part;
@@ -474,7 +502,7 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
   __shared__ uint32_t tmem_slot;
   __shared__ uint4 xch[kDg ? kEpiWarps : 1][32][2];
   __shared__ __align__(16) float bias[kDg ? 4 : 256];
-  __shared__ float rad[kHead ? kHeadGroups : 1][kHead ? kRadTile : 1];
+  __shared__ float4 rad[kHead ? kHeadGroups : 1][kHead ? kRadTile : 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tiles = (int)blockIdx.x < a.n_tiles ? (a.n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   if (warp == 0) tc::tmem_alloc(&tmem_slot, a.ncols);
@@ -635,12 +663,16 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
     // each tile's four accumulators.  A group must not be given a buffer
     // whose previous phase it cannot know to be complete, so there are no
     // more groups on alternate tiles than buffers.
-    const int g = (warp - kService) >> 2, groups = kUp ? 1 : min(kEpiWarps / 4, a.nbuf), g0 = kUp ? 0 : g;
+    const int g = (warp - kService) >> 2, groups = kUp ? 1 : min(kEpiWarps / 4, a.nbuf),
+              g0 = kUp ? 0 : g;
     double loss = 0.0;
     if (g0 < groups) {
       TileIter it(a, (int)(blockIdx.x + g0 * gridDim.x), groups * (int)gridDim.x);
-      for (int i = g0; i < n_tiles && ok; i += groups, it.next(a)) {
+      HeadIn in{};
+      if (kHead && g0 < n_tiles) head_load<kHead>(a, it.tile(kTH), warp, lane, in);
+      for (int i = g0; i < n_tiles && ok; i += groups) {
         const Tile t = it.tile(kTH);
+        it.next(a);
         const int buf = i % a.nbuf, lap = i / a.nbuf;
         auto wait = [&] {
           const bool w = warp_wait(&bars.accf[buf], (uint32_t)lap & 1u);
@@ -653,7 +685,12 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
         };
         const uint32_t acc = tmem + buf * NA * a.NT;
         if constexpr (kHead)
-          ok = head_epilogue<kHead>(a, t, acc, warp, lane, rad[g], bias, loss, wait, release);
+          ok = head_epilogue<kHead>(
+              a, t, acc, warp, lane, rad[g], bias, in, loss,
+              [&](HeadIn& n) {
+                if (i + groups < n_tiles) head_load<kHead>(a, it.tile(kTH), warp, lane, n);
+              },
+              wait, release);
         else
           ok = tile_epilogue<kUp, kDg>(a, t, acc, kUp ? g : 0, kUp ? g + 1 : MT, warp, lane,
                                        xch[kDg ? warp - kService : 0], bias, wait, release);
