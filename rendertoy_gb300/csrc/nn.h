@@ -51,6 +51,9 @@ struct ConvFwd {
   bf16* out;         // [P][Cout] or nullptr
   float* out_f32;    // [P][Cout] or nullptr
   int* err;
+  // [P / 4][Cout] or nullptr (only where conv_fwd_pools says so): the output's
+  // 2 x 2 averages, written beside it
+  bf16* pool = nullptr;
 };
 
 // The kernel-predicting output layer together with what its logits are for:
@@ -89,9 +92,11 @@ struct ConvWgrad {
   int pix_per_cta;   // pixels each CTA sums (multiple of 64)
   float* dw;         // [Cout][9][Cin], accumulated
   int* err;
+  float* db = nullptr;  // [Cout] or nullptr: the bias gradient, accumulated
 };
 
 cudaError_t conv_fwd(const ConvFwd& a, cudaStream_t st);
+bool conv_fwd_pools(const ConvFwd& a);
 // The output layer with its head in one launch; false: not a shape it takes
 // (rows of at least 64 pixels), nothing launched.
 bool conv_head(const ConvFwd& a, const KpHead& h, cudaStream_t st, cudaError_t* e);

@@ -31,6 +31,7 @@
 #include <algorithm>
 
 #include "nn.h"
+#include "nn_ops.h"
 #include "nn_tile.h"
 #include "tc_core.cuh"
 
@@ -761,6 +762,7 @@ cudaError_t conv_fwd(const ConvFwd& a, cudaStream_t st) {
   if (a.Cout % 16 || a.Cout > 256 || a.Cin % 8) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
   if (conv_tile_fwd(a, use_rows(a.W, a.Cin), st, &e)) return e;
+  if (a.pool) return cudaErrorNotSupported;  // only the tile kernels pool
   if (use_rows(a.W, a.Cin)) {
     const size_t wbytes = (size_t)9 * a.Cin * a.Cout * 2;
     const bool res = wbytes <= kResidentWeights;
@@ -773,6 +775,10 @@ cudaError_t conv_fwd(const ConvFwd& a, cudaStream_t st) {
   const dim3 grid((unsigned)((P + 127) / 128));
   return launch_staged(k_conv_fwd<4>, k_conv_fwd<3>, k_conv_fwd<2>, gather_stages(a.Cout, grid, stage), grid,
                        stage, a, st);
+}
+
+bool conv_fwd_pools(const ConvFwd& a) {
+  return conv_tile_takes_fwd(a, use_rows(a.W, a.Cin)) && !a.s1.up && a.out && a.H % 2 == 0 && a.W % 2 == 0;
 }
 
 bool conv_head(const ConvFwd& a, const KpHead& h, cudaStream_t st, cudaError_t* e) {
@@ -811,6 +817,7 @@ cudaError_t conv_wgrad(const ConvWgrad& a, cudaStream_t st) {
   if (P >= (1LL << 31) || a.Cout % 16 || a.Cout > 256) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
   if (conv_tile_wgrad(a, st, &e)) return e;
+  if (a.db && (e = bias_grad(a.dout, P, a.Cout, a.db, st))) return e;
   size_t stage = 128 * kSlice * 2 + (size_t)a.Cout * kSlice * 2;
   dim3 grid((9 * a.Cin + 127) / 128, (unsigned)((P + a.pix_per_cta - 1) / a.pix_per_cta));
   return launch_staged(k_conv_wgrad<4>, k_conv_wgrad<3>, k_conv_wgrad<2>, stages_for(a.Cout), grid, stage, a, st);

@@ -84,6 +84,7 @@ struct TileArgs {
   int relu;
   bf16* out;
   float* out_f32;
+  bf16* pool;               // 2 x 2 averages of the output
   // data gradient: the sources (ReLU mask), and where the gradient goes
   Src s1, s2;
   int mask_relu;
@@ -158,9 +159,34 @@ struct TileIter {
   __device__ __forceinline__ Tile tile(int th) const { return Tile{n, x * 8, y * th, nt}; }
 };
 
+// The FP32 sums, in row order, of the 2 x 2 blocks of a warp's 8 x 4 pixels:
+// each lane gives its pixel's 16 BF16 channels (u) and receives four channels
+// (4 sub ..) of its block's sum.  Warp-wide.
+__device__ __forceinline__ int block_sums(const uint32_t* u, int lane, uint4 (*xch)[2], float* s) {
+  xch[lane][0] = make_uint4(u[0], u[1], u[2], u[3]);
+  xch[lane][1] = make_uint4(u[4], u[5], u[6], u[7]);
+  __syncwarp();
+  const int lx = lane & 7, ly = lane >> 3, sub = (ly & 1) * 2 + (lx & 1);
+  const int base = (ly & ~1) * 8 + (lx & ~1);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) s[k] = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint2 g = reinterpret_cast<const uint2*>(xch[base + (k >> 1) * 8 + (k & 1)])[sub];
+    const float2 g0 = unpack2(g.x), g1 = unpack2(g.y);
+    s[0] += g0.x;
+    s[1] += g0.y;
+    s[2] += g1.x;
+    s[3] += g1.y;
+  }
+  __syncwarp();
+  return sub;
+}
+
 // 16 output columns (channels c .. c + 15 of this lane's pixel p) of a
-// forward convolution
-__device__ __forceinline__ void store_fwd(const TileArgs& a, float* v, int c, size_t p, bool ok, const float* bias) {
+// forward convolution.  Warp-wide.
+__device__ __forceinline__ void store_fwd(const TileArgs& a, float* v, int c, size_t p, size_t plow, bool ok, int lane,
+                                          uint4 (*xch)[2], const float* bias) {
   if (a.bias) {
 #pragma unroll
     for (int k = 0; k < 16; k += 4) {
@@ -175,14 +201,20 @@ __device__ __forceinline__ void store_fwd(const TileArgs& a, float* v, int c, si
 #pragma unroll
     for (int k = 0; k < 16; ++k) v[k] = fmaxf(v[k], 0.0f);
   }
-  if (!ok) return;
   if (a.out) {
     uint32_t u[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) u[k] = pack2(v[2 * k], v[2 * k + 1]);
-    st32(a.out + p * a.Nout + c, u, (reinterpret_cast<uintptr_t>(a.out) & 31) == 0);
+    if (ok) st32(a.out + p * a.Nout + c, u, (reinterpret_cast<uintptr_t>(a.out) & 31) == 0);
+    if (a.pool) {
+      float s[4];
+      const int sub = block_sums(u, lane, xch, s);
+      if (ok)
+        *reinterpret_cast<uint2*>(a.pool + plow * a.Nout + c + 4 * sub) =
+            make_uint2(pack2(s[0] * 0.25f, s[1] * 0.25f), pack2(s[2] * 0.25f, s[3] * 0.25f));
+    }
   }
-  if (a.out_f32) {
+  if (ok && a.out_f32) {
     float* d = a.out_f32 + p * a.Nout + c;
     const uintptr_t al = reinterpret_cast<uintptr_t>(a.out_f32);
     if ((al & 15) == 0) {
@@ -216,25 +248,9 @@ __device__ __forceinline__ void store_dgrad(const TileArgs& a, float* v, const u
   } else if (c >= a.s1.C) {
     if (ok) st32(a.dskip + p * a.s2.C + (c - a.s1.C), u, (reinterpret_cast<uintptr_t>(a.dskip) & 31) == 0);
   } else {
-    // gradient of nearest upsampling: the 2 x 2 blocks of the warp's 8 x 4
-    // pixels, summed in FP32 in row order from the BF16 values; each of a
-    // block's four lanes sums four channels
-    xch[lane][0] = make_uint4(u[0], u[1], u[2], u[3]);
-    xch[lane][1] = make_uint4(u[4], u[5], u[6], u[7]);
-    __syncwarp();
-    const int lx = lane & 7, ly = lane >> 3, sub = (ly & 1) * 2 + (lx & 1);
-    const int base = (ly & ~1) * 8 + (lx & ~1);
-    float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint2 g = reinterpret_cast<const uint2*>(xch[base + (k >> 1) * 8 + (k & 1)])[sub];
-      const float2 g0 = unpack2(g.x), g1 = unpack2(g.y);
-      s[0] += g0.x;
-      s[1] += g0.y;
-      s[2] += g1.x;
-      s[3] += g1.y;
-    }
-    __syncwarp();
+    // gradient of nearest upsampling: the 2 x 2 blocks' sums of the BF16 values
+    float s[4];
+    const int sub = block_sums(u, lane, xch, s);
     if (ok)
       *reinterpret_cast<uint2*>(a.dlow + plow * a.s1.C + c + 4 * sub) = make_uint2(pack2(s[0], s[1]), pack2(s[2], s[3]));
   }
@@ -455,14 +471,14 @@ __device__ __forceinline__ bool tile_epilogue(const TileArgs& a, const Tile& t, 
         float v[32];
         tmem_ld32(taddr + c, v);
         if (acc == acc1 - 1 && c + 32 == nt) release();
-        store_fwd(a, v, n0 + c, p, ok, bias);
-        store_fwd(a, v + 16, n0 + c + 16, p, ok, bias);
+        store_fwd(a, v, n0 + c, p, plow, ok, lane, xch, bias);
+        store_fwd(a, v + 16, n0 + c + 16, p, plow, ok, lane, xch, bias);
       }
       if (c < nt) {
         float v[16];
         tmem_ld16(taddr + c, v);
         if (acc == acc1 - 1) release();
-        store_fwd(a, v, n0 + c, p, ok, bias);
+        store_fwd(a, v, n0 + c, p, plow, ok, lane, xch, bias);
       }
     }
   }
@@ -500,7 +516,8 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) Bars bars;
   __shared__ uint32_t tmem_slot;
-  __shared__ uint4 xch[kDg ? kEpiWarps : 1][32][2];
+  constexpr bool kXch = !kUp && !kHead;  // exchanges between a 2 x 2 block's lanes
+  __shared__ uint4 xch[kXch ? kEpiWarps : 1][32][2];
   __shared__ __align__(16) float bias[kDg ? 4 : 256];
   __shared__ float4 rad[kHead ? kHeadGroups : 1][kHead ? kRadTile : 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -693,7 +710,7 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
               wait, release);
         else
           ok = tile_epilogue<kUp, kDg>(a, t, acc, kUp ? g : 0, kUp ? g + 1 : MT, warp, lane,
-                                       xch[kDg ? warp - kService : 0], bias, wait, release);
+                                       xch[kXch ? warp - kService : 0], bias, wait, release);
       }
       if (kHead == 2 && lane == 0) atomicAdd(a.head.loss, loss);
     }
@@ -723,7 +740,7 @@ __global__ void __launch_bounds__(kThreadsN, 1) k_conv_narrow(const TileArgs a, 
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) NarrowBars bars;
   __shared__ uint32_t tmem_slot;
-  __shared__ uint4 xch[kDg ? kNarrowEpi : 1][32][2];
+  __shared__ uint4 xch[kNarrowEpi][32][2];
   __shared__ __align__(16) float bias[kDg ? 4 : 256];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_tiles = (int)blockIdx.x < a.n_tiles ? (a.n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
@@ -873,7 +890,7 @@ __global__ void __launch_bounds__(kThreadsN, 1) k_conv_narrow(const TileArgs a, 
     for (int i = g; i < n_tiles && ok; i += 2, it.next(a)) {
       const Tile t = it.tile(16);
       ok = tile_epilogue<false, kDg>(
-          a, t, tmem + (i & 1) * a.NT, 0, 1, warp, lane, xch[kDg ? warp - 2 - kExpandWarps : 0], bias,
+          a, t, tmem + (i & 1) * a.NT, 0, 1, warp, lane, xch[warp - 2 - kExpandWarps], bias,
           [&] {
             const bool w = warp_wait(&bars.accf[i & 1], (uint32_t)(i >> 1) & 1u);
             tc::fence_after();
@@ -1104,10 +1121,16 @@ static bool plan_narrow(TileArgs a, const Src& x1, const Src& x2, const bf16* w,
   return true;
 }
 
-bool conv_tile_fwd(const ConvFwd& c, bool wide, cudaStream_t st, cudaError_t* e) {
+bool conv_tile_takes_fwd(const ConvFwd& c, bool wide) {
   const int g = c.s2.ptr ? (c.s1.C | c.s2.C) : c.s1.C;
   if (g % 16 || c.Cout % 16 || c.s2.up || (c.s1.up && (c.H % 2 || c.W % 2))) return false;
   if (c.out && (reinterpret_cast<uintptr_t>(c.out) & 15)) return false;
+  return wide || narrow_fits(g % 32 == 0 ? 32 : 16, c.Cin);
+}
+
+bool conv_tile_fwd(const ConvFwd& c, bool wide, cudaStream_t st, cudaError_t* e) {
+  if (!conv_tile_takes_fwd(c, wide)) return false;
+  const int g = c.s2.ptr ? (c.s1.C | c.s2.C) : c.s1.C;
   TileArgs a{};
   a.H = c.H;
   a.W = c.W;
@@ -1116,6 +1139,7 @@ bool conv_tile_fwd(const ConvFwd& c, bool wide, cudaStream_t st, cudaError_t* e)
   a.relu = c.relu;
   a.out = c.out;
   a.out_f32 = c.out_f32;
+  a.pool = c.pool;
   a.err = c.err;
   const Src s2 = c.s2.ptr ? c.s2 : Src{nullptr, 0, 0};
   if (!wide)

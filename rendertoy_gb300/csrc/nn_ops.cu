@@ -344,14 +344,6 @@ __global__ void __launch_bounds__(256) k_bias_grad(const bf16* __restrict__ dout
   bias_grad_block(dout, P, C, per_block, blockIdx.x, db);
 }
 
-// Every layer's bias gradient in one launch: blockIdx.y picks the layer,
-// blockIdx.x its pixel range (blocks past a layer's own count return).
-__global__ void __launch_bounds__(256) k_bias_grads(BiasGrads j) {
-  const int i = blockIdx.y;
-  if ((long long)blockIdx.x * j.per_block[i] >= j.P[i]) return;
-  bias_grad_block(j.dout[i], j.P[i], j.C[i], j.per_block[i], blockIdx.x, j.db[i]);
-}
-
 // Adam (Kingma & Ba) on the FP32 master parameters
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                        float* __restrict__ v, long long n, float lr, float b1, float b2, float eps,
@@ -462,18 +454,6 @@ cudaError_t bias_grad(const bf16* dout, long long P, int C, float* db, cudaStrea
   long long nb = std::min<long long>(2 * 152, (P + 255) / 256);
   long long per = (P + nb - 1) / nb;
   k_bias_grad<<<(unsigned)nb, 256, 0, st>>>(dout, P, C, per, db);
-  return cudaGetLastError();
-}
-cudaError_t bias_grads(BiasGrads j, cudaStream_t st) {
-  if (j.n <= 0 || j.n > BiasGrads::kMax) return cudaErrorInvalidValue;
-  long long nbmax = 1;
-  for (int i = 0; i < j.n; ++i) {
-    if (j.C[i] % 8 || j.C[i] > 256) return cudaErrorInvalidValue;
-    const long long nb = std::min<long long>(2 * 152, (j.P[i] + 255) / 256);
-    j.per_block[i] = (j.P[i] + nb - 1) / nb;
-    nbmax = std::max(nbmax, nb);
-  }
-  k_bias_grads<<<dim3((unsigned)nbmax, (unsigned)j.n), 256, 0, st>>>(j);
   return cudaGetLastError();
 }
 cudaError_t adam(float* p, const float* g, float* m, float* v, long long n, float lr, int step,

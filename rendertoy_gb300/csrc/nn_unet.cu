@@ -254,13 +254,7 @@ cudaError_t UNet::forward(const float* d_raw, int N, int H, int W, int* err, cud
   for (int i = 0; i < kNumLayers; ++i) {
     const Impl::Layer& l = I.L[i];
     int lev = kTL[l.d.out >= 0 ? l.d.out : tU0];
-    // pooled inputs are produced just before their consumer
-    if (l.d.s1 == tP1 || l.d.s1 == tP2 || l.d.s1 == tP3 || l.d.s1 == tP4) {
-      int from = l.d.s1 - 1;  // S0 -> P1, S1 -> P2, ...
-      if ((e = avgpool(I.act[from], I.act[l.d.s1], N, H >> (lev - 1), W >> (lev - 1), kTC[from], st))) return e;
-      ++I.launches;
-    }
-    ConvFwd c;
+    ConvFwd c{};
     c.s1 = I.src(l.d.s1, l.d.s1_up);
     c.s2 = l.d.s2 >= 0 ? I.src(l.d.s2, 0) : Src{nullptr, 0, 0};
     c.N = N;
@@ -279,7 +273,14 @@ cudaError_t UNet::forward(const float* d_raw, int N, int H, int W, int* err, cud
       *fused = true;
       return e;
     }
+    // a skip tensor's 2 x 2 averages feed the next level
+    const bool skip = l.d.out == tS0 || l.d.out == tS1 || l.d.out == tS2 || l.d.out == tS3;
+    if (skip && conv_fwd_pools(c)) c.pool = I.act[l.d.out + 1];
     if ((e = conv_fwd(c, st))) return e;
+    if (skip && !c.pool) {
+      if ((e = avgpool(I.act[l.d.out], I.act[l.d.out + 1], N, c.H, c.W, kTC[l.d.out], st))) return e;
+      ++I.launches;
+    }
   }
   return cudaSuccess;
 }
@@ -289,10 +290,6 @@ cudaError_t UNet::backward(int N, int H, int W, int* err, cudaStream_t st) {
   cudaError_t e;
   if ((e = cudaMemsetAsync(I.grad, 0, I.n_params * 4, st))) return e;
   I.launches = 0;
-  // Bias gradients are summed for all layers in one launch at the end: each
-  // layer's output gradient holds its final value once its own step is done
-  // (later steps write only the gradients of earlier layers' outputs).
-  BiasGrads bias;
   for (int i = kNumLayers - 1; i >= 0; --i) {
     const Impl::Layer& l = I.L[i];
     int lev = kTL[l.d.out >= 0 ? l.d.out : tU0];
@@ -302,7 +299,7 @@ cudaError_t UNet::backward(int N, int H, int W, int* err, cudaStream_t st) {
     Src s1 = I.src(l.d.s1, l.d.s1_up);
     Src s2 = l.d.s2 >= 0 ? I.src(l.d.s2, 0) : Src{nullptr, 0, 0};
     // weight and bias gradients
-    ConvWgrad g;
+    ConvWgrad g{};
     g.dout = dout;
     g.Cout = l.d.cout_pad;
     g.s1 = s1;
@@ -313,13 +310,9 @@ cudaError_t UNet::backward(int N, int H, int W, int* err, cudaStream_t st) {
     g.Cin = l.cin_pad;
     g.pix_per_cta = wgrad_pixels_per_cta(P, l.d.cout_pad, l.cin_pad);
     g.dw = I.grad + l.w_off;
+    g.db = I.grad + l.b_off;
     g.err = err;
     if ((e = conv_wgrad(g, st))) return e;
-    bias.dout[bias.n] = dout;
-    bias.P[bias.n] = P;
-    bias.C[bias.n] = l.d.cout_pad;
-    bias.db[bias.n] = I.grad + l.b_off;
-    ++bias.n;
     ++I.launches;
     if (i == 0) break;  // the input needs no gradient
     // data gradient into the sources
@@ -362,8 +355,6 @@ cudaError_t UNet::backward(int N, int H, int W, int* err, cudaStream_t st) {
       }
     }
   }
-  if ((e = bias_grads(bias, st))) return e;
-  ++I.launches;
   return cudaSuccess;
 }
 

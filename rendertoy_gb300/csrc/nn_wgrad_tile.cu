@@ -22,6 +22,12 @@
 // layout by the eight warps that later run the epilogue: 16-byte cp.async
 // copies, one unit ahead.
 //
+// The bias gradient (sums of dout over the pixels) comes from the same tiles:
+// the epilogue warps of the last channel column (the one with least to expand)
+// add up each unit's dout rows from shared memory (instead of 131 us of reading
+// every dout again per step of 32 x 256^2; in the first column, behind the
+// expansion, d1's launch grew from 100 to 174 us).
+//
 // A CTA owns one or more groups of CB channels for its outputs, keeps their
 // accumulators in TMEM over a run of tiles and adds them to dw with FP32
 // atomics at the run's end.  FP32 accumulation in the tensor core truncates: a
@@ -58,7 +64,7 @@ struct WgradArgs {
   int S;
   uint32_t stage, dbytes, sbytes, src_off;  // ring stage; bytes of one dout / source box (1 KB steps); source offset
   uint32_t ncols;
-  float* dw;
+  float *dw, *db;
   int* err;
 };
 struct WgradMaps {
@@ -109,17 +115,19 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) uint64_t full[kMaxSW], empty[kMaxSW], done[2], drained[2];
   __shared__ uint32_t tmem_slot;
+  __shared__ float sdb[256];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int gc = (int)blockIdx.x % a.ngc, go = (int)blockIdx.x / a.ngc;
   const int g0 = gc * a.G, gn = min(a.G, a.ng - g0);               // channel groups g0 .. g0 + gn - 1
   const int nup = a.up1 ? max(0, min(gn, a.ng1 - g0)) : 0;         // of which expanded (the first ones)
   const int ob0 = go * a.ao, on = min(a.ao, a.Cout / a.KO - ob0);  // o-blocks
+  const bool bias = a.db && gc == a.ngc - 1;                       // this CTA sums dout
   const int t0 = (int)blockIdx.y * a.per, n = max(0, min(a.per, a.tiles - t0));
   if (warp == 0) tc::tmem_alloc(&tmem_slot, a.ncols);
   if (tid == 0) {
     for (int i = 0; i < a.S; ++i) {
       tc::mbar_init(&full[i], 1 + (nup ? kExpanders : 0));
-      tc::mbar_init(&empty[i], 1);
+      tc::mbar_init(&empty[i], 1 + (bias ? kExpanders : 0));
     }
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&done[i], 1);
@@ -131,6 +139,8 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = tmem_slot, s0 = tc::smem_u32(smem);
+  for (int k = tid; k < 256; k += kThreadsW) sdb[k] = 0.0f;
+  __syncthreads();
   const uint32_t ncb = 3 * a.CB;  // accumulator columns of a block
   bool ok = true;
   if (warp == 0) {
@@ -221,10 +231,42 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&full[stage]);
     };
+    // bias: thread -> 8 outputs of one pixel out of every `bps`
+    const int bch = a.KO >> 3, bcols = on * bch, bc = (tid - 64) % bcols, bp0 = (tid - 64) / bcols,
+              bps = kExpanders * 32 / bcols;
+    float bsum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    int bst = 0;
+    uint32_t bph = 0;
+    auto sum_bias = [&] {
+      if (!warp_wait(&full[bst], bph)) return false;
+      const uint32_t sd = s0 + bst * a.stage + (bc / bch) * a.dbytes;
+      if (bp0 < bps)
+        for (int h = 8 + bp0; h < 8 + 8 * a.TR; h += bps) {  // the halo's rows 1 .. TR
+          const int ch = (bc % bch) ^ (a.KO == 32 ? (h >> 1) & 3 : (h >> 2) & 1);
+          uint4 v;
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                       : "r"(sd + h * a.KO * 2 + (ch << 4)));
+          const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            bsum[2 * k] += __uint_as_float(w[k] << 16);
+            bsum[2 * k + 1] += __uint_as_float(w[k] & 0xffff0000u);
+          }
+        }
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&empty[bst]);
+      if (++bst == a.S) {
+        bst = 0;
+        bph ^= 1u;
+      }
+      return true;
+    };
     for (int u0 = 0; u0 < n && ok; u0 += a.run) {
+      const int u1 = min(n, u0 + a.run);
       if (nup) {
         int prev = -1;
-        for (int u = u0; u < min(n, u0 + a.run); ++u, w.next(a)) {
+        for (int u = u0; u < u1; ++u, w.next(a)) {
           ok = warp_wait(&empty[st], ph);
           if (!ok) break;
           const uint32_t ss = s0 + st * a.stage + a.src_off;
@@ -244,6 +286,7 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
           if (prev >= 0) {
             tc::cp_async_wait<1>();
             arrive(prev);
+            if (bias && !(ok = sum_bias())) break;
           }
           prev = st;
           if (++st == a.S) {
@@ -252,7 +295,12 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
           }
         }
         tc::cp_async_wait<0>();
-        if (ok && prev >= 0) arrive(prev);
+        if (ok && prev >= 0) {
+          arrive(prev);
+          if (bias) ok = sum_bias();
+        }
+      } else if (bias) {
+        for (int u = u0; u < u1 && ok; ++u) ok = sum_bias();
       }
       if (++set == a.sets) {
         set = 0;
@@ -279,8 +327,12 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
       tc::fence_before();
       tc::mbar_arrive(&drained[set]);
     }
+    if (bias && bp0 < bps)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) atomicAdd(&sdb[8 * bc + k], bsum[k]);
   }
   if (!__syncthreads_and(ok) && lane == 0) atomicOr(a.err, tc::kErrMbarTimeout);
+  if (bias && tid < on * a.KO) atomicAdd(a.db + ob0 * a.KO + tid, sdb[tid]);
   tc::fence_before();
   __syncthreads();
   if (warp == 0) tc::tmem_dealloc(tmem, a.ncols);
@@ -331,6 +383,7 @@ bool conv_tile_wgrad(const ConvWgrad& c, cudaStream_t st, cudaError_t* e) {
   a.H = c.H;
   a.W = c.W;
   a.dw = c.dw;
+  a.db = c.db;
   a.err = c.err;
   a.KO = c.Cout % 32 == 0 ? 32 : 16;
   const int at = c.Cout / a.KO;
