@@ -249,39 +249,48 @@ struct SepAcc {
   }
 };
 
-// Add window pixels j0 .. j0 + kSepR - 1 into the accumulators.  Which (pixel,
-// output) pairs of the chunk are taps: kAny, tested at run time; kAll of them;
-// or, where the size is a multiple of kSepR plus one, the triangles s >= o of
-// the first chunk and s <= o of the last, known at compile time (the tests
-// took 58 % of the ALU).
-enum Taps { kAny, kAll, kFirst, kLast };
-template <int kTaps>
-RTX_DEV constexpr bool tap_in(int s, int o) {
-  return kTaps == kAll || (kTaps == kFirst && s >= o) || (kTaps == kLast && s <= o);
-}
-template <Taps kTaps, bool kFma, class Px>
-RTX_DEV void sep_chunk(SepAcc& A, const float* __restrict__ wsm, int size, int j0, int nj, f2_t nz, Px px) {
-  float wv[2 * kSepR - 1];  // wv[k]: weight of tap j0 - (kSepR - 1) + k
-#pragma unroll
-  for (int k = 0; k < 2 * kSepR - 1; ++k) {
-    int ii = j0 - (kSepR - 1) + k;
-    if (kTaps != kAll) ii = min(max(ii, 0), size - 1);
-    wv[k] = wsm[ii];
+// Add window pixels j0 .. j0 + kSepR - 1 into the accumulators; output o takes
+// pixel j0 + s as tap j0 + s - o - kLead.  The (pixel, output) pairs that are
+// taps: all of them, those with kLo <= s - o <= kHi, or (kTest) those a run-time
+// test of the tap's index finds.  (The tests of the edge chunks took 58 % of
+// the horizontal pass's ALU.)
+template <int kLo_, int kHi_, int kLead_ = 0, bool kTest_ = false>
+struct Taps {
+  static constexpr int kLo = kLo_, kHi = kHi_, kLead = kLead_;
+  static constexpr bool kTest = kTest_, kAll = !kTest && kLo <= 1 - kSepR && kHi >= kSepR - 1;
+  static RTX_DEV bool in(int s, int o, int j0, int size) {
+    return kTest ? (j0 + s - o >= 0 && j0 + s - o < size) : (s - o >= kLo && s - o <= kHi);
   }
+};
+using TapsAll = Taps<1 - kSepR, kSepR - 1>;
+using TapsTest = Taps<0, 0, 0, true>;
+
+template <class T>
+RTX_DEV void tap_weights(float (&wv)[2 * kSepR - 1], const float* __restrict__ wsm, int size, int j0) {
+#pragma unroll
+  for (int k = 0; k < 2 * kSepR - 1; ++k) {  // wv[k]: the weight of s - o = k - (kSepR - 1)
+    const int ii = j0 - (kSepR - 1) + k - T::kLead;
+    wv[k] = wsm[T::kAll ? ii : min(max(ii, 0), size - 1)];
+  }
+}
+
+template <class T, bool kFma, class Px>
+RTX_DEV void sep_chunk(SepAcc& A, const float* __restrict__ wsm, int size, int j0, int nj, f2_t nz, Px px) {
+  float wv[2 * kSepR - 1];
+  tap_weights<T>(wv, wsm, size, j0);
   f2_t wp[2 * kSepR - 1];  // wp[k] = (wv[k], wv[k - 1]): the taps of an output pair
 #pragma unroll
   for (int k = 1; k < 2 * kSepR - 1; ++k) wp[k] = f2_pack(wv[k], wv[k - 1]);
 #pragma unroll
   for (int s = 0; s < kSepR; ++s) {
-    const int j = j0 + s;
-    if (kTaps == kAny && j >= nj) break;
-    const F3 p = px(j);
+    if (T::kTest && j0 + s >= nj) break;
+    const F3 p = px(j0 + s);
     const f2_t pp[3] = {f2_pack(p.x, p.x), f2_pack(p.y, p.y), f2_pack(p.z, p.z)};
 #pragma unroll
     for (int q = 0; q < kSepQ; ++q) {
       const int o0 = 2 * q, o1 = 2 * q + 1, k0 = s - o0 + kSepR - 1;
-      const bool v0 = kTaps == kAny ? (j - o0 >= 0 && j - o0 < size) : tap_in<kTaps>(s, o0);
-      const bool v1 = kTaps == kAny ? (j - o1 >= 0 && j - o1 < size) : tap_in<kTaps>(s, o1);
+      const bool v0 = T::in(s, o0, j0, size);
+      const bool v1 = T::in(s, o1, j0, size);
       if (v0 && v1) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) A.v[c][q] = f2_tap<kFma>(A.v[c][q], pp[c], wp[k0], nz);
@@ -300,6 +309,32 @@ RTX_DEV void sep_chunk(SepAcc& A, const float* __restrict__ wsm, int size, int j
   }
 }
 
+// The taps of chunk c of a filter of size 8 m + 1 - 2 kLead, whose windows start
+// kLead pixels early.
+template <int kLead, class Fn>
+RTX_DEV void chunk_taps(int c, int m, Fn f) {
+  constexpr int kN = kSepR;
+  if (c == 0) {
+    if (m == 1)
+      f(Taps<kLead, kN - kLead, kLead>());
+    else
+      f(Taps<kLead, kN - 1, kLead>());
+  } else if (c == m) {
+    if (m == 1)
+      f(Taps<kLead - kN, -kLead, kLead>());
+    else
+      f(Taps<1 - kN, -kLead, kLead>());
+  } else if (kLead < 2 || (c > 1 && c < m - 1)) {
+    f(Taps<1 - kN, kN - 1, kLead>());
+  } else if (c > 1) {
+    f(Taps<1 - kN, kN - kLead, kLead>());
+  } else if (c < m - 1) {
+    f(Taps<kLead - kN, kN - 1, kLead>());
+  } else {
+    f(Taps<kLead - kN, kN - kLead, kLead>());
+  }
+}
+
 template <bool kFma, class Px>
 RTX_DEV void sep_window(SepAcc& A, const float* __restrict__ wsm, int size, float negzero, Px px) {
   const f2_t nz = f2_pack(negzero, negzero);
@@ -310,9 +345,9 @@ RTX_DEV void sep_window(SepAcc& A, const float* __restrict__ wsm, int size, floa
   const int nj = size + kSepR - 1;
   for (int j0 = 0; j0 < nj; j0 += kSepR) {
     if (j0 >= kSepR - 1 && j0 + kSepR - 1 < size)
-      sep_chunk<kAll, kFma>(A, wsm, size, j0, nj, nz, px);
+      sep_chunk<TapsAll, kFma>(A, wsm, size, j0, nj, nz, px);
     else
-      sep_chunk<kAny, kFma>(A, wsm, size, j0, nj, nz, px);
+      sep_chunk<TapsTest, kFma>(A, wsm, size, j0, nj, nz, px);
   }
 }
 
@@ -423,7 +458,7 @@ __global__ void __launch_bounds__(kColThreads, 7) k_gauss_y(const float* __restr
 
 // ---------------------------------------------------------------------------
 // The separable passes on 16-byte accesses: images whose rows are a multiple
-// of four pixels (48 bytes) and, across, filters whose half width is.  Same
+// of four pixels (48 bytes) and, across, odd sizes.  Same
 // taps in the same order with the same roundings; what differs is how pixels
 // reach the registers.  The passes are FP32-issue bound (7.7 us each for 49
 // taps at 1,024^2); the 4-byte staging copies with their 64-bit reflection
@@ -450,10 +485,12 @@ RTX_DEV void st_row(float* p, const float* v, bool wide) {  // 24 floats
 
 // Horizontal: staged pixels sit in groups of eight (24 floats) 28 floats apart,
 // so that a window chunk is six 16-byte loads and eight neighbouring threads'
-// loads fall in distinct banks.  Eight outputs are 96 contiguous bytes.
+// loads fall in distinct banks.  Eight outputs are 96 contiguous bytes.  The
+// window starts at a pixel that is a multiple of four, kLead pixels before its
+// first tap.
 constexpr int kRowGroup = 28;
 
-template <bool kFma>
+template <int kLead, bool kFma>
 __global__ void __launch_bounds__(kRowThreads, 7) k_gauss_x16(const float* __restrict__ in, float* __restrict__ out,
                                                              int W, int H, const float* __restrict__ w, int size,
                                                              int extract_mode, float thr, float negzero, int wide) {
@@ -461,12 +498,12 @@ __global__ void __launch_bounds__(kRowThreads, 7) k_gauss_x16(const float* __res
   float* wsm = sm;
   float* tile = sm + ((size + 3) & ~3);
   const int y = blockIdx.y, x0 = blockIdx.x * kRowTile, r = size >> 1, tid = threadIdx.x;
-  const int n_out = min(kRowTile, W - x0), groups = (n_out + size - 1 + 7) / 8;
+  const int m = (size + 2 * kLead) >> 3, n_out = min(kRowTile, W - x0), groups = (n_out + 7) / 8 + m;
   for (int j = tid; j < size; j += kRowThreads) wsm[j] = w[j];
-  // chunk c: floats 4 c .. 4 c + 3 from pixel x0 - r on; the row's ends fall on
+  // chunk c: floats 4 c .. 4 c + 3 from pixel x0 - r - kLead on; the row's ends fall on
   // chunk boundaries
   const float* row = in + 3 * (size_t)W * y;
-  const int f0 = 3 * (x0 - r), f1 = 3 * W;
+  const int f0 = 3 * (x0 - r - kLead), f1 = 3 * W;
   const unsigned td = (unsigned)__cvta_generic_to_shared(tile);
   for (int c = tid; c < 6 * groups; c += kRowThreads) {
     const int f = f0 + 4 * c, d = (c / 6) * kRowGroup + (c % 6) * 4;
@@ -475,7 +512,7 @@ __global__ void __launch_bounds__(kRowThreads, 7) k_gauss_x16(const float* __res
     } else {
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const int g = f + k + 3 * size, x = g / 3 - size;  // floor for negative f
+        const int g = f + k + 3 * (size + 3), x = g / 3 - (size + 3);  // floor for negative f
         const long long idx = reflect_index(y, x, W, H);
         tile[d + k] = idx < 0 ? 0.0f : __ldg(in + 3 * idx + (g - 3 * (g / 3)));
       }
@@ -501,9 +538,8 @@ __global__ void __launch_bounds__(kRowThreads, 7) k_gauss_x16(const float* __res
   for (int c = 0; c < 3; ++c)
 #pragma unroll
     for (int q = 0; q < kSepQ; ++q) A.v[c][q] = f2_pack(0.0f, 0.0f);
-  const int nj = size + kSepR - 1;
-  for (int j0 = 0; j0 < nj; j0 += kSepR) {
-    const float4* s = reinterpret_cast<const float4*>(tile + (tid + (j0 >> 3)) * kRowGroup);
+  for (int c = 0; c <= m; ++c) {
+    const float4* s = reinterpret_cast<const float4*>(tile + (tid + c) * kRowGroup);
     float px[24];
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
@@ -513,13 +549,12 @@ __global__ void __launch_bounds__(kRowThreads, 7) k_gauss_x16(const float* __res
       px[4 * k + 2] = v.z;
       px[4 * k + 3] = v.w;
     }
-    auto get = [&](int j) { return f3(px[3 * (j - j0)], px[3 * (j - j0) + 1], px[3 * (j - j0) + 2]); };
-    if (j0 == 0)  // size = 8 m + 1, m >= 1
-      sep_chunk<kFirst, kFma>(A, wsm, size, j0, nj, nz, get);
-    else if (j0 + kSepR < nj)
-      sep_chunk<kAll, kFma>(A, wsm, size, j0, nj, nz, get);
-    else
-      sep_chunk<kLast, kFma>(A, wsm, size, j0, nj, nz, get);
+    const int j0 = kSepR * c;
+    chunk_taps<kLead>(c, m, [&](auto taps) {
+      sep_chunk<decltype(taps), kFma>(A, wsm, size, j0, 0, nz, [&](int j) {
+        return f3(px[3 * (j - j0)], px[3 * (j - j0) + 1], px[3 * (j - j0) + 2]);
+      });
+    });
   }
   float* o = out + 3 * ((size_t)y * W + x0 + b);
   float v[24];
@@ -545,22 +580,18 @@ __global__ void __launch_bounds__(kRowThreads, 7) k_gauss_x16(const float* __res
 // first ones.
 constexpr int kColQ = 32, kCol16Threads = 128, kCol16Groups = kCol16Threads / kColQ, kCol16H = kCol16Groups * kSepR;
 
-template <Taps kTaps, bool kFma>
+template <class T, bool kFma>
 RTX_DEV void col_chunk(f2_t (&acc)[2][kSepR], const float* __restrict__ wsm, int size, int j0, f2_t nz,
                        const float4* s) {
-  float wv[2 * kSepR - 1];  // wv[k]: weight of tap j0 - (kSepR - 1) + k
-#pragma unroll
-  for (int k = 0; k < 2 * kSepR - 1; ++k) {
-    const int ii = j0 - (kSepR - 1) + k;
-    wv[k] = wsm[kTaps == kAll ? ii : min(max(ii, 0), size - 1)];
-  }
+  float wv[2 * kSepR - 1];
+  tap_weights<T>(wv, wsm, size, j0);
 #pragma unroll
   for (int k = 0; k < kSepR; ++k) {
     const float4 v = s[k * kColQ];
     const f2_t a = f2_pack(v.x, v.y), b = f2_pack(v.z, v.w);
 #pragma unroll
     for (int o = 0; o < kSepR; ++o) {
-      if (kTaps == kAny ? (j0 + k - o >= 0 && j0 + k - o < size) : tap_in<kTaps>(k, o)) {
+      if (T::in(k, o, j0, size)) {
         const float ww = wv[k - o + kSepR - 1];
         const f2_t w2 = f2_pack(ww, ww);
         acc[0][o] = f2_tap<kFma>(acc[0][o], a, w2, nz);
@@ -572,17 +603,19 @@ RTX_DEV void col_chunk(f2_t (&acc)[2][kSepR], const float* __restrict__ wsm, int
 
 // The image bloom adds back is fetched into staged rows no warp reads any
 // more, two chunks before it is needed.
-template <bool kFma>
+// kLead < 0: an even size, whose edge chunks test their taps.
+template <int kLead, bool kFma>
 __global__ void __launch_bounds__(kCol16Threads, 5) k_gauss_y16(const float* __restrict__ in,
                                                                const float* __restrict__ orig, float* __restrict__ out,
                                                                int W, int H, const float* __restrict__ w, int size,
                                                                float negzero) {
   extern __shared__ __align__(16) float sm[];
-  float4* strip = reinterpret_cast<float4*>(sm);  // (kCol16H + size - 1, rounded to chunks) rows x kColQ
-  const int rows = kCol16H + size - 1, chunks = (rows + kSepR - 1) / kSepR;
+  float4* strip = reinterpret_cast<float4*>(sm);  // chunks * kSepR rows x kColQ
+  const int nc = (size + 2 * kSepR - 2) / kSepR;  // chunks of a window, kLead or not
+  const int chunks = nc + kCol16Groups - 1;
   float* wsm = sm + 4 * (size_t)chunks * kSepR * kColQ;
   const int tid = threadIdx.x, q = tid % kColQ, g = tid / kColQ;
-  const int nq = 3 * W / 4, q0 = blockIdx.x * kColQ, y0 = blockIdx.y * kCol16H, r = size >> 1;
+  const int nq = 3 * W / 4, q0 = blockIdx.x * kColQ, y0 = blockIdx.y * kCol16H, r = (size >> 1) + max(kLead, 0);
   for (int j = tid; j < size; j += kCol16Threads) wsm[j] = w[j];
   const bool live = q0 + q < nq;
   const unsigned sd = (unsigned)__cvta_generic_to_shared(strip);
@@ -608,8 +641,6 @@ __global__ void __launch_bounds__(kCol16Threads, 5) k_gauss_y16(const float* __r
   f2_t acc[2][kSepR];
 #pragma unroll
   for (int o = 0; o < kSepR; ++o) acc[0][o] = acc[1][o] = f2_pack(0.0f, 0.0f);
-  const int nj = size + kSepR - 1, nc = (nj + kSepR - 1) / kSepR;
-  const bool tri = size % kSepR == 1 && size > kSepR;
   // after chunk c's barrier no warp reads rows below kSepR * c
   const int c_orig = orig && nc - 1 >= kCol16Groups ? max(kCol16Groups, nc - 2) : -1;
   for (int c = 0; c < nc; ++c) {
@@ -626,14 +657,13 @@ __global__ void __launch_bounds__(kCol16Threads, 5) k_gauss_y16(const float* __r
     }
     const int j0 = c * kSepR;
     const float4* s = strip + (size_t)(kSepR * (g + c)) * kColQ + q;
-    if (tri && c == 0)
-      col_chunk<kFirst, kFma>(acc, wsm, size, j0, nz, s);
-    else if (tri && c == nc - 1)
-      col_chunk<kLast, kFma>(acc, wsm, size, j0, nz, s);
+    if (kLead >= 0)
+      chunk_taps<kLead < 0 ? 0 : kLead>(
+          c, nc - 1, [&](auto taps) { col_chunk<decltype(taps), kFma>(acc, wsm, size, j0, nz, s); });
     else if (j0 >= kSepR - 1 && j0 + kSepR - 1 < size)
-      col_chunk<kAll, kFma>(acc, wsm, size, j0, nz, s);
+      col_chunk<TapsAll, kFma>(acc, wsm, size, j0, nz, s);
     else
-      col_chunk<kAny, kFma>(acc, wsm, size, j0, nz, s);
+      col_chunk<TapsTest, kFma>(acc, wsm, size, j0, nz, s);
   }
   cp_wait_all();
   if (!live) return;
@@ -727,6 +757,25 @@ static size_t smem_y(int size) {
   return sizeof(float) * (((size_t)size + 3 & ~(size_t)3) + 3 * ((size_t)kColH + size - 1) * kColW);
 }
 
+// The 16-byte passes' instance for a lead (kLead).
+static decltype(&k_gauss_x16<0, false>) by_lead_x(int lead, bool fma) {
+  switch (lead) {
+    case 0: return fma ? k_gauss_x16<0, true> : k_gauss_x16<0, false>;
+    case 1: return fma ? k_gauss_x16<1, true> : k_gauss_x16<1, false>;
+    case 2: return fma ? k_gauss_x16<2, true> : k_gauss_x16<2, false>;
+    default: return fma ? k_gauss_x16<3, true> : k_gauss_x16<3, false>;
+  }
+}
+static decltype(&k_gauss_y16<0, false>) by_lead_y(int lead, bool fma) {
+  switch (lead) {
+    case 0: return fma ? k_gauss_y16<0, true> : k_gauss_y16<0, false>;
+    case 1: return fma ? k_gauss_y16<1, true> : k_gauss_y16<1, false>;
+    case 2: return fma ? k_gauss_y16<2, true> : k_gauss_y16<2, false>;
+    case 3: return fma ? k_gauss_y16<3, true> : k_gauss_y16<3, false>;
+    default: return fma ? k_gauss_y16<-1, true> : k_gauss_y16<-1, false>;
+  }
+}
+
 // GaussianBlur(size) on `in` (extract_mode: bloom's Extract fused into the
 // first pass, and the second pass adds `in` back: Image::Bloom).
 // Kernels too large for a shared-memory strip take the direct path, with
@@ -749,13 +798,15 @@ cudaError_t launch_gaussian(const float* in, float* tmp, float* tmp2, float* out
     return cudaGetLastError();
   }
   // 16-byte forms: rows of a multiple of four pixels, 16-byte aligned images,
-  // and (across) a half width that is a multiple of four (size 8 m + 1)
+  // and (across) an odd size
   auto al = [](const void* p, uintptr_t m) { return (reinterpret_cast<uintptr_t>(p) & (m - 1)) == 0; };
   const bool quads = W % 4 == 0 && al(in, 16) && al(tmp, 16) && al(out, 16);
-  const size_t sx16 = sizeof(float) * (((size_t)size + 3 & ~(size_t)3) + (size_t)kRowGroup * ((kRowTile + size + 6) / 8));
-  const size_t sy16 = sizeof(float) * ((size_t)size + 4 * (size_t)kColQ * kSepR * ((kCol16H + size - 1 + kSepR - 1) / kSepR));
-  if (quads && size % 8 == 1 && size > 8 && sx16 <= kMaxSmem) {
-    auto kx = fma ? k_gauss_x16<true> : k_gauss_x16<false>;
+  const int lead = size % 2 == 0 ? -1 : (4 - (size >> 1) % 4) % 4;
+  const size_t ws16 = (size_t)size + 3 & ~(size_t)3;
+  const size_t sx16 = sizeof(float) * (ws16 + (size_t)kRowGroup * (kRowTile / 8 + (size + 6) / 8));
+  const size_t sy16 = sizeof(float) * (ws16 + 4 * (size_t)kColQ * kSepR * ((size + 2 * kSepR - 2) / kSepR + kCol16Groups - 1));
+  if (quads && lead >= 0 && size > 1 && sx16 <= kMaxSmem) {
+    auto kx = by_lead_x(lead, fma);
     if (sx16 > 48 * 1024 && (e = cudaFuncSetAttribute(kx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx16)))
       return e;
     kx<<<dim3((W + kRowTile - 1) / kRowTile, H), kRowThreads, sx16, st>>>(in, tmp, W, H, d_w, size, extract_mode,
@@ -771,7 +822,7 @@ cudaError_t launch_gaussian(const float* in, float* tmp, float* tmp2, float* out
   }
   ++*launches;
   if (quads && sy16 <= kMaxSmem) {
-    auto ky = fma ? k_gauss_y16<true> : k_gauss_y16<false>;
+    auto ky = by_lead_y(size > 1 ? lead : -1, fma);
     if (sy16 > 48 * 1024 && (e = cudaFuncSetAttribute(ky, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sy16)))
       return e;
     ky<<<dim3((3 * W / 4 + kColQ - 1) / kColQ, (H + kCol16H - 1) / kCol16H), kCol16Threads, sy16, st>>>(

@@ -3,9 +3,9 @@
 The shapes sit where the passes can go wrong: widths that are a multiple of
 four pixels but not of eight, around the 1,024-pixel row tiles; heights around
 the 32-row strips; images smaller than the filter (RenderToy's reflection wraps
-into the neighbouring row there); sizes 8 m + 1, whose first and last window
-chunks are known at compile time, and the others, which take the 16-byte pass
-only down the columns; pixels that are NaN or infinite; an image that starts
+into the neighbouring row there); odd sizes of each remainder, whose first and
+last window chunks are known at compile time, and even ones, which take the
+16-byte pass only down the columns; NaN and infinite pixels; an image that starts
 off a 16-byte boundary, which takes the 4-byte passes.
 """
 import numpy as np
@@ -15,7 +15,7 @@ from helpers import bits
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 2, 3, 7, 8, 9, 17, 33, 49, 65, 101]
+SIZES = [1, 2, 3, 5, 7, 8, 9, 11, 13, 15, 17, 19, 21, 27, 29, 31, 33, 49, 101]
 
 
 def same(gpu, orc, what):
