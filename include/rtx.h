@@ -79,9 +79,10 @@ enum rtx_option {
   RTX_OPT_WAVE_PATHS = 2,     /* max paths in flight per wavefront (0 = auto:
                                  the whole render up to 2^26 paths and a
                                  quarter of the free device memory) */
-  RTX_OPT_BLOCK = 3,          /* threads per block of the persistent wavefront
-                                 kernels (extend, shade, connect): 64 or 128
-                                 (their register budgets cap blocks at 128) */
+  RTX_OPT_BLOCK = 3,          /* threads per block of the persistent traversal
+                                 kernels (extend, connect): 64 or 128 (their
+                                 register budgets cap blocks at 128); shading
+                                 blocks follow the wave's size */
   RTX_OPT_SORT_MATERIAL = 4,  /* 0 off, 1 on, 2 (default) on for scenes with a
                                  refracting material (spec_trans != 0) or 8
                                  materials or more: sort hits by material

@@ -35,23 +35,45 @@ constexpr int kCounterInts = 4 * kMaxDepthSlots;
 constexpr int kMaxSortBins = 4096;
 // Minimum resident blocks of 128 threads per SM, i.e. the register budget
 // (measured on the 1.3M-triangle frame: the traversal kernels are latency
-// bound and gain from more warps until spills begin; shading, with the
-// lobe-set variants, is fastest at 7 blocks (72 registers): 1.7 % faster
-// than 8, 4 % faster than 6).
-#ifndef RTX_SHADE_MINB
-#define RTX_SHADE_MINB 7
-#endif
-// the batch variants (frames of several scenes in one wavefront): 8 blocks,
-// 64 registers (1.4 % faster than 7 on the 16-scene batch)
-#ifndef RTX_SHADE_MINB_JOBS
-#define RTX_SHADE_MINB_JOBS 8
-#endif
+// bound and gain from more warps until spills begin).
 #ifndef RTX_EXTEND_MINB
 #define RTX_EXTEND_MINB 10
 #endif
 #ifndef RTX_CONNECT_MINB
 #define RTX_CONNECT_MINB 8
 #endif
+// Threads per SM of the shading kernel (72 registers; 1,024 threads at 64
+// spill more, 768 at 80 are within 1 % either way), as blocks of
+// shade_block() threads.
+constexpr int kShadeThreads = 896;
+
+// Threads per block of a shading launch.  A vertex executes some 2,600
+// instructions of straight-line code, more than an SM's instruction cache
+// holds: blocks of 128 threads at 28 unrelated places of it missed that cache
+// on 39 % of their fetches, kept the GPC's instruction cache 94 % busy and
+// left 45 % of the issue slots empty.  So the threads of a block begin each
+// vertex together (a barrier), and blocks are as large as the wave allows:
+//                                      128 x 7, none   448 x 2    896 x 1
+//   Cornell box  64^2 x 4 (2^14 paths)     0.323 ms      0.337      0.363
+//               256^2 x 16 (2^20)          1.034         1.025      1.055
+//             1,024^2 x 32 (2^25)         25.68         24.65      24.90
+//   nine materials 1,024^2 x 16 (2^24)    23.52         22.18      22.25
+//   1.3M triangles 1,024^2 x 4 (2^22)      9.24          8.99       8.97
+//                          x 16 (2^24)    26.71         25.69      25.42
+//                          x 64 (2^26)    99.06         95.13      93.02
+//   eight-scene batch 8 spp (2^23.6)      28.6          27.0       26.8
+//                    32 spp (2^25.6)      97.9          92.3       90.2
+// One block per SM waits for its slowest warp with nothing else to run; it
+// pays where the code is longest (batches, materials with a clear coat or
+// refraction) and the wave long.  A wave that would leave SMs without a block
+// keeps small ones.  (More barriers within a vertex, its lobes compiled once
+// and called, or one loop body for the light's and the BSDF's direction:
+// all slower, by 1 to 12 %.)
+static int shade_block(bool jobs, int lobes, long long n_wave) {
+  if (n_wave < 1LL << 18) return 128;
+  return (jobs || lobes) && n_wave >= 1LL << 23 ? 896 : 448;
+}
+
 // path state 6 x 16 B + shadow record 4 x 16 B + six 4-byte entries (two
 // queues, the material order, the ray order, the ray keys, the shadow order)
 constexpr size_t kPathBytes = 6 * 16 + 4 * 16 + 7 * 4;
@@ -78,7 +100,7 @@ struct PtWorkspace {
   float4* shadow = nullptr;
   int* counters = nullptr;  // counts[64] | shadow_counts[64] | work[2 * 64]
   int num_sms = 0;
-  int occ_extend = 0, occ_connect = 0, occ_shade = 0, occ_shade_jobs = 0, block_cached = 0;
+  int occ_extend = 0, occ_connect = 0, block_cached = 0;
   long long last_wave = 0;  // paths per wave of the last render
 };
 
@@ -460,166 +482,174 @@ constexpr int kShadeTex = 4;
 // path i of the wave taking its camera ray and cached primary hit directly
 // -- the state k_raygen would have written and this launch would have read
 // back.
-template <bool kJobs, int kFeat, bool kFirst = false>
-__global__ void __launch_bounds__(128, kJobs ? RTX_SHADE_MINB_JOBS : RTX_SHADE_MINB) k_shade(PtArgs a, DeviceScene s) {
+template <bool kJobs, int kFeat, bool kFirst>
+RTX_DEV void shade_vertex(const PtArgs& a, const DeviceScene& s, int i) {
   constexpr bool kTex = (kFeat & kShadeTex) != 0;
   constexpr int kLobes = kFeat & kLobeAll;
+  const int depth = a.depth;
+  const int p = kFirst ? i : a.queue_in[i];
+  const JobView J = job_of<kJobs>(a, s, a.q0 + p);
+  float4 ro, rd, h, th;
+  if (kFirst) {
+    // the frame's pixel of the path, as k_raygen numbers it
+    const PtJob* pj = kJobs ? a.jobs + J.job : nullptr;
+    const int pix = kJobs ? (int)(J.q % pj->npix) : (int)((a.q0 + p) % a.npix);
+    const int W = kJobs ? pj->W : a.W;
+    F3 co, cd;
+    camera_ray(kJobs ? pj->cam : a.cam, pix % W, pix / W, co, cd);
+    ro = make_float4(co.x, co.y, co.z, 0.0f);
+    rd = make_float4(cd.x, cd.y, cd.z, __int_as_float(-1));
+    h = __ldg(a.prim + (kJobs ? pj->pix_begin : 0) + pix);
+    th = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(0u));
+  } else {
+    ro = a.ray_o[p];
+    rd = a.ray_d[p];
+    h = a.hit[p];
+    th = a.thr[p];
+  }
+  F3 o = f3(ro.x, ro.y, ro.z), d = f3(rd.x, rd.y, rd.z);
+  float last_pdf = ro.w;
+  int tri = __float_as_int(h.x);
+  F3 T = f3(th.x, th.y, th.z);
+  // The path's radiance is read and written back only when this vertex
+  // adds a term that is not exactly zero: the sum starts at +0 and never
+  // becomes -0 (x + y is -0 only when both are), so adding +-0 leaves it
+  // unchanged, bit for bit; a NaN term is added.  The first vertex always
+  // writes it (no earlier value exists).
+  F3 acc = f3s(0.0f);
+  bool touched = kFirst;
+  auto add_rad = [&](F3 x) {
+    if (x.x == 0.0f && x.y == 0.0f && x.z == 0.0f) return;
+    if (!touched) {
+      const float4 r0 = a.rad[p];
+      acc = f3(r0.x, r0.y, r0.z);
+      touched = true;
+    }
+    acc = acc + x;
+  };
+  if (tri < 0) {
+    // World::GetDefaultEmission (world.cpp:39-42) of -direction
+    F3 env = (-d.z < 0.0f) ? f3(J.sky[0], J.sky[1], J.sky[2])
+                           : f3(J.ground[0], J.ground[1], J.ground[2]);
+    add_rad(T * env);
+    if (touched) a.rad[p] = make_float4(acc.x, acc.y, acc.z, 0.0f);
+    return;
+  }
+  // bit 31 of the RNG counter word: the path carries an absorption that
+  // is not +-0 (only then was it stored); +-0 reads as +0, which gives
+  // the same transmittance (pow(e, +-0) = 1, and +-0 * inf = NaN either way)
+  const uint32_t thw = __float_as_uint(th.w);
+  float4 ab = (kFirst || !(thw >> 31)) ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : a.absb[p];
+  F3 absorption = f3(ab.x, ab.y, ab.z);
+  float t = h.y, u = h.z, v = h.w;
+  float4 s0 = __ldg(s.shade + 4 * (size_t)tri), s1 = __ldg(s.shade + 4 * (size_t)tri + 1);
+  int info = __float_as_int(s1.w);
+  const float* mrec = s.mats + 24 * (size_t)(info & 0x7fffffff);
+  Mat m = load_mat(mrec);
+  F3 pos = o + d * t;  // BVH::Intersect: src + t * direction
+  F3 N = shading_normal(s, tri, u, v, s0, s1, info < 0);
+  if (kTex && __ldg(mrec + 21) != 0.0f) m.base_color = textured_base(mrec, pos, N, s.perm);
+  F3 ff = N;
+  float eta;
+  if (dot(d, ff) > 0.0f) {  // renderer.cpp:288-298
+    ff = -ff;
+    eta = m.ior;
+    absorption = f3s(0.0f);
+  } else {
+    eta = 1.0f / m.ior;
+  }
+  // SurfacePoint::GetEmission<true> (surfacepoint.h:21-45) toward the ray source
+  F3 re = o - pos;
+  float d2 = dot(re, re);
+  float cos_area = dot(-d, N) * s0.w;
+  float self_pdf = fabsf(d2 / cos_area);
+  F3 E = m.emission;
+  if (depth > 0) E = E * PowerHeuristic(last_pdf, self_pdf);
+  add_rad(T * E);
+  float dist = length(pos - o);
+  F3 expo = (-absorption) * dist;
+  // pow(e, +-0) is exactly 1: no call for the common no-absorption case
+  F3 br = (expo.x == 0.0f && expo.y == 0.0f && expo.z == 0.0f) ? f3s(1.0f) : transmittance(expo);
+  ShadingFrame fr = make_frame(m, eta, ff, -d);
+
+  long long q = J.q;
+  Rng rng{J.k0, J.k1, (uint32_t)(q % J.npix), (uint32_t)(J.first_sample + q / J.npix),
+          thw & 0x7fffffffu};
+  // the vertex's draws, in the reference's order: Int (emitter), Float,
+  // Float (point on it) when there are emitters, then Float, Float (BSDF)
+  uint32_t dv[5];
+  rng.draw5(dv);
+  const bool nee = J.n_emitters > 0;
+  rng.draw += nee ? 5u : 2u;
+  if (nee) {
+    // World::SampleEmitter + Triangle::GetSamplePoint (world.cpp:5-17, object.cpp:169-178)
+    int e = __ldg(J.emitters + Rng::to_int(dv[0], 0, J.n_emitters - 1));
+    float sqr1 = sqrtf(Rng::to_uniform(dv[1]));
+    float r2 = Rng::to_uniform(dv[2]);
+    float aa = 1.0f - sqr1;
+    float bb = (1.0f - r2) * sqr1;
+    const float4* g = s.geo + 3 * (size_t)e;
+    float4 g0 = __ldg(g), g1 = __ldg(g + 1), g2 = __ldg(g + 2);
+    F3 emit_pos = (f3(g1.x, g1.y, g1.z) * aa + f3(g2.x, g2.y, g2.z) * bb) + f3(g0.x, g0.y, g0.z);
+    F3 dl = normalized(emit_pos - pos);
+    float bpdf;
+    F3 f = BsdfEvalFrame<kLobes>(m, eta, fr, dl, bpdf);
+    if (bpdf > 0.0f) {
+      int slot = warp_append(a.shadow_counts + depth);
+      F3 tb = T * br;
+      float4* r = a.shadow + 4 * (size_t)slot;
+      r[0] = make_float4(pos.x, pos.y, pos.z, __int_as_float(p));
+      r[1] = make_float4(emit_pos.x, emit_pos.y, emit_pos.z, __int_as_float(e));
+      r[2] = make_float4(f.x, f.y, f.z, bpdf);
+      r[3] = make_float4(tb.x, tb.y, tb.z, __int_as_float(tri));
+      if (a.skeys) a.skeys[slot] = shadow_sort_key(kJobs ? a.jobs[J.job].keyb : s.keyb, pos);
+    }
+  }
+  float r1 = Rng::to_uniform(nee ? dv[3] : dv[0]);
+  float r2 = Rng::to_uniform(nee ? dv[4] : dv[1]);
+  F3 nd, color;
+  float pdf;
+  bool cont = false;
+  if (BsdfSampleFrame<kLobes>(m, eta, fr, r1, r2, nd, color, pdf)) {
+    // log(1) is exactly +0: no call for the default extinction
+    F3 lg = (m.extinction.x == 1.0f && m.extinction.y == 1.0f && m.extinction.z == 1.0f)
+                ? f3s(0.0f)
+                : log_extinction(m.extinction);
+    absorption = (-lg) / m.at_distance;
+    if (pdf > 0.0f) {
+      F3 w = (br * color) / pdf;
+      if (depth + 1 < a.max_depth) {
+        T = T * w;
+        cont = true;
+      } else {
+        // the reference multiplies by the (zero) radiance beyond the cap,
+        // which keeps an infinite or NaN weight visible as NaN
+        add_rad(T * (w * 0.0f));
+      }
+    }
+  }
+  if (touched) a.rad[p] = make_float4(acc.x, acc.y, acc.z, 0.0f);
+  if (cont) {
+    a.ray_o[p] = make_float4(pos.x, pos.y, pos.z, pdf);
+    a.ray_d[p] = make_float4(nd.x, nd.y, nd.z, __int_as_float(tri));
+    const bool ab_zero = absorption.x == 0.0f && absorption.y == 0.0f && absorption.z == 0.0f;
+    a.thr[p] = make_float4(T.x, T.y, T.z, __uint_as_float(rng.draw | (ab_zero ? 0u : 0x80000000u)));
+    if (!ab_zero) a.absb[p] = make_float4(absorption.x, absorption.y, absorption.z, 0.0f);
+    int slot = warp_append(a.counts + depth + 1);
+    a.queue_out[slot] = p;
+    if (a.ekeys) a.ekeys[slot] = ext_sort_key(kJobs ? a.jobs[J.job].keyb : s.keyb, pos, nd);
+  }
+}
+
+template <bool kJobs, int kFeat, bool kFirst = false>
+__global__ void __launch_bounds__(kShadeThreads, 1) k_shade(PtArgs a, DeviceScene s) {
   const int n = kFirst ? a.n_wave : a.counts[a.depth];
   if (kFirst && blockIdx.x == 0 && threadIdx.x == 0) a.counts[0] = a.n_wave;
-  const int depth = a.depth;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int p = kFirst ? i : a.queue_in[i];
-    const JobView J = job_of<kJobs>(a, s, a.q0 + p);
-    float4 ro, rd, h, th;
-    if (kFirst) {
-      // the frame's pixel of the path, as k_raygen numbers it
-      const PtJob* pj = kJobs ? a.jobs + J.job : nullptr;
-      const int pix = kJobs ? (int)(J.q % pj->npix) : (int)((a.q0 + p) % a.npix);
-      const int W = kJobs ? pj->W : a.W;
-      F3 co, cd;
-      camera_ray(kJobs ? pj->cam : a.cam, pix % W, pix / W, co, cd);
-      ro = make_float4(co.x, co.y, co.z, 0.0f);
-      rd = make_float4(cd.x, cd.y, cd.z, __int_as_float(-1));
-      h = __ldg(a.prim + (kJobs ? pj->pix_begin : 0) + pix);
-      th = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(0u));
-    } else {
-      ro = a.ray_o[p];
-      rd = a.ray_d[p];
-      h = a.hit[p];
-      th = a.thr[p];
-    }
-    F3 o = f3(ro.x, ro.y, ro.z), d = f3(rd.x, rd.y, rd.z);
-    float last_pdf = ro.w;
-    int tri = __float_as_int(h.x);
-    F3 T = f3(th.x, th.y, th.z);
-    // The path's radiance is read and written back only when this vertex
-    // adds a term that is not exactly zero: the sum starts at +0 and never
-    // becomes -0 (x + y is -0 only when both are), so adding +-0 leaves it
-    // unchanged, bit for bit; a NaN term is added.  The first vertex always
-    // writes it (no earlier value exists).
-    F3 acc = f3s(0.0f);
-    bool touched = kFirst;
-    auto add_rad = [&](F3 x) {
-      if (x.x == 0.0f && x.y == 0.0f && x.z == 0.0f) return;
-      if (!touched) {
-        const float4 r0 = a.rad[p];
-        acc = f3(r0.x, r0.y, r0.z);
-        touched = true;
-      }
-      acc = acc + x;
-    };
-    if (tri < 0) {
-      // World::GetDefaultEmission (world.cpp:39-42) of -direction
-      F3 env = (-d.z < 0.0f) ? f3(J.sky[0], J.sky[1], J.sky[2])
-                             : f3(J.ground[0], J.ground[1], J.ground[2]);
-      add_rad(T * env);
-      if (touched) a.rad[p] = make_float4(acc.x, acc.y, acc.z, 0.0f);
-      continue;
-    }
-    // bit 31 of the RNG counter word: the path carries an absorption that
-    // is not +-0 (only then was it stored); +-0 reads as +0, which gives
-    // the same transmittance (pow(e, +-0) = 1, and +-0 * inf = NaN either way)
-    const uint32_t thw = __float_as_uint(th.w);
-    float4 ab = (kFirst || !(thw >> 31)) ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : a.absb[p];
-    F3 absorption = f3(ab.x, ab.y, ab.z);
-    float t = h.y, u = h.z, v = h.w;
-    float4 s0 = __ldg(s.shade + 4 * (size_t)tri), s1 = __ldg(s.shade + 4 * (size_t)tri + 1);
-    int info = __float_as_int(s1.w);
-    const float* mrec = s.mats + 24 * (size_t)(info & 0x7fffffff);
-    Mat m = load_mat(mrec);
-    F3 pos = o + d * t;  // BVH::Intersect: src + t * direction
-    F3 N = shading_normal(s, tri, u, v, s0, s1, info < 0);
-    if (kTex && __ldg(mrec + 21) != 0.0f) m.base_color = textured_base(mrec, pos, N, s.perm);
-    F3 ff = N;
-    float eta;
-    if (dot(d, ff) > 0.0f) {  // renderer.cpp:288-298
-      ff = -ff;
-      eta = m.ior;
-      absorption = f3s(0.0f);
-    } else {
-      eta = 1.0f / m.ior;
-    }
-    // SurfacePoint::GetEmission<true> (surfacepoint.h:21-45) toward the ray source
-    F3 re = o - pos;
-    float d2 = dot(re, re);
-    float cos_area = dot(-d, N) * s0.w;
-    float self_pdf = fabsf(d2 / cos_area);
-    F3 E = m.emission;
-    if (depth > 0) E = E * PowerHeuristic(last_pdf, self_pdf);
-    add_rad(T * E);
-    float dist = length(pos - o);
-    F3 expo = (-absorption) * dist;
-    // pow(e, +-0) is exactly 1: no call for the common no-absorption case
-    F3 br = (expo.x == 0.0f && expo.y == 0.0f && expo.z == 0.0f) ? f3s(1.0f) : transmittance(expo);
-    ShadingFrame fr = make_frame(m, eta, ff, -d);
-
-    long long q = J.q;
-    Rng rng{J.k0, J.k1, (uint32_t)(q % J.npix), (uint32_t)(J.first_sample + q / J.npix),
-            thw & 0x7fffffffu};
-    // the vertex's draws, in the reference's order: Int (emitter), Float,
-    // Float (point on it) when there are emitters, then Float, Float (BSDF)
-    uint32_t dv[5];
-    rng.draw5(dv);
-    const bool nee = J.n_emitters > 0;
-    rng.draw += nee ? 5u : 2u;
-    if (nee) {
-      // World::SampleEmitter + Triangle::GetSamplePoint (world.cpp:5-17, object.cpp:169-178)
-      int e = __ldg(J.emitters + Rng::to_int(dv[0], 0, J.n_emitters - 1));
-      float sqr1 = sqrtf(Rng::to_uniform(dv[1]));
-      float r2 = Rng::to_uniform(dv[2]);
-      float aa = 1.0f - sqr1;
-      float bb = (1.0f - r2) * sqr1;
-      const float4* g = s.geo + 3 * (size_t)e;
-      float4 g0 = __ldg(g), g1 = __ldg(g + 1), g2 = __ldg(g + 2);
-      F3 emit_pos = (f3(g1.x, g1.y, g1.z) * aa + f3(g2.x, g2.y, g2.z) * bb) + f3(g0.x, g0.y, g0.z);
-      F3 dl = normalized(emit_pos - pos);
-      float bpdf;
-      F3 f = BsdfEvalFrame<kLobes>(m, eta, fr, dl, bpdf);
-      if (bpdf > 0.0f) {
-        int slot = warp_append(a.shadow_counts + depth);
-        F3 tb = T * br;
-        float4* r = a.shadow + 4 * (size_t)slot;
-        r[0] = make_float4(pos.x, pos.y, pos.z, __int_as_float(p));
-        r[1] = make_float4(emit_pos.x, emit_pos.y, emit_pos.z, __int_as_float(e));
-        r[2] = make_float4(f.x, f.y, f.z, bpdf);
-        r[3] = make_float4(tb.x, tb.y, tb.z, __int_as_float(tri));
-        if (a.skeys) a.skeys[slot] = shadow_sort_key(kJobs ? a.jobs[J.job].keyb : s.keyb, pos);
-      }
-    }
-    float r1 = Rng::to_uniform(nee ? dv[3] : dv[0]);
-    float r2 = Rng::to_uniform(nee ? dv[4] : dv[1]);
-    F3 nd, color;
-    float pdf;
-    bool cont = false;
-    if (BsdfSampleFrame<kLobes>(m, eta, fr, r1, r2, nd, color, pdf)) {
-      // log(1) is exactly +0: no call for the default extinction
-      F3 lg = (m.extinction.x == 1.0f && m.extinction.y == 1.0f && m.extinction.z == 1.0f)
-                  ? f3s(0.0f)
-                  : log_extinction(m.extinction);
-      absorption = (-lg) / m.at_distance;
-      if (pdf > 0.0f) {
-        F3 w = (br * color) / pdf;
-        if (depth + 1 < a.max_depth) {
-          T = T * w;
-          cont = true;
-        } else {
-          // the reference multiplies by the (zero) radiance beyond the cap,
-          // which keeps an infinite or NaN weight visible as NaN
-          add_rad(T * (w * 0.0f));
-        }
-      }
-    }
-    if (touched) a.rad[p] = make_float4(acc.x, acc.y, acc.z, 0.0f);
-    if (cont) {
-      a.ray_o[p] = make_float4(pos.x, pos.y, pos.z, pdf);
-      a.ray_d[p] = make_float4(nd.x, nd.y, nd.z, __int_as_float(tri));
-      const bool ab_zero = absorption.x == 0.0f && absorption.y == 0.0f && absorption.z == 0.0f;
-      a.thr[p] = make_float4(T.x, T.y, T.z, __uint_as_float(rng.draw | (ab_zero ? 0u : 0x80000000u)));
-      if (!ab_zero) a.absb[p] = make_float4(absorption.x, absorption.y, absorption.z, 0.0f);
-      int slot = warp_append(a.counts + depth + 1);
-      a.queue_out[slot] = p;
-      if (a.ekeys) a.ekeys[slot] = ext_sort_key(kJobs ? a.jobs[J.job].keyb : s.keyb, pos, nd);
-    }
+  const int step = gridDim.x * blockDim.x;
+  for (int base = blockIdx.x * blockDim.x; base < n; base += step) {
+    __syncthreads();  // in step through the instruction cache: see shade_block
+    const int i = base + threadIdx.x;
+    if (i < n) shade_vertex<kJobs, kFeat, kFirst>(a, s, i);
   }
 }
 
@@ -651,18 +681,6 @@ static void launch_shade(int feat, dim3 grid, dim3 block, cudaStream_t st, const
     case 6: k_shade<kJobs, 6><<<grid, block, 0, st>>>(a, s); break;
     default: k_shade<kJobs, 7><<<grid, block, 0, st>>>(a, s); break;
   }
-}
-
-// resident blocks per SM of the least-resident shading variant
-template <bool kJobs>
-static int shade_occupancy(int block) {
-  int occ = 1 << 30, o = 0;
-  for (auto k : {k_shade<kJobs, 0>, k_shade<kJobs, 1>, k_shade<kJobs, 2>, k_shade<kJobs, 3>, k_shade<kJobs, 4>,
-                 k_shade<kJobs, 5>, k_shade<kJobs, 6>, k_shade<kJobs, 7>}) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k, block, 0);
-    occ = std::min(occ, o);
-  }
-  return occ;
 }
 
 // Emitter's own exact test for a shadow record: the emitter is the target of
@@ -1105,12 +1123,14 @@ __global__ void __launch_bounds__(256) k_raykey_scatter(PtArgs a, const int* key
 template <bool kJobs>
 static cudaError_t wave_launches(const PtParams& p, PtArgs& a, const DeviceScene& s, const CamParams& cam,
                                  const float4* prim, PtWorkspace* ws, KernelTimer* timer, cudaStream_t st,
-                                 int grid_ext, int grid_con, int grid_sh, int block, int nw, int* launches,
+                                 int grid_ext, int grid_con, int grid_sort, int block, int nw, int* launches,
                                  int* extend_launches, int* vertex_launches, bool overlap) {
   cudaError_t e;
   a.queue_in = ws->queue[0];
   a.queue_out = ws->queue[1];
   a.depth = 0;
+  const int feat = shade_features(s), block_sh = shade_block(kJobs, feat & kLobeAll, nw);
+  const int grid_sh = ws->num_sms * (kShadeThreads / block_sh);
   // A render with cached primary hits and path-order shading needs no path
   // state before its first shading launch, which makes the camera rays
   // itself; otherwise k_raygen writes the state (and the cached hits).
@@ -1135,9 +1155,9 @@ static cudaError_t wave_launches(const PtParams& p, PtArgs& a, const DeviceScene
     if (p.sort_rays && depth > 0) {
       static_assert(kRayKeyBins <= kMaxSortBins, "ray keys use the sort histogram");
       if ((e = cudaMemsetAsync(ws->mat_hist, 0, (kMaxSortBins + 1) * sizeof(int), st))) return e;
-      k_raykey_hist<false><<<grid_sh, 256, 0, st>>>(a, ws->keys, ws->mat_hist);
+      k_raykey_hist<false><<<grid_sort, 256, 0, st>>>(a, ws->keys, ws->mat_hist);
       k_sort_scan<<<1, 1024, 0, st>>>(kRayKeyBins, ws->mat_hist);
-      k_raykey_scatter<false><<<grid_sh, 256, 0, st>>>(a, ws->keys, ws->mat_hist, ws->ray_sorted);
+      k_raykey_scatter<false><<<grid_sort, 256, 0, st>>>(a, ws->keys, ws->mat_hist, ws->ray_sorted);
       *launches += 3;
       a.queue_in = ws->ray_sorted;  // the closest-hit kernel visits paths in key order
     }
@@ -1171,15 +1191,15 @@ static cudaError_t wave_launches(const PtParams& p, PtArgs& a, const DeviceScene
       // the shading kernel reads the sorted queue; its output queue is unchanged
       if ((e = cudaMemsetAsync(ws->mat_hist, 0, (kMaxSortBins + 1) * sizeof(int), st))) return e;
       size_t shm = (size_t)(s.n_mats + 1) * sizeof(int);
-      k_sort_hist<<<grid_sh, 256, shm, st>>>(a, s, ws->mat_hist);
+      k_sort_hist<<<grid_sort, 256, shm, st>>>(a, s, ws->mat_hist);
       k_sort_scan<<<1, 1024, 0, st>>>(s.n_mats + 1, ws->mat_hist);
-      k_sort_scatter<<<grid_sh, 256, 0, st>>>(a, s, ws->mat_hist, ws->sorted);
+      k_sort_scatter<<<grid_sort, 256, 0, st>>>(a, s, ws->mat_hist, ws->sorted);
       *launches += 3;
       PtArgs as = a;
       as.queue_in = ws->sorted;
-      launch_shade<kJobs>(shade_features(s), grid_sh, block, st, as, s);
+      launch_shade<kJobs>(feat, grid_sh, block_sh, st, as, s);
     } else {
-      launch_shade<kJobs>(shade_features(s), grid_sh, block, st, a, s, first_in_shade && depth == 0);
+      launch_shade<kJobs>(feat, grid_sh, block_sh, st, a, s, first_in_shade && depth == 0);
     }
     if ((e = timer->mark(1, st, false))) return e;
     // The vertex's shadow rays: sorted and traced on the side stream, beside
@@ -1196,9 +1216,9 @@ static cudaError_t wave_launches(const PtParams& p, PtArgs& a, const DeviceScene
     a.shadow_order = nullptr;
     if (p.sort_rays) {
       if ((e = cudaMemsetAsync(shist, 0, (kMaxSortBins + 1) * sizeof(int), cs))) return e;
-      k_raykey_hist<true><<<grid_sh, 256, 0, cs>>>(a, ws->keys2, shist);
+      k_raykey_hist<true><<<grid_sort, 256, 0, cs>>>(a, ws->keys2, shist);
       k_sort_scan<<<1, 1024, 0, cs>>>(kRayKeyBins, shist);
-      k_raykey_scatter<true><<<grid_sh, 256, 0, cs>>>(a, ws->keys2, shist, ws->shadow_order);
+      k_raykey_scatter<true><<<grid_sort, 256, 0, cs>>>(a, ws->keys2, shist, ws->shadow_order);
       *launches += 3;
       a.shadow_order = ws->shadow_order;  // the occlusion kernel visits records in key order
     }
@@ -1292,8 +1312,6 @@ cudaError_t pt_render(PtWorkspace* ws, const DeviceScene& s, const CamParams& ca
     ws->occ_connect = std::min(ws->occ_connect, o2);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o2, k_connect_batch<false, true, true>, block, 0);
     ws->occ_connect = std::min(ws->occ_connect, o2);
-    ws->occ_shade = shade_occupancy<false>(block);
-    ws->occ_shade_jobs = shade_occupancy<true>(block);
     ws->block_cached = block;
   }
   // The side stream and its events are made outside any stream capture (a
@@ -1312,9 +1330,7 @@ cudaError_t pt_render(PtWorkspace* ws, const DeviceScene& s, const CamParams& ca
   }
   int grid_ext = ws->num_sms * std::max(ws->occ_extend, 1);
   int grid_con = ws->num_sms * std::max(ws->occ_connect, 1);
-  // the shading grid (also the sorts' grid) at the residency of the variant
-  // this render launches
-  int grid_sh = ws->num_sms * std::max(jobs ? ws->occ_shade_jobs : ws->occ_shade, 1);
+  const int grid_sort = ws->num_sms * 8;  // 256-thread blocks
 
   PtArgs a;
   a.ray_o = ws->ray_o;
@@ -1370,9 +1386,9 @@ cudaError_t pt_render(PtWorkspace* ws, const DeviceScene& s, const CamParams& ca
     a.q0 = q0;
     a.n_wave = nw;
     if ((e = cudaMemsetAsync(ws->counters, 0, kCounterInts * sizeof(int), st))) return e;
-    e = jobs ? wave_launches<true>(p, a, s, cam, prim, ws, timer, st, grid_ext, grid_con, grid_sh, block, nw, launches,
+    e = jobs ? wave_launches<true>(p, a, s, cam, prim, ws, timer, st, grid_ext, grid_con, grid_sort, block, nw, launches,
                                    extend_launches, vertex_launches, overlap)
-             : wave_launches<false>(p, a, s, cam, prim, ws, timer, st, grid_ext, grid_con, grid_sh, block, nw, launches,
+             : wave_launches<false>(p, a, s, cam, prim, ws, timer, st, grid_ext, grid_con, grid_sort, block, nw, launches,
                                     extend_launches, vertex_launches, overlap);
     if (e) return e;
     if (jobs) {
