@@ -249,21 +249,27 @@ struct SepAcc {
   }
 };
 
+// A window starts kLead pixels before its first tap, so that its first pixel is
+// kSepR m / 2 (a multiple of four) pixels before the first output and the
+// windows' chunks of kSepR pixels number m + 1.  Window<k>: sizes with
+// kLead = k % 4; k >= 4: even ones, whose last tap is missing on the right.
+template <int k>
+struct Window {
+  static constexpr int kLead = k & 3, kTail = kLead + (k >> 2);
+};
+static int window_kind(int size) { return (4 - (size >> 1) % 4) % 4 + (size % 2 == 0 ? 4 : 0); }
+RTX_DEV int window_chunks(int size, int lead) { return ((size | 1) + 2 * lead) >> 3; }  // m
+
 // Add window pixels j0 .. j0 + kSepR - 1 into the accumulators; output o takes
-// pixel j0 + s as tap j0 + s - o - kLead.  The (pixel, output) pairs that are
-// taps: all of them, those with kLo <= s - o <= kHi, or (kTest) those a run-time
-// test of the tap's index finds.  (The tests of the edge chunks took 58 % of
-// the horizontal pass's ALU.)
-template <int kLo_, int kHi_, int kLead_ = 0, bool kTest_ = false>
+// pixel j0 + s as tap j0 + s - o - kLead.  Which (pixel, output) pairs of a
+// chunk are taps is known at compile time: those with kLo <= s - o <= kHi.
+// (Run-time tests of the edge chunks took 58 % of the horizontal pass's ALU.)
+template <int kLo_, int kHi_, int kLead_>
 struct Taps {
   static constexpr int kLo = kLo_, kHi = kHi_, kLead = kLead_;
-  static constexpr bool kTest = kTest_, kAll = !kTest && kLo <= 1 - kSepR && kHi >= kSepR - 1;
-  static RTX_DEV bool in(int s, int o, int j0, int size) {
-    return kTest ? (j0 + s - o >= 0 && j0 + s - o < size) : (s - o >= kLo && s - o <= kHi);
-  }
+  static constexpr bool kAll = kLo <= 1 - kSepR && kHi >= kSepR - 1;
+  static RTX_DEV constexpr bool in(int s, int o) { return s - o >= kLo && s - o <= kHi; }
 };
-using TapsAll = Taps<1 - kSepR, kSepR - 1>;
-using TapsTest = Taps<0, 0, 0, true>;
 
 template <class T>
 RTX_DEV void tap_weights(float (&wv)[2 * kSepR - 1], const float* __restrict__ wsm, int size, int j0) {
@@ -275,7 +281,7 @@ RTX_DEV void tap_weights(float (&wv)[2 * kSepR - 1], const float* __restrict__ w
 }
 
 template <class T, bool kFma, class Px>
-RTX_DEV void sep_chunk(SepAcc& A, const float* __restrict__ wsm, int size, int j0, int nj, f2_t nz, Px px) {
+RTX_DEV void sep_chunk(SepAcc& A, const float* __restrict__ wsm, int size, int j0, f2_t nz, Px px) {
   float wv[2 * kSepR - 1];
   tap_weights<T>(wv, wsm, size, j0);
   f2_t wp[2 * kSepR - 1];  // wp[k] = (wv[k], wv[k - 1]): the taps of an output pair
@@ -283,14 +289,13 @@ RTX_DEV void sep_chunk(SepAcc& A, const float* __restrict__ wsm, int size, int j
   for (int k = 1; k < 2 * kSepR - 1; ++k) wp[k] = f2_pack(wv[k], wv[k - 1]);
 #pragma unroll
   for (int s = 0; s < kSepR; ++s) {
-    if (T::kTest && j0 + s >= nj) break;
     const F3 p = px(j0 + s);
     const f2_t pp[3] = {f2_pack(p.x, p.x), f2_pack(p.y, p.y), f2_pack(p.z, p.z)};
 #pragma unroll
     for (int q = 0; q < kSepQ; ++q) {
       const int o0 = 2 * q, o1 = 2 * q + 1, k0 = s - o0 + kSepR - 1;
-      const bool v0 = T::in(s, o0, j0, size);
-      const bool v1 = T::in(s, o1, j0, size);
+      const bool v0 = T::in(s, o0);
+      const bool v1 = T::in(s, o1);
       if (v0 && v1) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) A.v[c][q] = f2_tap<kFma>(A.v[c][q], pp[c], wp[k0], nz);
@@ -309,46 +314,43 @@ RTX_DEV void sep_chunk(SepAcc& A, const float* __restrict__ wsm, int size, int j
   }
 }
 
-// The taps of chunk c of a filter of size 8 m + 1 - 2 kLead, whose windows start
-// kLead pixels early.
-template <int kLead, class Fn>
+// The taps of chunk c of Window<k>'s chunks 0 .. m.
+template <int k, class Fn>
 RTX_DEV void chunk_taps(int c, int m, Fn f) {
-  constexpr int kN = kSepR;
+  constexpr int kN = kSepR, kLead = Window<k>::kLead, kTail = Window<k>::kTail;
   if (c == 0) {
-    if (m == 1)
-      f(Taps<kLead, kN - kLead, kLead>());
+    if (k == 0 && m == 0)
+      f(Taps<0, 0, 0>());
+    else if (m == 1)
+      f(Taps<kLead, kN - kTail, kLead>());
     else
       f(Taps<kLead, kN - 1, kLead>());
   } else if (c == m) {
     if (m == 1)
-      f(Taps<kLead - kN, -kLead, kLead>());
+      f(Taps<kLead - kN, -kTail, kLead>());
     else
-      f(Taps<1 - kN, -kLead, kLead>());
-  } else if (kLead < 2 || (c > 1 && c < m - 1)) {
+      f(Taps<1 - kN, -kTail, kLead>());
+  } else if ((kLead < 2 || c > 1) && (kTail < 2 || c < m - 1)) {
     f(Taps<1 - kN, kN - 1, kLead>());
   } else if (c > 1) {
-    f(Taps<1 - kN, kN - kLead, kLead>());
+    f(Taps<1 - kN, kN - kTail, kLead>());
   } else if (c < m - 1) {
     f(Taps<kLead - kN, kN - 1, kLead>());
   } else {
-    f(Taps<kLead - kN, kN - kLead, kLead>());
+    f(Taps<kLead - kN, kN - kTail, kLead>());
   }
 }
 
-template <bool kFma, class Px>
+template <int k, bool kFma, class Px>
 RTX_DEV void sep_window(SepAcc& A, const float* __restrict__ wsm, int size, float negzero, Px px) {
   const f2_t nz = f2_pack(negzero, negzero);
 #pragma unroll
   for (int c = 0; c < 3; ++c)
 #pragma unroll
     for (int q = 0; q < kSepQ; ++q) A.v[c][q] = f2_pack(0.0f, 0.0f);
-  const int nj = size + kSepR - 1;
-  for (int j0 = 0; j0 < nj; j0 += kSepR) {
-    if (j0 >= kSepR - 1 && j0 + kSepR - 1 < size)
-      sep_chunk<TapsAll, kFma>(A, wsm, size, j0, nj, nz, px);
-    else
-      sep_chunk<TapsTest, kFma>(A, wsm, size, j0, nj, nz, px);
-  }
+  const int m = window_chunks(size, Window<k>::kLead);
+  for (int c = 0; c <= m; ++c)
+    chunk_taps<k>(c, m, [&](auto taps) { sep_chunk<decltype(taps), kFma>(A, wsm, size, kSepR * c, nz, px); });
 }
 
 // Horizontal pass (1 x size kernel): a block computes kRowTile pixels of one
@@ -358,17 +360,18 @@ RTX_DEV void sep_window(SepAcc& A, const float* __restrict__ wsm, int size, floa
 constexpr int kRowThreads = 128, kRowTile = kRowThreads * kSepR;
 RTX_DEV int row_slot(int i) { return 3 * (i + i / kSepR); }
 
-template <bool kFma>
+template <int k, bool kFma>
 __global__ void __launch_bounds__(kRowThreads, 8) k_gauss_x(const float* __restrict__ in,
                                                          float* __restrict__ out, int W, int H,
                                                          const float* __restrict__ w, int size,
                                                          int extract_mode, float thr, float negzero) {
   extern __shared__ float sm[];
   float* wsm = sm;                       // size weights
-  float* tile = sm + ((size + 3) & ~3);  // row_slot(kRowTile + size - 1) floats
-  const int y = blockIdx.y, x0 = blockIdx.x * kRowTile, r = size >> 1, tid = threadIdx.x;
+  float* tile = sm + ((size + 3) & ~3);  // row_slot(kRowTile + halo) floats
+  const int y = blockIdx.y, x0 = blockIdx.x * kRowTile, tid = threadIdx.x;
+  const int r = (size >> 1) + Window<k>::kLead;
   const int n_out = min(kRowTile, W - x0);
-  const int span = n_out + size - 1, cap = kRowTile + size - 1;
+  const int halo = kSepR * window_chunks(size, Window<k>::kLead), span = n_out + halo, cap = kRowTile + halo;
   for (int j = tid; j < size; j += kRowThreads) wsm[j] = w[j];
   for (int j = tid; j < cap; j += kRowThreads)
     stage_px(tile + row_slot(j), in, j < span ? reflect_index(y, (long long)x0 - r + j, W, H) : -1);
@@ -386,7 +389,7 @@ __global__ void __launch_bounds__(kRowThreads, 8) k_gauss_x(const float* __restr
   SepAcc acc;
   const int b = kSepR * tid;
   if (b < n_out) {
-    sep_window<kFma>(acc, wsm, size, negzero, [&](int j) {
+    sep_window<k, kFma>(acc, wsm, size, negzero, [&](int j) {
       const float* s = tile + row_slot(b + j);
       return f3(s[0], s[1], s[2]);
     });
@@ -415,7 +418,7 @@ __global__ void __launch_bounds__(kRowThreads, 8) k_gauss_x(const float* __restr
 // from a shared-memory strip of kColH + size - 1 rows.
 constexpr int kColW = 32, kColThreads = 128, kColH = (kColThreads / kColW) * kSepR;
 
-template <bool kFma>
+template <int k, bool kFma>
 __global__ void __launch_bounds__(kColThreads, 7) k_gauss_y(const float* __restrict__ in,
                                                          const float* __restrict__ orig,
                                                          float* __restrict__ out, int W, int H,
@@ -423,10 +426,11 @@ __global__ void __launch_bounds__(kColThreads, 7) k_gauss_y(const float* __restr
                                                          float negzero) {
   extern __shared__ float sm[];
   float* wsm = sm;
-  float* strip = sm + ((size + 3) & ~3);  // (kColH + size - 1) rows x kColW x 3
-  const int x0 = blockIdx.x * kColW, y0 = blockIdx.y * kColH, r = size >> 1, tid = threadIdx.x;
+  float* strip = sm + ((size + 3) & ~3);  // rows x kColW x 3
+  const int x0 = blockIdx.x * kColW, y0 = blockIdx.y * kColH, tid = threadIdx.x;
+  const int r = (size >> 1) + Window<k>::kLead;
   for (int j = tid; j < size; j += kColThreads) wsm[j] = w[j];
-  const int rows = kColH + size - 1;
+  const int rows = kColH + kSepR * window_chunks(size, Window<k>::kLead);
   for (int e = tid; e < rows * kColW; e += kColThreads) {
     const int rr = e / kColW, cc = e - rr * kColW;
     const int x = x0 + cc;
@@ -438,7 +442,7 @@ __global__ void __launch_bounds__(kColThreads, 7) k_gauss_y(const float* __restr
   const int x = x0 + cc, yb = y0 + kSepR * g;
   if (x >= W || yb >= H) return;
   SepAcc acc;
-  sep_window<kFma>(acc, wsm, size, negzero, [&](int j) {
+  sep_window<k, kFma>(acc, wsm, size, negzero, [&](int j) {
     const float* s = strip + 3 * ((kSepR * g + j) * kColW + cc);
     return f3(s[0], s[1], s[2]);
   });
@@ -458,9 +462,8 @@ __global__ void __launch_bounds__(kColThreads, 7) k_gauss_y(const float* __restr
 
 // ---------------------------------------------------------------------------
 // The separable passes on 16-byte accesses: images whose rows are a multiple
-// of four pixels (48 bytes) and, across, odd sizes.  Same
-// taps in the same order with the same roundings; what differs is how pixels
-// reach the registers.  The passes are FP32-issue bound (7.7 us each for 49
+// of four pixels (48 bytes).  Same taps in the same order with the same
+// roundings; what differs is how pixels reach the registers.  The passes are FP32-issue bound (7.7 us each for 49
 // taps at 1,024^2); the 4-byte staging copies with their 64-bit reflection
 // arithmetic, three scalar shared loads and six register moves per pixel, and
 // loads that all finished before any arithmetic began cost as much again.
@@ -490,20 +493,21 @@ RTX_DEV void st_row(float* p, const float* v, bool wide) {  // 24 floats
 // first tap.
 constexpr int kRowGroup = 28;
 
-template <int kLead, bool kFma>
+template <int k, bool kFma>
 __global__ void __launch_bounds__(kRowThreads, 7) k_gauss_x16(const float* __restrict__ in, float* __restrict__ out,
                                                              int W, int H, const float* __restrict__ w, int size,
                                                              int extract_mode, float thr, float negzero, int wide) {
   extern __shared__ __align__(16) float sm[];
   float* wsm = sm;
   float* tile = sm + ((size + 3) & ~3);
-  const int y = blockIdx.y, x0 = blockIdx.x * kRowTile, r = size >> 1, tid = threadIdx.x;
-  const int m = (size + 2 * kLead) >> 3, n_out = min(kRowTile, W - x0), groups = (n_out + 7) / 8 + m;
+  const int y = blockIdx.y, x0 = blockIdx.x * kRowTile, tid = threadIdx.x;
+  const int r = (size >> 1) + Window<k>::kLead;
+  const int m = window_chunks(size, Window<k>::kLead), n_out = min(kRowTile, W - x0), groups = (n_out + 7) / 8 + m;
   for (int j = tid; j < size; j += kRowThreads) wsm[j] = w[j];
-  // chunk c: floats 4 c .. 4 c + 3 from pixel x0 - r - kLead on; the row's ends fall on
+  // chunk c: floats 4 c .. 4 c + 3 from pixel x0 - r on; the row's ends fall on
   // chunk boundaries
   const float* row = in + 3 * (size_t)W * y;
-  const int f0 = 3 * (x0 - r - kLead), f1 = 3 * W;
+  const int f0 = 3 * (x0 - r), f1 = 3 * W;
   const unsigned td = (unsigned)__cvta_generic_to_shared(tile);
   for (int c = tid; c < 6 * groups; c += kRowThreads) {
     const int f = f0 + 4 * c, d = (c / 6) * kRowGroup + (c % 6) * 4;
@@ -511,10 +515,10 @@ __global__ void __launch_bounds__(kRowThreads, 7) k_gauss_x16(const float* __res
       cp16(td + 4 * d, row + f);
     } else {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int g = f + k + 3 * (size + 3), x = g / 3 - (size + 3);  // floor for negative f
+      for (int e = 0; e < 4; ++e) {
+        const int g = f + e + 3 * (size + 3), x = g / 3 - (size + 3);  // floor for negative f
         const long long idx = reflect_index(y, x, W, H);
-        tile[d + k] = idx < 0 ? 0.0f : __ldg(in + 3 * idx + (g - 3 * (g / 3)));
+        tile[d + e] = idx < 0 ? 0.0f : __ldg(in + 3 * idx + (g - 3 * (g / 3)));
       }
     }
   }
@@ -542,16 +546,16 @@ __global__ void __launch_bounds__(kRowThreads, 7) k_gauss_x16(const float* __res
     const float4* s = reinterpret_cast<const float4*>(tile + (tid + c) * kRowGroup);
     float px[24];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      const float4 v = s[k];
-      px[4 * k] = v.x;
-      px[4 * k + 1] = v.y;
-      px[4 * k + 2] = v.z;
-      px[4 * k + 3] = v.w;
+    for (int e = 0; e < 6; ++e) {
+      const float4 v = s[e];
+      px[4 * e] = v.x;
+      px[4 * e + 1] = v.y;
+      px[4 * e + 2] = v.z;
+      px[4 * e + 3] = v.w;
     }
     const int j0 = kSepR * c;
-    chunk_taps<kLead>(c, m, [&](auto taps) {
-      sep_chunk<decltype(taps), kFma>(A, wsm, size, j0, 0, nz, [&](int j) {
+    chunk_taps<k>(c, m, [&](auto taps) {
+      sep_chunk<decltype(taps), kFma>(A, wsm, size, j0, nz, [&](int j) {
         return f3(px[3 * (j - j0)], px[3 * (j - j0) + 1], px[3 * (j - j0) + 2]);
       });
     });
@@ -559,17 +563,17 @@ __global__ void __launch_bounds__(kRowThreads, 7) k_gauss_x16(const float* __res
   float* o = out + 3 * ((size_t)y * W + x0 + b);
   float v[24];
 #pragma unroll
-  for (int k = 0; k < kSepR; ++k) {
-    const F3 p = A.out(k);
-    v[3 * k] = p.x;
-    v[3 * k + 1] = p.y;
-    v[3 * k + 2] = p.z;
+  for (int e = 0; e < kSepR; ++e) {
+    const F3 p = A.out(e);
+    v[3 * e] = p.x;
+    v[3 * e + 1] = p.y;
+    v[3 * e + 2] = p.z;
   }
   if (b + kSepR <= n_out) {
     st_row(o, v, wide != 0);
   } else {  // n_out is a multiple of four pixels
 #pragma unroll
-    for (int k = 0; k < 12; k += 4) *reinterpret_cast<float4*>(o + k) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    for (int e = 0; e < 12; e += 4) *reinterpret_cast<float4*>(o + e) = make_float4(v[e], v[e + 1], v[e + 2], v[e + 3]);
   }
 }
 
@@ -591,7 +595,7 @@ RTX_DEV void col_chunk(f2_t (&acc)[2][kSepR], const float* __restrict__ wsm, int
     const f2_t a = f2_pack(v.x, v.y), b = f2_pack(v.z, v.w);
 #pragma unroll
     for (int o = 0; o < kSepR; ++o) {
-      if (T::in(k, o, j0, size)) {
+      if (T::in(k, o)) {
         const float ww = wv[k - o + kSepR - 1];
         const f2_t w2 = f2_pack(ww, ww);
         acc[0][o] = f2_tap<kFma>(acc[0][o], a, w2, nz);
@@ -603,19 +607,18 @@ RTX_DEV void col_chunk(f2_t (&acc)[2][kSepR], const float* __restrict__ wsm, int
 
 // The image bloom adds back is fetched into staged rows no warp reads any
 // more, two chunks before it is needed.
-// kLead < 0: an even size, whose edge chunks test their taps.
-template <int kLead, bool kFma>
+template <int k, bool kFma>
 __global__ void __launch_bounds__(kCol16Threads, 5) k_gauss_y16(const float* __restrict__ in,
                                                                const float* __restrict__ orig, float* __restrict__ out,
                                                                int W, int H, const float* __restrict__ w, int size,
                                                                float negzero) {
   extern __shared__ __align__(16) float sm[];
   float4* strip = reinterpret_cast<float4*>(sm);  // chunks * kSepR rows x kColQ
-  const int nc = (size + 2 * kSepR - 2) / kSepR;  // chunks of a window, kLead or not
+  const int nc = window_chunks(size, Window<k>::kLead) + 1;
   const int chunks = nc + kCol16Groups - 1;
   float* wsm = sm + 4 * (size_t)chunks * kSepR * kColQ;
   const int tid = threadIdx.x, q = tid % kColQ, g = tid / kColQ;
-  const int nq = 3 * W / 4, q0 = blockIdx.x * kColQ, y0 = blockIdx.y * kCol16H, r = (size >> 1) + max(kLead, 0);
+  const int nq = 3 * W / 4, q0 = blockIdx.x * kColQ, y0 = blockIdx.y * kCol16H, r = (size >> 1) + Window<k>::kLead;
   for (int j = tid; j < size; j += kCol16Threads) wsm[j] = w[j];
   const bool live = q0 + q < nq;
   const unsigned sd = (unsigned)__cvta_generic_to_shared(strip);
@@ -623,13 +626,13 @@ __global__ void __launch_bounds__(kCol16Threads, 5) k_gauss_y16(const float* __r
   auto stage = [&](int c) {  // rows 8 c .. 8 c + 7; warp g takes two of them
     if (c < chunks)
 #pragma unroll
-      for (int k = g; k < kSepR; k += kCol16Groups) {
-        int yy = abs(y0 - r + kSepR * c + k);
+      for (int e = g; e < kSepR; e += kCol16Groups) {
+        int yy = abs(y0 - r + kSepR * c + e);
         if (yy >= H) yy = 2 * H - yy;
         if (live && yy >= 0 && yy < H)
-          cp16(sd + 16 * ((kSepR * c + k) * kColQ + q), col + (size_t)yy * nq);
+          cp16(sd + 16 * ((kSepR * c + e) * kColQ + q), col + (size_t)yy * nq);
         else
-          strip[(kSepR * c + k) * kColQ + q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+          strip[(kSepR * c + e) * kColQ + q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -657,13 +660,7 @@ __global__ void __launch_bounds__(kCol16Threads, 5) k_gauss_y16(const float* __r
     }
     const int j0 = c * kSepR;
     const float4* s = strip + (size_t)(kSepR * (g + c)) * kColQ + q;
-    if (kLead >= 0)
-      chunk_taps<kLead < 0 ? 0 : kLead>(
-          c, nc - 1, [&](auto taps) { col_chunk<decltype(taps), kFma>(acc, wsm, size, j0, nz, s); });
-    else if (j0 >= kSepR - 1 && j0 + kSepR - 1 < size)
-      col_chunk<TapsAll, kFma>(acc, wsm, size, j0, nz, s);
-    else
-      col_chunk<TapsTest, kFma>(acc, wsm, size, j0, nz, s);
+    chunk_taps<k>(c, nc - 1, [&](auto taps) { col_chunk<decltype(taps), kFma>(acc, wsm, size, j0, nz, s); });
   }
   cp_wait_all();
   if (!live) return;
@@ -749,32 +746,35 @@ cudaError_t launch_convolve(const float* in, float* out, int W, int H, const flo
   return cudaGetLastError();
 }
 
+// pixels of a window beyond its first output's: kSepR m
+static size_t window_halo(int size) { return (size_t)((size | 1) + 2 * (window_kind(size) & 3)) / 8 * 8; }
 static size_t smem_x(int size) {
-  const size_t cap = (size_t)kRowTile + size - 1;
+  const size_t cap = (size_t)kRowTile + window_halo(size);
   return sizeof(float) * (((size_t)size + 3 & ~(size_t)3) + 3 * (cap + cap / kSepR));
 }
 static size_t smem_y(int size) {
-  return sizeof(float) * (((size_t)size + 3 & ~(size_t)3) + 3 * ((size_t)kColH + size - 1) * kColW);
+  return sizeof(float) * (((size_t)size + 3 & ~(size_t)3) + 3 * ((size_t)kColH + window_halo(size)) * kColW);
 }
 
-// The 16-byte passes' instance for a lead (kLead).
-static decltype(&k_gauss_x16<0, false>) by_lead_x(int lead, bool fma) {
-  switch (lead) {
-    case 0: return fma ? k_gauss_x16<0, true> : k_gauss_x16<0, false>;
-    case 1: return fma ? k_gauss_x16<1, true> : k_gauss_x16<1, false>;
-    case 2: return fma ? k_gauss_x16<2, true> : k_gauss_x16<2, false>;
-    default: return fma ? k_gauss_x16<3, true> : k_gauss_x16<3, false>;
+// A separable pass' instance for a size.
+#define RTX_BY_SIZE(name, kernel)                               \
+  static decltype(&kernel<0, false>) name(int size, bool fma) { \
+    switch (window_kind(size)) {                                \
+      case 0: return fma ? kernel<0, true> : kernel<0, false>;  \
+      case 1: return fma ? kernel<1, true> : kernel<1, false>;  \
+      case 2: return fma ? kernel<2, true> : kernel<2, false>;  \
+      case 3: return fma ? kernel<3, true> : kernel<3, false>;  \
+      case 4: return fma ? kernel<4, true> : kernel<4, false>;  \
+      case 5: return fma ? kernel<5, true> : kernel<5, false>;  \
+      case 6: return fma ? kernel<6, true> : kernel<6, false>;  \
+      default: return fma ? kernel<7, true> : kernel<7, false>; \
+    }                                                           \
   }
-}
-static decltype(&k_gauss_y16<0, false>) by_lead_y(int lead, bool fma) {
-  switch (lead) {
-    case 0: return fma ? k_gauss_y16<0, true> : k_gauss_y16<0, false>;
-    case 1: return fma ? k_gauss_y16<1, true> : k_gauss_y16<1, false>;
-    case 2: return fma ? k_gauss_y16<2, true> : k_gauss_y16<2, false>;
-    case 3: return fma ? k_gauss_y16<3, true> : k_gauss_y16<3, false>;
-    default: return fma ? k_gauss_y16<-1, true> : k_gauss_y16<-1, false>;
-  }
-}
+RTX_BY_SIZE(gauss_x, k_gauss_x)
+RTX_BY_SIZE(gauss_y, k_gauss_y)
+RTX_BY_SIZE(gauss_x16, k_gauss_x16)
+RTX_BY_SIZE(gauss_y16, k_gauss_y16)
+#undef RTX_BY_SIZE
 
 // GaussianBlur(size) on `in` (extract_mode: bloom's Extract fused into the
 // first pass, and the second pass adds `in` back: Image::Bloom).
@@ -785,7 +785,7 @@ cudaError_t launch_gaussian(const float* in, float* tmp, float* tmp2, float* out
                             const float* d_w, int size, int extract_mode, float threshold, bool fma,
                             cudaStream_t st, int* launches) {
   cudaError_t e;
-  size_t sx = smem_x(size), sy = smem_y(size);
+  const size_t sx = smem_x(size), sy = smem_y(size);
   const size_t kMaxSmem = 227 * 1024;
   size_t n = (size_t)W * H;
   if (extract_mode && (sx > kMaxSmem || sy > kMaxSmem)) {
@@ -797,22 +797,21 @@ cudaError_t launch_gaussian(const float* in, float* tmp, float* tmp2, float* out
     *launches += 4;
     return cudaGetLastError();
   }
-  // 16-byte forms: rows of a multiple of four pixels, 16-byte aligned images,
-  // and (across) an odd size
+  // 16-byte forms: rows of a multiple of four pixels, 16-byte aligned images
+  // (size 3 at 64^2: 17.8 -> 15.8 us per call, 49 at 1,024^2: 31 -> 22.4)
   auto al = [](const void* p, uintptr_t m) { return (reinterpret_cast<uintptr_t>(p) & (m - 1)) == 0; };
   const bool quads = W % 4 == 0 && al(in, 16) && al(tmp, 16) && al(out, 16);
-  const int lead = size % 2 == 0 ? -1 : (4 - (size >> 1) % 4) % 4;
   const size_t ws16 = (size_t)size + 3 & ~(size_t)3;
-  const size_t sx16 = sizeof(float) * (ws16 + (size_t)kRowGroup * (kRowTile / 8 + (size + 6) / 8));
-  const size_t sy16 = sizeof(float) * (ws16 + 4 * (size_t)kColQ * kSepR * ((size + 2 * kSepR - 2) / kSepR + kCol16Groups - 1));
-  if (quads && lead >= 0 && size > 1 && sx16 <= kMaxSmem) {
-    auto kx = by_lead_x(lead, fma);
+  const size_t sx16 = sizeof(float) * (ws16 + kRowGroup * ((size_t)kRowTile + window_halo(size)) / 8);
+  const size_t sy16 = sizeof(float) * (ws16 + 4 * (size_t)kColQ * (kCol16H + window_halo(size)));
+  if (quads && sx16 <= kMaxSmem) {
+    auto kx = gauss_x16(size, fma);
     if (sx16 > 48 * 1024 && (e = cudaFuncSetAttribute(kx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx16)))
       return e;
     kx<<<dim3((W + kRowTile - 1) / kRowTile, H), kRowThreads, sx16, st>>>(in, tmp, W, H, d_w, size, extract_mode,
                                                                          threshold, -0.0f, W % 8 == 0 && al(tmp, 32));
   } else if (sx <= kMaxSmem) {
-    auto kx = fma ? k_gauss_x<true> : k_gauss_x<false>;
+    auto kx = gauss_x(size, fma);
     if (sx > 48 * 1024 && (e = cudaFuncSetAttribute(kx, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sx)))
       return e;
     kx<<<dim3((W + kRowTile - 1) / kRowTile, H), kRowThreads, sx, st>>>(in, tmp, W, H, d_w, size, extract_mode,
@@ -822,13 +821,13 @@ cudaError_t launch_gaussian(const float* in, float* tmp, float* tmp2, float* out
   }
   ++*launches;
   if (quads && sy16 <= kMaxSmem) {
-    auto ky = by_lead_y(size > 1 ? lead : -1, fma);
+    auto ky = gauss_y16(size, fma);
     if (sy16 > 48 * 1024 && (e = cudaFuncSetAttribute(ky, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sy16)))
       return e;
     ky<<<dim3((3 * W / 4 + kColQ - 1) / kColQ, (H + kCol16H - 1) / kCol16H), kCol16Threads, sy16, st>>>(
         tmp, extract_mode ? in : nullptr, out, W, H, d_w, size, -0.0f);
   } else if (sy <= kMaxSmem) {
-    auto ky = fma ? k_gauss_y<true> : k_gauss_y<false>;
+    auto ky = gauss_y(size, fma);
     if (sy > 48 * 1024 && (e = cudaFuncSetAttribute(ky, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sy)))
       return e;
     ky<<<dim3((W + kColW - 1) / kColW, (H + kColH - 1) / kColH), kColThreads, sy, st>>>(

@@ -1,12 +1,10 @@
-"""The separable filters' 16-byte passes, bit for bit against the oracle.
-
-The shapes sit where the passes can go wrong: widths that are a multiple of
-four pixels but not of eight, around the 1,024-pixel row tiles; heights around
-the 32-row strips; images smaller than the filter (RenderToy's reflection wraps
-into the neighbouring row there); odd sizes of each remainder, whose first and
-last window chunks are known at compile time, and even ones, which take the
-16-byte pass only down the columns; NaN and infinite pixels; an image that starts
-off a 16-byte boundary, which takes the 4-byte passes.
+"""The separable filters, bit for bit against the oracle where their passes can go
+wrong: widths that are a multiple of four pixels but not of eight, around the
+1,024-pixel row tiles; heights around the 32-row strips; images smaller than
+the filter (RenderToy's reflection wraps into the neighbouring row there);
+sizes of each remainder, whose first and last window chunks are known at
+compile time; NaN and infinite pixels; an image that starts off a 16-byte
+boundary or has rows of another length, which take the 4-byte passes.
 """
 import numpy as np
 import pytest
@@ -15,7 +13,7 @@ from helpers import bits
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1, 2, 3, 5, 7, 8, 9, 11, 13, 15, 17, 19, 21, 27, 29, 31, 33, 49, 101]
+SIZES = [1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 21, 22, 24, 27, 29, 32, 49, 101]
 
 
 def same(gpu, orc, what):
@@ -24,7 +22,7 @@ def same(gpu, orc, what):
     assert np.array_equal(bits(gpu)[~nan], bits(orc)[~nan]), what
 
 
-@pytest.mark.parametrize("shape", [(1, 4), (3, 12), (31, 8), (33, 44), (65, 36), (5, 1020), (2, 1024), (9, 1028),
+@pytest.mark.parametrize("shape", [(1, 1), (3, 13), (33, 31), (65, 33), (5, 1023), (9, 1030), (31, 2061), (1, 4), (3, 12), (31, 8), (33, 44), (65, 36), (5, 1020), (2, 1024), (9, 1028),
                                    (32, 2052)])
 def test_quad_passes_bit_exact(ctx, oracle, shape):
     import torch
