@@ -1,5 +1,6 @@
 // nn_conv.cu — 3 x 3 convolutions of the denoiser as implicit GEMMs on the
-// tcgen05 tensor cores (BF16 operands, FP32 accumulation in TMEM).
+// tcgen05 tensor cores (BF16 operands, FP32 accumulation in TMEM): the choice
+// of kernel, and the kernels for channel counts the tiles do not take.
 //
 // Tensors are NHWC BF16 with channel counts padded to multiples of 8.  A
 // convolution reads one or two sources: s1 (optionally at half resolution,
@@ -21,13 +22,13 @@
 // off(t) = (t / 3 - 1, t % 3 - 1).  Out-of-image taps read zero ("same"
 // zero padding).
 //
-// Pipeline (all three): the K (or pixel) range is cut into slices of 64;
-// every thread copies its 16-byte chunks of a slice straight into shared
-// memory with cp.async (zero-filled where the tap falls outside the image),
-// S - 1 slices ahead, into a ring of S stages.  Thread 0 issues the slice's
-// MMAs and commits them to the stage's mbarrier; a stage is refilled once the
-// MMAs that read it have completed.  The gathers of later slices therefore
-// overlap the MMAs of earlier ones, and no thread stalls on its own loads.
+// Channel counts that are multiples of 16 run as tiles (nn_conv_tile.cu,
+// nn_wgrad_tile.cu).  The gather kernels here: the K (or pixel) range is cut
+// into slices of 64; every thread copies its 16-byte chunks of a slice straight
+// into shared memory with cp.async (zero-filled where the tap falls outside
+// the image), S - 1 slices ahead, into a ring of S stages.  Thread 0 issues the
+// slice's MMAs and commits them to the stage's mbarrier; a stage is refilled
+// once the MMAs that read it have completed.
 #include <algorithm>
 
 #include "nn.h"

@@ -33,9 +33,9 @@ class UNet {
   cudaError_t set_state(const float* host_m, const float* host_v, int step, cudaStream_t st);
 
   // raw [N*H*W][kRawCh] = radiance 3, albedo 3, normal 3, depth 1, spp 1 (FP32)
-  // (nullptr: the encoded input is already in input()).  With a head the
-  // output layer applies it to its logits; *fused tells whether it could (else
-  // the logits are in prediction()).
+  // (nullptr: the input tensor already holds the encoded input).  With a head
+  // the output layer applies it to its logits; *fused tells whether it could
+  // (else the logits are in the output layer's tensor).
   cudaError_t forward(const float* d_raw, int N, int H, int W, int* err, cudaStream_t st,
                       const KpHead* head = nullptr, bool* fused = nullptr);
   // gradients of the loss of the last forward (d_pred set by the loss)
