@@ -116,10 +116,13 @@ struct rtx_context {
   DeviceScene bds{};
   DevBuf b_nodes, b_nodes4, b_tris, b_shade, b_geo, b_mats, b_emit, b_jobs, b_jobq;
   std::vector<BatchScene> bscenes;
-  // CUDA graph of the last batch frame, keyed by its launch shape
+  // CUDA graph of the last batch frame, keyed by its launch shape and the
+  // buffers whose addresses its kernels hold (the path workspace's by its
+  // generation: any render of this context may move it)
   bool use_graph = false;
   cudaGraphExec_t graph = nullptr;
   std::vector<int64_t> graph_key;
+  long long graph_generation = 0;
   PtJob* h_jobs_pinned = nullptr;
   long long* h_jobq_pinned = nullptr;
   int pinned_cap = 0;
@@ -1206,16 +1209,17 @@ int rtx_render_batch(rtx_context* c, int n_jobs, const rtx_job* jobs, int max_de
   p.h_jobs = hj.data();
   RTX_CUDA(cudaMemsetAsync(c->d_counters, 0, sizeof(Counters), c->stream), "reset counters");
   c->timer.reset();
-  // the launch shape: everything the captured kernels bake in
+  // the launch shape and addresses: everything the captured kernels bake in
   std::vector<int64_t> key = {n_jobs, max_depth, c->wave_paths, c->block, c->primary_cache, c->count_visits,
                               c->accumulate, (int64_t)p.sort_material, (int64_t)p.sort_rays, c->traversal, c->overlap,
-                              c->stack_limit, (int64_t)(intptr_t)o.dev};
+                              c->stack_limit, (int64_t)(intptr_t)o.dev, (int64_t)(intptr_t)p.d_jobs,
+                              (int64_t)(intptr_t)p.d_job_q};
   for (int j = 0; j < n_jobs; ++j) key.insert(key.end(), {jobs[j].scene, jobs[j].W, jobs[j].H, jobs[j].spp});
   int launches = 0, ext_launches = 0, vtx_launches = 0;
   std::string why;
   cudaError_t e = cudaSuccess;
   const bool graphable = c->use_graph && !c->timer.on;
-  if (graphable && c->graph && key == c->graph_key) {
+  if (graphable && c->graph && key == c->graph_key && c->graph_generation == pt_generation(c->pt)) {
     e = cudaGraphLaunch(c->graph, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "cudaGraphLaunch");
     c->stats.kernel_launches = 0;  // kernels are graph nodes
@@ -1255,6 +1259,7 @@ int rtx_render_batch(rtx_context* c, int n_jobs, const rtx_job* jobs, int max_de
         return cuda_fail(c, ee, "cudaGraphInstantiate");
       }
       c->graph_key = key;
+      c->graph_generation = pt_generation(c->pt);
     }
   }
   if ((r = copy_back(c, o))) return r;

@@ -102,9 +102,11 @@ struct PtWorkspace {
   int num_sms = 0;
   int occ_extend = 0, occ_connect = 0, block_cached = 0;
   long long last_wave = 0;  // paths per wave of the last render
+  long long generation = 0;  // counts reallocations: a captured launch holds the buffers' addresses
 };
 
 long long pt_last_wave(const PtWorkspace* ws) { return ws->last_wave; }
+long long pt_generation(const PtWorkspace* ws) { return ws->generation; }
 
 PtWorkspace* pt_workspace_create() { return new PtWorkspace(); }
 
@@ -142,6 +144,7 @@ void pt_workspace_destroy(PtWorkspace* ws) {
 
 static cudaError_t ws_reserve(PtWorkspace* w, size_t cap) {
   if (w->cap >= cap && w->counters) return cudaSuccess;
+  ++w->generation;
   ws_free(w);
   cudaError_t e;
   float4** f[] = {&w->ray_o, &w->ray_d, &w->thr, &w->rad, &w->absb, &w->hit};
@@ -1402,6 +1405,7 @@ cudaError_t pt_render(PtWorkspace* ws, const DeviceScene& s, const CamParams& ca
   const float4* prim = nullptr;
   if (p.primary_cache) {
     if (ws->prim_cap < (size_t)npix) {
+      ++ws->generation;
       if (ws->prim) cudaFree(ws->prim);
       ws->prim = nullptr;
       ws->prim_cap = 0;

@@ -241,6 +241,7 @@ struct PtParams {
 };
 PtWorkspace* pt_workspace_create();
 long long pt_last_wave(const PtWorkspace* ws);
+long long pt_generation(const PtWorkspace* ws);  // changes whenever one of its buffers moves
 void pt_workspace_destroy(PtWorkspace* ws);
 cudaError_t pt_render(PtWorkspace* ws, const DeviceScene& s, const CamParams& cam,
                       const PtParams& p, float* d_out, int* err, Counters* d_counters,
