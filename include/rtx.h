@@ -374,8 +374,9 @@ int rtx_probe_read_bandwidth(rtx_context* ctx, size_t bytes, int passes,
 
 /* Diagnostic, no RenderToy counterpart: one block waits on a shared-memory
  * mbarrier that nothing arrives on, through the bounded wait every
- * tensor-core kernel uses, giving up after `polls` polls (1..2^20).  The
- * call then returns what such a kernel's failed wait returns:
+ * tensor-core kernel uses, giving up after `polls` polls (1..2^20), and
+ * groups of four warps that share a barrier per tile lose one warp's wait.
+ * The call then returns what such a kernel's failed wait returns:
  * RTX_ERR_DEVICE with "tensor-core barrier wait timed out", and the context
  * stays usable. */
 int rtx_selftest_wait_timeout(rtx_context* ctx, int polls);

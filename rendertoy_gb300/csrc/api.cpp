@@ -1653,8 +1653,8 @@ int rtx_selftest_wait_timeout(rtx_context* c, int polls) {
   if (polls < 1 || polls > (1 << 20)) return fail(c, RTX_ERR_INVALID, "polls must be in [1, 2^20]");
   int r;
   if ((r = begin(c))) return r;
-  RTX_CUDA(launch_wait_timeout(polls, c->d_err, c->stream), "wait kernel");
-  c->stats.kernel_launches = 1;
+  RTX_CUDA(launch_wait_timeout(polls, c->d_err, c->stream), "wait kernels");
+  c->stats.kernel_launches = 2;
   return finish(c, false);
 }
 

@@ -369,6 +369,8 @@ __device__ __forceinline__ void head_load(const TileArgs& a, const Tile& t, int 
   }
 }
 
+// The group's previous tile must be behind it (its taps are read).  Returns
+// false when this warp's wait ran out.
 template <int kHead, class Next, class Wait, class Release>
 __device__ __forceinline__ bool head_epilogue(const TileArgs& a, const Tile& t, uint32_t tmem, int warp, int lane,
                                               float4* rad, const float* bias, HeadIn& in, double& loss, Next&& next,
@@ -379,7 +381,6 @@ __device__ __forceinline__ bool head_epilogue(const TileArgs& a, const Tile& t, 
   const int x = t.x0 + mx, y = t.y0 + my;
   const bool ok = x < h.Wc && y < h.Hc;
   const size_t p = ((size_t)t.n * a.H + y) * a.W + x, pc = ((size_t)t.n * h.Hc + y) * h.Wc + x;
-  asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");  // the previous tile's taps are read
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int i = tid + 128 * j, yy = i / 12, xx = i - 12 * yy;
@@ -389,7 +390,7 @@ __device__ __forceinline__ bool head_epilogue(const TileArgs& a, const Tile& t, 
   const float tgt[3] = {in.tgt[0], in.tgt[1], in.tgt[2]};
   asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");
   next(in);
-  const bool w = wait();
+  if (!wait()) return false;
   float v[32];
   tmem_ld32(tmem + ((uint32_t)(q * 32) << 16), v);
   release();
@@ -407,7 +408,7 @@ __device__ __forceinline__ bool head_epilogue(const TileArgs& a, const Tile& t, 
     for (int o = 16; o > 0; o >>= 1) part += __shfl_down_sync(0xffffffffu, part, o);
     loss += (double)part;
   }
-  return w;
+  return true;
 }
 
 // The epilogue of accumulators [acc0, acc1) of a tile for one warp (its 32
@@ -687,7 +688,9 @@ __global__ void __launch_bounds__(kThreadsT, 1) k_conv_tile(const TileArgs a, co
       TileIter it(a, (int)(blockIdx.x + g0 * gridDim.x), groups * (int)gridDim.x);
       HeadIn in{};
       if (kHead && g0 < n_tiles) head_load<kHead>(a, it.tile(kTH), warp, lane, in);
-      for (int i = g0; i < n_tiles && ok; i += groups) {
+      for (int i = g0; i < n_tiles && (kHead || ok); i += groups) {
+        // the head's warps share barriers within a tile: they leave together
+        if (kHead && !(ok = tc::group_all(1 + g, ok))) break;
         const Tile t = it.tile(kTH);
         it.next(a);
         const int buf = i % a.nbuf, lap = i / a.nbuf;

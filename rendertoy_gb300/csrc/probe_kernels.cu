@@ -59,10 +59,38 @@ __global__ void k_wait_timeout(int polls, int* err) {
   if (!ok && (threadIdx.x & 31) == 0) atomicOr(err, tc::kErrMbarTimeout);
 }
 
+// Four warps that share a barrier per tile, as the fused output layer's do,
+// where the wait of one (warp b of block b, at tile b) runs out while the
+// others' succeed: all must leave at the next tile (kErrBadIndex otherwise).
+__global__ void k_group_timeout(int polls, int* err) {
+  constexpr int kTiles = 8;
+  __shared__ uint64_t never, done;
+  __shared__ int left[4];
+  const int warp = threadIdx.x >> 5, b = blockIdx.x;
+  if (threadIdx.x == 0) {
+    tc::mbar_init(&never, 1);
+    tc::mbar_init(&done, 1);
+    tc::mbar_arrive(&done);  // phase 0 is complete
+  }
+  __syncthreads();
+  bool ok = true;
+  int t = 0;
+  for (; t < kTiles; ++t) {
+    if (!(ok = tc::group_all(1, ok))) break;
+    ok = tc::mbar_wait_bounded(warp == b && t == b ? &never : &done, 0, polls);
+  }
+  if ((threadIdx.x & 31) == 0) left[warp] = t;
+  if (!__syncthreads_and(ok) && threadIdx.x == 0) atomicOr(err, tc::kErrMbarTimeout);
+  if (threadIdx.x == 0)
+    for (int w = 0; w < 4; ++w)
+      if (left[w] != b + 1) atomicOr(err, kErrBadIndex);
+}
+
 }  // namespace
 
 cudaError_t launch_wait_timeout(int polls, int* err, cudaStream_t st) {
   k_wait_timeout<<<1, 64, 0, st>>>(polls, err);
+  k_group_timeout<<<4, 128, 0, st>>>(polls, err);
   return cudaGetLastError();
 }
 

@@ -105,6 +105,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   return mbar_wait_bounded(bar, parity, kWaitLimit);
 }
 
+// The 128 threads of a group of four warps meet at named barrier `id`; true
+// when all of them passed ok.  Warps that wait on an mbarrier each by itself
+// and then share barriers must also agree here before one of them leaves: a
+// warp whose wait alone ran out would otherwise be missing at the next one.
+__device__ __forceinline__ bool group_all(int id, bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.u32 p, %1, 0;\n bar.red.and.pred q, %2, 128, p;\n selp.u32 %0, 1, 0, q;\n}\n"
+      : "=r"(r)
+      : "r"((uint32_t)ok), "r"(id)
+      : "memory");
+  return r != 0;
+}
+
 // Arrive on the barrier and add `bytes` to the transaction count its phase
 // waits for (the bytes of the tensor copies that complete on it).
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
