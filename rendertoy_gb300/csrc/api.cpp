@@ -251,6 +251,7 @@ int finish(rtx_context* c, bool may_async) {
 struct Arg {
   void* dev = nullptr;
   void* host = nullptr;
+  void* moved = nullptr;  // a device output that is staged (bind_out16)
   size_t bytes = 0;
 };
 
@@ -280,9 +281,34 @@ int bind_out(rtx_context* c, void* p, size_t bytes, int slot, Arg& a) {
   return RTX_OK;
 }
 
+// The same for an operand that kernels read or write 16 bytes at a time (BF16
+// tensors): a device pointer off a 16-byte boundary -- a view into a larger
+// tensor -- goes through stage[slot] too.
+bool off16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; }
+
+int bind_in16(rtx_context* c, const void* p, size_t bytes, int slot, Arg& a) {
+  int r = bind_in(c, p, bytes, slot, a);
+  if (r || !off16(a.dev)) return r;
+  RTX_CUDA(c->stage[slot].ensure(bytes), "stage alloc");
+  RTX_CUDA(cudaMemcpyAsync(c->stage[slot].p, p, bytes, cudaMemcpyDeviceToDevice, c->stream), "D2D");
+  a.dev = c->stage[slot].p;
+  return RTX_OK;
+}
+
+int bind_out16(rtx_context* c, void* p, size_t bytes, int slot, Arg& a) {
+  int r = bind_out(c, p, bytes, slot, a);
+  if (r || !off16(a.dev)) return r;
+  RTX_CUDA(c->stage[slot].ensure(bytes), "stage alloc");
+  a.moved = a.dev;
+  a.dev = c->stage[slot].p;
+  return RTX_OK;
+}
+
 int copy_back(rtx_context* c, const Arg& a) {
   if (a.host)
     RTX_CUDA(cudaMemcpyAsync(a.host, a.dev, a.bytes, cudaMemcpyDeviceToHost, c->stream), "D2H");
+  if (a.moved)
+    RTX_CUDA(cudaMemcpyAsync(a.moved, a.dev, a.bytes, cudaMemcpyDeviceToDevice, c->stream), "D2D");
   return RTX_OK;
 }
 
@@ -1751,8 +1777,8 @@ int rtx_nn_gemm_bf16(rtx_context* c, int M, int N, int K, const void* A, const v
   int r;
   if ((r = begin(c))) return r;
   Arg aa, ab, ac;
-  if ((r = bind_in(c, A, (size_t)M * K * 2, 0, aa))) return r;
-  if ((r = bind_in(c, B, (size_t)N * K * 2, 1, ab))) return r;
+  if ((r = bind_in16(c, A, (size_t)M * K * 2, 0, aa))) return r;
+  if ((r = bind_in16(c, B, (size_t)N * K * 2, 1, ab))) return r;
   if ((r = bind_out(c, C, (size_t)M * N * 4, 2, ac))) return r;
   cudaError_t e = launch_gemm_bf16(aa.dev, ab.dev, (float*)ac.dev, M, N, K, a_mn, b_mn, c->d_err, c->stream);
   c->stats.kernel_launches = 1;
@@ -1777,8 +1803,8 @@ static int bind_srcs(rtx_context* c, int N, int H, int W, const void* x1, int C1
                      int C2, int slot, Arg& a1, Arg& a2, rtx::nn::Src& s1, rtx::nn::Src& s2) {
   int r;
   size_t p1 = up1 ? (size_t)N * (H / 2) * (W / 2) : (size_t)N * H * W;
-  if ((r = bind_in(c, x1, p1 * C1 * 2, slot, a1))) return r;
-  if ((r = bind_in(c, x2, (size_t)N * H * W * C2 * 2, slot + 1, a2))) return r;
+  if ((r = bind_in16(c, x1, p1 * C1 * 2, slot, a1))) return r;
+  if ((r = bind_in16(c, x2, (size_t)N * H * W * C2 * 2, slot + 1, a2))) return r;
   s1 = rtx::nn::Src{(const rtx::nn::bf16*)a1.dev, C1, up1 ? 1 : 0};
   s2 = rtx::nn::Src{(const rtx::nn::bf16*)a2.dev, C2, 0};
   return RTX_OK;
@@ -1798,7 +1824,7 @@ int rtx_nn_conv3x3_fwd(rtx_context* c, int N, int H, int W, const void* x1, int 
   Arg a1, a2, aw, ab, ao;
   rtx::nn::Src s1, s2;
   if ((r = bind_srcs(c, N, H, W, x1, C1, up1, x2, C2, 0, a1, a2, s1, s2))) return r;
-  if ((r = bind_in(c, w, (size_t)Cout * 9 * Cin * 2, 2, aw))) return r;
+  if ((r = bind_in16(c, w, (size_t)Cout * 9 * Cin * 2, 2, aw))) return r;
   if ((r = bind_in(c, bias, bias ? (size_t)Cout * 4 : 0, 3, ab))) return r;
   if ((r = bind_out(c, out, P * Cout * 4, 4, ao))) return r;
   rtx::nn::ConvFwd a{};
@@ -1837,9 +1863,9 @@ int rtx_nn_conv3x3_dgrad(rtx_context* c, int N, int H, int W, const void* dout, 
   Arg a1, a2, ad, aw, ao;
   rtx::nn::Src s1, s2;
   if ((r = bind_srcs(c, N, H, W, x1, C1, up1, x2, C2, 0, a1, a2, s1, s2))) return r;
-  if ((r = bind_in(c, dout, P * Cout * 2, 2, ad))) return r;
-  if ((r = bind_in(c, wt, (size_t)Cin * 9 * Cout * 2, 3, aw))) return r;
-  if ((r = bind_out(c, din, P * Cin * 2, 4, ao))) return r;
+  if ((r = bind_in16(c, dout, P * Cout * 2, 2, ad))) return r;
+  if ((r = bind_in16(c, wt, (size_t)Cin * 9 * Cout * 2, 3, aw))) return r;
+  if ((r = bind_out16(c, din, P * Cin * 2, 4, ao))) return r;
   rtx::nn::ConvDgrad a{};
   a.dout = (const rtx::nn::bf16*)ad.dev;
   a.Cout = Cout;
@@ -1874,7 +1900,7 @@ int rtx_nn_conv3x3_wgrad(rtx_context* c, int N, int H, int W, const void* dout, 
   Arg a1, a2, ad, ao;
   rtx::nn::Src s1, s2;
   if ((r = bind_srcs(c, N, H, W, x1, C1, up1, x2, C2, 0, a1, a2, s1, s2))) return r;
-  if ((r = bind_in(c, dout, (size_t)P * Cout * 2, 2, ad))) return r;
+  if ((r = bind_in16(c, dout, (size_t)P * Cout * 2, 2, ad))) return r;
   if ((r = bind_out(c, dw, (size_t)Cout * 9 * Cin * 4, 4, ao))) return r;
   RTX_CUDA(cudaMemsetAsync(ao.dev, 0, ao.bytes, c->stream), "zero dw");
   rtx::nn::ConvWgrad a{};
