@@ -97,10 +97,16 @@ struct rtx_context {
   DevBuf nodes, nodes4, tris, shade, geo, mats, emit;
   std::vector<int32_t> emitters;
   // device scratch
-  // Error word: mapped pinned host memory that kernels touch only to report
-  // an error, so a synchronous call clears and reads it without a memset and
-  // a copy of its own (5x5 convolution of a 256^2 image: 32.5 -> 21.7 us per call).
-  int* d_err = nullptr;          // device address
+  // Error words, which kernels touch only to report an error.  A synchronous
+  // call's is mapped pinned host memory, cleared and read without a memset and
+  // a copy of its own (5x5 convolution of a 256^2 image: 32.5 -> 21.7 us per
+  // call).  An asynchronous call's is device memory, cleared in stream order:
+  // an error that a replay of a captured call reports after that call is not
+  // taken for another call's, and the memset costs 1 to 3 us less than one of
+  // host memory (16 -> 32 channels at 64^2, enqueued: 14.7 -> 12.6 us per call).
+  int* d_err = nullptr;           // the current call's, one of the two below
+  int* async_err = nullptr;       // device memory
+  int* sync_err = nullptr;        // mapped memory: device address
   volatile int* h_err = nullptr;  // the same word on the host
   Counters* d_counters = nullptr;
   PtWorkspace* pt = nullptr;
@@ -133,7 +139,7 @@ struct rtx_context {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   rtx_stats stats{};
   bool pending_timing = false;
-  bool err_busy = false;  // work that may still write the error word was enqueued and not waited for
+  bool err_busy = false;  // a synchronous call left before its wait: its kernels may still write its error word
 };
 
 namespace {
@@ -207,17 +213,23 @@ static SortKeyBounds sort_key_bounds(const Float4Array& nodes4, int root4) {
 
 int begin(rtx_context* c) {
   RTX_CUDA(cudaSetDevice(c->device), "cudaSetDevice");
-  // Cleared from the host when no earlier call of this context can still be
-  // running; in stream order otherwise (asynchronous calls, captures).
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  RTX_CUDA(cudaStreamIsCapturing(c->stream, &cap), "cudaStreamIsCapturing");
-  if (c->err_busy || cap != cudaStreamCaptureStatusNone)
+  c->d_err = c->async ? c->async_err : c->sync_err;
+  if (c->async || c->err_busy)
     RTX_CUDA(cudaMemsetAsync(c->d_err, 0, sizeof(int), c->stream), "cudaMemsetAsync(err)");
   else
     *c->h_err = 0;
-  c->err_busy = true;
+  if (!c->async) c->err_busy = true;
   RTX_CUDA(cudaEventRecord(c->ev0, c->stream), "cudaEventRecord");
   c->stats.kernel_launches = 0;
+  return RTX_OK;
+}
+
+// The last call's error word; its work has been waited for.
+int read_err(rtx_context* c, int* v) {
+  if (c->d_err == c->sync_err)
+    *v = *c->h_err;
+  else
+    RTX_CUDA(cudaMemcpy(v, c->d_err, sizeof(int), cudaMemcpyDeviceToHost), "read error word");
   return RTX_OK;
 }
 
@@ -233,8 +245,9 @@ int finish(rtx_context* c, bool may_async) {
   RTX_CUDA(cudaEventElapsedTime(&ms, c->ev0, c->ev1), "cudaEventElapsedTime");
   c->stats.last_gpu_ms = ms;
   c->pending_timing = false;
-  c->err_busy = false;
-  const int herr = *c->h_err;
+  if (c->d_err == c->sync_err) c->err_busy = false;
+  int herr = 0;
+  if (int r = read_err(c, &herr)) return r;
   if (herr) {
     std::string m = "kernel error:";
     if (herr & kErrStackOverflow) m += " traversal stack overflow";
@@ -431,7 +444,9 @@ int rtx_create(rtx_context** out, int device) {
   if ((e = cudaEventCreate(&c->ev1)) != cudaSuccess) return bail(e);
   if ((e = cudaHostAlloc((void**)&c->h_err, sizeof(int), cudaHostAllocMapped)) != cudaSuccess) return bail(e);
   *c->h_err = 0;
-  if ((e = cudaHostGetDevicePointer((void**)&c->d_err, (void*)c->h_err, 0)) != cudaSuccess) return bail(e);
+  if ((e = cudaHostGetDevicePointer((void**)&c->sync_err, (void*)c->h_err, 0)) != cudaSuccess) return bail(e);
+  if ((e = cudaMalloc(&c->async_err, sizeof(int))) != cudaSuccess) return bail(e);
+  c->d_err = c->sync_err;
   if ((e = cudaMalloc(&c->d_counters, sizeof(Counters))) != cudaSuccess) return bail(e);
   if ((e = cudaMemset(c->d_counters, 0, sizeof(Counters))) != cudaSuccess) return bail(e);
   {
@@ -470,6 +485,7 @@ void rtx_destroy(rtx_context* c) {
   c->weights_valid = false;
   if (c->pt) pt_workspace_destroy(c->pt);
   if (c->h_err) cudaFreeHost((void*)c->h_err);
+  if (c->async_err) cudaFree(c->async_err);
   if (c->d_counters) cudaFree(c->d_counters);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
@@ -567,8 +583,9 @@ int rtx_synchronize(rtx_context* c) {
     c->stats.last_gpu_ms = ms;
     c->pending_timing = false;
   }
-  c->err_busy = false;
-  if (*c->h_err) return fail(c, RTX_ERR_DEVICE, "kernel error reported by an asynchronous call");
+  int herr = 0;
+  if (int r = read_err(c, &herr)) return r;
+  if (herr) return fail(c, RTX_ERR_DEVICE, "kernel error reported by an asynchronous call");
   return RTX_OK;
 }
 
@@ -1239,7 +1256,7 @@ int rtx_render_batch(rtx_context* c, int n_jobs, const rtx_job* jobs, int max_de
   std::vector<int64_t> key = {n_jobs, max_depth, c->wave_paths, c->block, c->primary_cache, c->count_visits,
                               c->accumulate, (int64_t)p.sort_material, (int64_t)p.sort_rays, c->traversal, c->overlap,
                               c->stack_limit, (int64_t)(intptr_t)o.dev, (int64_t)(intptr_t)p.d_jobs,
-                              (int64_t)(intptr_t)p.d_job_q};
+                              (int64_t)(intptr_t)p.d_job_q, (int64_t)(intptr_t)c->d_err};
   for (int j = 0; j < n_jobs; ++j) key.insert(key.end(), {jobs[j].scene, jobs[j].W, jobs[j].H, jobs[j].spp});
   int launches = 0, ext_launches = 0, vtx_launches = 0;
   std::string why;
