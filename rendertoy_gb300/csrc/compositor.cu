@@ -356,7 +356,9 @@ RTX_DEV void sep_window(SepAcc& A, const float* __restrict__ wsm, int size, floa
 // Horizontal pass (1 x size kernel): a block computes kRowTile pixels of one
 // row.  The row segment and its halo sit in shared memory as RGB triples with
 // one spare triple after every kSepR pixels, so the kSepR-pixel strides of a
-// warp's lanes (27 words apart) fall in distinct banks.
+// warp's lanes (27 words apart) fall in distinct banks.  Only pixels that are
+// taps are staged (size - 1 beyond the outputs; the window's kLead before them
+// have no slot), so that the segment fits up to 12,493 taps.
 constexpr int kRowThreads = 128, kRowTile = kRowThreads * kSepR;
 RTX_DEV int row_slot(int i) { return 3 * (i + i / kSepR); }
 
@@ -367,18 +369,19 @@ __global__ void __launch_bounds__(kRowThreads, 8) k_gauss_x(const float* __restr
                                                          int extract_mode, float thr, float negzero) {
   extern __shared__ float sm[];
   float* wsm = sm;                       // size weights
-  float* tile = sm + ((size + 3) & ~3);  // row_slot(kRowTile + halo) floats
-  const int y = blockIdx.y, x0 = blockIdx.x * kRowTile, tid = threadIdx.x;
-  const int r = (size >> 1) + Window<k>::kLead;
+  float* tile = sm + ((size + 3) & ~3);
+  constexpr int kLead = Window<k>::kLead;
+  auto slot = [&](int i) { return tile + row_slot(i) - row_slot(kLead); };  // of window pixel i >= kLead
+  const int y = blockIdx.y, x0 = blockIdx.x * kRowTile, r = size >> 1, tid = threadIdx.x;
   const int n_out = min(kRowTile, W - x0);
-  const int halo = kSepR * window_chunks(size, Window<k>::kLead), span = n_out + halo, cap = kRowTile + halo;
+  const int span = n_out + size - 1, cap = kRowTile + size - 1;
   for (int j = tid; j < size; j += kRowThreads) wsm[j] = w[j];
   for (int j = tid; j < cap; j += kRowThreads)
-    stage_px(tile + row_slot(j), in, j < span ? reflect_index(y, (long long)x0 - r + j, W, H) : -1);
+    stage_px(slot(kLead + j), in, j < span ? reflect_index(y, (long long)x0 - r + j, W, H) : -1);
   cp_wait_all();
   if (extract_mode) {  // bloom: Extract applied to the staged pixels
     for (int j = tid; j < span; j += kRowThreads) {
-      float* s = tile + row_slot(j);
+      float* s = slot(kLead + j);
       const F3 p = extract(f3(s[0], s[1], s[2]), thr);
       s[0] = p.x;
       s[1] = p.y;
@@ -390,11 +393,11 @@ __global__ void __launch_bounds__(kRowThreads, 8) k_gauss_x(const float* __restr
   const int b = kSepR * tid;
   if (b < n_out) {
     sep_window<k, kFma>(acc, wsm, size, negzero, [&](int j) {
-      const float* s = tile + row_slot(b + j);
+      const float* s = slot(b + j);
       return f3(s[0], s[1], s[2]);
     });
   }
-  __syncthreads();  // the tile now holds the outputs, in the same slots
+  __syncthreads();  // the tile now holds the outputs
   if (b < n_out) {
 #pragma unroll
     for (int o = 0; o < kSepR; ++o) {
@@ -415,7 +418,8 @@ __global__ void __launch_bounds__(kRowThreads, 8) k_gauss_x(const float* __restr
 
 // Vertical pass (size x 1 kernel): a block computes kColW columns x kColH
 // rows; lanes take neighbouring columns, each thread kSepR consecutive rows,
-// from a shared-memory strip of kColH + size - 1 rows.
+// from a shared-memory strip of kColH + size - 1 rows (those that are taps; the
+// window's kLead rows before them are not staged): up to 568 taps.
 constexpr int kColW = 32, kColThreads = 128, kColH = (kColThreads / kColW) * kSepR;
 
 template <int k, bool kFma>
@@ -427,10 +431,9 @@ __global__ void __launch_bounds__(kColThreads, 7) k_gauss_y(const float* __restr
   extern __shared__ float sm[];
   float* wsm = sm;
   float* strip = sm + ((size + 3) & ~3);  // rows x kColW x 3
-  const int x0 = blockIdx.x * kColW, y0 = blockIdx.y * kColH, tid = threadIdx.x;
-  const int r = (size >> 1) + Window<k>::kLead;
+  const int x0 = blockIdx.x * kColW, y0 = blockIdx.y * kColH, r = size >> 1, tid = threadIdx.x;
   for (int j = tid; j < size; j += kColThreads) wsm[j] = w[j];
-  const int rows = kColH + kSepR * window_chunks(size, Window<k>::kLead);
+  const int rows = kColH + size - 1;
   for (int e = tid; e < rows * kColW; e += kColThreads) {
     const int rr = e / kColW, cc = e - rr * kColW;
     const int x = x0 + cc;
@@ -443,7 +446,7 @@ __global__ void __launch_bounds__(kColThreads, 7) k_gauss_y(const float* __restr
   if (x >= W || yb >= H) return;
   SepAcc acc;
   sep_window<k, kFma>(acc, wsm, size, negzero, [&](int j) {
-    const float* s = strip + 3 * ((kSepR * g + j) * kColW + cc);
+    const float* s = strip + 3 * ((kSepR * g + j - Window<k>::kLead) * kColW + cc);
     return f3(s[0], s[1], s[2]);
   });
 #pragma unroll
@@ -749,11 +752,11 @@ cudaError_t launch_convolve(const float* in, float* out, int W, int H, const flo
 // pixels of a window beyond its first output's: kSepR m
 static size_t window_halo(int size) { return (size_t)((size | 1) + 2 * (window_kind(size) & 3)) / 8 * 8; }
 static size_t smem_x(int size) {
-  const size_t cap = (size_t)kRowTile + window_halo(size);
-  return sizeof(float) * (((size_t)size + 3 & ~(size_t)3) + 3 * (cap + cap / kSepR));
+  const size_t cap = (size_t)kRowTile + size - 1, lead = window_kind(size) & 3;
+  return sizeof(float) * (((size_t)size + 3 & ~(size_t)3) + 3 * (cap + (lead + cap - 1) / kSepR));
 }
 static size_t smem_y(int size) {
-  return sizeof(float) * (((size_t)size + 3 & ~(size_t)3) + 3 * ((size_t)kColH + window_halo(size)) * kColW);
+  return sizeof(float) * (((size_t)size + 3 & ~(size_t)3) + 3 * ((size_t)kColH + size - 1) * kColW);
 }
 
 // A separable pass' instance for a size.
