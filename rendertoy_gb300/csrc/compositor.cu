@@ -801,7 +801,11 @@ cudaError_t launch_gaussian(const float* in, float* tmp, float* tmp2, float* out
     return cudaGetLastError();
   }
   // 16-byte forms: rows of a multiple of four pixels, 16-byte aligned images
-  // (size 3 at 64^2: 17.8 -> 15.8 us per call, 49 at 1,024^2: 31 -> 22.4)
+  // (size 3 at 64^2: 17.8 -> 15.8 us per call, 49 at 1,024^2: 31 -> 22.4).
+  // Down the columns their strips are a third larger: where only one fits an
+  // SM but two of the 4-byte form's do (194 to 267 taps), that form is
+  // faster (512^2: 201 taps 52.0 -> 45.2 us, 261 taps 63.9 -> 55.4; 1,024^2:
+  // 129 -> 121, 166 -> 156; 1920 x 1080: 238 -> 229, 307 -> 299).
   auto al = [](const void* p, uintptr_t m) { return (reinterpret_cast<uintptr_t>(p) & (m - 1)) == 0; };
   const bool quads = W % 4 == 0 && al(in, 16) && al(tmp, 16) && al(out, 16);
   const size_t ws16 = (size_t)size + 3 & ~(size_t)3;
@@ -823,7 +827,8 @@ cudaError_t launch_gaussian(const float* in, float* tmp, float* tmp2, float* out
     k_convolve<<<dim3((W + 127) / 128, H), 128, 0, st>>>(in, tmp, W, H, d_w, 1, size, 0);
   }
   ++*launches;
-  if (quads && sy16 <= kMaxSmem) {
+  const size_t kHalfSmem = 113 * 1024;  // two blocks on an SM, 1 KB each reserved
+  if (quads && sy16 <= kMaxSmem && (sy16 <= kHalfSmem || sy > kHalfSmem)) {
     auto ky = gauss_y16(size, fma);
     if (sy16 > 48 * 1024 && (e = cudaFuncSetAttribute(ky, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sy16)))
       return e;

@@ -35,3 +35,12 @@ def test_longest_row_windows(ctx, oracle, size):
     assert np.array_equal(bits(got), bits(ref))
     assert not np.array_equal(bits(fused), bits(got))
     np.testing.assert_allclose(fused, ref, rtol=1e-5)
+
+
+@pytest.mark.parametrize("size", [180, 181, 189, 190, 200, 201, 264, 265, 266, 269, 281])
+def test_column_forms_by_strip_size(ctx, oracle, size):
+    """Rows of a multiple of four pixels: the 16-byte and the 4-byte column
+    passes on both sides of where one gives way to the other."""
+    img = np.random.RandomState(size).exponential(0.7, (43, 36, 3)).astype(np.float32)
+    assert np.array_equal(bits(ctx.gaussian_blur(img, size, size / 6.0)), bits(oracle.gaussian_blur(img, size, size / 6.0)))
+    assert np.array_equal(bits(ctx.bloom(img, size, size / 6.0, 0.8)), bits(oracle.bloom(img, size, size / 6.0, 0.8)))
