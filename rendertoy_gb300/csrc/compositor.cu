@@ -363,7 +363,7 @@ constexpr int kRowThreads = 128, kRowTile = kRowThreads * kSepR;
 RTX_DEV int row_slot(int i) { return 3 * (i + i / kSepR); }
 
 template <int k, bool kFma>
-__global__ void __launch_bounds__(kRowThreads, 8) k_gauss_x(const float* __restrict__ in,
+__global__ void __launch_bounds__(kRowThreads, 7) k_gauss_x(const float* __restrict__ in,
                                                          float* __restrict__ out, int W, int H,
                                                          const float* __restrict__ w, int size,
                                                          int extract_mode, float thr, float negzero) {
@@ -420,10 +420,14 @@ __global__ void __launch_bounds__(kRowThreads, 8) k_gauss_x(const float* __restr
 // rows; lanes take neighbouring columns, each thread kSepR consecutive rows,
 // from a shared-memory strip of kColH + size - 1 rows (those that are taps; the
 // window's kLead rows before them are not staged): up to 568 taps.
+// Registers for five blocks per SM: at seven (72) the compile-time windows
+// spilled or were scheduled with loads late, which showed where strips leave few
+// blocks on an SM (1,024^2: 520 taps 375 -> 342 us, 568 taps 408 -> 371; run-time
+// windows took 362, 390) and at small sizes too (513 x 511: 49 taps 26.7 -> 25.1).
 constexpr int kColW = 32, kColThreads = 128, kColH = (kColThreads / kColW) * kSepR;
 
 template <int k, bool kFma>
-__global__ void __launch_bounds__(kColThreads, 7) k_gauss_y(const float* __restrict__ in,
+__global__ void __launch_bounds__(kColThreads, 5) k_gauss_y(const float* __restrict__ in,
                                                          const float* __restrict__ orig,
                                                          float* __restrict__ out, int W, int H,
                                                          const float* __restrict__ w, int size,
