@@ -28,15 +28,17 @@
 // every dout again per step of 32 x 256^2; in the first column, behind the
 // expansion, d1's launch grew from 100 to 174 us).
 //
-// A CTA owns one or more groups of CB channels for its outputs, keeps their
-// accumulators in TMEM over a run of tiles and adds them to dw with FP32
-// atomics at the run's end.  FP32 accumulation in the tensor core truncates: a
-// run of n MMAs loses about n 2^-26 of a sum that grows steadily (measured
-// 1.3e-5 after 864 of them), so a CTA's range is cut into runs no longer than
-// the earlier kernels' (run_pixels), alternating between two sets of
-// accumulators where TMEM holds them.
+// A CTA owns one or more groups of CB channels for one or more blocks of
+// outputs and keeps their accumulators in TMEM over a run of tiles.  FP32
+// accumulation in the tensor core truncates: a run of n MMAs loses about n 2^-26
+// of a sum that grows steadily (measured 1.3e-5 after 864 of them), so a CTA's
+// range is cut into runs no longer than the earlier kernels' (run_pixels).  The
+// epilogue warps add the runs up in registers, or as many as TMEM holds side by
+// side when they flush, and the sums go to dw with FP32 atomics: no more partial
+// sums than before either.  Runs of at least 512 pixels, added to dw each, had
+// made narrow layers less exact (128 -> 512 pixels: 153 -> 502e-9 relative at
+// 8 x 32^2, 96 + 64 -> 64; now 152).
 #include <algorithm>
-#include <cmath>
 #include <cuda.h>
 
 #include "nn.h"
@@ -49,6 +51,9 @@ namespace nn {
 namespace {
 
 constexpr int kThreadsW = 320, kMaxSW = 8;
+constexpr int kExpanders = 8;     // warps that expand, sum the bias and run the epilogue
+constexpr uint32_t kPad = 4096;   // MMA reads of padding atoms past the last stage
+constexpr uint32_t kXch = 2 * 16 * 12 * 4;  // bytes an epilogue warp passes rows through
 
 struct WgradArgs {
   int KO, CB, ao, G;        // block sizes; o-blocks and channel groups of a CTA
@@ -60,7 +65,7 @@ struct WgradArgs {
   int ngc;                  // CTA columns: sets of G channel groups (x o-block sets)
   int TR, tx, ty;           // tile rows, tiles per image row / column
   int tiles, per;           // all tiles, tiles per CTA
-  int run, sets;            // tiles per run, accumulator sets that runs alternate between
+  int run, batch, halves;   // tiles per run; runs flushed together, each in its own accumulators; alternating halves of these
   int S;
   uint32_t stage, dbytes, sbytes, src_off;  // ring stage; bytes of one dout / source box (1 KB steps); source offset
   uint32_t ncols;
@@ -77,16 +82,68 @@ __device__ __forceinline__ uint64_t mn_desc(uint32_t addr, uint32_t atom, uint32
          ((uint64_t)((group >> 4) & 0x3FFFu) << 32) | (1ull << 46) | (layout << 61);
 }
 
-// dw[o, t, c .. c + 7] += v
-__device__ __forceinline__ void add8(const WgradArgs& a, int o, int t, int c, const float* v) {
-  float* d = a.dw + ((size_t)o * 9 + t) * a.Cin + c;
+__device__ __forceinline__ void add4(float* d, float4 v) {
   if ((reinterpret_cast<uintptr_t>(d) & 15) == 0) {
-    atomicAdd(reinterpret_cast<float4*>(d), make_float4(v[0], v[1], v[2], v[3]));
-    atomicAdd(reinterpret_cast<float4*>(d + 4), make_float4(v[4], v[5], v[6], v[7]));
+    atomicAdd(reinterpret_cast<float4*>(d), v);
   } else {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) atomicAdd(d + k, v[k]);
+    atomicAdd(d, v.x);
+    atomicAdd(d + 1, v.y);
+    atomicAdd(d + 2, v.z);
+    atomicAdd(d + 3, v.w);
   }
+}
+
+// Adds a warp's 32 rows x NC columns (v: this lane's row, m0 the first) to dw
+// at tap column d, channels c0 .. of the nc left in the source.  A row is one
+// (output, tap), 9 Cin floats from the next, so rows pass through shared memory
+// (xw, this warp's): an instruction then adds whole 64-byte (NC = 8: 32-byte)
+// pieces of 8 (16) rows instead of 16 bytes of 32 rows (32 x 32^2, 128 -> 128:
+// 41.0 -> 26.8 us together with the sums held).  xw holds two
+// turns' rows, used alternately: one __syncwarp a turn, an even number of turns.
+template <int NC>
+__device__ __forceinline__ void add_rows(const WgradArgs& a, float* xw, const float* v, int o0, int m0, int d, int c0,
+                                         int nc, int lane) {
+  constexpr int kRow = NC + 4, kCh = NC / 4, kRows = 32 / kCh;  // floats a row (padded: distinct banks), pieces, rows a turn
+#pragma unroll
+  for (int p = 0; p < 32 / kRows; ++p) {
+    float* const x = xw + (p & 1) * (kXch / 8);
+    if (lane / kRows == p)
+#pragma unroll
+      for (int e = 0; e < kCh; ++e)
+        *reinterpret_cast<float4*>(x + (lane % kRows) * kRow + 4 * e) =
+            make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+    __syncwarp();
+    const int r = lane / kCh, ch = lane % kCh, m = m0 + kRows * p + r;
+    const int atom = a.KO == 32 ? m >> 5 : m >> 4, o = o0 + (m & (a.KO - 1));
+    if (atom < 3 && 4 * ch < nc)
+      add4(a.dw + ((size_t)o * 9 + (2 - atom) * 3 + d) * a.Cin + c0 + 4 * ch,
+           *reinterpret_cast<const float4*>(x + r * kRow + 4 * ch));
+  }
+}
+
+// NC of a lane's accumulator columns at each of the three tap columns, `step` apart
+template <int NC>
+__device__ __forceinline__ void load3(uint32_t t, uint32_t step, float (&v)[3][16]) {
+  uint32_t r[3][NC];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    uint32_t* const q = r[d];
+    if constexpr (NC == 16)
+      asm volatile(
+          "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+          : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7]), "=r"(q[8]),
+            "=r"(q[9]), "=r"(q[10]), "=r"(q[11]), "=r"(q[12]), "=r"(q[13]), "=r"(q[14]), "=r"(q[15])
+          : "r"(t + d * step)
+          : "memory");
+    else
+      asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]), "=r"(q[7])
+                   : "r"(t + d * step)
+                   : "memory");
+  }
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int k = 0; k < 3 * NC; ++k) v[k / NC][k % NC] = __uint_as_float(r[k / NC][k % NC]);
 }
 
 // Walks a CTA's tiles in order
@@ -109,8 +166,9 @@ struct Walk {
   }
 };
 
-constexpr int kExpanders = 8;  // warps
-
+// kHeld: blocks whose sums over the CTA's runs stay in registers (0: each run's,
+// or each batch of runs', accumulators go to dw)
+template <int kHeld>
 __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, const __grid_constant__ WgradMaps tm) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) uint64_t full[kMaxSW], empty[kMaxSW], done[2], drained[2];
@@ -147,19 +205,22 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
     const uint32_t idesc = tc::make_idesc_bf16(128, ncb, true, true);
     const uint32_t drow = 8 * a.KO * 2, srow = 10 * a.CB * 2;       // a pixel row of the tile
     const uint32_t dstep = 2 * drow >> 4, sstep = 2 * srow >> 4;    // 16 pixels further
-    int st = 0, left = 0, set = a.sets - 1;
-    uint32_t ph = 0, set_ph = 0;  // fresh barriers: the phase before reads complete
+    int st = 0, left = 0, k = a.batch - 1, half = a.halves - 1;
+    uint32_t ph = 0, half_ph = 0;  // fresh barriers: the phase before reads complete
     for (int u = 0; u < n && ok; ++u) {
       const bool fresh = left == 0;  // first unit of a run
       if (fresh) {
         left = min(a.run, n - u);
-        if (++set == a.sets) {
-          set = 0;
-          set_ph ^= 1u;
+        if (++k == a.batch) {
+          k = 0;
+          if (++half == a.halves) {
+            half = 0;
+            half_ph ^= 1u;
+          }
+          ok = warp_wait(&drained[half], half_ph);
         }
-        ok = warp_wait(&drained[set], set_ph);
       }
-      const uint32_t set_col = set * a.ao * a.G * ncb;
+      const uint32_t set_col = (half * a.batch + k) * a.ao * a.G * ncb;
       --left;
       ok = ok && warp_wait(&full[st], ph);
       if (!ok) break;
@@ -177,7 +238,7 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
           }
         }
         tc::mma_commit(&empty[st]);
-        if (left == 0) tc::mma_commit(&done[set]);
+        if (left == 0 && (k == a.batch - 1 || u == n - 1)) tc::mma_commit(&done[half]);
       }
       __syncwarp();
       if (++st == a.S) {
@@ -218,13 +279,27 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
     // pxs-th pixel of the TR x 10 halo
     const int cpp = a.CB >> 3, ch = (tid - 64) % cpp, p0 = (tid - 64) / cpp, pxs = kExpanders * 32 / cpp;
     const int Hl = a.H >> 1, Wl = a.W >> 1;
-    // epilogue: two warps per 32 lanes, on alternate 8-column chunks
-    const int q = warp & 3, half = (warp - 2) >> 2;
-    const int m = q * 32 + lane, atom = m / a.KO, ol = m - atom * a.KO;
-    const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16);
-    const int nc8 = a.CB >> 3;
-    int st = 0, set = a.sets - 1;
-    uint32_t ph = 1, set_ph = 1;
+    // epilogue: two warps per 32 lanes, each half of a group's channels
+    const int q = warp & 3, odd = (warp - 2) >> 2;
+    const int nc2 = a.CB >> 1;
+    const uint32_t lanes = tmem + ((uint32_t)(q * 32) << 16) + odd * nc2;
+    const bool taps = q * 32 / a.KO < 3;  // some lane of the warp holds one
+    float held[kHeld ? kHeld : 1][3][16];
+#pragma unroll
+    for (int i = 0; i < 3 * 16 * (kHeld ? kHeld : 1); ++i) held[i / 48][i / 16 % 3][i % 16] = 0.0f;
+    float* const xw = reinterpret_cast<float*>(smem + (size_t)a.S * a.stage + kPad) + (warp - 2) * (kXch / 4);
+    // block (o, g)'s tap column d
+    auto flush = [&](int o, int g, int d, const float* v) {
+      const bool first = g0 + g < a.ng1;
+      const int cl = (g0 + g - (first ? 0 : a.ng1)) * a.CB + odd * nc2;  // channel within its source
+      const int c0 = (first ? 0 : a.C1) + cl, nc = (first ? a.C1 : a.C2) - cl;
+      if (a.CB == 32)
+        add_rows<16>(a, xw, v, (ob0 + o) * a.KO, q * 32, d, c0, nc, lane);
+      else
+        add_rows<8>(a, xw, v, (ob0 + o) * a.KO, q * 32, d, c0, nc, lane);
+    };
+    int st = 0, half = a.halves - 1;
+    uint32_t ph = 1, half_ph = 1;
     Walk w(a, t0);
     auto arrive = [&](int stage) {
       tc::fence_proxy_async();
@@ -262,8 +337,8 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
       }
       return true;
     };
-    for (int u0 = 0; u0 < n && ok; u0 += a.run) {
-      const int u1 = min(n, u0 + a.run);
+    for (int u0 = 0; u0 < n && ok; u0 += a.run * a.batch) {
+      const int u1 = min(n, u0 + a.run * a.batch), runs = (u1 - u0 + a.run - 1) / a.run;
       if (nup) {
         int prev = -1;
         for (int u = u0; u < u1; ++u, w.next(a)) {
@@ -302,30 +377,60 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
       } else if (bias) {
         for (int u = u0; u < u1 && ok; ++u) ok = sum_bias();
       }
-      if (++set == a.sets) {
-        set = 0;
-        set_ph ^= 1u;
+      if (++half == a.halves) {
+        half = 0;
+        half_ph ^= 1u;
       }
-      ok = ok && warp_wait(&done[set], set_ph);
+      ok = ok && warp_wait(&done[half], half_ph);
       tc::fence_after();
-      if (ok && q * 32 / a.KO < 3) {  // some lane of the warp holds a tap
-        for (int o = 0; o < on; ++o)
-          for (int g = 0; g < gn; ++g) {
-            const bool first = g0 + g < a.ng1;
-            const int cl = (g0 + g - (first ? 0 : a.ng1)) * a.CB;  // channel within its source
-            for (int k = half; k < nc8; k += 2) {
-              const int c = cl + 8 * k;
-              const bool live = atom < 3 && c < (first ? a.C1 : a.C2);
+      if (ok && taps) {
+        const uint32_t set = a.ao * a.G * ncb, t = lanes + half * a.batch * set;  // a run's columns
+        if constexpr (kHeld > 0) {
+#pragma unroll
+          for (int b = 0; b < kHeld; ++b)
+            if (b / a.G < on && b % a.G < gn)
+#pragma unroll
               for (int d = 0; d < 3; ++d) {
-                float v[8];
-                tc::tmem_ld8(lanes + ((set * a.ao + o) * a.G + g) * ncb + d * a.CB + 8 * k, v);
-                if (live) add8(a, (ob0 + o) * a.KO + ol, (2 - atom) * 3 + d, (first ? 0 : a.C1) + c, v);
+                float v[16];
+                if (a.CB == 32) {
+                  tmem_ld16(t + b * ncb + d * a.CB, v);
+#pragma unroll
+                  for (int k = 0; k < 16; ++k) held[b][d][k] += v[k];
+                } else {
+                  tc::tmem_ld8(t + b * ncb + d * a.CB, v);
+#pragma unroll
+                  for (int k = 0; k < 8; ++k) held[b][d][k] += v[k];
+                }
               }
+        } else {
+          for (int b = 0; b < a.ao * a.G; ++b) {
+            if (b / a.G >= on || b % a.G >= gn) continue;
+            float v[3][16] = {};
+            for (int r = 0; r < runs; ++r) {
+              float w[3][16];
+              const uint32_t tr = t + r * set + b * ncb;
+              if (a.CB == 32)
+                load3<16>(tr, a.CB, w);
+              else
+                load3<8>(tr, a.CB, w);
+#pragma unroll
+              for (int k = 0; k < 48; ++k) v[k / 16][k % 16] += k % 16 < nc2 ? w[k / 16][k % 16] : 0.0f;
             }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) flush(b / a.G, b % a.G, d, v[d]);
           }
+        }
       }
       tc::fence_before();
-      tc::mbar_arrive(&drained[set]);
+      tc::mbar_arrive(&drained[half]);
+    }
+    if constexpr (kHeld > 0) {
+      if (ok && taps)
+#pragma unroll
+        for (int b = 0; b < kHeld; ++b)
+          if (b / a.G < on && b % a.G < gn)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) flush(b / a.G, b % a.G, d, held[b][d]);
     }
     if (bias && bp0 < bps)
 #pragma unroll
@@ -338,32 +443,39 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
   if (warp == 0) tc::tmem_dealloc(tmem, a.ncols);
 }
 
-constexpr uint32_t kSmemW = 216 * 1024, kPad = 4096;  // kPad: MMA reads of padding atoms past the last stage
+// Clocks of the split's estimate, from forced splits of 37 layers: a unit costs
+// kUnit and an MMA kMma32 (kMma16 with 16-channel groups), adding a block's sums
+// to dw kFlush, taking them into registers kHold, a CTA's start kStart.
+constexpr double kUnit = 590, kMma32 = 80, kMma16 = 65, kFlush = 3000, kHold = 300, kStart = 6000;
+constexpr uint32_t kSmemW = 216 * 1024;  // the ring and kPad
 
 // Pixels an accumulator may sum before it is added to dw (see the file
-// comment): the range a CTA of the kernels before this one summed.  Rows of
-// 64 pixels or more: one CTA per SM and set of channels -- all of up to 128
-// where outputs are few, else the width (48, 32 or 16) that weighed a set's
-// fixed cost against its number -- two for 16 channels.  Narrower rows: the
-// gather kernel's, but at least 512 (32 MMAs lose about 4e-7).
+// comment): no more than a CTA of the kernels before this one summed, so that
+// no weight loses more to truncation than it did.  Rows of 64 pixels or more:
+// those kernels' row tiles (32, 64 or 128 pixels wide) shared out over one CTA
+// per SM and set of channels -- all of up to 128 where outputs are few, else
+// the width (48, 32 or 16) that weighed a set's fixed cost against its number
+// -- two for 16 channels.  Narrower rows: about eight CTAs per SM, multiples of
+// 64 pixels.
 long long run_pixels(const ConvWgrad& c) {
   const long long P = (long long)c.N * c.H * c.W;
-  long long px;
+  int nr = 0, tw = 0, per_sm = 1;
   if (c.W >= 64 && c.Cin % 16 == 0 && 9 * c.Cout <= 512 && c.Cin >= 64) {
-    px = P * ((c.Cin + 127) / 128) / tile_sm_count();
+    nr = (c.Cin + 127) / 128;
+    tw = 32;
   } else if (c.W >= 64 && c.Cin % 16 == 0 && c.Cout <= 128) {
-    int nr = 1;
     long long best = -1;
     for (int cr : {48, 32, 16}) {
       const int k = (c.Cin + cr - 1) / cr;
       const long long cost = (long long)k * (cr + c.Cout / 4 + 8);
       if (cr <= c.Cin && (best < 0 || cost < best)) best = cost, nr = k;
     }
-    px = P * nr / (tile_sm_count() * (c.Cin <= 16 ? 2 : 1));
-  } else {
-    px = wgrad_pixels_per_cta(P, c.Cout, c.Cin);
+    tw = c.W >= 128 ? 128 : 64;
+    per_sm = c.Cin <= 16 ? 2 : 1;
   }
-  return std::max(px, 512LL);
+  if (!nr) return wgrad_pixels_per_cta(P, c.Cout, c.Cin);
+  const long long row = (c.W + tw - 1) / tw, npg = std::max(1, tile_sm_count() * per_sm / nr);
+  return ((long long)c.N * c.H * row + npg - 1) / npg * c.W / row;
 }
 
 }  // namespace
@@ -389,8 +501,6 @@ bool conv_tile_wgrad(const ConvWgrad& c, cudaStream_t st, cudaError_t* e) {
   const int at = c.Cout / a.KO;
   a.CB = std::max(a.C1, a.C2) > 16 ? 32 : 16;
   if (at * 3 * a.CB > 512) a.CB = 16;  // the accumulators of all outputs in 512 columns
-  a.ao = std::min(at, 512 / (3 * a.CB));
-  const int ngo = (at + a.ao - 1) / a.ao;
   a.ng1 = (a.C1 + a.CB - 1) / a.CB;
   a.ng = a.ng1 + (a.C2 + a.CB - 1) / a.CB;
   auto plan = [&](int TR, int G) {
@@ -403,40 +513,79 @@ bool conv_tile_wgrad(const ConvWgrad& c, cudaStream_t st, cudaError_t* e) {
     a.S = (int)std::min<uint32_t>(kMaxSW, (kSmemW - kPad) / a.stage);
     return a.S;
   };
-  // One block of outputs (up to 32): a CTA takes every channel group its
-  // accumulators and a three-stage ring allow, so dout is read once; more
-  // outputs: one group per CTA.
-  int G = 1;
-  if (at == 1)
-    while (G < a.ng && (G + 1) * 3 * a.CB <= 512 && plan(8, G + 1) >= 3) ++G;
-  // the tallest tile (up to 32 rows) that leaves three stages
-  int TR = 32;
-  while (TR > 8 && (plan(TR, G) < 3 || c.H <= TR / 2)) TR /= 2;
-  if (plan(TR, G) < 2) return false;
-  a.ngc = (a.ng + G - 1) / G;
-  a.tx = (c.W + 7) / 8;
-  a.ty = (c.H + TR - 1) / TR;
-  const long long T = (long long)c.N * a.tx * a.ty;
-  if (T > (1LL << 30)) return false;
-  a.tiles = (int)T;
-  const int columns = a.ngc * ngo, ranges = std::max(1, tile_sm_count() / columns);
-  a.per = (a.tiles + ranges - 1) / ranges;
-  // equal runs; a tenth over the limit is within what the limit's own
-  // rounding to whole tiles varied by
-  const double over = (double)a.per * 8 * TR / (1.1 * (double)run_pixels(c));
-  const int runs = std::min(a.per, std::max(1, (int)std::ceil(over)));
-  a.run = (a.per + runs - 1) / runs;
-  a.sets = runs > 1 && 2 * a.ao * G * 3 * a.CB <= 512 ? 2 : 1;
-  const uint32_t cols = (uint32_t)(a.sets * a.ao * G * 3 * a.CB);
+  // The split (tile rows TR, channel groups G and output blocks ao of a CTA)
+  // with the shortest estimate.  One block of outputs (up to 32) may take
+  // several channel groups, so that dout is read once; more take one.  No split
+  // whose number of partial sums exceeds the earlier kernels' (their FP32
+  // additions round), unless all do.  Every block of outputs in one CTA, and
+  // tiles as tall as fit, left small layers to a handful of CTAs with long
+  // flushes (1 x 16^2, 128 -> 160: 23.2 -> 16.6 us per enqueued call; 64 + 32 ->
+  // 32: 20.6 -> 16.6; 32 x 64^2, 96 -> 96: 51.9 -> 41.2).
+  const long long limit = run_pixels(c), P = (long long)c.N * c.H * c.W, most = (P + limit - 1) / limit;
+  const int at_max = std::min(at, 512 / (3 * a.CB));
+  int G = 1, held = 0;
+  // false: not a split
+  auto split = [&](int TR, int g, int o, double* cost, bool* over) {
+    a.ao = o;
+    G = g;
+    if (o * g * 3 * a.CB > 512 || (TR > 8 && c.H <= TR / 2) || plan(TR, g) < (TR > 8 ? 3 : 2)) return false;
+    const int px = std::min(8, c.W) * std::min(TR, c.H);  // a full tile's
+    if (TR > 8 && px > limit) return false;
+    a.tx = (c.W + 7) / 8;
+    a.ty = (c.H + TR - 1) / TR;
+    const long long tiles = (long long)c.N * a.tx * a.ty;
+    if (tiles > (1LL << 30)) return false;
+    a.tiles = (int)tiles;
+    a.ngc = (a.ng + g - 1) / g;
+    const int columns = a.ngc * ((at + o - 1) / o);
+    const int ranges = (int)std::min<long long>(std::max(1, tile_sm_count() / columns), most);
+    a.per = (a.tiles + ranges - 1) / ranges;
+    const int run = (int)std::max(1LL, std::min<long long>(a.per, limit / px)), runs = (a.per + run - 1) / run;
+    a.run = (a.per + runs - 1) / runs;  // equal runs
+    // several runs: held in registers where a CTA has one or two blocks, else
+    // as many to a flush as TMEM has accumulators
+    const int sets = 512 / (o * g * 3 * a.CB);
+    held = runs > 1 && o * g <= 2 ? o * g : 0;
+    a.halves = held || (runs > sets && sets > 1) ? 2 : 1;
+    a.batch = held ? 1 : std::min(runs, sets / a.halves);
+    const int flushes = held ? 1 : (runs + a.batch - 1) / a.batch, used = (a.tiles + a.per - 1) / a.per;
+    *over = (long long)flushes * used > most;
+    const double mmas = (TR / 2) * o * g, unit = kUnit + mmas * (a.CB == 32 ? kMma32 : kMma16);
+    const double work = a.per * unit, flush = o * g * kFlush;
+    const double waves = (columns * used + tile_sm_count() - 1) / tile_sm_count();
+    *cost = waves * (kStart + (a.halves == 1 ? work + flushes * flush
+                               : held        ? std::max(work, runs * o * g * kHold) + flush
+                                             : std::max(work, flushes * flush) + flush));
+    return true;
+  };
+  double best = 0, cost;
+  bool best_over = true, over;
+  int pick[3] = {0, 0, 0};
+  for (int o = 1; o <= at_max; ++o)
+    for (int g = 1; g <= (at == 1 ? a.ng : 1); ++g)
+      for (int TR : {32, 16, 8})
+        if (split(TR, g, o, &cost, &over) && (!pick[0] || over < best_over || (over == best_over && cost < best))) {
+          best = cost;
+          best_over = over;
+          pick[0] = TR, pick[1] = g, pick[2] = o;
+        }
+  if (!pick[0] || !split(pick[0], pick[1], pick[2], &cost, &over)) return false;
+  const int TR = pick[0];
+  const int columns = a.ngc * ((at + a.ao - 1) / a.ao);
+  const uint32_t cols = (uint32_t)(a.halves * a.batch * a.ao * G * 3 * a.CB);
   for (a.ncols = 32; a.ncols < cols;) a.ncols *= 2;
   WgradMaps m{};
   if (!pixel_map(&m.dout, c.dout, c.N, c.H, c.W, c.Cout, 1, 1, a.KO, 8, TR + 2)) return false;
   if (!c.s1.up && !pixel_map(&m.src[0], c.s1.ptr, c.N, c.H, c.W, a.C1, 1, 1, a.CB, 10, TR)) return false;
   if (a.C2 && !pixel_map(&m.src[1], c.s2.ptr, c.N, c.H, c.W, a.C2, 1, 1, a.CB, 10, TR)) return false;
-  // past half the SM's shared memory: one CTA per SM (TMEM columns)
-  const size_t smem = std::max<size_t>((size_t)a.S * a.stage + kPad, 116 * 1024);
-  if ((*e = cudaFuncSetAttribute(k_wgrad_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))) return true;
-  k_wgrad_tile<<<dim3(columns, (a.tiles + a.per - 1) / a.per), kThreadsW, smem, st>>>(a, m);
+  // no more stages than units; past half the SM's shared memory where two CTAs'
+  // TMEM columns do not fit side by side
+  a.S = std::min(a.S, std::max(2, a.per));
+  const size_t ring = (size_t)a.S * a.stage + kPad + kExpanders * kXch;
+  const size_t smem = a.ncols > 256 ? std::max<size_t>(ring, 116 * 1024) : ring;
+  auto k = held == 2 ? k_wgrad_tile<2> : (held == 1 ? k_wgrad_tile<1> : k_wgrad_tile<0>);
+  if ((*e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))) return true;
+  k<<<dim3(columns, (a.tiles + a.per - 1) / a.per), kThreadsW, smem, st>>>(a, m);
   *e = cudaGetLastError();
   return true;
 }
