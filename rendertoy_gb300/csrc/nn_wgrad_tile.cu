@@ -447,7 +447,8 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
 // kUnit and an MMA kMma32 (kMma16 with 16-channel groups), adding a block's sums
 // to dw kFlush, taking them into registers kHold, a CTA's start kStart.
 constexpr double kUnit = 590, kMma32 = 80, kMma16 = 65, kFlush = 3000, kHold = 300, kStart = 6000;
-constexpr uint32_t kSmemW = 216 * 1024;  // the ring and kPad
+constexpr uint32_t kSmemW = 212 * 1024;  // the ring and kPad; rows in passing and static arrays take the rest of 227 KB
+static_assert(kSmemW + kExpanders * kXch + 3072 <= 227 * 1024, "shared memory of a block");
 
 // Pixels an accumulator may sum before it is added to dw (see the file
 // comment): no more than a CTA of the kernels before this one summed, so that

@@ -57,6 +57,7 @@ def test_error_of_sums_of_one_sign(ctx, c):
     (40, 8, 8, 32, 1, 32, 32),      # tiles of one image each, many per CTA
     (200, 2, 6, 32, 0, 0, 32),      # images smaller than a tile
     (2, 272, 96, 64, 0, 0, 64),     # tall tiles, several runs
+    (15, 80, 96, 136, 0, 8, 16),    # a ring that fills shared memory
 ])
 def test_splits(ctx, c):
     """Every way a layer is shared out, against the oracle; tolerance as for
