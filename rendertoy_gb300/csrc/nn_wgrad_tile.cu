@@ -28,14 +28,23 @@
 // every dout again per step of 32 x 256^2; in the first column, behind the
 // expansion, d1's launch grew from 100 to 174 us).
 //
+// An infinite or NaN source value in an image's first or last row meets dout's
+// zero halo rows (in the last column of a width that is not a multiple of
+// eight, dout's zero columns): 0 x inf is NaN, in taps that do not read the
+// value.  So rows of sums of those taps that are not all finite are left out and
+// formed again from memory, over the pixels of dout alone, once the CTA is done;
+// while all values are finite nothing is read twice.  The reverse is not made
+// good: an infinite dout value in those rows leaves taps that would read the
+// padding beside it as they are, where multiplying the padding would give NaN.
+//
 // A CTA owns one or more groups of CB channels for one or more blocks of
 // outputs and keeps their accumulators in TMEM over a run of tiles.  FP32
 // accumulation in the tensor core truncates: a run of n MMAs loses about n 2^-26
 // of a sum that grows steadily (measured 1.3e-5 after 864 of them), so a CTA's
 // range is cut into runs no longer than the earlier kernels' (run_pixels).  The
-// epilogue warps add the runs up in registers, or as many as TMEM holds side by
-// side when they flush, and the sums go to dw with FP32 atomics: no more partial
-// sums than before either.  Runs of at least 512 pixels, added to dw each, had
+// epilogue warps add the runs up in registers, or TMEM holds them side by side,
+// and a CTA's sums go to dw once, with FP32 atomics: no more partial sums than
+// before either.  Runs of at least 512 pixels, added to dw each, had
 // made narrow layers less exact (128 -> 512 pixels: 153 -> 502e-9 relative at
 // 8 x 32^2, 96 + 64 -> 64; now 152).
 #include <algorithm>
@@ -50,7 +59,7 @@ namespace nn {
 
 namespace {
 
-constexpr int kThreadsW = 320, kMaxSW = 8;
+constexpr int kThreadsW = 320, kMaxSW = 8, kMaxBlocks = 10;
 constexpr int kExpanders = 8;     // warps that expand, sum the bias and run the epilogue
 constexpr uint32_t kPad = 4096;   // MMA reads of padding atoms past the last stage
 constexpr uint32_t kXch = 2 * 16 * 12 * 4;  // bytes an epilogue warp passes rows through
@@ -60,12 +69,12 @@ struct WgradArgs {
   int Cout, Cin;            // outputs; dw's channel stride
   int C1, C2, ng1, ng;      // the sources' channels; channel groups of the first, of both
   int up1;                  // the first source is expanded from half resolution
-  const bf16* x1;
+  const bf16 *x1, *x2, *dout;
   int H, W;
   int ngc;                  // CTA columns: sets of G channel groups (x o-block sets)
   int TR, tx, ty;           // tile rows, tiles per image row / column
   int tiles, per;           // all tiles, tiles per CTA
-  int run, batch, halves;   // tiles per run; runs flushed together, each in its own accumulators; alternating halves of these
+  int run, sets;            // tiles per run; accumulator sets (of all runs, or two that runs alternate between)
   int S;
   uint32_t stage, dbytes, sbytes, src_off;  // ring stage; bytes of one dout / source box (1 KB steps); source offset
   uint32_t ncols;
@@ -166,14 +175,18 @@ struct Walk {
   }
 };
 
-// kHeld: blocks whose sums over the CTA's runs stay in registers (0: each run's,
-// or each batch of runs', accumulators go to dw)
+// kHeld: blocks whose sums over the CTA's runs stay in registers (0: every run
+// has accumulators of its own)
 template <int kHeld>
 __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, const __grid_constant__ WgradMaps tm) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) uint64_t full[kMaxSW], empty[kMaxSW], done[2], drained[2];
   __shared__ uint32_t tmem_slot;
   __shared__ float sdb[256];
+  // rows (outputs and tap rows) of a block's tap column and an epilogue warp
+  // whose sums are formed again
+  __shared__ uint32_t redo[kMaxBlocks * 3 * kExpanders];
+  __shared__ int again;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int gc = (int)blockIdx.x % a.ngc, go = (int)blockIdx.x / a.ngc;
   const int g0 = gc * a.G, gn = min(a.G, a.ng - g0);               // channel groups g0 .. g0 + gn - 1
@@ -197,7 +210,11 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = tmem_slot, s0 = tc::smem_u32(smem);
-  for (int k = tid; k < 256; k += kThreadsW) sdb[k] = 0.0f;
+  for (int k = tid; k < 256; k += kThreadsW) {
+    sdb[k] = 0.0f;
+    if (k < kMaxBlocks * 3 * kExpanders) redo[k] = 0;
+  }
+  if (tid == 0) again = 0;
   __syncthreads();
   const uint32_t ncb = 3 * a.CB;  // accumulator columns of a block
   bool ok = true;
@@ -205,22 +222,19 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
     const uint32_t idesc = tc::make_idesc_bf16(128, ncb, true, true);
     const uint32_t drow = 8 * a.KO * 2, srow = 10 * a.CB * 2;       // a pixel row of the tile
     const uint32_t dstep = 2 * drow >> 4, sstep = 2 * srow >> 4;    // 16 pixels further
-    int st = 0, left = 0, k = a.batch - 1, half = a.halves - 1;
-    uint32_t ph = 0, half_ph = 0;  // fresh barriers: the phase before reads complete
+    int st = 0, left = 0, set = a.sets - 1;
+    uint32_t ph = 0, set_ph = 0;  // fresh barriers: the phase before reads complete
     for (int u = 0; u < n && ok; ++u) {
       const bool fresh = left == 0;  // first unit of a run
       if (fresh) {
         left = min(a.run, n - u);
-        if (++k == a.batch) {
-          k = 0;
-          if (++half == a.halves) {
-            half = 0;
-            half_ph ^= 1u;
-          }
-          ok = warp_wait(&drained[half], half_ph);
+        if (++set == a.sets) {
+          set = 0;
+          set_ph ^= 1u;
         }
+        if (kHeld) ok = warp_wait(&drained[set], set_ph);
       }
-      const uint32_t set_col = (half * a.batch + k) * a.ao * a.G * ncb;
+      const uint32_t set_col = set * a.ao * a.G * ncb;
       --left;
       ok = ok && warp_wait(&full[st], ph);
       if (!ok) break;
@@ -238,7 +252,7 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
           }
         }
         tc::mma_commit(&empty[st]);
-        if (left == 0 && (k == a.batch - 1 || u == n - 1)) tc::mma_commit(&done[half]);
+        if (left == 0 && (kHeld || u == n - 1)) tc::mma_commit(&done[kHeld ? set : 0]);
       }
       __syncwarp();
       if (++st == a.S) {
@@ -288,18 +302,31 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
 #pragma unroll
     for (int i = 0; i < 3 * 16 * (kHeld ? kHeld : 1); ++i) held[i / 48][i / 16 % 3][i % 16] = 0.0f;
     float* const xw = reinterpret_cast<float*>(smem + (size_t)a.S * a.stage + kPad) + (warp - 2) * (kXch / 4);
-    // block (o, g)'s tap column d
-    auto flush = [&](int o, int g, int d, const float* v) {
+    // block b's tap column d
+    auto flush = [&](int b, int d, float* v) {
+      const int o = b / a.G, g = b % a.G;
       const bool first = g0 + g < a.ng1;
       const int cl = (g0 + g - (first ? 0 : a.ng1)) * a.CB + odd * nc2;  // channel within its source
       const int c0 = (first ? 0 : a.C1) + cl, nc = (first ? a.C1 : a.C2) - cl;
+      const int m = q * 32 + lane, atom = a.KO == 32 ? m >> 5 : m >> 4;
+      float t = 0.0f;  // 0, or NaN once a sum is not finite
+#pragma unroll
+      for (int k = 0; k < 16; ++k) t = __fmaf_rn(v[k], 0.0f, t);
+      const bool bad = !(t == 0.0f) && atom < 3 && (atom != 1 || (d == 0 && a.W % 8));  // a tap that may have met dout's zeros
+      const uint32_t rows = __ballot_sync(0xffffffffu, bad);
+      if (rows) {
+        if (lane == 0) redo[(b * 3 + d) * kExpanders + warp - 2] = rows, again = 1;
+        if (bad)
+#pragma unroll
+          for (int k = 0; k < 16; ++k) v[k] = 0.0f;
+      }
       if (a.CB == 32)
         add_rows<16>(a, xw, v, (ob0 + o) * a.KO, q * 32, d, c0, nc, lane);
       else
         add_rows<8>(a, xw, v, (ob0 + o) * a.KO, q * 32, d, c0, nc, lane);
     };
-    int st = 0, half = a.halves - 1;
-    uint32_t ph = 1, half_ph = 1;
+    int st = 0, set = 1;
+    uint32_t ph = 1, set_ph = 1;
     Walk w(a, t0);
     auto arrive = [&](int stage) {
       tc::fence_proxy_async();
@@ -337,8 +364,9 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
       }
       return true;
     };
-    for (int u0 = 0; u0 < n && ok; u0 += a.run * a.batch) {
-      const int u1 = min(n, u0 + a.run * a.batch), runs = (u1 - u0 + a.run - 1) / a.run;
+    const int step = kHeld ? a.run : n, runs = kHeld ? 1 : (n + a.run - 1) / a.run;
+    for (int u0 = 0; u0 < n && ok; u0 += step) {
+      const int u1 = min(n, u0 + step);
       if (nup) {
         int prev = -1;
         for (int u = u0; u < u1; ++u, w.next(a)) {
@@ -377,14 +405,14 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
       } else if (bias) {
         for (int u = u0; u < u1 && ok; ++u) ok = sum_bias();
       }
-      if (++half == a.halves) {
-        half = 0;
-        half_ph ^= 1u;
+      if (!kHeld || ++set == a.sets) {
+        set = 0;
+        set_ph ^= 1u;
       }
-      ok = ok && warp_wait(&done[half], half_ph);
+      ok = ok && warp_wait(&done[set], set_ph);
       tc::fence_after();
       if (ok && taps) {
-        const uint32_t set = a.ao * a.G * ncb, t = lanes + half * a.batch * set;  // a run's columns
+        const uint32_t cols = a.ao * a.G * ncb, t = lanes + set * cols;
         if constexpr (kHeld > 0) {
 #pragma unroll
           for (int b = 0; b < kHeld; ++b)
@@ -408,7 +436,7 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
             float v[3][16] = {};
             for (int r = 0; r < runs; ++r) {
               float w[3][16];
-              const uint32_t tr = t + r * set + b * ncb;
+              const uint32_t tr = t + r * cols + b * ncb;
               if (a.CB == 32)
                 load3<16>(tr, a.CB, w);
               else
@@ -417,12 +445,12 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
               for (int k = 0; k < 48; ++k) v[k / 16][k % 16] += k % 16 < nc2 ? w[k / 16][k % 16] : 0.0f;
             }
 #pragma unroll
-            for (int d = 0; d < 3; ++d) flush(b / a.G, b % a.G, d, v[d]);
+            for (int d = 0; d < 3; ++d) flush(b, d, v[d]);
           }
         }
       }
       tc::fence_before();
-      tc::mbar_arrive(&drained[half]);
+      tc::mbar_arrive(&drained[set]);
     }
     if constexpr (kHeld > 0) {
       if (ok && taps)
@@ -430,13 +458,44 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
         for (int b = 0; b < kHeld; ++b)
           if (b / a.G < on && b % a.G < gn)
 #pragma unroll
-            for (int d = 0; d < 3; ++d) flush(b / a.G, b % a.G, d, held[b][d]);
+            for (int d = 0; d < 3; ++d) flush(b, d, held[b][d]);
     }
     if (bias && bp0 < bps)
 #pragma unroll
       for (int k = 0; k < 8; ++k) atomicAdd(&sdb[8 * bc + k], bsum[k]);
   }
-  if (!__syncthreads_and(ok) && lane == 0) atomicOr(a.err, tc::kErrMbarTimeout);
+  const bool all = __syncthreads_and(ok);
+  if (!all && lane == 0) atomicOr(a.err, tc::kErrMbarTimeout);
+  // rows to form again: a warp each, pixel by pixel with zeros outside the image
+  for (int i = warp; all && again && i < a.ao * a.G * 3 * kExpanders; i += kThreadsW / 32) {
+    for (uint32_t rows = redo[i]; rows; rows &= rows - 1) {
+      const int ew = i % kExpanders, d = i / kExpanders % 3, b = i / (3 * kExpanders), g = b % a.G;
+      const int m = ((ew + 2) & 3) * 32 + __ffs(rows) - 1, atom = m / a.KO;  // epilogue warp ew + 2's row
+      const bool first = g0 + g < a.ng1;
+      const int c = (g0 + g - (first ? 0 : a.ng1)) * a.CB + (ew >> 2) * (a.CB >> 1), C = first ? a.C1 : a.C2;
+      const int o = (ob0 + b / a.G) * a.KO + m % a.KO, dy = 1 - atom, up = first ? a.up1 : 0;
+      const bf16* const src = first ? a.x1 : a.x2;
+      for (int ck = c; ck < min(C, c + (a.CB >> 1)); ++ck) {
+        float s = 0.0f;
+        bool nan = false;
+        Walk w(a, t0);
+        for (int u = 0; u < n && !nan; ++u, w.next(a)) {
+          for (int h = lane; h < 8 * a.TR; h += 32) {
+            // the tile's pairs: its columns of dout, its rows of the source
+            const int x = w.x * 8 + (h & 7), Y = w.y * a.TR + (h >> 3), y = Y - dy, X = x + d - 1;
+            if (x < a.W && Y < a.H && y >= 0 && y < a.H) {
+              const float v = __bfloat162float(a.dout[(((size_t)w.img * a.H + y) * a.W + x) * a.Cout + o]);
+              const size_t p = ((size_t)w.img * (a.H >> up) + (Y >> up)) * (a.W >> up) + (X >> up);
+              s += v * (X >= 0 && X < a.W ? __bfloat162float(src[p * C + ck]) : 0.0f);
+            }
+          }
+          nan = __any_sync(0xffffffffu, s != s);  // and stays so
+        }
+        for (int j = 16; j > 0; j >>= 1) s += __shfl_xor_sync(0xffffffffu, s, j);
+        if (lane == 0) atomicAdd(a.dw + ((size_t)o * 9 + (2 - atom) * 3 + d) * a.Cin + (first ? 0 : a.C1) + ck, s);
+      }
+    }
+  }
   if (bias && tid < on * a.KO) atomicAdd(a.db + ob0 * a.KO + tid, sdb[tid]);
   tc::fence_before();
   __syncthreads();
@@ -493,6 +552,8 @@ bool conv_tile_wgrad(const ConvWgrad& c, cudaStream_t st, cudaError_t* e) {
   a.C2 = c.s2.ptr ? c.s2.C : 0;
   a.up1 = c.s1.up ? 1 : 0;
   a.x1 = c.s1.ptr;
+  a.x2 = c.s2.ptr;
+  a.dout = c.dout;
   a.H = c.H;
   a.W = c.W;
   a.dw = c.dw;
@@ -541,22 +602,22 @@ bool conv_tile_wgrad(const ConvWgrad& c, cudaStream_t st, cudaError_t* e) {
     const int columns = a.ngc * ((at + o - 1) / o);
     const int ranges = (int)std::min<long long>(std::max(1, tile_sm_count() / columns), most);
     a.per = (a.tiles + ranges - 1) / ranges;
-    const int run = (int)std::max(1LL, std::min<long long>(a.per, limit / px)), runs = (a.per + run - 1) / run;
+    // a run of a few tiles counts them as full, a longer one as full as they are on average
+    long long run = limit / px;
+    if (run >= 4) run = limit * a.tx * a.ty / ((long long)c.H * c.W);
+    run = std::max(1LL, std::min<long long>(a.per, run));
+    const int runs = (int)((a.per + run - 1) / run), used = (a.tiles + a.per - 1) / a.per;
     a.run = (a.per + runs - 1) / runs;  // equal runs
     // several runs: held in registers where a CTA has one or two blocks, else
-    // as many to a flush as TMEM has accumulators
-    const int sets = 512 / (o * g * 3 * a.CB);
+    // no more than TMEM has accumulators for
     held = runs > 1 && o * g <= 2 ? o * g : 0;
-    a.halves = held || (runs > sets && sets > 1) ? 2 : 1;
-    a.batch = held ? 1 : std::min(runs, sets / a.halves);
-    const int flushes = held ? 1 : (runs + a.batch - 1) / a.batch, used = (a.tiles + a.per - 1) / a.per;
-    *over = (long long)flushes * used > most;
+    a.sets = held ? 2 : runs;
+    if (a.sets * o * g * 3 * a.CB > 512) return false;
+    *over = used > most;
     const double mmas = (TR / 2) * o * g, unit = kUnit + mmas * (a.CB == 32 ? kMma32 : kMma16);
     const double work = a.per * unit, flush = o * g * kFlush;
     const double waves = (columns * used + tile_sm_count() - 1) / tile_sm_count();
-    *cost = waves * (kStart + (a.halves == 1 ? work + flushes * flush
-                               : held        ? std::max(work, runs * o * g * kHold) + flush
-                                             : std::max(work, flushes * flush) + flush));
+    *cost = waves * (kStart + (held ? std::max(work, runs * o * g * kHold) : work) + flush);
     return true;
   };
   double best = 0, cost;
@@ -573,7 +634,7 @@ bool conv_tile_wgrad(const ConvWgrad& c, cudaStream_t st, cudaError_t* e) {
   if (!pick[0] || !split(pick[0], pick[1], pick[2], &cost, &over)) return false;
   const int TR = pick[0];
   const int columns = a.ngc * ((at + a.ao - 1) / a.ao);
-  const uint32_t cols = (uint32_t)(a.halves * a.batch * a.ao * G * 3 * a.CB);
+  const uint32_t cols = (uint32_t)(a.sets * a.ao * G * 3 * a.CB);
   for (a.ncols = 32; a.ncols < cols;) a.ncols *= 2;
   WgradMaps m{};
   if (!pixel_map(&m.dout, c.dout, c.N, c.H, c.W, c.Cout, 1, 1, a.KO, 8, TR + 2)) return false;

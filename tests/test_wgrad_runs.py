@@ -50,8 +50,8 @@ def test_error_of_sums_of_one_sign(ctx, c):
     (32, 16, 16, 128, 0, 0, 160),   # two blocks of outputs held, the last CTA's alone
     (8, 16, 16, 16, 0, 0, 48),      # 16-channel groups, blocks of 16 outputs
     (16, 32, 32, 16, 0, 0, 80),     # the same, several runs
-    (6, 100, 68, 64, 1, 32, 32),    # three channel groups, two flushes of one run
-    (5, 68, 100, 160, 1, 0, 16),    # five groups of one block of 16 outputs
+    (6, 100, 68, 64, 1, 32, 32),    # three channel groups shared out over CTAs
+    (5, 68, 100, 160, 1, 0, 16),    # five groups, one block of 16 outputs
     (3, 24, 40, 24, 0, 8, 96),      # part-filled groups over several runs
     (16, 40, 24, 96, 0, 0, 256),    # eight blocks of outputs
     (40, 8, 8, 32, 1, 32, 32),      # tiles of one image each, many per CTA
