@@ -317,10 +317,11 @@ RTX_DEV int4 node4(const RayBox4& r, const float4* n, float tmax, float (&k)[4])
 
 constexpr int kNoNode = 0x76543210;  // above every node index
 
-// Closest hit over the 4-wide tree; same result as closest_hit.
-template <bool kAnyHit, bool kCount>
+// Closest hit over the 4-wide tree; same result as closest_hit.  A stack that
+// is full ends the walk with a call of `full`.
+template <bool kAnyHit, bool kCount, class Full>
 RTX_DEV int trace4(const DeviceScene& s, F3 o, F3 d, int exclude, int target, float& t, float& u,
-                   float& v, int* err, VisitCount& vc) {
+                   float& v, VisitCount& vc, Full full) {
   // closest hit: t starts at 1e7, returns the triangle; occlusion: t is the
   // limit, returns 1 when occluded, -1 otherwise
   if (!kAnyHit) t = kInf;
@@ -439,7 +440,7 @@ RTX_DEV int trace4(const DeviceScene& s, F3 o, F3 d, int exclude, int target, fl
   while (node != kNoNode || leaf < 0) {
     while ((unsigned)node < (unsigned)kNoNode) {
       if (!descend()) {
-        atomicOr(err, kErrStackOverflow);
+        full();
         return kAnyHit ? 1 : best;
       }
       if (node < 0 && leaf >= 0) {
@@ -460,12 +461,25 @@ RTX_DEV int trace4(const DeviceScene& s, F3 o, F3 d, int exclude, int target, fl
   return best;
 }
 
-// Closest hit over the tree RTX_OPT_TRAVERSAL selects
+template <bool kAnyHit, bool kCount>
+RTX_DEV int trace4(const DeviceScene& s, F3 o, F3 d, int exclude, int target, float& t, float& u,
+                   float& v, int* err, VisitCount& vc) {
+  return trace4<kAnyHit, kCount>(s, o, d, exclude, target, t, u, v, vc, [&] { atomicOr(err, kErrStackOverflow); });
+}
+
+// Closest hit of a primary pass or a ray query over the tree RTX_OPT_TRAVERSAL
+// selects.  A 4-wide walk keeps up to three entries a level where the binary
+// one keeps one, so a ray that fills its stack starts again on the binary tree:
+// no ray is refused that the binary walk answers.
 template <bool kWide>
 RTX_DEV int first_hit(const DeviceScene& s, F3 o, F3 d, int exclude, float& t, float& u, float& v, int* err,
                       VisitCount& vc) {
-  return kWide ? trace4<false, false>(s, o, d, exclude, -1, t, u, v, err, vc)
-               : closest_hit<false>(s, o, d, exclude, t, u, v, err, vc);
+  if constexpr (kWide) {
+    bool full = false;
+    const int h = trace4<false, false>(s, o, d, exclude, -1, t, u, v, vc, [&] { full = true; });
+    if (!full) return h;
+  }
+  return closest_hit<false>(s, o, d, exclude, t, u, v, err, vc);
 }
 
 // ---------------------------------------------------------------------------
