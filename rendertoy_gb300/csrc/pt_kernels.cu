@@ -1026,11 +1026,31 @@ constexpr int kMatPer = 8;
 // warp and key queued at a handful of addresses: the eight scatters of the
 // nine-material frame (1.8 M paths) 311 -> 58 us, the frame 2.86 -> 2.62 ms,
 // at 1,024^2 x 16 21.8 -> 19.4 ms, the eight-scene batch 21.2 -> 19.4 ms.
+// With fewer than 64 entries per key a chunk's sweep over all counts costs more
+// than such atomics do, and chunks are too few: there a warp's lanes take their
+// places themselves (16,384 paths: 1,024 materials 6.9 -> 4.6 us, 4,095
+// materials 11.7 -> 5.0; 4.2 M paths of 1,024: 155 us that way, 27 in chunks).
 __global__ void __launch_bounds__(256) k_sort_scatter(PtArgs a, DeviceScene s, int* hist, const int* keys, int* sorted) {
   extern __shared__ int sh[];
   int* offs = hist + kMaxSortBins + 1;
   const int n = a.counts[a.depth], bins = s.n_mats + 1, tid = threadIdx.x;
   int *cnt = sh, *run = sh + bins;
+  // lanes with equal keys: the first adds their number to *count(key); each
+  // lane's place
+  auto place = [&](int key, int* count) {
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    const int leader = __ffs(peers) - 1, lane = tid & 31;
+    int r = 0;
+    if (lane == leader && key >= 0) r = atomicAdd(&count[key], __popc(peers));
+    return __shfl_sync(0xffffffffu, r, leader) + __popc(peers & ((1u << lane) - 1u));
+  };
+  if (n < 64 * bins) {
+    for (int base = blockIdx.x * 256; base < n; base += gridDim.x * 256) {
+      const int i = base + tid, key = i < n ? keys[i] : -1, at = place(key, offs);
+      if (key >= 0) sorted[at] = a.queue_in[i];
+    }
+    return;
+  }
   for (int c0 = blockIdx.x * 256 * kMatPer; c0 < n; c0 += gridDim.x * 256 * kMatPer) {
     for (int b = tid; b < bins; b += 256) cnt[b] = 0;
     int key[kMatPer], rank[kMatPer], path[kMatPer];
@@ -1042,13 +1062,7 @@ __global__ void __launch_bounds__(256) k_sort_scatter(PtArgs a, DeviceScene s, i
     }
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < kMatPer; ++j) {
-      const unsigned peers = __match_any_sync(0xffffffffu, key[j]);
-      const int leader = __ffs(peers) - 1, lane = tid & 31;
-      int r = 0;
-      if (lane == leader && key[j] >= 0) r = atomicAdd(&cnt[key[j]], __popc(peers));
-      rank[j] = __shfl_sync(0xffffffffu, r, leader) + __popc(peers & ((1u << lane) - 1u));
-    }
+    for (int j = 0; j < kMatPer; ++j) rank[j] = place(key[j], cnt);
     __syncthreads();
     for (int b = tid; b < bins; b += 256)
       if (cnt[b]) run[b] = atomicAdd(&offs[b], cnt[b]);
