@@ -1929,7 +1929,6 @@ int rtx_nn_conv3x3_wgrad(rtx_context* c, int N, int H, int W, const void* dout, 
   a.H = H;
   a.W = W;
   a.Cin = Cin;
-  a.pix_per_cta = rtx::nn::wgrad_pixels_per_cta(P, Cout, Cin);
   a.dw = (float*)ao.dev;
   a.err = c->d_err;
   cudaError_t e = rtx::nn::conv_wgrad(a, c->stream);

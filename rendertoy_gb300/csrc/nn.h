@@ -51,8 +51,8 @@ struct ConvFwd {
   bf16* out;         // [P][Cout] or nullptr
   float* out_f32;    // [P][Cout] or nullptr
   int* err;
-  // [P / 4][Cout] or nullptr (only where conv_fwd_pools says so): the output's
-  // 2 x 2 averages, written beside it
+  // [P / 4][Cout] or nullptr: the output's 2 x 2 averages, written beside it
+  // (tile kernels, a full-resolution source, even H and W)
   bf16* pool = nullptr;
 };
 
@@ -78,7 +78,7 @@ struct ConvDgrad {
   int mask_relu;
   bf16* din;         // [P][Cin] (s1's channels upsampled when s1.up)
   int* err;
-  // Both given (only where conv_dgrad_splits says so): instead of din, s1's
+  // Both given (tile kernels, s1 upsampled and s2 a skip source): instead of din, s1's
   // channels go to dlow [P / 4][C1], summed over each 2 x 2 block (nearest
   // upsampling's gradient), and s2's to dskip [P][C2].
   bf16 *dlow = nullptr, *dskip = nullptr;
@@ -89,25 +89,17 @@ struct ConvWgrad {
   int Cout;
   Src s1, s2;
   int N, H, W, Cin;
-  int pix_per_cta;   // pixels each CTA sums (multiple of 64)
   float* dw;         // [Cout][9][Cin], accumulated
   int* err;
   float* db = nullptr;  // [Cout] or nullptr: the bias gradient, accumulated
 };
 
 cudaError_t conv_fwd(const ConvFwd& a, cudaStream_t st);
-bool conv_fwd_pools(const ConvFwd& a);
 // The output layer with its head in one launch; false: not a shape it takes
 // (rows of at least 64 pixels), nothing launched.
 bool conv_head(const ConvFwd& a, const KpHead& h, cudaStream_t st, cudaError_t* e);
 cudaError_t conv_dgrad(const ConvDgrad& a, cudaStream_t st);
-// whether conv_dgrad can write an upsampled + skip concatenation's gradient
-// straight to its two sources (dlow, dskip)
-bool conv_dgrad_splits(const ConvDgrad& a);
 cudaError_t conv_wgrad(const ConvWgrad& a, cudaStream_t st);
-// pixels per weight-gradient CTA: enough CTAs for about eight per SM, each
-// summing a multiple of 64 pixels
-int wgrad_pixels_per_cta(long long P, int Cout, int Cin);
 
 }  // namespace nn
 }  // namespace rtx

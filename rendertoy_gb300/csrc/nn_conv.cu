@@ -14,17 +14,14 @@
 //             GEMM M = pixels, N = Cin (tiles of <= 256), K = 9 * Cout, with
 //             the weights re-laid out as wt[c, t, o]; mask = (src > 0) when
 //             the source is a ReLU output
-//   wgrad   : dw[o, t, c] += sum_p dout[p, o] src[p + off(t), c]
-//             GEMM M = 9 * Cin (128 (t, c) rows per CTA), N = Cout (<= 256),
-//             K = the CTA's range of pixels; both operands staged MN-major
-//             (16-byte chunks = 8 channels of one pixel); FP32 atomics
-//             combine the ranges
+//   wgrad   : dw[o, t, c] += sum_p dout[p, o] src[p + off(t), c], all of it in
+//             nn_wgrad_tile.cu
 // off(t) = (t / 3 - 1, t % 3 - 1).  Out-of-image taps read zero ("same"
 // zero padding).
 //
 // Channel counts that are multiples of 16 run as tiles (nn_conv_tile.cu,
-// nn_wgrad_tile.cu).  The gather kernels here: the K (or pixel) range is cut
-// into slices of 64; every thread copies its 16-byte chunks of a slice straight
+// nn_wgrad_tile.cu).  The gather kernels here: the K range is cut into slices of
+// 64; every thread copies its 16-byte chunks of a slice straight
 // into shared memory with cp.async (zero-filled where the tap falls outside
 // the image), S - 1 slices ahead, into a ring of S stages.  Thread 0 issues the
 // slice's MMAs and commits them to the stage's mbarrier; a stage is refilled
@@ -32,7 +29,6 @@
 #include <algorithm>
 
 #include "nn.h"
-#include "nn_ops.h"
 #include "nn_tile.h"
 #include "tc_core.cuh"
 
@@ -593,82 +589,6 @@ __global__ void __launch_bounds__(kThreads, 2) k_conv_dgrad(ConvDgrad a) {
 }
 
 // ---------------------------------------------------------------------------
-// weight gradient
-// ---------------------------------------------------------------------------
-template <int S>
-__global__ void __launch_bounds__(kThreads, 2) k_conv_wgrad(ConvWgrad a) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  __shared__ __align__(8) uint64_t bars[S];
-  __shared__ uint32_t tmem_slot;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int P = a.N * a.H * a.W;  // < 2^31 (checked by the host)
-  const int J = 9 * a.Cin;
-  const int j0 = blockIdx.x * 128;
-  const int pb = blockIdx.y * a.pix_per_cta;
-  const int pe = min(P, pb + a.pix_per_cta);
-  const uint32_t ncols = a.Cout <= 32 ? 32 : (a.Cout <= 64 ? 64 : (a.Cout <= 128 ? 128 : 256));
-  const uint32_t a_bytes = 128 * kSlice * 2, stage = a_bytes + (uint32_t)a.Cout * kSlice * 2;
-  tc_begin(&tmem_slot, bars, S, ncols);
-  const uint32_t tmem = tmem_slot;
-  const uint32_t idesc = tc::make_idesc_bf16(128, a.Cout, true, true);
-  const uint32_t s0 = tc::smem_u32(smem);
-  const int n_slices = pe > pb ? (pe - pb + kSlice - 1) / kSlice : 0;
-  // this thread's 8 rows of the A tile: (tap, channel) j = j0 + 8 rg
-  const int rg = tid & 15;
-  const int j = j0 + rg * 8;
-  const bool jv = j < J;
-  const int t = jv ? j / a.Cin : 0, c = jv ? j - t * a.Cin : 0;
-  const int dy = t / 3 - 1, dx = t % 3 - 1;
-  const int HW = a.H * a.W;
-  const int ng = a.Cout >> 3;
-  auto load = [&](int slice, int st) {
-    if (slice >= n_slices) return;
-    const uint32_t sa = s0 + st * stage, sb = sa + a_bytes;
-    const int q0 = pb + slice * kSlice;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int kp = (tid >> 4) + 16 * i;  // pixel within the slice
-      const int p = q0 + kp;
-      const bf16* src = nullptr;
-      if (p < pe && jv) {
-        const int n = p / HW, rem = p - n * HW;
-        const int y = rem / a.W, x = rem - y * a.W;
-        src = src_ptr(a.s1, a.s2, a.H, a.W, n, y + dy, x + dx, c);
-      }
-      chunk_async(sa + tc::tile_offset_mn(rg * 8, kp, 128), src, a.s1.ptr);
-    }
-    for (int ch = tid; ch < ng * kSlice; ch += kThreads) {
-      const int og = ch % ng, kp = ch / ng;
-      const int p = q0 + kp;
-      const bf16* src = p < pe ? a.dout + (size_t)p * a.Cout + og * 8 : nullptr;
-      chunk_async(sb + tc::tile_offset_mn(og * 8, kp, a.Cout), src, a.dout);
-    }
-  };
-  auto mma = [&](int st, bool first) {
-    const uint32_t a0 = s0 + st * stage, b0 = a0 + a_bytes;
-    const uint64_t ad = tc::make_desc(a0, 16 * 128, 128), bd = tc::make_desc(b0, 16 * a.Cout, 128);
-#pragma unroll
-    for (int s = 0; s < kSlice / 16; ++s)
-      tc::mma_bf16(tmem, ad + s * 2 * 128, bd + s * 2 * a.Cout, idesc, !first || s > 0);
-  };
-  const bool ok = conv_pipeline<S>(n_slices, bars, load, mma, a.err);
-  tc::fence_after();
-  if (ok && n_slices > 0) {
-    const int lw = warp & 3, half = a.Cout >> 1;
-    const int jj = j0 + lw * 32 + lane;  // this thread's accumulator row
-    const uint32_t taddr = tmem + ((uint32_t)(lw * 32) << 16);
-    for (int c0 = (warp >> 2) * half; c0 < (warp >> 2) * half + half; c0 += 8) {
-      float v[8];
-      tc::tmem_ld8(taddr + c0, v);
-      if (jj < J)
-#pragma unroll
-        for (int i = 0; i < 8; ++i) atomicAdd(a.dw + (size_t)(c0 + i) * J + jj, v[i]);
-    }
-  }
-  tc_end(tmem, ncols);
-}
-
-// ---------------------------------------------------------------------------
 // Stages of the ring for a B tile of nb rows: 3 stages up to 128 rows, 2
 // beyond (72 KB per CTA for nb <= 64, at most 96 KB otherwise).
 static int stages_for(int nb) { return nb <= 128 ? 3 : 2; }
@@ -761,6 +681,7 @@ constexpr size_t kResidentWeights = 128 * 1024;
 cudaError_t conv_fwd(const ConvFwd& a, cudaStream_t st) {
   long long P = (long long)a.N * a.H * a.W;
   if (a.Cout % 16 || a.Cout > 256 || a.Cin % 8) return cudaErrorInvalidValue;
+  if (a.pool && (a.s1.up || !a.out || a.H % 2 || a.W % 2)) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
   if (conv_tile_fwd(a, use_rows(a.W, a.Cin), st, &e)) return e;
   if (a.pool) return cudaErrorNotSupported;  // only the tile kernels pool
@@ -778,22 +699,14 @@ cudaError_t conv_fwd(const ConvFwd& a, cudaStream_t st) {
                        stage, a, st);
 }
 
-bool conv_fwd_pools(const ConvFwd& a) {
-  return conv_tile_takes_fwd(a, use_rows(a.W, a.Cin)) && !a.s1.up && a.out && a.H % 2 == 0 && a.W % 2 == 0;
-}
-
 bool conv_head(const ConvFwd& a, const KpHead& h, cudaStream_t st, cudaError_t* e) {
   return use_rows(a.W, a.Cin) && conv_tile_head(a, h, st, e);
-}
-
-bool conv_dgrad_splits(const ConvDgrad& a) {
-  return conv_tile_takes_dgrad(a, use_rows(a.W, a.Cout)) && a.s1.up && a.s2.ptr && a.s1.C % 16 == 0 &&
-         a.H % 2 == 0 && a.W % 2 == 0;
 }
 
 cudaError_t conv_dgrad(const ConvDgrad& a, cudaStream_t st) {
   long long P = (long long)a.N * a.H * a.W;
   if (a.Cin % 16 || a.Cout % 8) return cudaErrorInvalidValue;
+  if (a.dlow && (!a.s1.up || !a.s2.ptr || a.s1.C % 16 || a.H % 2 || a.W % 2)) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
   if (conv_tile_dgrad(a, use_rows(a.W, a.Cout), st, &e)) return e;
   if (a.dlow || a.dskip) return cudaErrorNotSupported;  // only the tile kernel splits its output
@@ -804,24 +717,11 @@ cudaError_t conv_dgrad(const ConvDgrad& a, cudaStream_t st) {
                        stage, a, st);
 }
 
-int wgrad_pixels_per_cta(long long P, int Cout, int Cin) {
-  (void)Cout;
-  int tiles = (9 * Cin + 127) / 128;
-  long long ranges = std::max(1, 8 * 152 / tiles);
-  long long per = (P + ranges - 1) / ranges;
-  per = (per + 63) / 64 * 64;
-  return (int)std::max(64LL, std::min(per, 1LL << 30));
-}
-
 cudaError_t conv_wgrad(const ConvWgrad& a, cudaStream_t st) {
   long long P = (long long)a.N * a.H * a.W;
   if (P >= (1LL << 31) || a.Cout % 16 || a.Cout > 256) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
-  if (conv_tile_wgrad(a, st, &e)) return e;
-  if (a.db && (e = bias_grad(a.dout, P, a.Cout, a.db, st))) return e;
-  size_t stage = 128 * kSlice * 2 + (size_t)a.Cout * kSlice * 2;
-  dim3 grid((9 * a.Cin + 127) / 128, (unsigned)((P + a.pix_per_cta - 1) / a.pix_per_cta));
-  return launch_staged(k_conv_wgrad<4>, k_conv_wgrad<3>, k_conv_wgrad<2>, stages_for(a.Cout), grid, stage, a, st);
+  return conv_tile_wgrad(a, st, &e) ? e : cudaErrorNotSupported;  // it takes every shape allowed here
 }
 
 }  // namespace nn

@@ -77,7 +77,6 @@ struct TileArgs {
   int nslab1, nslab;        // slabs of the first source, of both
   int R, S, nbuf;           // service warps, stages of each one's ring, accumulator buffers
   uint32_t stage, w_off;    // ring stage bytes, weights within a streamed stage
-  int flip;                 // data gradient: taps mirrored
   uint32_t ncols;           // TMEM columns allocated
   // epilogue
   const float* bias;
@@ -1124,7 +1123,7 @@ static bool plan_narrow(TileArgs a, const Src& x1, const Src& x2, const bf16* w,
   return true;
 }
 
-bool conv_tile_takes_fwd(const ConvFwd& c, bool wide) {
+static bool takes_fwd(const ConvFwd& c, bool wide) {
   const int g = c.s2.ptr ? (c.s1.C | c.s2.C) : c.s1.C;
   if (g % 16 || c.Cout % 16 || c.s2.up || (c.s1.up && (c.H % 2 || c.W % 2))) return false;
   if (c.out && (reinterpret_cast<uintptr_t>(c.out) & 15)) return false;
@@ -1132,7 +1131,7 @@ bool conv_tile_takes_fwd(const ConvFwd& c, bool wide) {
 }
 
 bool conv_tile_fwd(const ConvFwd& c, bool wide, cudaStream_t st, cudaError_t* e) {
-  if (!conv_tile_takes_fwd(c, wide)) return false;
+  if (!takes_fwd(c, wide)) return false;
   const int g = c.s2.ptr ? (c.s1.C | c.s2.C) : c.s1.C;
   TileArgs a{};
   a.H = c.H;
@@ -1167,13 +1166,13 @@ bool conv_tile_head(const ConvFwd& c, const KpHead& h, cudaStream_t st, cudaErro
                : plan_wide<32, false, 2>(a, c.s1, none, c.w, c.N, st, e);
 }
 
-bool conv_tile_takes_dgrad(const ConvDgrad& c, bool wide) {
+static bool takes_dgrad(const ConvDgrad& c, bool wide) {
   if (c.Cout % 16 || c.Cin % 16) return false;
   return wide || narrow_fits(c.Cout % 32 == 0 ? 32 : 16, c.Cout);
 }
 
 bool conv_tile_dgrad(const ConvDgrad& c, bool wide, cudaStream_t st, cudaError_t* e) {
-  if (!conv_tile_takes_dgrad(c, wide)) return false;
+  if (!takes_dgrad(c, wide)) return false;
   TileArgs a{};
   a.H = c.H;
   a.W = c.W;
@@ -1184,7 +1183,6 @@ bool conv_tile_dgrad(const ConvDgrad& c, bool wide, cudaStream_t st, cudaError_t
   a.din = c.din;
   a.dlow = c.dlow;
   a.dskip = c.dskip;
-  a.flip = 1;
   a.err = c.err;
   const Src d{c.dout, c.Cout, 0}, none{nullptr, 0, 0};
   if (!wide)

@@ -139,64 +139,6 @@ __global__ void k_encode_passes(const float* __restrict__ rad, const float* __re
   encode_px(f, x + 16 * ((long long)py * Wp + px));
 }
 
-__global__ void k_avgpool(const bf16* __restrict__ in, bf16* __restrict__ out, int N, int H, int W, int C) {
-  int h = H >> 1, w = W >> 1, c8 = C >> 3;
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  long long total = (long long)N * h * w * c8;
-  if (i >= total) return;
-  int c = (int)(i % c8) * 8;
-  long long q = i / c8;
-  int x = (int)(q % w);
-  long long r = q / w;
-  int y = (int)(r % h);
-  int n = (int)(r / h);
-  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}, v[8];
-  for (int dy = 0; dy < 2; ++dy)
-    for (int dx = 0; dx < 2; ++dx) {
-      ld8(in + (((size_t)n * H + 2 * y + dy) * W + 2 * x + dx) * C + c, v);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc[k] += v[k];
-    }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) acc[k] *= 0.25f;
-  st8(out + q * C + c, acc);
-}
-
-// d_low[n, y, x, c] = sum over the 2 x 2 block of dcat[.., c0 + c] (nearest
-// upsampling's gradient), channels [c0, c0 + C) of a Ccat-channel tensor
-__global__ void k_upsample_grad(const bf16* __restrict__ dcat, int Ccat, int c0, bf16* __restrict__ dlow,
-                                int N, int H, int W, int C) {
-  int h = H >> 1, w = W >> 1, c8 = C >> 3;
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  long long total = (long long)N * h * w * c8;
-  if (i >= total) return;
-  int c = (int)(i % c8) * 8;
-  long long q = i / c8;
-  int x = (int)(q % w);
-  long long r = q / w;
-  int y = (int)(r % h);
-  int n = (int)(r / h);
-  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}, v[8];
-  for (int dy = 0; dy < 2; ++dy)
-    for (int dx = 0; dx < 2; ++dx) {
-      ld8(dcat + (((size_t)n * H + 2 * y + dy) * W + 2 * x + dx) * Ccat + c0 + c, v);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc[k] += v[k];
-    }
-  st8(dlow + q * C + c, acc);
-}
-
-// dst[p, c] = dcat[p, c0 + c] (a skip connection's share of a concatenation)
-__global__ void k_take_channels(const bf16* __restrict__ dcat, int Ccat, int c0, bf16* __restrict__ dst,
-                                long long P, int C) {
-  int c8 = C >> 3;
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= P * c8) return;
-  long long p = i / c8;
-  int c = (int)(i % c8) * 8;
-  *reinterpret_cast<uint4*>(dst + p * C + c) = *reinterpret_cast<const uint4*>(dcat + p * Ccat + c0 + c);
-}
-
 // dskip[p, c] += (skip[p, c] > 0) * 0.25 * dpool[p / 2, c]: the pooled path's
 // gradient reaching a ReLU output
 __global__ void k_pool_grad_acc(const bf16* __restrict__ dpool, const bf16* __restrict__ skip,
@@ -310,40 +252,6 @@ __global__ void __launch_bounds__(kKpBlock) k_kp_loss(const float* __restrict__ 
   if ((threadIdx.x & 31) == 0) atomicAdd(loss, (double)part);
 }
 
-// db[c] += sum_p dout[p, c].  Thread t of a 256-thread block owns the
-// 8-channel group t % (C / 8) and walks pixels t / (C / 8), + 256 / (C / 8),
-// ... of the block's range; the block then sums its partials in shared memory
-// and adds one value per channel (C <= 256).
-__device__ __forceinline__ void bias_grad_block(const bf16* __restrict__ dout, long long P, int C,
-                                                long long per_block, int block, float* __restrict__ db) {
-  __shared__ float part[256][9];
-  const int groups = C >> 3, lanes = 256 / groups, tid = threadIdx.x;
-  const int g = tid % groups, l = tid / groups;
-  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}, v[8];
-  if (l < lanes) {
-    long long p0 = block * per_block, p1 = min(P, p0 + per_block);
-    for (long long p = p0 + l; p < p1; p += lanes) {
-      ld8(dout + p * C + 8 * g, v);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc[k] += v[k];
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 8; ++k) part[tid][k] = acc[k];
-  __syncthreads();
-  if (tid < C) {
-    int gg = tid >> 3, k = tid & 7;
-    float s = 0.0f;
-    for (int j = 0; j < lanes; ++j) s += part[j * groups + gg][k];
-    atomicAdd(db + tid, s);
-  }
-}
-
-__global__ void __launch_bounds__(256) k_bias_grad(const bf16* __restrict__ dout, long long P, int C,
-                                                   long long per_block, float* __restrict__ db) {
-  bias_grad_block(dout, P, C, per_block, blockIdx.x, db);
-}
-
 // Adam (Kingma & Ba) on the FP32 master parameters
 __global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                        float* __restrict__ v, long long n, float lr, float b1, float b2, float eps,
@@ -420,21 +328,6 @@ cudaError_t encode_input(const float* raw, bf16* x, long long P, cudaStream_t st
   k_encode_input<<<blocks(P), 256, 0, st>>>(raw, x, P);
   return cudaGetLastError();
 }
-cudaError_t avgpool(const bf16* in, bf16* out, int N, int H, int W, int C, cudaStream_t st) {
-  long long n = (long long)N * (H / 2) * (W / 2) * (C / 8);
-  k_avgpool<<<blocks(n), 256, 0, st>>>(in, out, N, H, W, C);
-  return cudaGetLastError();
-}
-cudaError_t upsample_grad(const bf16* dcat, int Ccat, int c0, bf16* dlow, int N, int H, int W, int C,
-                          cudaStream_t st) {
-  long long n = (long long)N * (H / 2) * (W / 2) * (C / 8);
-  k_upsample_grad<<<blocks(n), 256, 0, st>>>(dcat, Ccat, c0, dlow, N, H, W, C);
-  return cudaGetLastError();
-}
-cudaError_t take_channels(const bf16* dcat, int Ccat, int c0, bf16* dst, long long P, int C, cudaStream_t st) {
-  k_take_channels<<<blocks(P * (C / 8)), 256, 0, st>>>(dcat, Ccat, c0, dst, P, C);
-  return cudaGetLastError();
-}
 cudaError_t pool_grad_acc(const bf16* dpool, const bf16* skip, bf16* dskip, int N, int H, int W, int C,
                           cudaStream_t st) {
   long long n = (long long)N * H * W * (C / 8);
@@ -447,13 +340,6 @@ cudaError_t kp_loss(const float* pred, const float* raw, const float* target, bf
     k_kp_loss<true><<<blocks((long long)N * H * W), kKpBlock, 0, st>>>(pred, raw, target, dpred, N, H, W, loss);
   else
     k_kp_loss<false><<<blocks((long long)N * H * W), kKpBlock, 0, st>>>(pred, raw, target, dpred, N, H, W, loss);
-  return cudaGetLastError();
-}
-cudaError_t bias_grad(const bf16* dout, long long P, int C, float* db, cudaStream_t st) {
-  if (C % 8 || C > 256) return cudaErrorInvalidValue;
-  long long nb = std::min<long long>(2 * 152, (P + 255) / 256);
-  long long per = (P + nb - 1) / nb;
-  k_bias_grad<<<(unsigned)nb, 256, 0, st>>>(dout, P, C, per, db);
   return cudaGetLastError();
 }
 cudaError_t adam(float* p, const float* g, float* m, float* v, long long n, float lr, int step,

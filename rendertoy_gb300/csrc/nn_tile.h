@@ -12,10 +12,8 @@ namespace nn {
 
 // wide: additions in slab-major order (the rule for rows of 64 pixels or
 // more), else tap-major
-bool conv_tile_takes_fwd(const ConvFwd& a, bool wide);
 bool conv_tile_fwd(const ConvFwd& a, bool wide, cudaStream_t st, cudaError_t* e);
 bool conv_tile_head(const ConvFwd& a, const KpHead& h, cudaStream_t st, cudaError_t* e);
-bool conv_tile_takes_dgrad(const ConvDgrad& a, bool wide);
 bool conv_tile_dgrad(const ConvDgrad& a, bool wide, cudaStream_t st, cudaError_t* e);
 
 bool conv_tile_wgrad(const ConvWgrad& a, cudaStream_t st, cudaError_t* e);

@@ -78,7 +78,6 @@ struct UNet::Impl {
   long long cap = 0;
   bf16* act[kTensors] = {};
   bf16* dact[kTensors] = {};
-  bf16* dcat = nullptr;
   float* pred = nullptr;     // filter logits [P][kPredCh]
   bf16* dpred = nullptr;
   double* loss = nullptr;
@@ -91,10 +90,9 @@ struct UNet::Impl {
       if (dact[t]) cudaFree(dact[t]);
       act[t] = dact[t] = nullptr;
     }
-    void* ps[] = {dcat, pred, dpred};
+    void* ps[] = {pred, dpred};
     for (void* p : ps)
       if (p) cudaFree(p);
-    dcat = nullptr;
     pred = nullptr;
     dpred = nullptr;
     cap = 0;
@@ -118,9 +116,6 @@ struct UNet::Impl {
       if ((e = cudaMalloc(&act[t], n * sizeof(bf16)))) return e;
       if ((e = cudaMalloc(&dact[t], n * sizeof(bf16)))) return e;
     }
-    size_t ncat = std::max({(size_t)P0 * 96, (size_t)(P0 >> 2) * 160, (size_t)(P0 >> 4) * 224,
-                            (size_t)(P0 >> 6) * 288});
-    if ((e = cudaMalloc(&dcat, ncat * sizeof(bf16)))) return e;
     if ((e = cudaMalloc(&pred, (size_t)P0 * kPredCh * sizeof(float)))) return e;
     if ((e = cudaMalloc(&dpred, (size_t)P0 * kPredCh * sizeof(bf16)))) return e;
     cap = P0;
@@ -275,12 +270,8 @@ cudaError_t UNet::forward(const float* d_raw, int N, int H, int W, int* err, cud
     }
     // a skip tensor's 2 x 2 averages feed the next level
     const bool skip = l.d.out == tS0 || l.d.out == tS1 || l.d.out == tS2 || l.d.out == tS3;
-    if (skip && conv_fwd_pools(c)) c.pool = I.act[l.d.out + 1];
+    if (skip) c.pool = I.act[l.d.out + 1];
     if ((e = conv_fwd(c, st))) return e;
-    if (skip && !c.pool) {
-      if ((e = avgpool(I.act[l.d.out], I.act[l.d.out + 1], N, c.H, c.W, kTC[l.d.out], st))) return e;
-      ++I.launches;
-    }
   }
   return cudaSuccess;
 }
@@ -308,7 +299,6 @@ cudaError_t UNet::backward(int N, int H, int W, int* err, cudaStream_t st) {
     g.H = h;
     g.W = w;
     g.Cin = l.cin_pad;
-    g.pix_per_cta = wgrad_pixels_per_cta(P, l.d.cout_pad, l.cin_pad);
     g.dw = I.grad + l.w_off;
     g.db = I.grad + l.b_off;
     g.err = err;
@@ -330,19 +320,10 @@ cudaError_t UNet::backward(int N, int H, int W, int* err, cudaStream_t st) {
     d.mask_relu = pooled ? 0 : 1;  // pooled inputs are not ReLU outputs
     d.err = err;
     if (l.d.s2 >= 0) {
-      if (conv_dgrad_splits(d)) {
-        d.dlow = I.dact[l.d.s1];
-        d.dskip = I.dact[l.d.s2];
-        if ((e = conv_dgrad(d, st))) return e;
-        ++I.launches;
-      } else {
-        d.din = I.dcat;
-        if ((e = conv_dgrad(d, st))) return e;
-        int c1 = kTC[l.d.s1], c2 = kTC[l.d.s2];
-        if ((e = upsample_grad(I.dcat, l.cin_pad, 0, I.dact[l.d.s1], N, h, w, c1, st))) return e;
-        if ((e = take_channels(I.dcat, l.cin_pad, c1, I.dact[l.d.s2], P, c2, st))) return e;
-        I.launches += 3;
-      }
+      d.dlow = I.dact[l.d.s1];
+      d.dskip = I.dact[l.d.s2];
+      if ((e = conv_dgrad(d, st))) return e;
+      ++I.launches;
     } else {
       d.din = I.dact[l.d.s1];
       if ((e = conv_dgrad(d, st))) return e;

@@ -533,7 +533,10 @@ long long run_pixels(const ConvWgrad& c) {
     tw = c.W >= 128 ? 128 : 64;
     per_sm = c.Cin <= 16 ? 2 : 1;
   }
-  if (!nr) return wgrad_pixels_per_cta(P, c.Cout, c.Cin);
+  if (!nr) {
+    const long long ranges = std::max(1, 8 * 152 / ((9 * c.Cin + 127) / 128)), per = (P + ranges - 1) / ranges;
+    return std::max(64LL, (per + 63) / 64 * 64);
+  }
   const long long row = (c.W + tw - 1) / tw, npg = std::max(1, tile_sm_count() * per_sm / nr);
   return ((long long)c.N * c.H * row + npg - 1) / npg * c.W / row;
 }
@@ -595,9 +598,7 @@ bool conv_tile_wgrad(const ConvWgrad& c, cudaStream_t st, cudaError_t* e) {
     if (TR > 8 && px > limit) return false;
     a.tx = (c.W + 7) / 8;
     a.ty = (c.H + TR - 1) / TR;
-    const long long tiles = (long long)c.N * a.tx * a.ty;
-    if (tiles > (1LL << 30)) return false;
-    a.tiles = (int)tiles;
+    a.tiles = (int)((long long)c.N * a.tx * a.ty);  // at most the pixels, which are fewer than 2^31
     a.ngc = (a.ng + g - 1) / g;
     const int columns = a.ngc * ((at + o - 1) / o);
     const int ranges = (int)std::min<long long>(std::max(1, tile_sm_count() / columns), most);
