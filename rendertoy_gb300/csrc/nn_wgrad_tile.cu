@@ -155,6 +155,10 @@ __device__ __forceinline__ void load3(uint32_t t, uint32_t step, float (&v)[3][1
   for (int k = 0; k < 3 * NC; ++k) v[k / NC][k % NC] = __uint_as_float(r[k / NC][k % NC]);
 }
 
+__device__ __forceinline__ void prefetch_map(const void* m) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
+}
+
 // Walks a CTA's tiles in order
 struct Walk {
   int x, y, img;
@@ -194,8 +198,12 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
   const int ob0 = go * a.ao, on = min(a.ao, a.Cout / a.KO - ob0);  // o-blocks
   const bool bias = a.db && gc == a.ngc - 1;                       // this CTA sums dout
   const int t0 = (int)blockIdx.y * a.per, n = max(0, min(a.per, a.tiles - t0));
+  if (tid == 64) {  // the maps' fetches overlap what follows
+    prefetch_map(&tm.dout);
+    if (nup < gn) prefetch_map(&tm.src[g0 + nup < a.ng1 ? 0 : 1]);
+  }
   if (warp == 0) tc::tmem_alloc(&tmem_slot, a.ncols);
-  if (tid == 0) {
+  if (tid == 32) {
     for (int i = 0; i < a.S; ++i) {
       tc::mbar_init(&full[i], 1 + (nup ? kExpanders : 0));
       tc::mbar_init(&empty[i], 1 + (bias ? kExpanders : 0));
@@ -206,16 +214,15 @@ __global__ void __launch_bounds__(kThreadsW, 1) k_wgrad_tile(const WgradArgs a, 
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  tc::fence_before();
-  __syncthreads();
-  tc::fence_after();
-  const uint32_t tmem = tmem_slot, s0 = tc::smem_u32(smem);
   for (int k = tid; k < 256; k += kThreadsW) {
     sdb[k] = 0.0f;
     if (k < kMaxBlocks * 3 * kExpanders) redo[k] = 0;
   }
   if (tid == 0) again = 0;
+  tc::fence_before();
   __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = tmem_slot, s0 = tc::smem_u32(smem);
   const uint32_t ncb = 3 * a.CB;  // accumulator columns of a block
   bool ok = true;
   if (warp == 0) {
