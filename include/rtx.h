@@ -115,7 +115,9 @@ enum rtx_option {
                                  cost more than they save) */
   RTX_OPT_STACK_LIMIT = 14,   /* traversal stack entries a ray may use, 2..64
                                  (default 64, the whole stack).  A ray that
-                                 needs more stops, and the call returns
+                                 needs more stops (primary passes and
+                                 rtx_intersect first start it again on the
+                                 binary tree), and the call returns
                                  RTX_ERR_DEVICE "traversal stack overflow".
                                  Lower values exist to exercise that error
                                  path; results are undefined after it. */
