@@ -619,21 +619,10 @@ static cudaError_t launch_staged(K4 k4, K3 k3, K2 k2, int stages, dim3 grid, siz
   return cudaGetLastError();
 }
 
-static int sm_count() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
-      n = 148;
-  }
-  return n;
-}
-
 static int gather_stages(int nb, dim3 grid, size_t stage_bytes) {
   const int base = stages_for(nb);
   const long long ctas = (long long)grid.x * grid.y * grid.z;
-  return (base == 2 && ctas < sm_count() && 4 * stage_bytes <= 200 * 1024) ? 4 : base;
+  return (base == 2 && ctas < tile_sm_count() && 4 * stage_bytes <= 200 * 1024) ? 4 : base;
 }
 
 // Row tiles pay off once a row holds at least half a tile; they need input
@@ -655,7 +644,7 @@ static cudaError_t launch_tiles(KR kr, K6 k6, K4 k4, K2 k2, bool res, size_t sta
     smem = S * stage;
   }
   smem = std::max(smem, (size_t)116 * 1024);
-  const unsigned grid = (unsigned)std::min<long long>(T, sm_count());
+  const unsigned grid = (unsigned)std::min<long long>(T, tile_sm_count());
   cudaError_t e;
 #define RTX_LAUNCH_TILES(K)                                                                          \
   if ((e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))) return e; \

@@ -959,14 +959,14 @@ static bool tap_map(CUtensorMap* m, const bf16* base, int rows, int K, int KC, i
 }
 
 int tile_sm_count() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
+  static const int count = [] {  // once, also with several threads
+    int dev = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
       n = 152;
-  }
-  return n;
+    return n;
+  }();
+  return count;
 }
 
 static uint32_t pow2_cols(uint32_t c) {
